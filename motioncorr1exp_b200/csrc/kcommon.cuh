@@ -46,7 +46,8 @@ __device__ __forceinline__ const void* fwd_frame(const FwdRowsArgs& a) {
 //   X[k2 + N2 k1]  = sum_n1 Y[n1][k2] W_N1^(n1 k1)                    thread k2: N1-point codelet
 // so a whole transform costs one shared-memory exchange.  N1 = 53 uses the
 // generated radix-53 butterfly.  One CTA (a team of `T2L` threads) per
-// transform; W_N comes from the global twiddle table through the L1.
+// transform; step A's factors W_N^(n1 k2) come from a global table laid out
+// [k2][n1] (fft_tables), so the threads n1 of a warp read consecutive words.
 template <int N1, bool INV>
 __device__ __forceinline__ void fft_n1(float2* v) {
   if constexpr (N1 == 53) dft_r53<INV>(v);
@@ -71,11 +72,12 @@ struct TwoLevel {
   static constexpr int T = ((N1 > N2 ? N1 : N2) + 31) / 32 * 32;
 
   // step A + exchange + step B; load(i) gives x[i], store(k, X[k]) takes the
-  // result; tw[TWS * j] = exp(-2 pi i j / N).  For N1 = 53 only the outputs
-  // with k1 or N1 - k1 <= kmax are formed (pruned transforms).  T >= N2, so each thread owns at most one k2 in step B; with
+  // result; tw[k2 * N1 + n1] = exp(-2 pi i n1 k2 / N).  For N1 = 53 only the
+  // outputs with k1 or N1 - k1 <= kmax are formed (pruned transforms).
+  // T >= N2, so each thread owns at most one k2 in step B; with
   // SYNC_STORE a barrier follows every thread's step-B reads of ysm, which
   // lets store() write back into ysm.
-  template <bool INV, bool SYNC_STORE, bool PAIRED = false, int TWS = 1, class Load, class Store>
+  template <bool INV, bool SYNC_STORE, bool PAIRED = false, class Load, class Store>
   __device__ static void run(float2* ysm, const float2* __restrict__ tw, Load&& load, Store&& store,
                              int kmax = (N1 - 1) / 2, int lt_team = -1) {
     static_assert(T >= N2, "one k2 per thread");
@@ -89,7 +91,7 @@ struct TwoLevel {
       fft_reg<N2, INV>(x);
 #pragma unroll
       for (int k2 = 0; k2 < N2; k2++) {
-        float2 w = __ldg(tw + TWS * lt * k2);
+        float2 w = __ldg(tw + k2 * N1 + lt);
         if (INV) w.y = -w.y;
         ysm[k2 * N1 + lt] = k2 ? cmul(x[k2], w) : x[k2];
       }

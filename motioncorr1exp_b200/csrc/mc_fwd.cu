@@ -156,12 +156,12 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_rows_
   if constexpr (PLAIN) {
     // every output kept, unscaled (the forward column pass without a Fourier
     // crop): no per-output crop test or multiply (2.47 -> 2.15 ms per c2 movie)
-    TL::template run<INV, false, PAIRED>(ysm, a.tw, [&](int i) { return __ldg(in + i); },
+    TL::template run<INV, false, PAIRED>(ysm, a.tw + TL::N, [&](int i) { return __ldg(in + i); },
                                          [&](int k, float2 v) { out[k] = v; });
   } else {
     const int shift = TL::N - a.n_out, keep = a.keep_lo;
     const float sc = a.scale;
-    TL::template run<INV, false, PAIRED>(ysm, a.tw, [&](int i) { return __ldg(in + i); },
+    TL::template run<INV, false, PAIRED>(ysm, a.tw + TL::N, [&](int i) { return __ldg(in + i); },
                           [&](int k, float2 v) {
                             int o;
                             if (k < keep) o = k;

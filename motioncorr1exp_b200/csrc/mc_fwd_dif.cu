@@ -12,7 +12,8 @@ namespace mc {
 //   A[m] = FFT_N(z_n + z_{n+N})[m] = Z[2m],
 //   B[m] = FFT_N((z_n - z_{n+N}) W_L^n)[m] = Z[2m+1],
 // then the two N-point two-level transforms, whose outputs go straight to
-// the kept indices.  tw is the L-entry table exp(-2 pi i j / L).
+// the kept indices.  tw is the L-entry table exp(-2 pi i j / L), followed by
+// the N-point transforms' own factors (fft_tables).
 
 // Output pairs (k1, N1 - k1) of the N1-point step a radix-2 split transform
 // needs when only its outputs below `lo` (2m < lo) and their mirror images
@@ -56,15 +57,15 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_r
   // wanted A/B outputs: m < hk/2 or m > N - hk/2, i.e. m = k2 + N2*k1 with
   // k1 or N1 - 1 - k1 at most (hk/2)/N2
   const int kmax = dif_kmax<N1, N2>(hk);
-  TL::template run<false, false, false, 2>(
-      ysm, tw,
+  TL::template run<false, false, false>(
+      ysm, tw + L,
       [&](int n) {
         return make_float2((float)p0[n] + (float)p0[n + N], (float)p1[n] + (float)p1[n + N]);
       },
       [&](int m, float2 v) { keep(2 * m, v); }, kmax);
   __syncthreads();
-  TL::template run<false, false, false, 2>(
-      ysm, tw,
+  TL::template run<false, false, false>(
+      ysm, tw + L,
       [&](int n) {
         const float2 d = make_float2((float)p0[n] - (float)p0[n + N], (float)p1[n] - (float)p1[n + N]);
         return cmul(d, __ldg(tw + n));
@@ -101,12 +102,12 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_rows_
   };
   // wanted outputs i < keep or i >= keep + shift: with no crop all of them
   const int kmax = shift == 0 ? (N1 - 1) / 2 : dif_kmax<N1, N2>(keep + 1);
-  TL::template run<false, false, false, 2>(
-      ysm, tw, [&](int n) { return cadd(__ldg(in + n), __ldg(in + n + N)); },
+  TL::template run<false, false, false>(
+      ysm, tw + L, [&](int n) { return cadd(__ldg(in + n), __ldg(in + n + N)); },
       [&](int m, float2 v) { put(2 * m, v); }, kmax);
   __syncthreads();
-  TL::template run<false, false, false, 2>(
-      ysm, tw,
+  TL::template run<false, false, false>(
+      ysm, tw + L,
       [&](int n) {
         const float2 x0 = __ldg(in + n), x1 = __ldg(in + n + N);
         return cmul(make_float2(x0.x - x1.x, x0.y - x1.y), __ldg(tw + n));

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS / 2)
   const Px* p1 =
       reinterpret_cast<const Px*>(rawb + (2 * team + 1) * RB + (reinterpret_cast<uintptr_t>(row(2 * team + 1)) & 15));
   TL::template run<false, true, PAIRED>(
-      ysm, a.tw, [&](int x) { return make_float2((float)p0[x], (float)p1[x]); },
+      ysm, a.tw + N, [&](int x) { return make_float2((float)p0[x], (float)p1[x]); },
       [&](int k, float2 v) { ysm[k] = v; }, (N1 - 1) / 2, lt);
   __syncthreads();
   const int nh = two ? 2 : 1;
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_r
   // between the steps, and step B reads only ysm
   float2* zsm = xin;
   TL::template run<false, false>(
-      ysm, a.tw, [&](int x) { return xin[x]; }, [&](int k, float2 v) { zsm[k] = v; });
+      ysm, a.tw + N, [&](int x) { return xin[x]; }, [&](int k, float2 v) { zsm[k] = v; });
   __syncthreads();
   for (int k = threadIdx.x; k < a.hk; k += TL::T) {
     const float2 z = zsm[k];

@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kThreads) k_shift_sum2l(ShiftSumArgs a, const 
   __syncthreads();
   float2* out = a.out;
   const long long ld = a.ld_out;
-  TL::template run<true, false>(ysm, a.tw, [&](int i) { return col[i]; },
+  TL::template run<true, false>(ysm, a.tw + N, [&](int i) { return col[i]; },
                                 [&](int k, float2 v) { out[(long long)k * ld + kx] = v; });
 }
 
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS)
   __shared__ float2 ysm[TL::N];
   const int kx = blockIdx.x;
   const float2* col = in + (long long)kx * ld_in;
-  TL::template run<true, false>(ysm, tw, [&](int i) { return __ldg(col + i); },
+  TL::template run<true, false>(ysm, tw + TL::N, [&](int i) { return __ldg(col + i); },
                                 [&](int k, float2 v) { out[(long long)k * ld_out + kx] = v; });
 }
 
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T) k_c2r_rows2l(C2rRowsArgs 
   float* i1 = a.image + (long long)y1 * N;
   const float sc = a.scale;
   TL::template run<true, false>(
-      ysm, a.tw,
+      ysm, a.tw + N,
       [&](int k) {
         float2 u, v;
         if (k <= N / 2) {
