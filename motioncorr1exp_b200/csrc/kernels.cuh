@@ -292,6 +292,5 @@ size_t pair_cols_smem(int n, int P, int Q, int box);
 inline bool pair_cols_tabn(int n, int P, int box) { return (long long)P * box > n; }
 size_t shift_sum_smem(int n, int nsum);
 size_t c2r_rows_smem(int n);
-size_t peak_smem();
 
 }  // namespace mc

@@ -3,21 +3,39 @@
 // accumulate with the inverse column FFT (cufunc.cu:372-393), final C2R rows
 // (DFAlign.cu:1287-1292), exact count sums and the objective of the gradient
 // refinement.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "kcommon.cuh"
 
 namespace mc {
 
+namespace cg = cooperative_groups;
+
 // ==================================================================== peak ==
+// A cluster of C CTAs serves one pair: every CTA finds the integer peak and
+// the masked sub-box spectrum (both cheap), then searches its share of the
+// 512 grid rows; CTA 0 merges the C maxima through distributed shared memory.
+//
+// The grid values are f(X, Y) = G0(Y).x + sum_k 2 (G_k.x cos - G_k.y sin)(2 pi
+// k X / 512), k = 1..7.  What bounds the search is FP64 issue, 64 lanes per SM
+// and cycle, so a thread forms four columns at once: X, 512 - X, 256 - X and
+// 256 + X share their cosine and sine products up to sign, by the parity of k
+// (26 FP64 operations for four values, 14 multiply-adds each before).  The rows
+// likewise: G(Y) and G(512 - Y) share theirs.  Rows ascend within a thread, so
+// the strict comparison keeps the first of equal values.
+// Measured per launch, one CTA per pair before / now: 21 pairs 179 -> 27 us,
+// 55 pairs 186 -> 35 us, 105 pairs 185 -> 52 us, 378 pairs 417 -> 123 us.
 constexpr int kSub = 16;
 constexpr int kPad = 512;
 constexpr int kUp = 32;
 
 struct PeakSmem {
-  double2 g1[kPad][8];     // column-inverse of the masked sub-box spectrum
   double2 tw[kPad];        // exp(+2 pi i m / 512)
   double2 s[kSub][9];      // masked 16x16 half spectrum
+  double2 sp[8][8];        // s[j] + s[16 - j] (row 0: s[0])
+  double2 sn[8][8];        // s[j] - s[16 - j]
   double2 rx[kSub][9];     // row transforms of the sub-box
   double sub[kSub][kSub];
   double rv[kThreads / 32];
@@ -25,9 +43,10 @@ struct PeakSmem {
   float fv[kThreads / 32];
   int fi[kThreads / 32];
   double f00;
+  double2 g1[1][8];        // G_k of this CTA's grid rows, k >= 1 doubled (kPad / C + 2 rows)
 };
 
-size_t peak_smem() { return sizeof(PeakSmem); }
+size_t peak_smem(int cluster) { return sizeof(PeakSmem) + sizeof(double2) * 8 * (kPad / cluster + 1); }
 
 // (v, i) beats (bv, bi): larger value, or equal value and earlier scan index.
 template <typename T>
@@ -35,10 +54,10 @@ __device__ __forceinline__ bool better(T v, int i, T bv, int bi) {
   return v > bv || (v == bv && i < bi);
 }
 
-__global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a) {
+__global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a, int C) {
   extern __shared__ __align__(16) unsigned char smraw[];
   PeakSmem& S = *reinterpret_cast<PeakSmem*>(smraw);
-  const int p = blockIdx.x;
+  const int p = blockIdx.x / C, rank = blockIdx.x - p * C;
   const int box = a.box;
   const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, wid = tid >> 5;
   const float* bm = a.boxes + (long long)p * box * box;
@@ -48,11 +67,15 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a) {
   // ---- integer peak (cufunc.cu:409-424): strict '>' from -1e9, y outer, x inner
   float bv = -1e9f;
   int bi = 0x7fffffff;
+#pragma unroll 8
   for (int idx = tid; idx < box * box; idx += nth) {
-    const int yy = idx / box, xx = idx - yy * box;
-    if (abs(xx - hb) <= wnoise && abs(yy - hb) <= wnoise) continue;
     const float v = bm[idx];
-    if (v > -1e9f && better(v, idx, bv, bi)) {
+    bool out = false;
+    if (wnoise >= 0) {
+      const int yy = idx / box, xx = idx - yy * box;
+      out = abs(xx - hb) <= wnoise && abs(yy - hb) <= wnoise;
+    }
+    if (!out && v > -1e9f && better(v, idx, bv, bi)) {
       bv = v;
       bi = idx;
     }
@@ -68,6 +91,11 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a) {
   if (lane == 0) {
     S.fv[wid] = bv;
     S.fi[wid] = bi;
+  }
+  for (int m = tid; m < kPad; m += nth) {
+    double sn, cn;
+    sincospi((double)m / (kPad / 2), &sn, &cn);
+    S.tw[m] = make_double2(cn, sn);
   }
   __syncthreads();
   bv = S.fv[0];
@@ -88,15 +116,10 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a) {
   if (offy + kSub > box) offy = box - kSub;
   else if (offy < 0) offy = 0;
 
-  // ---- sub-box, tables
+  // ---- sub-box
   for (int t = tid; t < kSub * kSub; t += nth) {
     const int yy = t / kSub, xx = t - yy * kSub;
     S.sub[yy][xx] = (double)bm[(offy + yy) * box + offx + xx];
-  }
-  for (int m = tid; m < kPad; m += nth) {
-    double sn, cn;
-    sincospi((double)m / (kPad / 2), &sn, &cn);
-    S.tw[m] = make_double2(cn, sn);
   }
   __syncthreads();
   // R2C along x: rx[y][kx] = sum_x sub[y][x] exp(-2 pi i kx x / 16)
@@ -125,44 +148,122 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a) {
     S.s[j][k] = make_double2(re * wt, im * wt);
   }
   __syncthreads();
-  // zero-padded inverse along y: g1[Y][kx] = sum_j s[j][kx] exp(+2 pi i ky_j Y / 512)
-  for (int t = tid; t < kPad * 8; t += nth) {
-    const int Y = t >> 3, k = t & 7;
-    double re = 0.0, im = 0.0;
-    for (int j = 0; j < kSub; j++) {
-      const int ky = j < kSub / 2 ? j : j - kSub;
-      const double2 w = S.tw[(ky * Y) & (kPad - 1)];
-      const double2 v = S.s[j][k];
-      re += v.x * w.x - v.y * w.y;
-      im += v.x * w.y + v.y * w.x;
+  // rows j and 16 - j together (the mask leaves nothing of row 8, ky = -8)
+  if (tid < 64) {
+    const int j = tid >> 3, k = tid & 7;
+    const double2 u = S.s[j][k], v = j ? S.s[kSub - j][k] : make_double2(0.0, 0.0);
+    S.sp[j][k] = make_double2(u.x + v.x, u.y + v.y);
+    S.sn[j][k] = make_double2(u.x - v.x, u.y - v.y);
+  }
+  __syncthreads();
+  // zero-padded inverse along y, G_k(Y) = sum_j s[j][k] exp(+2 pi i ky_j Y / 512).
+  // This CTA's rows: Y = y0 .. y0 + hr - 1, then the mirrored rows
+  // 512 - Y in ascending order, then Y = 256 (the last CTA; the first has no
+  // mirror of Y = 0).
+  const int hr = kPad / 2 / C, y0 = rank * hr;
+  const bool first = rank == 0, last = rank == C - 1;
+  const int nmir = first ? hr - 1 : hr;  // mirrored rows
+  const int nrow = hr + nmir + (last ? 1 : 0);
+  // local row l -> Y, ascending: direct rows, Y = 256, mirrored rows
+  auto row_y = [&](int l) {
+    if (l < hr) return y0 + l;
+    l -= hr;
+    if (last) {
+      if (l == 0) return kPad / 2;
+      l--;
     }
-    S.g1[Y][k] = make_double2(re, im);
+    return kPad - (y0 + hr - 1) + l;
+  };
+  for (int t = tid; t < (hr + (last ? 1 : 0)) * 8; t += nth) {
+    const int l = t >> 3, k = t & 7, Y = y0 + l;  // l = hr only for Y = 256
+    const double2 s0 = S.s[0][k];
+    double pr = s0.x, pi = s0.y, qr = 0.0, qi = 0.0;
+#pragma unroll
+    for (int j = 1; j < 8; j++) {
+      const double2 w = S.tw[(j * Y) & (kPad - 1)];
+      const double2 u = S.sp[j][k], v = S.sn[j][k];
+      pr += u.x * w.x;
+      pi += u.y * w.x;
+      qr -= v.y * w.y;
+      qi += v.x * w.y;
+    }
+    const double two = k ? 2.0 : 1.0;
+    S.g1[l][k] = make_double2(two * (pr + qr), two * (pi + qi));
+    if (l < hr && Y > 0) {
+      // 512 - Y: the mirrored rows end with Y = y0 (first: y0 + 1)
+      const int m = hr + (last ? 1 : 0) + (hr - 1 - l);
+      S.g1[m][k] = make_double2(two * (pr - qr), two * (pi - qi));
+    }
   }
   __syncthreads();
   // C2R along x on the 512 grid and the argmax (cufunc.cu:457-476)
   const int ox = (hb - offx) * kUp, oy = (hb - offy) * kUp, wns = kUp * wnoise;
-  double best = -INFINITY;
-  int bidx = 0x7fffffff;
-  for (int X = tid; X < kPad; X += nth) {
-    double2 c[8];
+  const int X = tid & 127;
+  double2 c[8];
 #pragma unroll
-    for (int k = 1; k < 8; k++) c[k] = S.tw[(k * X) & (kPad - 1)];
-    const bool xex = abs(X - ox) <= wns;
-    for (int Y = 0; Y < kPad; Y++) {
-      double f = S.g1[Y][0].x;
+  for (int k = 1; k < 8; k++) c[k] = S.tw[k * X & (kPad - 1)];
+  const int Xs[4] = {X, (kPad - X) & (kPad - 1), kPad / 2 - X, kPad / 2 + X};
+  double qb[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  int ql[4] = {-1, -1, -1, -1};
+  for (int l = tid >> 7; l < nrow; l += kThreads / 128) {
+    const double2* g = S.g1[l];
+    double ev = g[0].x, od, es, os;
+    {
+      const double2 g1 = g[1], g2 = g[2];
+      od = g1.x * c[1].x;
+      os = g1.y * c[1].y;
+      ev += g2.x * c[2].x;
+      es = g2.y * c[2].y;
+    }
 #pragma unroll
-      for (int k = 1; k < 8; k++) {
-        const double2 g = S.g1[Y][k];
-        f += 2.0 * (g.x * c[k].x - g.y * c[k].y);
-      }
-      if (X == 0 && Y == 0) S.f00 = f;
-      if (xex && abs(Y - oy) <= wns) continue;
-      const int idx = Y * kPad + X;
-      if (better(f, idx, best, bidx)) {
-        best = f;
-        bidx = idx;
+    for (int k = 3; k < 8; k += 2) {
+      const double2 go = g[k];
+      od += go.x * c[k].x;
+      os += go.y * c[k].y;
+      if (k < 7) {
+        const double2 ge = g[k + 1];
+        ev += ge.x * c[k + 1].x;
+        es += ge.y * c[k + 1].y;
       }
     }
+    const double pe = ev + od, me = ev - od, ps = es + os, ms = es - os;
+    const double f[4] = {pe - ps, pe + ps, me + ms, me - ms};
+    if (first && l == 0 && tid == 0) S.f00 = f[0];
+    if (wnoise >= 0 && abs(row_y(l) - oy) <= wns) {
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (abs(Xs[q] - ox) > wns && f[q] > qb[q]) {
+          qb[q] = f[q];
+          ql[q] = l;
+        }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (f[q] > qb[q]) {
+          qb[q] = f[q];
+          ql[q] = l;
+        }
+    }
+  }
+  double best = -INFINITY;
+  int bidx = 0x7fffffff;
+  auto take = [&](double v, int idx) {
+    if (better(v, idx, best, bidx)) {
+      best = v;
+      bidx = idx;
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    if (ql[q] >= 0) take(qb[q], row_y(ql[q]) * kPad + Xs[q]);
+  // columns 128 and 384: exp(+2 pi i k 128 / 512) = i^k
+  for (int l = tid; l < nrow; l += kThreads) {
+    const double2* g = S.g1[l];
+    const int Y = row_y(l);
+    const double ev = g[0].x - g[2].x + g[4].x - g[6].x, os = g[1].y - g[3].y + g[5].y - g[7].y;
+    const bool yex = wnoise >= 0 && abs(Y - oy) <= wns;
+    if (!(yex && abs(kPad / 4 - ox) <= wns)) take(ev - os, Y * kPad + kPad / 4);
+    if (!(yex && abs(3 * kPad / 4 - ox) <= wns)) take(ev + os, Y * kPad + 3 * kPad / 4);
   }
   for (int o = 16; o > 0; o >>= 1) {
     const double ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -172,18 +273,22 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a) {
       bidx = oi;
     }
   }
-  __syncthreads();
   if (lane == 0) {
     S.rv[wid] = best;
     S.ri[wid] = bidx;
   }
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < nth / 32; w++)
-      if (better(S.rv[w], S.ri[w], best, bidx)) {
-        best = S.rv[w];
-        bidx = S.ri[w];
-      }
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  if (rank == 0 && tid == 0) {
+    for (int r = 0; r < C; r++) {
+      const double* rv = cl.map_shared_rank(S.rv, r);
+      const int* ri = cl.map_shared_rank(S.ri, r);
+      for (int w = 0; w < nth / 32; w++)
+        if (better(rv[w], ri[w], best, bidx)) {
+          best = rv[w];
+          bidx = ri[w];
+        }
+    }
     int sxp = 0, syp = 0;
     double bestcc = S.f00;
     if (bidx != 0x7fffffff && best > S.f00) {
@@ -199,14 +304,31 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a) {
     a.peak[2 * p] = ix;
     a.peak[2 * p + 1] = iy;
   }
+  cl.sync();  // the other CTAs' maxima stay in place until CTA 0 has read them
 }
 
 cudaError_t launch_peak(const PeakArgs& a, cudaStream_t st) {
-  const size_t smem = peak_smem();
+  // CTAs per pair: four while they all run at once (two per SM), else two; the
+  // work every CTA of a pair repeats (table, sub-box) outweighs a finer split
+  // (C = 1 / 2 / 4 / 8: 21 pairs 62, 37, 27, 27 us; 55 pairs 64, 41, 35, 52;
+  // 105 pairs 66, 52, 62, 79; 378 pairs 142, 123, 150, 227)
+  const int C = a.npairs * 4 <= 148 * 2 ? 4 : 2;
+  const size_t smem = peak_smem(C);
   cudaError_t e = allow_smem((const void*)k_peak, smem);
   if (e != cudaSuccess) return e;
-  k_peak<<<a.npairs, kThreads, smem, st>>>(a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(a.npairs * C));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = C;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_peak, a, C);
 }
 
 // ============================================================== shift-sum ==
