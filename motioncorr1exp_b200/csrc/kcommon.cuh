@@ -33,11 +33,12 @@ __device__ __forceinline__ void copy_table(float2* dst, const float2* __restrict
 
 }  // namespace
 
-// Frame read by a forward launch (direct pointer, or the run's base from the
-// device-side slot plus this frame's offset).
+// Frame read by a forward CTA (direct pointer, or the run's base from the
+// device-side slot plus the first frame's offset; frame blockIdx.y of the launch).
 __device__ __forceinline__ const void* fwd_frame(const FwdRowsArgs& a) {
-  return a.frames_slot ? static_cast<const void*>(static_cast<const char*>(*a.frames_slot) + a.frame_offset)
-                       : a.frame;
+  const char* f = a.frames_slot ? static_cast<const char*>(*a.frames_slot) + a.frame_offset
+                                : static_cast<const char*>(a.frame);
+  return f + (long long)blockIdx.y * a.frame_stride;
 }
 
 // ================================================== two-level transforms ==

@@ -38,6 +38,10 @@ struct FwdRowsArgs {
   FftPlan1D plan;      // length nu, forward
   const float2* tw;    // nu twiddles exp(-2 pi i m / nu)
   int paired;          // radix-53 step: 0 built-in, 1 one output pair per loop pass, 2 two
+  // frames of one launch (blockIdx.y; 0 = 1): frame i at i * frame_stride
+  // bytes from the first, its output at i * out_stride elements
+  int nfr;
+  long long frame_stride, out_stride;
 };
 
 // Pass B and every other batched transform over contiguous rows:
@@ -54,6 +58,8 @@ struct RowsFftArgs {
   FftPlan1D plan;
   const float2* tw;
   int paired;          // radix-53 step: 0 built-in, 1 one output pair per loop pass, 2 two
+  int nfr;             // row sets of one launch (blockIdx.y; 0 = 1), at these strides (elements)
+  long long in_stride, out_stride;
 };
 
 // ------------------------------------------------------------------ pairs --

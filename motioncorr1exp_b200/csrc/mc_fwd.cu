@@ -55,6 +55,8 @@ __global__ void __launch_bounds__(kThreads) k_fwd_rows(FwdRowsArgs a) {
   }
   __syncthreads();
   float2* Z = fft_run<false, false>(b0, b1, a.plan, 1, nu, tw, tid, nth);
+  float2* outA = a.outA + blockIdx.y * a.out_stride;
+  float2* outB = a.two_outputs ? a.outB + blockIdx.y * a.out_stride : nullptr;
   // split the two real transforms: X = (Z(k) + conj Z(-k))/2, Y = -i (Z(k) - conj Z(-k))/2
   for (int k = tid; k < a.hk; k += nth) {
     const float2 z = Z[k];
@@ -62,10 +64,10 @@ __global__ void __launch_bounds__(kThreads) k_fwd_rows(FwdRowsArgs a) {
     const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
     const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
     if (a.two_outputs) {
-      a.outA[(long long)k * a.ldt + y0] = X;
-      a.outB[(long long)k * a.ldt + y0] = Y;
+      outA[(long long)k * a.ldt + y0] = X;
+      outB[(long long)k * a.ldt + y0] = Y;
     } else {
-      float4* dst = reinterpret_cast<float4*>(a.outA + (long long)k * a.ldt + y0);
+      float4* dst = reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0);
       *dst = make_float4(X.x, X.y, Y.x, Y.y);
     }
   }
@@ -90,7 +92,7 @@ cudaError_t launch_fwd_rows(const FwdRowsArgs& a, cudaStream_t st) {
   cudaError_t e = allow_smem((const void*)k_fwd_rows, smem);
   if (e != cudaSuccess) return e;
   const int grid = a.two_outputs ? a.nu : a.nu / 2;
-  k_fwd_rows<<<grid, kThreads, smem, st>>>(a);
+  k_fwd_rows<<<dim3(grid, std::max(a.nfr, 1)), kThreads, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -106,10 +108,12 @@ __global__ void __launch_bounds__(kThreads) k_rows_fft(RowsFftArgs a, int rows_p
   copy_table(tw, a.tw, n);
   const int tid = threadIdx.x, nth = blockDim.x;
   const int row0 = blockIdx.x * B;
+  const float2* in = a.in + blockIdx.y * a.in_stride;
+  float2* out = a.out + blockIdx.y * a.out_stride;
   const int nb = min(B, a.nrows - row0);
   for (int t = tid; t < B * n; t += nth) {
     const int b = t / n, i = t - b * n;
-    b0[t] = (b < nb) ? a.in[(long long)(row0 + b) * a.ld_in + i] : make_float2(0.f, 0.f);
+    b0[t] = (b < nb) ? in[(long long)(row0 + b) * a.ld_in + i] : make_float2(0.f, 0.f);
   }
   __syncthreads();
   float2* X = fft_run<INV, false>(b0, b1, a.plan, B, n, tw, tid, nth);
@@ -118,7 +122,7 @@ __global__ void __launch_bounds__(kThreads) k_rows_fft(RowsFftArgs a, int rows_p
     const int b = t / a.n_out, i = t - b * a.n_out;
     const int src = (i < a.keep_lo) ? i : i + shift;
     const float2 v = X[b * n + src];
-    a.out[(long long)(row0 + b) * a.ld_out + i] = make_float2(v.x * a.scale, v.y * a.scale);
+    out[(long long)(row0 + b) * a.ld_out + i] = make_float2(v.x * a.scale, v.y * a.scale);
   }
 }
 
@@ -131,7 +135,7 @@ cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, int rows_per_cta
   if (two_level_split(a.plan.n, n1, n2)) return launch_rows_fft2l(a, inverse, st);
   if (!inverse && dif_supported(a.plan.n)) return launch_rows_fft_dif(a, st);
   const size_t smem = rows_fft_smem(a.plan.n, rows_per_cta);
-  const int grid = (a.nrows + rows_per_cta - 1) / rows_per_cta;
+  const dim3 grid((a.nrows + rows_per_cta - 1) / rows_per_cta, std::max(a.nfr, 1));
   cudaError_t e;
   if (inverse) {
     e = allow_smem((const void*)k_rows_fft<true>, smem);
@@ -151,8 +155,8 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_rows_
   using TL = TwoLevel<N1, N2>;
   __shared__ float2 ysm[TL::N];
   const long long row = blockIdx.x;
-  const float2* in = a.in + row * a.ld_in;
-  float2* out = a.out + row * a.ld_out;
+  const float2* in = a.in + blockIdx.y * a.in_stride + row * a.ld_in;
+  float2* out = a.out + blockIdx.y * a.out_stride + row * a.ld_out;
   if constexpr (PLAIN) {
     // every output kept, unscaled (the forward column pass without a Fourier
     // crop): no per-output crop test or multiply (2.47 -> 2.15 ms per c2 movie)
@@ -188,16 +192,17 @@ bool two_level_split(int n, int& n1, int& n2) {
 // Forward column launch with the radix-53 pairing the schedule asks for
 template <int A, int B>
 void launch_cols_fwd(const RowsFftArgs& a, bool paired, cudaStream_t st) {
+  const dim3 grid(a.nrows, std::max(a.nfr, 1));
   const bool plain = a.n_out == A * B && a.keep_lo >= A * B && a.scale == 1.f;
   if constexpr (A == 53) {
     if (paired != kFwdColsPaired) {
-      if (plain) k_rows_fft2l<A, B, false, !kFwdColsPaired, true><<<a.nrows, TwoLevel<A, B>::T, 0, st>>>(a);
-      else k_rows_fft2l<A, B, false, !kFwdColsPaired><<<a.nrows, TwoLevel<A, B>::T, 0, st>>>(a);
+      if (plain) k_rows_fft2l<A, B, false, !kFwdColsPaired, true><<<grid, TwoLevel<A, B>::T, 0, st>>>(a);
+      else k_rows_fft2l<A, B, false, !kFwdColsPaired><<<grid, TwoLevel<A, B>::T, 0, st>>>(a);
       return;
     }
   }
-  if (plain) k_rows_fft2l<A, B, false, kFwdColsPaired, true><<<a.nrows, TwoLevel<A, B>::T, 0, st>>>(a);
-  else k_rows_fft2l<A, B, false, kFwdColsPaired><<<a.nrows, TwoLevel<A, B>::T, 0, st>>>(a);
+  if (plain) k_rows_fft2l<A, B, false, kFwdColsPaired, true><<<grid, TwoLevel<A, B>::T, 0, st>>>(a);
+  else k_rows_fft2l<A, B, false, kFwdColsPaired><<<grid, TwoLevel<A, B>::T, 0, st>>>(a);
 }
 
 cudaError_t launch_rows_fft2l(const RowsFftArgs& a, bool inverse, cudaStream_t st) {
@@ -207,7 +212,8 @@ cudaError_t launch_rows_fft2l(const RowsFftArgs& a, bool inverse, cudaStream_t s
   const bool paired = a.paired == 0 ? kFwdColsPaired : a.paired == 2;
 #define MC_TL_LAUNCH(A, B)                                                                   \
   if (n1 == (A) && n2 == (B)) {                                                              \
-    if (inverse) k_rows_fft2l<A, B, true, kFwdColsPaired><<<a.nrows, TwoLevel<A, B>::T, 0, st>>>(a); \
+    if (inverse)                                                                             \
+      k_rows_fft2l<A, B, true, kFwdColsPaired><<<dim3(a.nrows, std::max(a.nfr, 1)), TwoLevel<A, B>::T, 0, st>>>(a); \
     else launch_cols_fwd<A, B>(a, paired, st);                                               \
     return cudaGetLastError();                                                               \
   }

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_r
   unsigned char* raw0 = reinterpret_cast<unsigned char*>(zhi + hk);
   unsigned char* raw1 = raw0 + RB;
   const int y0 = 2 * blockIdx.x, y1 = y0 + 1;
+  float2* outA = a.outA + blockIdx.y * a.out_stride;
   const Px* f = reinterpret_cast<const Px*>(fwd_frame(a));
   const Px* row0 = f + (long long)(a.offy + y0) * a.nx + a.offx;
   const Px* row1 = f + (long long)(a.offy + y1) * a.nx + a.offx;
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_r
     const float2 zc = k == 0 ? zlo[0] : zhi[hk - 1 - k];
     const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
     const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
-    *reinterpret_cast<float4*>(a.outA + (long long)k * a.ldt + y0) = make_float4(X.x, X.y, Y.x, Y.y);
+    *reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0) = make_float4(X.x, X.y, Y.x, Y.y);
   }
 }
 
@@ -88,8 +89,8 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_rows_
   constexpr int N = TL::N, L = 2 * N;
   __shared__ float2 ysm[N];
   const long long row = blockIdx.x;
-  const float2* in = a.in + row * a.ld_in;
-  float2* out = a.out + row * a.ld_out;
+  const float2* in = a.in + blockIdx.y * a.in_stride + row * a.ld_in;
+  float2* out = a.out + blockIdx.y * a.out_stride + row * a.ld_out;
   const int shift = L - a.n_out, keep = a.keep_lo;
   const float sc = a.scale;
   const float2* tw = a.tw;
@@ -123,7 +124,7 @@ bool dif_supported(int n) {
 cudaError_t launch_fwd_rows_dif(const FwdRowsArgs& a, cudaStream_t st) {
   int n1 = 0, n2 = 0;
   if (a.nu % 2 || !two_level_split(a.nu / 2, n1, n2)) return cudaErrorInvalidValue;
-  const int grid = a.nu / 2;
+  const dim3 grid(a.nu / 2, std::max(a.nfr, 1));
 #define MC_DIF_RAW(A, B, PX)                                                                          \
   {                                                                                                   \
     const size_t smem = ((size_t)(A) * (B) + 2 * (size_t)a.hk) * sizeof(float2) +                     \
@@ -155,7 +156,7 @@ cudaError_t launch_rows_fft_dif(const RowsFftArgs& a, cudaStream_t st) {
   if (a.plan.n % 2 || !two_level_split(a.plan.n / 2, n1, n2)) return cudaErrorInvalidValue;
 #define MC_DIF_LAUNCH(A, B)                                                        \
   if (n1 == (A) && n2 == (B)) {                                                    \
-    k_rows_fft_dif<A, B><<<a.nrows, TwoLevel<A, B>::T, 0, st>>>(a);                \
+    k_rows_fft_dif<A, B><<<dim3(a.nrows, std::max(a.nfr, 1)), TwoLevel<A, B>::T, 0, st>>>(a); \
     return cudaGetLastError();                                                     \
   }
   MC_TWO_LEVEL_LIST(MC_DIF_LAUNCH)

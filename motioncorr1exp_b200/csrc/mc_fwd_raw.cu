@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS / 2)
   float2* ysm = dynraw + (size_t)team * N;
   unsigned char* rawb = reinterpret_cast<unsigned char*>(dynraw + 2 * N);  // four staged rows
   const int y0 = 4 * blockIdx.x;
+  float2* outA = a.outA + blockIdx.y * a.out_stride;
   const bool two = y0 + 2 < a.nu;  // the second row pair exists
   const Px* f = reinterpret_cast<const Px*>(fwd_frame(a));
   auto row = [&](int j) { return f + (long long)(a.offy + y0 + (two ? j : (j & 1))) * a.nx + a.offx; };
@@ -49,7 +50,7 @@ __global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS / 2)
       const float2 zc = zs[k == 0 ? 0 : N - k];
       const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
       const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
-      *reinterpret_cast<float4*>(a.outA + (long long)k * a.ldt + y0 + 2 * h) = make_float4(X.x, X.y, Y.x, Y.y);
+      *reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0 + 2 * h) = make_float4(X.x, X.y, Y.x, Y.y);
     }
   }
 }
@@ -88,16 +89,18 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_r
   TL::template run<false, false>(
       ysm, a.tw + N, [&](int x) { return xin[x]; }, [&](int k, float2 v) { zsm[k] = v; });
   __syncthreads();
+  float2* outA = a.outA + blockIdx.y * a.out_stride;
+  float2* outB = a.two_outputs ? a.outB + blockIdx.y * a.out_stride : nullptr;
   for (int k = threadIdx.x; k < a.hk; k += TL::T) {
     const float2 z = zsm[k];
     const float2 zc = zsm[k == 0 ? 0 : N - k];
     const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
     const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
     if (a.two_outputs) {
-      a.outA[(long long)k * a.ldt + y0] = X;
-      a.outB[(long long)k * a.ldt + y0] = Y;
+      outA[(long long)k * a.ldt + y0] = X;
+      outB[(long long)k * a.ldt + y0] = Y;
     } else {
-      *reinterpret_cast<float4*>(a.outA + (long long)k * a.ldt + y0) = make_float4(X.x, X.y, Y.x, Y.y);
+      *reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0) = make_float4(X.x, X.y, Y.x, Y.y);
     }
   }
 }
@@ -107,7 +110,7 @@ cudaError_t launch_raw_rows_p(const FwdRowsArgs& a, int grid, cudaStream_t st) {
   const size_t smem = 2 * (size_t)A * B * sizeof(float2) + 4 * (size_t)raw_row_bytes<PX>(A * B);
   cudaError_t e = allow_smem((const void*)k_fwd_rows2l_raw4<A, B, PX, PR>, smem);
   if (e != cudaSuccess) return e;
-  k_fwd_rows2l_raw4<A, B, PX, PR><<<(grid + 1) / 2, 2 * TwoLevel<A, B>::T, smem, st>>>(a);
+  k_fwd_rows2l_raw4<A, B, PX, PR><<<dim3((grid + 1) / 2, std::max(a.nfr, 1)), 2 * TwoLevel<A, B>::T, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -144,7 +147,7 @@ cudaError_t launch_fwd_rows2l(const FwdRowsArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)2 * (A) * (B) * sizeof(float2);                                      \
     cudaError_t e = allow_smem((const void*)k_fwd_rows2l<A, B>, smem);                               \
     if (e != cudaSuccess) return e;                                                                  \
-    k_fwd_rows2l<A, B><<<grid, TwoLevel<A, B>::T, smem, st>>>(a);                                    \
+    k_fwd_rows2l<A, B><<<dim3(grid, std::max(a.nfr, 1)), TwoLevel<A, B>::T, smem, st>>>(a);                                    \
     return cudaGetLastError();                                                                       \
   }
   MC_TWO_LEVEL_LIST(MC_TL_LAUNCH)

@@ -81,6 +81,7 @@ namespace {
 constexpr double kPi = 3.14159265358979323846;
 constexpr int kPairBatch = 512;
 constexpr int kPairsPerCta = 32;
+constexpr int kForwardCtas = 148 * 16;  // row CTAs (of four rows) a forward launch is filled to
 // spectrum slots: the fewest a plan works with (two blocks of two frames in
 // the pair stage), and the device memory the automatic choice leaves free
 // (kernel modules, captured graphs, first-use buffers, the caller's own)
@@ -1470,7 +1471,16 @@ static int enqueue_forward(mc_plan* pl, const std::vector<cudaEvent_t>* waits, i
   // play (binning's row buffer, the stretched frame); per-launch timing
   // events need the one stream
   const int njob = only ? (int)only->size() : pl->nframe;
-  const bool multi = !binned && !pl->stretch && njob > 1 && !(pl->profiling && !pl->capturing);
+  // frames of one launch: consecutive frames going to consecutive spectra,
+  // until the launch holds kForwardCtas row CTAs; a small frame alone does
+  // not fill the GPU and costs two launches.  Measured (whole pass, one frame
+  // per launch / this): 8 x 256^2 238 / 224 us, 30 x 520^2 878 / 810 us,
+  // 16 x 1024^2 484 / 469 us, 40 x 3710^2 10.32 / 10.25 ms; launches of
+  // 148 * 32 CTAs and more cost the batch runner's two lanes 8 %.
+  const int gmax = (binned || pl->stretch) ? 1 : std::max(1, std::min(njob, kForwardCtas * 4 / pl->nu));
+  auto frame_of = [&](int job) { return only ? (*only)[job].first : job; };
+  auto slot_of = [&](int job) { return only ? (*only)[job].second : job; };
+  const bool multi = !binned && !pl->stretch && njob > gmax && !(pl->profiling && !pl->capturing);
   const int NS = pl->nfs;
   if (multi) {
     for (int i = 0; i < NS; i++) {
@@ -1482,11 +1492,15 @@ static int enqueue_forward(mc_plan* pl, const std::vector<cudaEvent_t>* waits, i
     CK(cudaEventRecord(fork, pl->st));
     for (int i = 0; i < NS; i++) CK(cudaStreamWaitEvent(pl->fst[i], fork, 0));
   }
-  for (int job = 0; job < njob; job++) {
-    const int f = only ? (*only)[job].first : job;
-    const int slot = only ? (*only)[job].second : job;
-    cudaStream_t fs = multi ? pl->fst[job % NS] : pl->st;
-    if (waits && (multi || f % chunk == 0)) CK(cudaStreamWaitEvent(fs, (*waits)[f / chunk], 0));
+  int launch = 0;
+  for (int job = 0, cnt; job < njob; job += cnt, launch++) {
+    const int f = frame_of(job), slot = slot_of(job);
+    for (cnt = 1; cnt < gmax && job + cnt < njob && frame_of(job + cnt) == f + cnt &&
+                  slot_of(job + cnt) == slot + cnt && (!waits || (f + cnt) / chunk == f / chunk);
+         cnt++) {
+    }
+    cudaStream_t fs = multi ? pl->fst[launch % NS] : pl->st;
+    if (waits) CK(cudaStreamWaitEvent(fs, (*waits)[f / chunk], 0));
     mc::FwdRowsArgs a{};
     a.frame = (const char*)(pl->frames_src ? pl->frames_src : pl->d_frames) + (size_t)f * pl->frame_bytes;
     a.frames_slot = pl->d_src_slot;
@@ -1519,9 +1533,12 @@ static int enqueue_forward(mc_plan* pl, const std::vector<cudaEvent_t>* waits, i
     a.plan = pl->plan_nu;
     a.tw = pl->d_tw_nu;
     const int nrefs = (pl->d_dark ? 1 : 0) + (pl->d_dark2 ? 1 : 0) + (pl->d_norm ? 1 : 0) + (pl->d_norm2 ? 1 : 0);
-    const double crop_bytes = (double)pl->nu * pl->nu * (pl->wl + 4.0 * nrefs);
-    const double t_bytes = (double)pl->H * pl->nu * sizeof(float2);
-    const double s_bytes = (double)pl->H * pl->n * sizeof(float2);
+    a.nfr = cnt;
+    a.frame_stride = (long long)pl->frame_bytes;
+    a.out_stride = pl->fstride;
+    const double crop_bytes = (double)cnt * pl->nu * pl->nu * (pl->wl + 4.0 * nrefs);
+    const double t_bytes = (double)cnt * pl->H * pl->nu * sizeof(float2);
+    const double s_bytes = (double)cnt * pl->H * pl->n * sizeof(float2);
     float2* TB = nullptr;
     if (pl->two_sets) TB = binned ? nullptr : specB_at(pl, slot);
     if (pl->two_sets && binned) {
@@ -1569,6 +1586,8 @@ static int enqueue_forward(mc_plan* pl, const std::vector<cudaEvent_t>* waits, i
       c.plan = pl->plan_nu;
       c.tw = pl->d_tw_nu;
       c.paired = pl->fwd_cols_pairing;
+      c.nfr = cnt;
+      c.in_stride = c.out_stride = pl->fstride;
       LAUNCH(pl, MC_K_FWD_COLS, t_bytes + s_bytes, mc::launch_rows_fft(c, false, 1, fs));
     }
   }
