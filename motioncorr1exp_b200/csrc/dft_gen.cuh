@@ -9,7 +9,7 @@
 #define MC_PACKED_FMA 0
 #endif
 namespace mc {
-constexpr int kGeneratedOddRadices[] = {3, 5, 7, 11, 13, 53};
+constexpr int kGeneratedOddRadices[] = {3, 5, 7, 11, 13};
 template <bool INV> __device__ __forceinline__ void dft_r3(float2* v) {
   const float2 x0 = v[0];
 #if MC_PACKED_FMA
@@ -573,1822 +573,6 @@ template <bool INV> __device__ __forceinline__ void dft_r13(float2* v) {
     }
   }
 #endif
-}
-template <bool INV> __device__ __forceinline__ void dft_r53(float2* v) {
-  const float2 x0 = v[0];
-  const float2 s1 = padd(v[1], v[52]);
-  const float2 d1 = psub(v[1], v[52]);
-  const float2 s2 = padd(v[2], v[51]);
-  const float2 d2 = psub(v[2], v[51]);
-  const float2 s3 = padd(v[3], v[50]);
-  const float2 d3 = psub(v[3], v[50]);
-  const float2 s4 = padd(v[4], v[49]);
-  const float2 d4 = psub(v[4], v[49]);
-  const float2 s5 = padd(v[5], v[48]);
-  const float2 d5 = psub(v[5], v[48]);
-  const float2 s6 = padd(v[6], v[47]);
-  const float2 d6 = psub(v[6], v[47]);
-  const float2 s7 = padd(v[7], v[46]);
-  const float2 d7 = psub(v[7], v[46]);
-  const float2 s8 = padd(v[8], v[45]);
-  const float2 d8 = psub(v[8], v[45]);
-  const float2 s9 = padd(v[9], v[44]);
-  const float2 d9 = psub(v[9], v[44]);
-  const float2 s10 = padd(v[10], v[43]);
-  const float2 d10 = psub(v[10], v[43]);
-  const float2 s11 = padd(v[11], v[42]);
-  const float2 d11 = psub(v[11], v[42]);
-  const float2 s12 = padd(v[12], v[41]);
-  const float2 d12 = psub(v[12], v[41]);
-  const float2 s13 = padd(v[13], v[40]);
-  const float2 d13 = psub(v[13], v[40]);
-  const float2 s14 = padd(v[14], v[39]);
-  const float2 d14 = psub(v[14], v[39]);
-  const float2 s15 = padd(v[15], v[38]);
-  const float2 d15 = psub(v[15], v[38]);
-  const float2 s16 = padd(v[16], v[37]);
-  const float2 d16 = psub(v[16], v[37]);
-  const float2 s17 = padd(v[17], v[36]);
-  const float2 d17 = psub(v[17], v[36]);
-  const float2 s18 = padd(v[18], v[35]);
-  const float2 d18 = psub(v[18], v[35]);
-  const float2 s19 = padd(v[19], v[34]);
-  const float2 d19 = psub(v[19], v[34]);
-  const float2 s20 = padd(v[20], v[33]);
-  const float2 d20 = psub(v[20], v[33]);
-  const float2 s21 = padd(v[21], v[32]);
-  const float2 d21 = psub(v[21], v[32]);
-  const float2 s22 = padd(v[22], v[31]);
-  const float2 d22 = psub(v[22], v[31]);
-  const float2 s23 = padd(v[23], v[30]);
-  const float2 d23 = psub(v[23], v[30]);
-  const float2 s24 = padd(v[24], v[29]);
-  const float2 d24 = psub(v[24], v[29]);
-  const float2 s25 = padd(v[25], v[28]);
-  const float2 d25 = psub(v[25], v[28]);
-  const float2 s26 = padd(v[26], v[27]);
-  const float2 d26 = psub(v[26], v[27]);
-  v[0] = make_float2(x0.x + (s1.x + s2.x + s3.x + s4.x + s5.x + s6.x + s7.x + s8.x + s9.x + s10.x + s11.x + s12.x + s13.x + s14.x + s15.x + s16.x + s17.x + s18.x + s19.x + s20.x + s21.x + s22.x + s23.x + s24.x + s25.x + s26.x), x0.y + (s1.y + s2.y + s3.y + s4.y + s5.y + s6.y + s7.y + s8.y + s9.y + s10.y + s11.y + s12.y + s13.y + s14.y + s15.y + s16.y + s17.y + s18.y + s19.y + s20.y + s21.y + s22.y + s23.y + s24.y + s25.y + s26.y));
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.9929810762405396f, ar); ai = fmaf(s1.y, 0.9929810762405396f, ai); br = fmaf(d1.x, 0.11827316880226135f, br); bi = fmaf(d1.y, 0.11827316880226135f, bi);
-    ar = fmaf(s2.x, 0.9720228910446167f, ar); ai = fmaf(s2.y, 0.9720228910446167f, ai); br = fmaf(d2.x, 0.2348860502243042f, br); bi = fmaf(d2.y, 0.2348860502243042f, bi);
-    ar = fmaf(s3.x, 0.9374196529388428f, ar); ai = fmaf(s3.y, 0.9374196529388428f, ai); br = fmaf(d3.x, 0.3482016324996948f, br); bi = fmaf(d3.y, 0.3482016324996948f, bi);
-    ar = fmaf(s4.x, 0.8896570801734924f, ar); ai = fmaf(s4.y, 0.8896570801734924f, ai); br = fmaf(d4.x, 0.4566292464733124f, br); bi = fmaf(d4.y, 0.4566292464733124f, bi);
-    ar = fmaf(s5.x, 0.829405665397644f, ar); ai = fmaf(s5.y, 0.829405665397644f, ai); br = fmaf(d5.x, 0.5586467385292053f, br); bi = fmaf(d5.y, 0.5586467385292053f, bi);
-    ar = fmaf(s6.x, 0.7575112581253052f, ar); ai = fmaf(s6.y, 0.7575112581253052f, ai); br = fmaf(d6.x, 0.6528221368789673f, br); bi = fmaf(d6.y, 0.6528221368789673f, bi);
-    ar = fmaf(s7.x, 0.674983024597168f, ar); ai = fmaf(s7.y, 0.674983024597168f, ai); br = fmaf(d7.x, 0.7378332614898682f, br); bi = fmaf(d7.y, 0.7378332614898682f, bi);
-    ar = fmaf(s8.x, 0.5829795002937317f, ar); ai = fmaf(s8.y, 0.5829795002937317f, ai); br = fmaf(d8.x, 0.8124868869781494f, br); bi = fmaf(d8.y, 0.8124868869781494f, bi);
-    ar = fmaf(s9.x, 0.4827921986579895f, ar); ai = fmaf(s9.y, 0.4827921986579895f, ai); br = fmaf(d9.x, 0.8757349252700806f, br); bi = fmaf(d9.y, 0.8757349252700806f, bi);
-    ar = fmaf(s10.x, 0.3758275806903839f, ar); ai = fmaf(s10.y, 0.3758275806903839f, ai); br = fmaf(d10.x, 0.926689624786377f, br); bi = fmaf(d10.y, 0.926689624786377f, bi);
-    ar = fmaf(s11.x, 0.26358717679977417f, ar); ai = fmaf(s11.y, 0.26358717679977417f, ai); br = fmaf(d11.x, 0.9646356105804443f, br); bi = fmaf(d11.y, 0.9646356105804443f, bi);
-    ar = fmaf(s12.x, 0.14764656126499176f, ar); ai = fmaf(s12.y, 0.14764656126499176f, ai); br = fmaf(d12.x, 0.989040195941925f, br); bi = fmaf(d12.y, 0.989040195941925f, bi);
-    ar = fmaf(s13.x, 0.029633328318595886f, ar); ai = fmaf(s13.y, 0.029633328318595886f, ai); br = fmaf(d13.x, 0.9995608329772949f, br); bi = fmaf(d13.y, 0.9995608329772949f, bi);
-    ar = fmaf(s14.x, -0.08879589289426804f, ar); ai = fmaf(s14.y, -0.08879589289426804f, ai); br = fmaf(d14.x, 0.9960498213768005f, br); bi = fmaf(d14.y, 0.9960498213768005f, bi);
-    ar = fmaf(s15.x, -0.2059786170721054f, ar); ai = fmaf(s15.y, -0.2059786170721054f, ai); br = fmaf(d15.x, 0.9785565137863159f, br); bi = fmaf(d15.y, 0.9785565137863159f, bi);
-    ar = fmaf(s16.x, -0.3202698528766632f, ar); ai = fmaf(s16.y, -0.3202698528766632f, ai); br = fmaf(d16.x, 0.9473263621330261f, br); bi = fmaf(d16.y, 0.9473263621330261f, bi);
-    ar = fmaf(s17.x, -0.43006521463394165f, ar); ai = fmaf(s17.y, -0.43006521463394165f, ai); br = fmaf(d17.x, 0.9027978181838989f, br); bi = fmaf(d17.y, 0.9027978181838989f, bi);
-    ar = fmaf(s18.x, -0.5338233709335327f, ar); ai = fmaf(s18.y, -0.5338233709335327f, ai); br = fmaf(d18.x, 0.8455960154533386f, br); bi = fmaf(d18.y, 0.8455960154533386f, bi);
-    ar = fmaf(s19.x, -0.6300878524780273f, ar); ai = fmaf(s19.y, -0.6300878524780273f, ai); br = fmaf(d19.x, 0.7765238881111145f, br); bi = fmaf(d19.y, 0.7765238881111145f, bi);
-    ar = fmaf(s20.x, -0.7175072431564331f, ar); ai = fmaf(s20.y, -0.7175072431564331f, ai); br = fmaf(d20.x, 0.6965510249137878f, br); bi = fmaf(d20.y, 0.6965510249137878f, bi);
-    ar = fmaf(s21.x, -0.794854462146759f, ar); ai = fmaf(s21.y, -0.794854462146759f, ai); br = fmaf(d21.x, 0.6068001389503479f, br); bi = fmaf(d21.y, 0.6068001389503479f, bi);
-    ar = fmaf(s22.x, -0.8610436320304871f, ar); ai = fmaf(s22.y, -0.8610436320304871f, ai); br = fmaf(d22.x, 0.5085310935974121f, br); bi = fmaf(d22.y, 0.5085310935974121f, bi);
-    ar = fmaf(s23.x, -0.9151456356048584f, ar); ai = fmaf(s23.y, -0.9151456356048584f, ai); br = fmaf(d23.x, 0.4031234383583069f, br); bi = fmaf(d23.y, 0.4031234383583069f, bi);
-    ar = fmaf(s24.x, -0.956400990486145f, ar); ai = fmaf(s24.y, -0.956400990486145f, ai); br = fmaf(d24.x, 0.29205676913261414f, br); bi = fmaf(d24.y, 0.29205676913261414f, bi);
-    ar = fmaf(s25.x, -0.9842305779457092f, ar); ai = fmaf(s25.y, -0.9842305779457092f, ai); br = fmaf(d25.x, 0.1768902689218521f, br); bi = fmaf(d25.y, 0.1768902689218521f, bi);
-    ar = fmaf(s26.x, -0.9982437491416931f, ar); ai = fmaf(s26.y, -0.9982437491416931f, ai); br = fmaf(d26.x, 0.05924062803387642f, br); bi = fmaf(d26.y, 0.05924062803387642f, bi);
-    if (!INV) {
-      v[1] = make_float2(ar + bi, ai - br); v[52] = make_float2(ar - bi, ai + br);
-    } else {
-      v[1] = make_float2(ar - bi, ai + br); v[52] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.9720228910446167f, ar); ai = fmaf(s1.y, 0.9720228910446167f, ai); br = fmaf(d1.x, 0.2348860502243042f, br); bi = fmaf(d1.y, 0.2348860502243042f, bi);
-    ar = fmaf(s2.x, 0.8896570801734924f, ar); ai = fmaf(s2.y, 0.8896570801734924f, ai); br = fmaf(d2.x, 0.4566292464733124f, br); bi = fmaf(d2.y, 0.4566292464733124f, bi);
-    ar = fmaf(s3.x, 0.7575112581253052f, ar); ai = fmaf(s3.y, 0.7575112581253052f, ai); br = fmaf(d3.x, 0.6528221368789673f, br); bi = fmaf(d3.y, 0.6528221368789673f, bi);
-    ar = fmaf(s4.x, 0.5829795002937317f, ar); ai = fmaf(s4.y, 0.5829795002937317f, ai); br = fmaf(d4.x, 0.8124868869781494f, br); bi = fmaf(d4.y, 0.8124868869781494f, bi);
-    ar = fmaf(s5.x, 0.3758275806903839f, ar); ai = fmaf(s5.y, 0.3758275806903839f, ai); br = fmaf(d5.x, 0.926689624786377f, br); bi = fmaf(d5.y, 0.926689624786377f, bi);
-    ar = fmaf(s6.x, 0.14764656126499176f, ar); ai = fmaf(s6.y, 0.14764656126499176f, ai); br = fmaf(d6.x, 0.989040195941925f, br); bi = fmaf(d6.y, 0.989040195941925f, bi);
-    ar = fmaf(s7.x, -0.08879589289426804f, ar); ai = fmaf(s7.y, -0.08879589289426804f, ai); br = fmaf(d7.x, 0.9960498213768005f, br); bi = fmaf(d7.y, 0.9960498213768005f, bi);
-    ar = fmaf(s8.x, -0.3202698528766632f, ar); ai = fmaf(s8.y, -0.3202698528766632f, ai); br = fmaf(d8.x, 0.9473263621330261f, br); bi = fmaf(d8.y, 0.9473263621330261f, bi);
-    ar = fmaf(s9.x, -0.5338233709335327f, ar); ai = fmaf(s9.y, -0.5338233709335327f, ai); br = fmaf(d9.x, 0.8455960154533386f, br); bi = fmaf(d9.y, 0.8455960154533386f, bi);
-    ar = fmaf(s10.x, -0.7175072431564331f, ar); ai = fmaf(s10.y, -0.7175072431564331f, ai); br = fmaf(d10.x, 0.6965510249137878f, br); bi = fmaf(d10.y, 0.6965510249137878f, bi);
-    ar = fmaf(s11.x, -0.8610436320304871f, ar); ai = fmaf(s11.y, -0.8610436320304871f, ai); br = fmaf(d11.x, 0.5085310935974121f, br); bi = fmaf(d11.y, 0.5085310935974121f, bi);
-    ar = fmaf(s12.x, -0.956400990486145f, ar); ai = fmaf(s12.y, -0.956400990486145f, ai); br = fmaf(d12.x, 0.29205676913261414f, br); bi = fmaf(d12.y, 0.29205676913261414f, bi);
-    ar = fmaf(s13.x, -0.9982437491416931f, ar); ai = fmaf(s13.y, -0.9982437491416931f, ai); br = fmaf(d13.x, 0.05924062803387642f, br); bi = fmaf(d13.y, 0.05924062803387642f, bi);
-    ar = fmaf(s14.x, -0.9842305779457092f, ar); ai = fmaf(s14.y, -0.9842305779457092f, ai); br = fmaf(d14.x, -0.1768902689218521f, br); bi = fmaf(d14.y, -0.1768902689218521f, bi);
-    ar = fmaf(s15.x, -0.9151456356048584f, ar); ai = fmaf(s15.y, -0.9151456356048584f, ai); br = fmaf(d15.x, -0.4031234383583069f, br); bi = fmaf(d15.y, -0.4031234383583069f, bi);
-    ar = fmaf(s16.x, -0.794854462146759f, ar); ai = fmaf(s16.y, -0.794854462146759f, ai); br = fmaf(d16.x, -0.6068001389503479f, br); bi = fmaf(d16.y, -0.6068001389503479f, bi);
-    ar = fmaf(s17.x, -0.6300878524780273f, ar); ai = fmaf(s17.y, -0.6300878524780273f, ai); br = fmaf(d17.x, -0.7765238881111145f, br); bi = fmaf(d17.y, -0.7765238881111145f, bi);
-    ar = fmaf(s18.x, -0.43006521463394165f, ar); ai = fmaf(s18.y, -0.43006521463394165f, ai); br = fmaf(d18.x, -0.9027978181838989f, br); bi = fmaf(d18.y, -0.9027978181838989f, bi);
-    ar = fmaf(s19.x, -0.2059786170721054f, ar); ai = fmaf(s19.y, -0.2059786170721054f, ai); br = fmaf(d19.x, -0.9785565137863159f, br); bi = fmaf(d19.y, -0.9785565137863159f, bi);
-    ar = fmaf(s20.x, 0.029633328318595886f, ar); ai = fmaf(s20.y, 0.029633328318595886f, ai); br = fmaf(d20.x, -0.9995608329772949f, br); bi = fmaf(d20.y, -0.9995608329772949f, bi);
-    ar = fmaf(s21.x, 0.26358717679977417f, ar); ai = fmaf(s21.y, 0.26358717679977417f, ai); br = fmaf(d21.x, -0.9646356105804443f, br); bi = fmaf(d21.y, -0.9646356105804443f, bi);
-    ar = fmaf(s22.x, 0.4827921986579895f, ar); ai = fmaf(s22.y, 0.4827921986579895f, ai); br = fmaf(d22.x, -0.8757349252700806f, br); bi = fmaf(d22.y, -0.8757349252700806f, bi);
-    ar = fmaf(s23.x, 0.674983024597168f, ar); ai = fmaf(s23.y, 0.674983024597168f, ai); br = fmaf(d23.x, -0.7378332614898682f, br); bi = fmaf(d23.y, -0.7378332614898682f, bi);
-    ar = fmaf(s24.x, 0.829405665397644f, ar); ai = fmaf(s24.y, 0.829405665397644f, ai); br = fmaf(d24.x, -0.5586467385292053f, br); bi = fmaf(d24.y, -0.5586467385292053f, bi);
-    ar = fmaf(s25.x, 0.9374196529388428f, ar); ai = fmaf(s25.y, 0.9374196529388428f, ai); br = fmaf(d25.x, -0.3482016324996948f, br); bi = fmaf(d25.y, -0.3482016324996948f, bi);
-    ar = fmaf(s26.x, 0.9929810762405396f, ar); ai = fmaf(s26.y, 0.9929810762405396f, ai); br = fmaf(d26.x, -0.11827316880226135f, br); bi = fmaf(d26.y, -0.11827316880226135f, bi);
-    if (!INV) {
-      v[2] = make_float2(ar + bi, ai - br); v[51] = make_float2(ar - bi, ai + br);
-    } else {
-      v[2] = make_float2(ar - bi, ai + br); v[51] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.9374196529388428f, ar); ai = fmaf(s1.y, 0.9374196529388428f, ai); br = fmaf(d1.x, 0.3482016324996948f, br); bi = fmaf(d1.y, 0.3482016324996948f, bi);
-    ar = fmaf(s2.x, 0.7575112581253052f, ar); ai = fmaf(s2.y, 0.7575112581253052f, ai); br = fmaf(d2.x, 0.6528221368789673f, br); bi = fmaf(d2.y, 0.6528221368789673f, bi);
-    ar = fmaf(s3.x, 0.4827921986579895f, ar); ai = fmaf(s3.y, 0.4827921986579895f, ai); br = fmaf(d3.x, 0.8757349252700806f, br); bi = fmaf(d3.y, 0.8757349252700806f, bi);
-    ar = fmaf(s4.x, 0.14764656126499176f, ar); ai = fmaf(s4.y, 0.14764656126499176f, ai); br = fmaf(d4.x, 0.989040195941925f, br); bi = fmaf(d4.y, 0.989040195941925f, bi);
-    ar = fmaf(s5.x, -0.2059786170721054f, ar); ai = fmaf(s5.y, -0.2059786170721054f, ai); br = fmaf(d5.x, 0.9785565137863159f, br); bi = fmaf(d5.y, 0.9785565137863159f, bi);
-    ar = fmaf(s6.x, -0.5338233709335327f, ar); ai = fmaf(s6.y, -0.5338233709335327f, ai); br = fmaf(d6.x, 0.8455960154533386f, br); bi = fmaf(d6.y, 0.8455960154533386f, bi);
-    ar = fmaf(s7.x, -0.794854462146759f, ar); ai = fmaf(s7.y, -0.794854462146759f, ai); br = fmaf(d7.x, 0.6068001389503479f, br); bi = fmaf(d7.y, 0.6068001389503479f, bi);
-    ar = fmaf(s8.x, -0.956400990486145f, ar); ai = fmaf(s8.y, -0.956400990486145f, ai); br = fmaf(d8.x, 0.29205676913261414f, br); bi = fmaf(d8.y, 0.29205676913261414f, bi);
-    ar = fmaf(s9.x, -0.9982437491416931f, ar); ai = fmaf(s9.y, -0.9982437491416931f, ai); br = fmaf(d9.x, -0.05924062803387642f, br); bi = fmaf(d9.y, -0.05924062803387642f, bi);
-    ar = fmaf(s10.x, -0.9151456356048584f, ar); ai = fmaf(s10.y, -0.9151456356048584f, ai); br = fmaf(d10.x, -0.4031234383583069f, br); bi = fmaf(d10.y, -0.4031234383583069f, bi);
-    ar = fmaf(s11.x, -0.7175072431564331f, ar); ai = fmaf(s11.y, -0.7175072431564331f, ai); br = fmaf(d11.x, -0.6965510249137878f, br); bi = fmaf(d11.y, -0.6965510249137878f, bi);
-    ar = fmaf(s12.x, -0.43006521463394165f, ar); ai = fmaf(s12.y, -0.43006521463394165f, ai); br = fmaf(d12.x, -0.9027978181838989f, br); bi = fmaf(d12.y, -0.9027978181838989f, bi);
-    ar = fmaf(s13.x, -0.08879589289426804f, ar); ai = fmaf(s13.y, -0.08879589289426804f, ai); br = fmaf(d13.x, -0.9960498213768005f, br); bi = fmaf(d13.y, -0.9960498213768005f, bi);
-    ar = fmaf(s14.x, 0.26358717679977417f, ar); ai = fmaf(s14.y, 0.26358717679977417f, ai); br = fmaf(d14.x, -0.9646356105804443f, br); bi = fmaf(d14.y, -0.9646356105804443f, bi);
-    ar = fmaf(s15.x, 0.5829795002937317f, ar); ai = fmaf(s15.y, 0.5829795002937317f, ai); br = fmaf(d15.x, -0.8124868869781494f, br); bi = fmaf(d15.y, -0.8124868869781494f, bi);
-    ar = fmaf(s16.x, 0.829405665397644f, ar); ai = fmaf(s16.y, 0.829405665397644f, ai); br = fmaf(d16.x, -0.5586467385292053f, br); bi = fmaf(d16.y, -0.5586467385292053f, bi);
-    ar = fmaf(s17.x, 0.9720228910446167f, ar); ai = fmaf(s17.y, 0.9720228910446167f, ai); br = fmaf(d17.x, -0.2348860502243042f, br); bi = fmaf(d17.y, -0.2348860502243042f, bi);
-    ar = fmaf(s18.x, 0.9929810762405396f, ar); ai = fmaf(s18.y, 0.9929810762405396f, ai); br = fmaf(d18.x, 0.11827316880226135f, br); bi = fmaf(d18.y, 0.11827316880226135f, bi);
-    ar = fmaf(s19.x, 0.8896570801734924f, ar); ai = fmaf(s19.y, 0.8896570801734924f, ai); br = fmaf(d19.x, 0.4566292464733124f, br); bi = fmaf(d19.y, 0.4566292464733124f, bi);
-    ar = fmaf(s20.x, 0.674983024597168f, ar); ai = fmaf(s20.y, 0.674983024597168f, ai); br = fmaf(d20.x, 0.7378332614898682f, br); bi = fmaf(d20.y, 0.7378332614898682f, bi);
-    ar = fmaf(s21.x, 0.3758275806903839f, ar); ai = fmaf(s21.y, 0.3758275806903839f, ai); br = fmaf(d21.x, 0.926689624786377f, br); bi = fmaf(d21.y, 0.926689624786377f, bi);
-    ar = fmaf(s22.x, 0.029633328318595886f, ar); ai = fmaf(s22.y, 0.029633328318595886f, ai); br = fmaf(d22.x, 0.9995608329772949f, br); bi = fmaf(d22.y, 0.9995608329772949f, bi);
-    ar = fmaf(s23.x, -0.3202698528766632f, ar); ai = fmaf(s23.y, -0.3202698528766632f, ai); br = fmaf(d23.x, 0.9473263621330261f, br); bi = fmaf(d23.y, 0.9473263621330261f, bi);
-    ar = fmaf(s24.x, -0.6300878524780273f, ar); ai = fmaf(s24.y, -0.6300878524780273f, ai); br = fmaf(d24.x, 0.7765238881111145f, br); bi = fmaf(d24.y, 0.7765238881111145f, bi);
-    ar = fmaf(s25.x, -0.8610436320304871f, ar); ai = fmaf(s25.y, -0.8610436320304871f, ai); br = fmaf(d25.x, 0.5085310935974121f, br); bi = fmaf(d25.y, 0.5085310935974121f, bi);
-    ar = fmaf(s26.x, -0.9842305779457092f, ar); ai = fmaf(s26.y, -0.9842305779457092f, ai); br = fmaf(d26.x, 0.1768902689218521f, br); bi = fmaf(d26.y, 0.1768902689218521f, bi);
-    if (!INV) {
-      v[3] = make_float2(ar + bi, ai - br); v[50] = make_float2(ar - bi, ai + br);
-    } else {
-      v[3] = make_float2(ar - bi, ai + br); v[50] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.8896570801734924f, ar); ai = fmaf(s1.y, 0.8896570801734924f, ai); br = fmaf(d1.x, 0.4566292464733124f, br); bi = fmaf(d1.y, 0.4566292464733124f, bi);
-    ar = fmaf(s2.x, 0.5829795002937317f, ar); ai = fmaf(s2.y, 0.5829795002937317f, ai); br = fmaf(d2.x, 0.8124868869781494f, br); bi = fmaf(d2.y, 0.8124868869781494f, bi);
-    ar = fmaf(s3.x, 0.14764656126499176f, ar); ai = fmaf(s3.y, 0.14764656126499176f, ai); br = fmaf(d3.x, 0.989040195941925f, br); bi = fmaf(d3.y, 0.989040195941925f, bi);
-    ar = fmaf(s4.x, -0.3202698528766632f, ar); ai = fmaf(s4.y, -0.3202698528766632f, ai); br = fmaf(d4.x, 0.9473263621330261f, br); bi = fmaf(d4.y, 0.9473263621330261f, bi);
-    ar = fmaf(s5.x, -0.7175072431564331f, ar); ai = fmaf(s5.y, -0.7175072431564331f, ai); br = fmaf(d5.x, 0.6965510249137878f, br); bi = fmaf(d5.y, 0.6965510249137878f, bi);
-    ar = fmaf(s6.x, -0.956400990486145f, ar); ai = fmaf(s6.y, -0.956400990486145f, ai); br = fmaf(d6.x, 0.29205676913261414f, br); bi = fmaf(d6.y, 0.29205676913261414f, bi);
-    ar = fmaf(s7.x, -0.9842305779457092f, ar); ai = fmaf(s7.y, -0.9842305779457092f, ai); br = fmaf(d7.x, -0.1768902689218521f, br); bi = fmaf(d7.y, -0.1768902689218521f, bi);
-    ar = fmaf(s8.x, -0.794854462146759f, ar); ai = fmaf(s8.y, -0.794854462146759f, ai); br = fmaf(d8.x, -0.6068001389503479f, br); bi = fmaf(d8.y, -0.6068001389503479f, bi);
-    ar = fmaf(s9.x, -0.43006521463394165f, ar); ai = fmaf(s9.y, -0.43006521463394165f, ai); br = fmaf(d9.x, -0.9027978181838989f, br); bi = fmaf(d9.y, -0.9027978181838989f, bi);
-    ar = fmaf(s10.x, 0.029633328318595886f, ar); ai = fmaf(s10.y, 0.029633328318595886f, ai); br = fmaf(d10.x, -0.9995608329772949f, br); bi = fmaf(d10.y, -0.9995608329772949f, bi);
-    ar = fmaf(s11.x, 0.4827921986579895f, ar); ai = fmaf(s11.y, 0.4827921986579895f, ai); br = fmaf(d11.x, -0.8757349252700806f, br); bi = fmaf(d11.y, -0.8757349252700806f, bi);
-    ar = fmaf(s12.x, 0.829405665397644f, ar); ai = fmaf(s12.y, 0.829405665397644f, ai); br = fmaf(d12.x, -0.5586467385292053f, br); bi = fmaf(d12.y, -0.5586467385292053f, bi);
-    ar = fmaf(s13.x, 0.9929810762405396f, ar); ai = fmaf(s13.y, 0.9929810762405396f, ai); br = fmaf(d13.x, -0.11827316880226135f, br); bi = fmaf(d13.y, -0.11827316880226135f, bi);
-    ar = fmaf(s14.x, 0.9374196529388428f, ar); ai = fmaf(s14.y, 0.9374196529388428f, ai); br = fmaf(d14.x, 0.3482016324996948f, br); bi = fmaf(d14.y, 0.3482016324996948f, bi);
-    ar = fmaf(s15.x, 0.674983024597168f, ar); ai = fmaf(s15.y, 0.674983024597168f, ai); br = fmaf(d15.x, 0.7378332614898682f, br); bi = fmaf(d15.y, 0.7378332614898682f, bi);
-    ar = fmaf(s16.x, 0.26358717679977417f, ar); ai = fmaf(s16.y, 0.26358717679977417f, ai); br = fmaf(d16.x, 0.9646356105804443f, br); bi = fmaf(d16.y, 0.9646356105804443f, bi);
-    ar = fmaf(s17.x, -0.2059786170721054f, ar); ai = fmaf(s17.y, -0.2059786170721054f, ai); br = fmaf(d17.x, 0.9785565137863159f, br); bi = fmaf(d17.y, 0.9785565137863159f, bi);
-    ar = fmaf(s18.x, -0.6300878524780273f, ar); ai = fmaf(s18.y, -0.6300878524780273f, ai); br = fmaf(d18.x, 0.7765238881111145f, br); bi = fmaf(d18.y, 0.7765238881111145f, bi);
-    ar = fmaf(s19.x, -0.9151456356048584f, ar); ai = fmaf(s19.y, -0.9151456356048584f, ai); br = fmaf(d19.x, 0.4031234383583069f, br); bi = fmaf(d19.y, 0.4031234383583069f, bi);
-    ar = fmaf(s20.x, -0.9982437491416931f, ar); ai = fmaf(s20.y, -0.9982437491416931f, ai); br = fmaf(d20.x, -0.05924062803387642f, br); bi = fmaf(d20.y, -0.05924062803387642f, bi);
-    ar = fmaf(s21.x, -0.8610436320304871f, ar); ai = fmaf(s21.y, -0.8610436320304871f, ai); br = fmaf(d21.x, -0.5085310935974121f, br); bi = fmaf(d21.y, -0.5085310935974121f, bi);
-    ar = fmaf(s22.x, -0.5338233709335327f, ar); ai = fmaf(s22.y, -0.5338233709335327f, ai); br = fmaf(d22.x, -0.8455960154533386f, br); bi = fmaf(d22.y, -0.8455960154533386f, bi);
-    ar = fmaf(s23.x, -0.08879589289426804f, ar); ai = fmaf(s23.y, -0.08879589289426804f, ai); br = fmaf(d23.x, -0.9960498213768005f, br); bi = fmaf(d23.y, -0.9960498213768005f, bi);
-    ar = fmaf(s24.x, 0.3758275806903839f, ar); ai = fmaf(s24.y, 0.3758275806903839f, ai); br = fmaf(d24.x, -0.926689624786377f, br); bi = fmaf(d24.y, -0.926689624786377f, bi);
-    ar = fmaf(s25.x, 0.7575112581253052f, ar); ai = fmaf(s25.y, 0.7575112581253052f, ai); br = fmaf(d25.x, -0.6528221368789673f, br); bi = fmaf(d25.y, -0.6528221368789673f, bi);
-    ar = fmaf(s26.x, 0.9720228910446167f, ar); ai = fmaf(s26.y, 0.9720228910446167f, ai); br = fmaf(d26.x, -0.2348860502243042f, br); bi = fmaf(d26.y, -0.2348860502243042f, bi);
-    if (!INV) {
-      v[4] = make_float2(ar + bi, ai - br); v[49] = make_float2(ar - bi, ai + br);
-    } else {
-      v[4] = make_float2(ar - bi, ai + br); v[49] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.829405665397644f, ar); ai = fmaf(s1.y, 0.829405665397644f, ai); br = fmaf(d1.x, 0.5586467385292053f, br); bi = fmaf(d1.y, 0.5586467385292053f, bi);
-    ar = fmaf(s2.x, 0.3758275806903839f, ar); ai = fmaf(s2.y, 0.3758275806903839f, ai); br = fmaf(d2.x, 0.926689624786377f, br); bi = fmaf(d2.y, 0.926689624786377f, bi);
-    ar = fmaf(s3.x, -0.2059786170721054f, ar); ai = fmaf(s3.y, -0.2059786170721054f, ai); br = fmaf(d3.x, 0.9785565137863159f, br); bi = fmaf(d3.y, 0.9785565137863159f, bi);
-    ar = fmaf(s4.x, -0.7175072431564331f, ar); ai = fmaf(s4.y, -0.7175072431564331f, ai); br = fmaf(d4.x, 0.6965510249137878f, br); bi = fmaf(d4.y, 0.6965510249137878f, bi);
-    ar = fmaf(s5.x, -0.9842305779457092f, ar); ai = fmaf(s5.y, -0.9842305779457092f, ai); br = fmaf(d5.x, 0.1768902689218521f, br); bi = fmaf(d5.y, 0.1768902689218521f, bi);
-    ar = fmaf(s6.x, -0.9151456356048584f, ar); ai = fmaf(s6.y, -0.9151456356048584f, ai); br = fmaf(d6.x, -0.4031234383583069f, br); bi = fmaf(d6.y, -0.4031234383583069f, bi);
-    ar = fmaf(s7.x, -0.5338233709335327f, ar); ai = fmaf(s7.y, -0.5338233709335327f, ai); br = fmaf(d7.x, -0.8455960154533386f, br); bi = fmaf(d7.y, -0.8455960154533386f, bi);
-    ar = fmaf(s8.x, 0.029633328318595886f, ar); ai = fmaf(s8.y, 0.029633328318595886f, ai); br = fmaf(d8.x, -0.9995608329772949f, br); bi = fmaf(d8.y, -0.9995608329772949f, bi);
-    ar = fmaf(s9.x, 0.5829795002937317f, ar); ai = fmaf(s9.y, 0.5829795002937317f, ai); br = fmaf(d9.x, -0.8124868869781494f, br); bi = fmaf(d9.y, -0.8124868869781494f, bi);
-    ar = fmaf(s10.x, 0.9374196529388428f, ar); ai = fmaf(s10.y, 0.9374196529388428f, ai); br = fmaf(d10.x, -0.3482016324996948f, br); bi = fmaf(d10.y, -0.3482016324996948f, bi);
-    ar = fmaf(s11.x, 0.9720228910446167f, ar); ai = fmaf(s11.y, 0.9720228910446167f, ai); br = fmaf(d11.x, 0.2348860502243042f, br); bi = fmaf(d11.y, 0.2348860502243042f, bi);
-    ar = fmaf(s12.x, 0.674983024597168f, ar); ai = fmaf(s12.y, 0.674983024597168f, ai); br = fmaf(d12.x, 0.7378332614898682f, br); bi = fmaf(d12.y, 0.7378332614898682f, bi);
-    ar = fmaf(s13.x, 0.14764656126499176f, ar); ai = fmaf(s13.y, 0.14764656126499176f, ai); br = fmaf(d13.x, 0.989040195941925f, br); bi = fmaf(d13.y, 0.989040195941925f, bi);
-    ar = fmaf(s14.x, -0.43006521463394165f, ar); ai = fmaf(s14.y, -0.43006521463394165f, ai); br = fmaf(d14.x, 0.9027978181838989f, br); bi = fmaf(d14.y, 0.9027978181838989f, bi);
-    ar = fmaf(s15.x, -0.8610436320304871f, ar); ai = fmaf(s15.y, -0.8610436320304871f, ai); br = fmaf(d15.x, 0.5085310935974121f, br); bi = fmaf(d15.y, 0.5085310935974121f, bi);
-    ar = fmaf(s16.x, -0.9982437491416931f, ar); ai = fmaf(s16.y, -0.9982437491416931f, ai); br = fmaf(d16.x, -0.05924062803387642f, br); bi = fmaf(d16.y, -0.05924062803387642f, bi);
-    ar = fmaf(s17.x, -0.794854462146759f, ar); ai = fmaf(s17.y, -0.794854462146759f, ai); br = fmaf(d17.x, -0.6068001389503479f, br); bi = fmaf(d17.y, -0.6068001389503479f, bi);
-    ar = fmaf(s18.x, -0.3202698528766632f, ar); ai = fmaf(s18.y, -0.3202698528766632f, ai); br = fmaf(d18.x, -0.9473263621330261f, br); bi = fmaf(d18.y, -0.9473263621330261f, bi);
-    ar = fmaf(s19.x, 0.26358717679977417f, ar); ai = fmaf(s19.y, 0.26358717679977417f, ai); br = fmaf(d19.x, -0.9646356105804443f, br); bi = fmaf(d19.y, -0.9646356105804443f, bi);
-    ar = fmaf(s20.x, 0.7575112581253052f, ar); ai = fmaf(s20.y, 0.7575112581253052f, ai); br = fmaf(d20.x, -0.6528221368789673f, br); bi = fmaf(d20.y, -0.6528221368789673f, bi);
-    ar = fmaf(s21.x, 0.9929810762405396f, ar); ai = fmaf(s21.y, 0.9929810762405396f, ai); br = fmaf(d21.x, -0.11827316880226135f, br); bi = fmaf(d21.y, -0.11827316880226135f, bi);
-    ar = fmaf(s22.x, 0.8896570801734924f, ar); ai = fmaf(s22.y, 0.8896570801734924f, ai); br = fmaf(d22.x, 0.4566292464733124f, br); bi = fmaf(d22.y, 0.4566292464733124f, bi);
-    ar = fmaf(s23.x, 0.4827921986579895f, ar); ai = fmaf(s23.y, 0.4827921986579895f, ai); br = fmaf(d23.x, 0.8757349252700806f, br); bi = fmaf(d23.y, 0.8757349252700806f, bi);
-    ar = fmaf(s24.x, -0.08879589289426804f, ar); ai = fmaf(s24.y, -0.08879589289426804f, ai); br = fmaf(d24.x, 0.9960498213768005f, br); bi = fmaf(d24.y, 0.9960498213768005f, bi);
-    ar = fmaf(s25.x, -0.6300878524780273f, ar); ai = fmaf(s25.y, -0.6300878524780273f, ai); br = fmaf(d25.x, 0.7765238881111145f, br); bi = fmaf(d25.y, 0.7765238881111145f, bi);
-    ar = fmaf(s26.x, -0.956400990486145f, ar); ai = fmaf(s26.y, -0.956400990486145f, ai); br = fmaf(d26.x, 0.29205676913261414f, br); bi = fmaf(d26.y, 0.29205676913261414f, bi);
-    if (!INV) {
-      v[5] = make_float2(ar + bi, ai - br); v[48] = make_float2(ar - bi, ai + br);
-    } else {
-      v[5] = make_float2(ar - bi, ai + br); v[48] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.7575112581253052f, ar); ai = fmaf(s1.y, 0.7575112581253052f, ai); br = fmaf(d1.x, 0.6528221368789673f, br); bi = fmaf(d1.y, 0.6528221368789673f, bi);
-    ar = fmaf(s2.x, 0.14764656126499176f, ar); ai = fmaf(s2.y, 0.14764656126499176f, ai); br = fmaf(d2.x, 0.989040195941925f, br); bi = fmaf(d2.y, 0.989040195941925f, bi);
-    ar = fmaf(s3.x, -0.5338233709335327f, ar); ai = fmaf(s3.y, -0.5338233709335327f, ai); br = fmaf(d3.x, 0.8455960154533386f, br); bi = fmaf(d3.y, 0.8455960154533386f, bi);
-    ar = fmaf(s4.x, -0.956400990486145f, ar); ai = fmaf(s4.y, -0.956400990486145f, ai); br = fmaf(d4.x, 0.29205676913261414f, br); bi = fmaf(d4.y, 0.29205676913261414f, bi);
-    ar = fmaf(s5.x, -0.9151456356048584f, ar); ai = fmaf(s5.y, -0.9151456356048584f, ai); br = fmaf(d5.x, -0.4031234383583069f, br); bi = fmaf(d5.y, -0.4031234383583069f, bi);
-    ar = fmaf(s6.x, -0.43006521463394165f, ar); ai = fmaf(s6.y, -0.43006521463394165f, ai); br = fmaf(d6.x, -0.9027978181838989f, br); bi = fmaf(d6.y, -0.9027978181838989f, bi);
-    ar = fmaf(s7.x, 0.26358717679977417f, ar); ai = fmaf(s7.y, 0.26358717679977417f, ai); br = fmaf(d7.x, -0.9646356105804443f, br); bi = fmaf(d7.y, -0.9646356105804443f, bi);
-    ar = fmaf(s8.x, 0.829405665397644f, ar); ai = fmaf(s8.y, 0.829405665397644f, ai); br = fmaf(d8.x, -0.5586467385292053f, br); bi = fmaf(d8.y, -0.5586467385292053f, bi);
-    ar = fmaf(s9.x, 0.9929810762405396f, ar); ai = fmaf(s9.y, 0.9929810762405396f, ai); br = fmaf(d9.x, 0.11827316880226135f, br); bi = fmaf(d9.y, 0.11827316880226135f, bi);
-    ar = fmaf(s10.x, 0.674983024597168f, ar); ai = fmaf(s10.y, 0.674983024597168f, ai); br = fmaf(d10.x, 0.7378332614898682f, br); bi = fmaf(d10.y, 0.7378332614898682f, bi);
-    ar = fmaf(s11.x, 0.029633328318595886f, ar); ai = fmaf(s11.y, 0.029633328318595886f, ai); br = fmaf(d11.x, 0.9995608329772949f, br); bi = fmaf(d11.y, 0.9995608329772949f, bi);
-    ar = fmaf(s12.x, -0.6300878524780273f, ar); ai = fmaf(s12.y, -0.6300878524780273f, ai); br = fmaf(d12.x, 0.7765238881111145f, br); bi = fmaf(d12.y, 0.7765238881111145f, bi);
-    ar = fmaf(s13.x, -0.9842305779457092f, ar); ai = fmaf(s13.y, -0.9842305779457092f, ai); br = fmaf(d13.x, 0.1768902689218521f, br); bi = fmaf(d13.y, 0.1768902689218521f, bi);
-    ar = fmaf(s14.x, -0.8610436320304871f, ar); ai = fmaf(s14.y, -0.8610436320304871f, ai); br = fmaf(d14.x, -0.5085310935974121f, br); bi = fmaf(d14.y, -0.5085310935974121f, bi);
-    ar = fmaf(s15.x, -0.3202698528766632f, ar); ai = fmaf(s15.y, -0.3202698528766632f, ai); br = fmaf(d15.x, -0.9473263621330261f, br); bi = fmaf(d15.y, -0.9473263621330261f, bi);
-    ar = fmaf(s16.x, 0.3758275806903839f, ar); ai = fmaf(s16.y, 0.3758275806903839f, ai); br = fmaf(d16.x, -0.926689624786377f, br); bi = fmaf(d16.y, -0.926689624786377f, bi);
-    ar = fmaf(s17.x, 0.8896570801734924f, ar); ai = fmaf(s17.y, 0.8896570801734924f, ai); br = fmaf(d17.x, -0.4566292464733124f, br); bi = fmaf(d17.y, -0.4566292464733124f, bi);
-    ar = fmaf(s18.x, 0.9720228910446167f, ar); ai = fmaf(s18.y, 0.9720228910446167f, ai); br = fmaf(d18.x, 0.2348860502243042f, br); bi = fmaf(d18.y, 0.2348860502243042f, bi);
-    ar = fmaf(s19.x, 0.5829795002937317f, ar); ai = fmaf(s19.y, 0.5829795002937317f, ai); br = fmaf(d19.x, 0.8124868869781494f, br); bi = fmaf(d19.y, 0.8124868869781494f, bi);
-    ar = fmaf(s20.x, -0.08879589289426804f, ar); ai = fmaf(s20.y, -0.08879589289426804f, ai); br = fmaf(d20.x, 0.9960498213768005f, br); bi = fmaf(d20.y, 0.9960498213768005f, bi);
-    ar = fmaf(s21.x, -0.7175072431564331f, ar); ai = fmaf(s21.y, -0.7175072431564331f, ai); br = fmaf(d21.x, 0.6965510249137878f, br); bi = fmaf(d21.y, 0.6965510249137878f, bi);
-    ar = fmaf(s22.x, -0.9982437491416931f, ar); ai = fmaf(s22.y, -0.9982437491416931f, ai); br = fmaf(d22.x, 0.05924062803387642f, br); bi = fmaf(d22.y, 0.05924062803387642f, bi);
-    ar = fmaf(s23.x, -0.794854462146759f, ar); ai = fmaf(s23.y, -0.794854462146759f, ai); br = fmaf(d23.x, -0.6068001389503479f, br); bi = fmaf(d23.y, -0.6068001389503479f, bi);
-    ar = fmaf(s24.x, -0.2059786170721054f, ar); ai = fmaf(s24.y, -0.2059786170721054f, ai); br = fmaf(d24.x, -0.9785565137863159f, br); bi = fmaf(d24.y, -0.9785565137863159f, bi);
-    ar = fmaf(s25.x, 0.4827921986579895f, ar); ai = fmaf(s25.y, 0.4827921986579895f, ai); br = fmaf(d25.x, -0.8757349252700806f, br); bi = fmaf(d25.y, -0.8757349252700806f, bi);
-    ar = fmaf(s26.x, 0.9374196529388428f, ar); ai = fmaf(s26.y, 0.9374196529388428f, ai); br = fmaf(d26.x, -0.3482016324996948f, br); bi = fmaf(d26.y, -0.3482016324996948f, bi);
-    if (!INV) {
-      v[6] = make_float2(ar + bi, ai - br); v[47] = make_float2(ar - bi, ai + br);
-    } else {
-      v[6] = make_float2(ar - bi, ai + br); v[47] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.674983024597168f, ar); ai = fmaf(s1.y, 0.674983024597168f, ai); br = fmaf(d1.x, 0.7378332614898682f, br); bi = fmaf(d1.y, 0.7378332614898682f, bi);
-    ar = fmaf(s2.x, -0.08879589289426804f, ar); ai = fmaf(s2.y, -0.08879589289426804f, ai); br = fmaf(d2.x, 0.9960498213768005f, br); bi = fmaf(d2.y, 0.9960498213768005f, bi);
-    ar = fmaf(s3.x, -0.794854462146759f, ar); ai = fmaf(s3.y, -0.794854462146759f, ai); br = fmaf(d3.x, 0.6068001389503479f, br); bi = fmaf(d3.y, 0.6068001389503479f, bi);
-    ar = fmaf(s4.x, -0.9842305779457092f, ar); ai = fmaf(s4.y, -0.9842305779457092f, ai); br = fmaf(d4.x, -0.1768902689218521f, br); bi = fmaf(d4.y, -0.1768902689218521f, bi);
-    ar = fmaf(s5.x, -0.5338233709335327f, ar); ai = fmaf(s5.y, -0.5338233709335327f, ai); br = fmaf(d5.x, -0.8455960154533386f, br); bi = fmaf(d5.y, -0.8455960154533386f, bi);
-    ar = fmaf(s6.x, 0.26358717679977417f, ar); ai = fmaf(s6.y, 0.26358717679977417f, ai); br = fmaf(d6.x, -0.9646356105804443f, br); bi = fmaf(d6.y, -0.9646356105804443f, bi);
-    ar = fmaf(s7.x, 0.8896570801734924f, ar); ai = fmaf(s7.y, 0.8896570801734924f, ai); br = fmaf(d7.x, -0.4566292464733124f, br); bi = fmaf(d7.y, -0.4566292464733124f, bi);
-    ar = fmaf(s8.x, 0.9374196529388428f, ar); ai = fmaf(s8.y, 0.9374196529388428f, ai); br = fmaf(d8.x, 0.3482016324996948f, br); bi = fmaf(d8.y, 0.3482016324996948f, bi);
-    ar = fmaf(s9.x, 0.3758275806903839f, ar); ai = fmaf(s9.y, 0.3758275806903839f, ai); br = fmaf(d9.x, 0.926689624786377f, br); bi = fmaf(d9.y, 0.926689624786377f, bi);
-    ar = fmaf(s10.x, -0.43006521463394165f, ar); ai = fmaf(s10.y, -0.43006521463394165f, ai); br = fmaf(d10.x, 0.9027978181838989f, br); bi = fmaf(d10.y, 0.9027978181838989f, bi);
-    ar = fmaf(s11.x, -0.956400990486145f, ar); ai = fmaf(s11.y, -0.956400990486145f, ai); br = fmaf(d11.x, 0.29205676913261414f, br); bi = fmaf(d11.y, 0.29205676913261414f, bi);
-    ar = fmaf(s12.x, -0.8610436320304871f, ar); ai = fmaf(s12.y, -0.8610436320304871f, ai); br = fmaf(d12.x, -0.5085310935974121f, br); bi = fmaf(d12.y, -0.5085310935974121f, bi);
-    ar = fmaf(s13.x, -0.2059786170721054f, ar); ai = fmaf(s13.y, -0.2059786170721054f, ai); br = fmaf(d13.x, -0.9785565137863159f, br); bi = fmaf(d13.y, -0.9785565137863159f, bi);
-    ar = fmaf(s14.x, 0.5829795002937317f, ar); ai = fmaf(s14.y, 0.5829795002937317f, ai); br = fmaf(d14.x, -0.8124868869781494f, br); bi = fmaf(d14.y, -0.8124868869781494f, bi);
-    ar = fmaf(s15.x, 0.9929810762405396f, ar); ai = fmaf(s15.y, 0.9929810762405396f, ai); br = fmaf(d15.x, -0.11827316880226135f, br); bi = fmaf(d15.y, -0.11827316880226135f, bi);
-    ar = fmaf(s16.x, 0.7575112581253052f, ar); ai = fmaf(s16.y, 0.7575112581253052f, ai); br = fmaf(d16.x, 0.6528221368789673f, br); bi = fmaf(d16.y, 0.6528221368789673f, bi);
-    ar = fmaf(s17.x, 0.029633328318595886f, ar); ai = fmaf(s17.y, 0.029633328318595886f, ai); br = fmaf(d17.x, 0.9995608329772949f, br); bi = fmaf(d17.y, 0.9995608329772949f, bi);
-    ar = fmaf(s18.x, -0.7175072431564331f, ar); ai = fmaf(s18.y, -0.7175072431564331f, ai); br = fmaf(d18.x, 0.6965510249137878f, br); bi = fmaf(d18.y, 0.6965510249137878f, bi);
-    ar = fmaf(s19.x, -0.9982437491416931f, ar); ai = fmaf(s19.y, -0.9982437491416931f, ai); br = fmaf(d19.x, -0.05924062803387642f, br); bi = fmaf(d19.y, -0.05924062803387642f, bi);
-    ar = fmaf(s20.x, -0.6300878524780273f, ar); ai = fmaf(s20.y, -0.6300878524780273f, ai); br = fmaf(d20.x, -0.7765238881111145f, br); bi = fmaf(d20.y, -0.7765238881111145f, bi);
-    ar = fmaf(s21.x, 0.14764656126499176f, ar); ai = fmaf(s21.y, 0.14764656126499176f, ai); br = fmaf(d21.x, -0.989040195941925f, br); bi = fmaf(d21.y, -0.989040195941925f, bi);
-    ar = fmaf(s22.x, 0.829405665397644f, ar); ai = fmaf(s22.y, 0.829405665397644f, ai); br = fmaf(d22.x, -0.5586467385292053f, br); bi = fmaf(d22.y, -0.5586467385292053f, bi);
-    ar = fmaf(s23.x, 0.9720228910446167f, ar); ai = fmaf(s23.y, 0.9720228910446167f, ai); br = fmaf(d23.x, 0.2348860502243042f, br); bi = fmaf(d23.y, 0.2348860502243042f, bi);
-    ar = fmaf(s24.x, 0.4827921986579895f, ar); ai = fmaf(s24.y, 0.4827921986579895f, ai); br = fmaf(d24.x, 0.8757349252700806f, br); bi = fmaf(d24.y, 0.8757349252700806f, bi);
-    ar = fmaf(s25.x, -0.3202698528766632f, ar); ai = fmaf(s25.y, -0.3202698528766632f, ai); br = fmaf(d25.x, 0.9473263621330261f, br); bi = fmaf(d25.y, 0.9473263621330261f, bi);
-    ar = fmaf(s26.x, -0.9151456356048584f, ar); ai = fmaf(s26.y, -0.9151456356048584f, ai); br = fmaf(d26.x, 0.4031234383583069f, br); bi = fmaf(d26.y, 0.4031234383583069f, bi);
-    if (!INV) {
-      v[7] = make_float2(ar + bi, ai - br); v[46] = make_float2(ar - bi, ai + br);
-    } else {
-      v[7] = make_float2(ar - bi, ai + br); v[46] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.5829795002937317f, ar); ai = fmaf(s1.y, 0.5829795002937317f, ai); br = fmaf(d1.x, 0.8124868869781494f, br); bi = fmaf(d1.y, 0.8124868869781494f, bi);
-    ar = fmaf(s2.x, -0.3202698528766632f, ar); ai = fmaf(s2.y, -0.3202698528766632f, ai); br = fmaf(d2.x, 0.9473263621330261f, br); bi = fmaf(d2.y, 0.9473263621330261f, bi);
-    ar = fmaf(s3.x, -0.956400990486145f, ar); ai = fmaf(s3.y, -0.956400990486145f, ai); br = fmaf(d3.x, 0.29205676913261414f, br); bi = fmaf(d3.y, 0.29205676913261414f, bi);
-    ar = fmaf(s4.x, -0.794854462146759f, ar); ai = fmaf(s4.y, -0.794854462146759f, ai); br = fmaf(d4.x, -0.6068001389503479f, br); bi = fmaf(d4.y, -0.6068001389503479f, bi);
-    ar = fmaf(s5.x, 0.029633328318595886f, ar); ai = fmaf(s5.y, 0.029633328318595886f, ai); br = fmaf(d5.x, -0.9995608329772949f, br); bi = fmaf(d5.y, -0.9995608329772949f, bi);
-    ar = fmaf(s6.x, 0.829405665397644f, ar); ai = fmaf(s6.y, 0.829405665397644f, ai); br = fmaf(d6.x, -0.5586467385292053f, br); bi = fmaf(d6.y, -0.5586467385292053f, bi);
-    ar = fmaf(s7.x, 0.9374196529388428f, ar); ai = fmaf(s7.y, 0.9374196529388428f, ai); br = fmaf(d7.x, 0.3482016324996948f, br); bi = fmaf(d7.y, 0.3482016324996948f, bi);
-    ar = fmaf(s8.x, 0.26358717679977417f, ar); ai = fmaf(s8.y, 0.26358717679977417f, ai); br = fmaf(d8.x, 0.9646356105804443f, br); bi = fmaf(d8.y, 0.9646356105804443f, bi);
-    ar = fmaf(s9.x, -0.6300878524780273f, ar); ai = fmaf(s9.y, -0.6300878524780273f, ai); br = fmaf(d9.x, 0.7765238881111145f, br); bi = fmaf(d9.y, 0.7765238881111145f, bi);
-    ar = fmaf(s10.x, -0.9982437491416931f, ar); ai = fmaf(s10.y, -0.9982437491416931f, ai); br = fmaf(d10.x, -0.05924062803387642f, br); bi = fmaf(d10.y, -0.05924062803387642f, bi);
-    ar = fmaf(s11.x, -0.5338233709335327f, ar); ai = fmaf(s11.y, -0.5338233709335327f, ai); br = fmaf(d11.x, -0.8455960154533386f, br); bi = fmaf(d11.y, -0.8455960154533386f, bi);
-    ar = fmaf(s12.x, 0.3758275806903839f, ar); ai = fmaf(s12.y, 0.3758275806903839f, ai); br = fmaf(d12.x, -0.926689624786377f, br); bi = fmaf(d12.y, -0.926689624786377f, bi);
-    ar = fmaf(s13.x, 0.9720228910446167f, ar); ai = fmaf(s13.y, 0.9720228910446167f, ai); br = fmaf(d13.x, -0.2348860502243042f, br); bi = fmaf(d13.y, -0.2348860502243042f, bi);
-    ar = fmaf(s14.x, 0.7575112581253052f, ar); ai = fmaf(s14.y, 0.7575112581253052f, ai); br = fmaf(d14.x, 0.6528221368789673f, br); bi = fmaf(d14.y, 0.6528221368789673f, bi);
-    ar = fmaf(s15.x, -0.08879589289426804f, ar); ai = fmaf(s15.y, -0.08879589289426804f, ai); br = fmaf(d15.x, 0.9960498213768005f, br); bi = fmaf(d15.y, 0.9960498213768005f, bi);
-    ar = fmaf(s16.x, -0.8610436320304871f, ar); ai = fmaf(s16.y, -0.8610436320304871f, ai); br = fmaf(d16.x, 0.5085310935974121f, br); bi = fmaf(d16.y, 0.5085310935974121f, bi);
-    ar = fmaf(s17.x, -0.9151456356048584f, ar); ai = fmaf(s17.y, -0.9151456356048584f, ai); br = fmaf(d17.x, -0.4031234383583069f, br); bi = fmaf(d17.y, -0.4031234383583069f, bi);
-    ar = fmaf(s18.x, -0.2059786170721054f, ar); ai = fmaf(s18.y, -0.2059786170721054f, ai); br = fmaf(d18.x, -0.9785565137863159f, br); bi = fmaf(d18.y, -0.9785565137863159f, bi);
-    ar = fmaf(s19.x, 0.674983024597168f, ar); ai = fmaf(s19.y, 0.674983024597168f, ai); br = fmaf(d19.x, -0.7378332614898682f, br); bi = fmaf(d19.y, -0.7378332614898682f, bi);
-    ar = fmaf(s20.x, 0.9929810762405396f, ar); ai = fmaf(s20.y, 0.9929810762405396f, ai); br = fmaf(d20.x, 0.11827316880226135f, br); bi = fmaf(d20.y, 0.11827316880226135f, bi);
-    ar = fmaf(s21.x, 0.4827921986579895f, ar); ai = fmaf(s21.y, 0.4827921986579895f, ai); br = fmaf(d21.x, 0.8757349252700806f, br); bi = fmaf(d21.y, 0.8757349252700806f, bi);
-    ar = fmaf(s22.x, -0.43006521463394165f, ar); ai = fmaf(s22.y, -0.43006521463394165f, ai); br = fmaf(d22.x, 0.9027978181838989f, br); bi = fmaf(d22.y, 0.9027978181838989f, bi);
-    ar = fmaf(s23.x, -0.9842305779457092f, ar); ai = fmaf(s23.y, -0.9842305779457092f, ai); br = fmaf(d23.x, 0.1768902689218521f, br); bi = fmaf(d23.y, 0.1768902689218521f, bi);
-    ar = fmaf(s24.x, -0.7175072431564331f, ar); ai = fmaf(s24.y, -0.7175072431564331f, ai); br = fmaf(d24.x, -0.6965510249137878f, br); bi = fmaf(d24.y, -0.6965510249137878f, bi);
-    ar = fmaf(s25.x, 0.14764656126499176f, ar); ai = fmaf(s25.y, 0.14764656126499176f, ai); br = fmaf(d25.x, -0.989040195941925f, br); bi = fmaf(d25.y, -0.989040195941925f, bi);
-    ar = fmaf(s26.x, 0.8896570801734924f, ar); ai = fmaf(s26.y, 0.8896570801734924f, ai); br = fmaf(d26.x, -0.4566292464733124f, br); bi = fmaf(d26.y, -0.4566292464733124f, bi);
-    if (!INV) {
-      v[8] = make_float2(ar + bi, ai - br); v[45] = make_float2(ar - bi, ai + br);
-    } else {
-      v[8] = make_float2(ar - bi, ai + br); v[45] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.4827921986579895f, ar); ai = fmaf(s1.y, 0.4827921986579895f, ai); br = fmaf(d1.x, 0.8757349252700806f, br); bi = fmaf(d1.y, 0.8757349252700806f, bi);
-    ar = fmaf(s2.x, -0.5338233709335327f, ar); ai = fmaf(s2.y, -0.5338233709335327f, ai); br = fmaf(d2.x, 0.8455960154533386f, br); bi = fmaf(d2.y, 0.8455960154533386f, bi);
-    ar = fmaf(s3.x, -0.9982437491416931f, ar); ai = fmaf(s3.y, -0.9982437491416931f, ai); br = fmaf(d3.x, -0.05924062803387642f, br); bi = fmaf(d3.y, -0.05924062803387642f, bi);
-    ar = fmaf(s4.x, -0.43006521463394165f, ar); ai = fmaf(s4.y, -0.43006521463394165f, ai); br = fmaf(d4.x, -0.9027978181838989f, br); bi = fmaf(d4.y, -0.9027978181838989f, bi);
-    ar = fmaf(s5.x, 0.5829795002937317f, ar); ai = fmaf(s5.y, 0.5829795002937317f, ai); br = fmaf(d5.x, -0.8124868869781494f, br); bi = fmaf(d5.y, -0.8124868869781494f, bi);
-    ar = fmaf(s6.x, 0.9929810762405396f, ar); ai = fmaf(s6.y, 0.9929810762405396f, ai); br = fmaf(d6.x, 0.11827316880226135f, br); bi = fmaf(d6.y, 0.11827316880226135f, bi);
-    ar = fmaf(s7.x, 0.3758275806903839f, ar); ai = fmaf(s7.y, 0.3758275806903839f, ai); br = fmaf(d7.x, 0.926689624786377f, br); bi = fmaf(d7.y, 0.926689624786377f, bi);
-    ar = fmaf(s8.x, -0.6300878524780273f, ar); ai = fmaf(s8.y, -0.6300878524780273f, ai); br = fmaf(d8.x, 0.7765238881111145f, br); bi = fmaf(d8.y, 0.7765238881111145f, bi);
-    ar = fmaf(s9.x, -0.9842305779457092f, ar); ai = fmaf(s9.y, -0.9842305779457092f, ai); br = fmaf(d9.x, -0.1768902689218521f, br); bi = fmaf(d9.y, -0.1768902689218521f, bi);
-    ar = fmaf(s10.x, -0.3202698528766632f, ar); ai = fmaf(s10.y, -0.3202698528766632f, ai); br = fmaf(d10.x, -0.9473263621330261f, br); bi = fmaf(d10.y, -0.9473263621330261f, bi);
-    ar = fmaf(s11.x, 0.674983024597168f, ar); ai = fmaf(s11.y, 0.674983024597168f, ai); br = fmaf(d11.x, -0.7378332614898682f, br); bi = fmaf(d11.y, -0.7378332614898682f, bi);
-    ar = fmaf(s12.x, 0.9720228910446167f, ar); ai = fmaf(s12.y, 0.9720228910446167f, ai); br = fmaf(d12.x, 0.2348860502243042f, br); bi = fmaf(d12.y, 0.2348860502243042f, bi);
-    ar = fmaf(s13.x, 0.26358717679977417f, ar); ai = fmaf(s13.y, 0.26358717679977417f, ai); br = fmaf(d13.x, 0.9646356105804443f, br); bi = fmaf(d13.y, 0.9646356105804443f, bi);
-    ar = fmaf(s14.x, -0.7175072431564331f, ar); ai = fmaf(s14.y, -0.7175072431564331f, ai); br = fmaf(d14.x, 0.6965510249137878f, br); bi = fmaf(d14.y, 0.6965510249137878f, bi);
-    ar = fmaf(s15.x, -0.956400990486145f, ar); ai = fmaf(s15.y, -0.956400990486145f, ai); br = fmaf(d15.x, -0.29205676913261414f, br); bi = fmaf(d15.y, -0.29205676913261414f, bi);
-    ar = fmaf(s16.x, -0.2059786170721054f, ar); ai = fmaf(s16.y, -0.2059786170721054f, ai); br = fmaf(d16.x, -0.9785565137863159f, br); bi = fmaf(d16.y, -0.9785565137863159f, bi);
-    ar = fmaf(s17.x, 0.7575112581253052f, ar); ai = fmaf(s17.y, 0.7575112581253052f, ai); br = fmaf(d17.x, -0.6528221368789673f, br); bi = fmaf(d17.y, -0.6528221368789673f, bi);
-    ar = fmaf(s18.x, 0.9374196529388428f, ar); ai = fmaf(s18.y, 0.9374196529388428f, ai); br = fmaf(d18.x, 0.3482016324996948f, br); bi = fmaf(d18.y, 0.3482016324996948f, bi);
-    ar = fmaf(s19.x, 0.14764656126499176f, ar); ai = fmaf(s19.y, 0.14764656126499176f, ai); br = fmaf(d19.x, 0.989040195941925f, br); bi = fmaf(d19.y, 0.989040195941925f, bi);
-    ar = fmaf(s20.x, -0.794854462146759f, ar); ai = fmaf(s20.y, -0.794854462146759f, ai); br = fmaf(d20.x, 0.6068001389503479f, br); bi = fmaf(d20.y, 0.6068001389503479f, bi);
-    ar = fmaf(s21.x, -0.9151456356048584f, ar); ai = fmaf(s21.y, -0.9151456356048584f, ai); br = fmaf(d21.x, -0.4031234383583069f, br); bi = fmaf(d21.y, -0.4031234383583069f, bi);
-    ar = fmaf(s22.x, -0.08879589289426804f, ar); ai = fmaf(s22.y, -0.08879589289426804f, ai); br = fmaf(d22.x, -0.9960498213768005f, br); bi = fmaf(d22.y, -0.9960498213768005f, bi);
-    ar = fmaf(s23.x, 0.829405665397644f, ar); ai = fmaf(s23.y, 0.829405665397644f, ai); br = fmaf(d23.x, -0.5586467385292053f, br); bi = fmaf(d23.y, -0.5586467385292053f, bi);
-    ar = fmaf(s24.x, 0.8896570801734924f, ar); ai = fmaf(s24.y, 0.8896570801734924f, ai); br = fmaf(d24.x, 0.4566292464733124f, br); bi = fmaf(d24.y, 0.4566292464733124f, bi);
-    ar = fmaf(s25.x, 0.029633328318595886f, ar); ai = fmaf(s25.y, 0.029633328318595886f, ai); br = fmaf(d25.x, 0.9995608329772949f, br); bi = fmaf(d25.y, 0.9995608329772949f, bi);
-    ar = fmaf(s26.x, -0.8610436320304871f, ar); ai = fmaf(s26.y, -0.8610436320304871f, ai); br = fmaf(d26.x, 0.5085310935974121f, br); bi = fmaf(d26.y, 0.5085310935974121f, bi);
-    if (!INV) {
-      v[9] = make_float2(ar + bi, ai - br); v[44] = make_float2(ar - bi, ai + br);
-    } else {
-      v[9] = make_float2(ar - bi, ai + br); v[44] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.3758275806903839f, ar); ai = fmaf(s1.y, 0.3758275806903839f, ai); br = fmaf(d1.x, 0.926689624786377f, br); bi = fmaf(d1.y, 0.926689624786377f, bi);
-    ar = fmaf(s2.x, -0.7175072431564331f, ar); ai = fmaf(s2.y, -0.7175072431564331f, ai); br = fmaf(d2.x, 0.6965510249137878f, br); bi = fmaf(d2.y, 0.6965510249137878f, bi);
-    ar = fmaf(s3.x, -0.9151456356048584f, ar); ai = fmaf(s3.y, -0.9151456356048584f, ai); br = fmaf(d3.x, -0.4031234383583069f, br); bi = fmaf(d3.y, -0.4031234383583069f, bi);
-    ar = fmaf(s4.x, 0.029633328318595886f, ar); ai = fmaf(s4.y, 0.029633328318595886f, ai); br = fmaf(d4.x, -0.9995608329772949f, br); bi = fmaf(d4.y, -0.9995608329772949f, bi);
-    ar = fmaf(s5.x, 0.9374196529388428f, ar); ai = fmaf(s5.y, 0.9374196529388428f, ai); br = fmaf(d5.x, -0.3482016324996948f, br); bi = fmaf(d5.y, -0.3482016324996948f, bi);
-    ar = fmaf(s6.x, 0.674983024597168f, ar); ai = fmaf(s6.y, 0.674983024597168f, ai); br = fmaf(d6.x, 0.7378332614898682f, br); bi = fmaf(d6.y, 0.7378332614898682f, bi);
-    ar = fmaf(s7.x, -0.43006521463394165f, ar); ai = fmaf(s7.y, -0.43006521463394165f, ai); br = fmaf(d7.x, 0.9027978181838989f, br); bi = fmaf(d7.y, 0.9027978181838989f, bi);
-    ar = fmaf(s8.x, -0.9982437491416931f, ar); ai = fmaf(s8.y, -0.9982437491416931f, ai); br = fmaf(d8.x, -0.05924062803387642f, br); bi = fmaf(d8.y, -0.05924062803387642f, bi);
-    ar = fmaf(s9.x, -0.3202698528766632f, ar); ai = fmaf(s9.y, -0.3202698528766632f, ai); br = fmaf(d9.x, -0.9473263621330261f, br); bi = fmaf(d9.y, -0.9473263621330261f, bi);
-    ar = fmaf(s10.x, 0.7575112581253052f, ar); ai = fmaf(s10.y, 0.7575112581253052f, ai); br = fmaf(d10.x, -0.6528221368789673f, br); bi = fmaf(d10.y, -0.6528221368789673f, bi);
-    ar = fmaf(s11.x, 0.8896570801734924f, ar); ai = fmaf(s11.y, 0.8896570801734924f, ai); br = fmaf(d11.x, 0.4566292464733124f, br); bi = fmaf(d11.y, 0.4566292464733124f, bi);
-    ar = fmaf(s12.x, -0.08879589289426804f, ar); ai = fmaf(s12.y, -0.08879589289426804f, ai); br = fmaf(d12.x, 0.9960498213768005f, br); bi = fmaf(d12.y, 0.9960498213768005f, bi);
-    ar = fmaf(s13.x, -0.956400990486145f, ar); ai = fmaf(s13.y, -0.956400990486145f, ai); br = fmaf(d13.x, 0.29205676913261414f, br); bi = fmaf(d13.y, 0.29205676913261414f, bi);
-    ar = fmaf(s14.x, -0.6300878524780273f, ar); ai = fmaf(s14.y, -0.6300878524780273f, ai); br = fmaf(d14.x, -0.7765238881111145f, br); bi = fmaf(d14.y, -0.7765238881111145f, bi);
-    ar = fmaf(s15.x, 0.4827921986579895f, ar); ai = fmaf(s15.y, 0.4827921986579895f, ai); br = fmaf(d15.x, -0.8757349252700806f, br); bi = fmaf(d15.y, -0.8757349252700806f, bi);
-    ar = fmaf(s16.x, 0.9929810762405396f, ar); ai = fmaf(s16.y, 0.9929810762405396f, ai); br = fmaf(d16.x, 0.11827316880226135f, br); bi = fmaf(d16.y, 0.11827316880226135f, bi);
-    ar = fmaf(s17.x, 0.26358717679977417f, ar); ai = fmaf(s17.y, 0.26358717679977417f, ai); br = fmaf(d17.x, 0.9646356105804443f, br); bi = fmaf(d17.y, 0.9646356105804443f, bi);
-    ar = fmaf(s18.x, -0.794854462146759f, ar); ai = fmaf(s18.y, -0.794854462146759f, ai); br = fmaf(d18.x, 0.6068001389503479f, br); bi = fmaf(d18.y, 0.6068001389503479f, bi);
-    ar = fmaf(s19.x, -0.8610436320304871f, ar); ai = fmaf(s19.y, -0.8610436320304871f, ai); br = fmaf(d19.x, -0.5085310935974121f, br); bi = fmaf(d19.y, -0.5085310935974121f, bi);
-    ar = fmaf(s20.x, 0.14764656126499176f, ar); ai = fmaf(s20.y, 0.14764656126499176f, ai); br = fmaf(d20.x, -0.989040195941925f, br); bi = fmaf(d20.y, -0.989040195941925f, bi);
-    ar = fmaf(s21.x, 0.9720228910446167f, ar); ai = fmaf(s21.y, 0.9720228910446167f, ai); br = fmaf(d21.x, -0.2348860502243042f, br); bi = fmaf(d21.y, -0.2348860502243042f, bi);
-    ar = fmaf(s22.x, 0.5829795002937317f, ar); ai = fmaf(s22.y, 0.5829795002937317f, ai); br = fmaf(d22.x, 0.8124868869781494f, br); bi = fmaf(d22.y, 0.8124868869781494f, bi);
-    ar = fmaf(s23.x, -0.5338233709335327f, ar); ai = fmaf(s23.y, -0.5338233709335327f, ai); br = fmaf(d23.x, 0.8455960154533386f, br); bi = fmaf(d23.y, 0.8455960154533386f, bi);
-    ar = fmaf(s24.x, -0.9842305779457092f, ar); ai = fmaf(s24.y, -0.9842305779457092f, ai); br = fmaf(d24.x, -0.1768902689218521f, br); bi = fmaf(d24.y, -0.1768902689218521f, bi);
-    ar = fmaf(s25.x, -0.2059786170721054f, ar); ai = fmaf(s25.y, -0.2059786170721054f, ai); br = fmaf(d25.x, -0.9785565137863159f, br); bi = fmaf(d25.y, -0.9785565137863159f, bi);
-    ar = fmaf(s26.x, 0.829405665397644f, ar); ai = fmaf(s26.y, 0.829405665397644f, ai); br = fmaf(d26.x, -0.5586467385292053f, br); bi = fmaf(d26.y, -0.5586467385292053f, bi);
-    if (!INV) {
-      v[10] = make_float2(ar + bi, ai - br); v[43] = make_float2(ar - bi, ai + br);
-    } else {
-      v[10] = make_float2(ar - bi, ai + br); v[43] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.26358717679977417f, ar); ai = fmaf(s1.y, 0.26358717679977417f, ai); br = fmaf(d1.x, 0.9646356105804443f, br); bi = fmaf(d1.y, 0.9646356105804443f, bi);
-    ar = fmaf(s2.x, -0.8610436320304871f, ar); ai = fmaf(s2.y, -0.8610436320304871f, ai); br = fmaf(d2.x, 0.5085310935974121f, br); bi = fmaf(d2.y, 0.5085310935974121f, bi);
-    ar = fmaf(s3.x, -0.7175072431564331f, ar); ai = fmaf(s3.y, -0.7175072431564331f, ai); br = fmaf(d3.x, -0.6965510249137878f, br); bi = fmaf(d3.y, -0.6965510249137878f, bi);
-    ar = fmaf(s4.x, 0.4827921986579895f, ar); ai = fmaf(s4.y, 0.4827921986579895f, ai); br = fmaf(d4.x, -0.8757349252700806f, br); bi = fmaf(d4.y, -0.8757349252700806f, bi);
-    ar = fmaf(s5.x, 0.9720228910446167f, ar); ai = fmaf(s5.y, 0.9720228910446167f, ai); br = fmaf(d5.x, 0.2348860502243042f, br); bi = fmaf(d5.y, 0.2348860502243042f, bi);
-    ar = fmaf(s6.x, 0.029633328318595886f, ar); ai = fmaf(s6.y, 0.029633328318595886f, ai); br = fmaf(d6.x, 0.9995608329772949f, br); bi = fmaf(d6.y, 0.9995608329772949f, bi);
-    ar = fmaf(s7.x, -0.956400990486145f, ar); ai = fmaf(s7.y, -0.956400990486145f, ai); br = fmaf(d7.x, 0.29205676913261414f, br); bi = fmaf(d7.y, 0.29205676913261414f, bi);
-    ar = fmaf(s8.x, -0.5338233709335327f, ar); ai = fmaf(s8.y, -0.5338233709335327f, ai); br = fmaf(d8.x, -0.8455960154533386f, br); bi = fmaf(d8.y, -0.8455960154533386f, bi);
-    ar = fmaf(s9.x, 0.674983024597168f, ar); ai = fmaf(s9.y, 0.674983024597168f, ai); br = fmaf(d9.x, -0.7378332614898682f, br); bi = fmaf(d9.y, -0.7378332614898682f, bi);
-    ar = fmaf(s10.x, 0.8896570801734924f, ar); ai = fmaf(s10.y, 0.8896570801734924f, ai); br = fmaf(d10.x, 0.4566292464733124f, br); bi = fmaf(d10.y, 0.4566292464733124f, bi);
-    ar = fmaf(s11.x, -0.2059786170721054f, ar); ai = fmaf(s11.y, -0.2059786170721054f, ai); br = fmaf(d11.x, 0.9785565137863159f, br); bi = fmaf(d11.y, 0.9785565137863159f, bi);
-    ar = fmaf(s12.x, -0.9982437491416931f, ar); ai = fmaf(s12.y, -0.9982437491416931f, ai); br = fmaf(d12.x, 0.05924062803387642f, br); bi = fmaf(d12.y, 0.05924062803387642f, bi);
-    ar = fmaf(s13.x, -0.3202698528766632f, ar); ai = fmaf(s13.y, -0.3202698528766632f, ai); br = fmaf(d13.x, -0.9473263621330261f, br); bi = fmaf(d13.y, -0.9473263621330261f, bi);
-    ar = fmaf(s14.x, 0.829405665397644f, ar); ai = fmaf(s14.y, 0.829405665397644f, ai); br = fmaf(d14.x, -0.5586467385292053f, br); bi = fmaf(d14.y, -0.5586467385292053f, bi);
-    ar = fmaf(s15.x, 0.7575112581253052f, ar); ai = fmaf(s15.y, 0.7575112581253052f, ai); br = fmaf(d15.x, 0.6528221368789673f, br); bi = fmaf(d15.y, 0.6528221368789673f, bi);
-    ar = fmaf(s16.x, -0.43006521463394165f, ar); ai = fmaf(s16.y, -0.43006521463394165f, ai); br = fmaf(d16.x, 0.9027978181838989f, br); bi = fmaf(d16.y, 0.9027978181838989f, bi);
-    ar = fmaf(s17.x, -0.9842305779457092f, ar); ai = fmaf(s17.y, -0.9842305779457092f, ai); br = fmaf(d17.x, -0.1768902689218521f, br); bi = fmaf(d17.y, -0.1768902689218521f, bi);
-    ar = fmaf(s18.x, -0.08879589289426804f, ar); ai = fmaf(s18.y, -0.08879589289426804f, ai); br = fmaf(d18.x, -0.9960498213768005f, br); bi = fmaf(d18.y, -0.9960498213768005f, bi);
-    ar = fmaf(s19.x, 0.9374196529388428f, ar); ai = fmaf(s19.y, 0.9374196529388428f, ai); br = fmaf(d19.x, -0.3482016324996948f, br); bi = fmaf(d19.y, -0.3482016324996948f, bi);
-    ar = fmaf(s20.x, 0.5829795002937317f, ar); ai = fmaf(s20.y, 0.5829795002937317f, ai); br = fmaf(d20.x, 0.8124868869781494f, br); bi = fmaf(d20.y, 0.8124868869781494f, bi);
-    ar = fmaf(s21.x, -0.6300878524780273f, ar); ai = fmaf(s21.y, -0.6300878524780273f, ai); br = fmaf(d21.x, 0.7765238881111145f, br); bi = fmaf(d21.y, 0.7765238881111145f, bi);
-    ar = fmaf(s22.x, -0.9151456356048584f, ar); ai = fmaf(s22.y, -0.9151456356048584f, ai); br = fmaf(d22.x, -0.4031234383583069f, br); bi = fmaf(d22.y, -0.4031234383583069f, bi);
-    ar = fmaf(s23.x, 0.14764656126499176f, ar); ai = fmaf(s23.y, 0.14764656126499176f, ai); br = fmaf(d23.x, -0.989040195941925f, br); bi = fmaf(d23.y, -0.989040195941925f, bi);
-    ar = fmaf(s24.x, 0.9929810762405396f, ar); ai = fmaf(s24.y, 0.9929810762405396f, ai); br = fmaf(d24.x, -0.11827316880226135f, br); bi = fmaf(d24.y, -0.11827316880226135f, bi);
-    ar = fmaf(s25.x, 0.3758275806903839f, ar); ai = fmaf(s25.y, 0.3758275806903839f, ai); br = fmaf(d25.x, 0.926689624786377f, br); bi = fmaf(d25.y, 0.926689624786377f, bi);
-    ar = fmaf(s26.x, -0.794854462146759f, ar); ai = fmaf(s26.y, -0.794854462146759f, ai); br = fmaf(d26.x, 0.6068001389503479f, br); bi = fmaf(d26.y, 0.6068001389503479f, bi);
-    if (!INV) {
-      v[11] = make_float2(ar + bi, ai - br); v[42] = make_float2(ar - bi, ai + br);
-    } else {
-      v[11] = make_float2(ar - bi, ai + br); v[42] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.14764656126499176f, ar); ai = fmaf(s1.y, 0.14764656126499176f, ai); br = fmaf(d1.x, 0.989040195941925f, br); bi = fmaf(d1.y, 0.989040195941925f, bi);
-    ar = fmaf(s2.x, -0.956400990486145f, ar); ai = fmaf(s2.y, -0.956400990486145f, ai); br = fmaf(d2.x, 0.29205676913261414f, br); bi = fmaf(d2.y, 0.29205676913261414f, bi);
-    ar = fmaf(s3.x, -0.43006521463394165f, ar); ai = fmaf(s3.y, -0.43006521463394165f, ai); br = fmaf(d3.x, -0.9027978181838989f, br); bi = fmaf(d3.y, -0.9027978181838989f, bi);
-    ar = fmaf(s4.x, 0.829405665397644f, ar); ai = fmaf(s4.y, 0.829405665397644f, ai); br = fmaf(d4.x, -0.5586467385292053f, br); bi = fmaf(d4.y, -0.5586467385292053f, bi);
-    ar = fmaf(s5.x, 0.674983024597168f, ar); ai = fmaf(s5.y, 0.674983024597168f, ai); br = fmaf(d5.x, 0.7378332614898682f, br); bi = fmaf(d5.y, 0.7378332614898682f, bi);
-    ar = fmaf(s6.x, -0.6300878524780273f, ar); ai = fmaf(s6.y, -0.6300878524780273f, ai); br = fmaf(d6.x, 0.7765238881111145f, br); bi = fmaf(d6.y, 0.7765238881111145f, bi);
-    ar = fmaf(s7.x, -0.8610436320304871f, ar); ai = fmaf(s7.y, -0.8610436320304871f, ai); br = fmaf(d7.x, -0.5085310935974121f, br); bi = fmaf(d7.y, -0.5085310935974121f, bi);
-    ar = fmaf(s8.x, 0.3758275806903839f, ar); ai = fmaf(s8.y, 0.3758275806903839f, ai); br = fmaf(d8.x, -0.926689624786377f, br); bi = fmaf(d8.y, -0.926689624786377f, bi);
-    ar = fmaf(s9.x, 0.9720228910446167f, ar); ai = fmaf(s9.y, 0.9720228910446167f, ai); br = fmaf(d9.x, 0.2348860502243042f, br); bi = fmaf(d9.y, 0.2348860502243042f, bi);
-    ar = fmaf(s10.x, -0.08879589289426804f, ar); ai = fmaf(s10.y, -0.08879589289426804f, ai); br = fmaf(d10.x, 0.9960498213768005f, br); bi = fmaf(d10.y, 0.9960498213768005f, bi);
-    ar = fmaf(s11.x, -0.9982437491416931f, ar); ai = fmaf(s11.y, -0.9982437491416931f, ai); br = fmaf(d11.x, 0.05924062803387642f, br); bi = fmaf(d11.y, 0.05924062803387642f, bi);
-    ar = fmaf(s12.x, -0.2059786170721054f, ar); ai = fmaf(s12.y, -0.2059786170721054f, ai); br = fmaf(d12.x, -0.9785565137863159f, br); bi = fmaf(d12.y, -0.9785565137863159f, bi);
-    ar = fmaf(s13.x, 0.9374196529388428f, ar); ai = fmaf(s13.y, 0.9374196529388428f, ai); br = fmaf(d13.x, -0.3482016324996948f, br); bi = fmaf(d13.y, -0.3482016324996948f, bi);
-    ar = fmaf(s14.x, 0.4827921986579895f, ar); ai = fmaf(s14.y, 0.4827921986579895f, ai); br = fmaf(d14.x, 0.8757349252700806f, br); bi = fmaf(d14.y, 0.8757349252700806f, bi);
-    ar = fmaf(s15.x, -0.794854462146759f, ar); ai = fmaf(s15.y, -0.794854462146759f, ai); br = fmaf(d15.x, 0.6068001389503479f, br); bi = fmaf(d15.y, 0.6068001389503479f, bi);
-    ar = fmaf(s16.x, -0.7175072431564331f, ar); ai = fmaf(s16.y, -0.7175072431564331f, ai); br = fmaf(d16.x, -0.6965510249137878f, br); bi = fmaf(d16.y, -0.6965510249137878f, bi);
-    ar = fmaf(s17.x, 0.5829795002937317f, ar); ai = fmaf(s17.y, 0.5829795002937317f, ai); br = fmaf(d17.x, -0.8124868869781494f, br); bi = fmaf(d17.y, -0.8124868869781494f, bi);
-    ar = fmaf(s18.x, 0.8896570801734924f, ar); ai = fmaf(s18.y, 0.8896570801734924f, ai); br = fmaf(d18.x, 0.4566292464733124f, br); bi = fmaf(d18.y, 0.4566292464733124f, bi);
-    ar = fmaf(s19.x, -0.3202698528766632f, ar); ai = fmaf(s19.y, -0.3202698528766632f, ai); br = fmaf(d19.x, 0.9473263621330261f, br); bi = fmaf(d19.y, 0.9473263621330261f, bi);
-    ar = fmaf(s20.x, -0.9842305779457092f, ar); ai = fmaf(s20.y, -0.9842305779457092f, ai); br = fmaf(d20.x, -0.1768902689218521f, br); bi = fmaf(d20.y, -0.1768902689218521f, bi);
-    ar = fmaf(s21.x, 0.029633328318595886f, ar); ai = fmaf(s21.y, 0.029633328318595886f, ai); br = fmaf(d21.x, -0.9995608329772949f, br); bi = fmaf(d21.y, -0.9995608329772949f, bi);
-    ar = fmaf(s22.x, 0.9929810762405396f, ar); ai = fmaf(s22.y, 0.9929810762405396f, ai); br = fmaf(d22.x, -0.11827316880226135f, br); bi = fmaf(d22.y, -0.11827316880226135f, bi);
-    ar = fmaf(s23.x, 0.26358717679977417f, ar); ai = fmaf(s23.y, 0.26358717679977417f, ai); br = fmaf(d23.x, 0.9646356105804443f, br); bi = fmaf(d23.y, 0.9646356105804443f, bi);
-    ar = fmaf(s24.x, -0.9151456356048584f, ar); ai = fmaf(s24.y, -0.9151456356048584f, ai); br = fmaf(d24.x, 0.4031234383583069f, br); bi = fmaf(d24.y, 0.4031234383583069f, bi);
-    ar = fmaf(s25.x, -0.5338233709335327f, ar); ai = fmaf(s25.y, -0.5338233709335327f, ai); br = fmaf(d25.x, -0.8455960154533386f, br); bi = fmaf(d25.y, -0.8455960154533386f, bi);
-    ar = fmaf(s26.x, 0.7575112581253052f, ar); ai = fmaf(s26.y, 0.7575112581253052f, ai); br = fmaf(d26.x, -0.6528221368789673f, br); bi = fmaf(d26.y, -0.6528221368789673f, bi);
-    if (!INV) {
-      v[12] = make_float2(ar + bi, ai - br); v[41] = make_float2(ar - bi, ai + br);
-    } else {
-      v[12] = make_float2(ar - bi, ai + br); v[41] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, 0.029633328318595886f, ar); ai = fmaf(s1.y, 0.029633328318595886f, ai); br = fmaf(d1.x, 0.9995608329772949f, br); bi = fmaf(d1.y, 0.9995608329772949f, bi);
-    ar = fmaf(s2.x, -0.9982437491416931f, ar); ai = fmaf(s2.y, -0.9982437491416931f, ai); br = fmaf(d2.x, 0.05924062803387642f, br); bi = fmaf(d2.y, 0.05924062803387642f, bi);
-    ar = fmaf(s3.x, -0.08879589289426804f, ar); ai = fmaf(s3.y, -0.08879589289426804f, ai); br = fmaf(d3.x, -0.9960498213768005f, br); bi = fmaf(d3.y, -0.9960498213768005f, bi);
-    ar = fmaf(s4.x, 0.9929810762405396f, ar); ai = fmaf(s4.y, 0.9929810762405396f, ai); br = fmaf(d4.x, -0.11827316880226135f, br); bi = fmaf(d4.y, -0.11827316880226135f, bi);
-    ar = fmaf(s5.x, 0.14764656126499176f, ar); ai = fmaf(s5.y, 0.14764656126499176f, ai); br = fmaf(d5.x, 0.989040195941925f, br); bi = fmaf(d5.y, 0.989040195941925f, bi);
-    ar = fmaf(s6.x, -0.9842305779457092f, ar); ai = fmaf(s6.y, -0.9842305779457092f, ai); br = fmaf(d6.x, 0.1768902689218521f, br); bi = fmaf(d6.y, 0.1768902689218521f, bi);
-    ar = fmaf(s7.x, -0.2059786170721054f, ar); ai = fmaf(s7.y, -0.2059786170721054f, ai); br = fmaf(d7.x, -0.9785565137863159f, br); bi = fmaf(d7.y, -0.9785565137863159f, bi);
-    ar = fmaf(s8.x, 0.9720228910446167f, ar); ai = fmaf(s8.y, 0.9720228910446167f, ai); br = fmaf(d8.x, -0.2348860502243042f, br); bi = fmaf(d8.y, -0.2348860502243042f, bi);
-    ar = fmaf(s9.x, 0.26358717679977417f, ar); ai = fmaf(s9.y, 0.26358717679977417f, ai); br = fmaf(d9.x, 0.9646356105804443f, br); bi = fmaf(d9.y, 0.9646356105804443f, bi);
-    ar = fmaf(s10.x, -0.956400990486145f, ar); ai = fmaf(s10.y, -0.956400990486145f, ai); br = fmaf(d10.x, 0.29205676913261414f, br); bi = fmaf(d10.y, 0.29205676913261414f, bi);
-    ar = fmaf(s11.x, -0.3202698528766632f, ar); ai = fmaf(s11.y, -0.3202698528766632f, ai); br = fmaf(d11.x, -0.9473263621330261f, br); bi = fmaf(d11.y, -0.9473263621330261f, bi);
-    ar = fmaf(s12.x, 0.9374196529388428f, ar); ai = fmaf(s12.y, 0.9374196529388428f, ai); br = fmaf(d12.x, -0.3482016324996948f, br); bi = fmaf(d12.y, -0.3482016324996948f, bi);
-    ar = fmaf(s13.x, 0.3758275806903839f, ar); ai = fmaf(s13.y, 0.3758275806903839f, ai); br = fmaf(d13.x, 0.926689624786377f, br); bi = fmaf(d13.y, 0.926689624786377f, bi);
-    ar = fmaf(s14.x, -0.9151456356048584f, ar); ai = fmaf(s14.y, -0.9151456356048584f, ai); br = fmaf(d14.x, 0.4031234383583069f, br); bi = fmaf(d14.y, 0.4031234383583069f, bi);
-    ar = fmaf(s15.x, -0.43006521463394165f, ar); ai = fmaf(s15.y, -0.43006521463394165f, ai); br = fmaf(d15.x, -0.9027978181838989f, br); bi = fmaf(d15.y, -0.9027978181838989f, bi);
-    ar = fmaf(s16.x, 0.8896570801734924f, ar); ai = fmaf(s16.y, 0.8896570801734924f, ai); br = fmaf(d16.x, -0.4566292464733124f, br); bi = fmaf(d16.y, -0.4566292464733124f, bi);
-    ar = fmaf(s17.x, 0.4827921986579895f, ar); ai = fmaf(s17.y, 0.4827921986579895f, ai); br = fmaf(d17.x, 0.8757349252700806f, br); bi = fmaf(d17.y, 0.8757349252700806f, bi);
-    ar = fmaf(s18.x, -0.8610436320304871f, ar); ai = fmaf(s18.y, -0.8610436320304871f, ai); br = fmaf(d18.x, 0.5085310935974121f, br); bi = fmaf(d18.y, 0.5085310935974121f, bi);
-    ar = fmaf(s19.x, -0.5338233709335327f, ar); ai = fmaf(s19.y, -0.5338233709335327f, ai); br = fmaf(d19.x, -0.8455960154533386f, br); bi = fmaf(d19.y, -0.8455960154533386f, bi);
-    ar = fmaf(s20.x, 0.829405665397644f, ar); ai = fmaf(s20.y, 0.829405665397644f, ai); br = fmaf(d20.x, -0.5586467385292053f, br); bi = fmaf(d20.y, -0.5586467385292053f, bi);
-    ar = fmaf(s21.x, 0.5829795002937317f, ar); ai = fmaf(s21.y, 0.5829795002937317f, ai); br = fmaf(d21.x, 0.8124868869781494f, br); bi = fmaf(d21.y, 0.8124868869781494f, bi);
-    ar = fmaf(s22.x, -0.794854462146759f, ar); ai = fmaf(s22.y, -0.794854462146759f, ai); br = fmaf(d22.x, 0.6068001389503479f, br); bi = fmaf(d22.y, 0.6068001389503479f, bi);
-    ar = fmaf(s23.x, -0.6300878524780273f, ar); ai = fmaf(s23.y, -0.6300878524780273f, ai); br = fmaf(d23.x, -0.7765238881111145f, br); bi = fmaf(d23.y, -0.7765238881111145f, bi);
-    ar = fmaf(s24.x, 0.7575112581253052f, ar); ai = fmaf(s24.y, 0.7575112581253052f, ai); br = fmaf(d24.x, -0.6528221368789673f, br); bi = fmaf(d24.y, -0.6528221368789673f, bi);
-    ar = fmaf(s25.x, 0.674983024597168f, ar); ai = fmaf(s25.y, 0.674983024597168f, ai); br = fmaf(d25.x, 0.7378332614898682f, br); bi = fmaf(d25.y, 0.7378332614898682f, bi);
-    ar = fmaf(s26.x, -0.7175072431564331f, ar); ai = fmaf(s26.y, -0.7175072431564331f, ai); br = fmaf(d26.x, 0.6965510249137878f, br); bi = fmaf(d26.y, 0.6965510249137878f, bi);
-    if (!INV) {
-      v[13] = make_float2(ar + bi, ai - br); v[40] = make_float2(ar - bi, ai + br);
-    } else {
-      v[13] = make_float2(ar - bi, ai + br); v[40] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.08879589289426804f, ar); ai = fmaf(s1.y, -0.08879589289426804f, ai); br = fmaf(d1.x, 0.9960498213768005f, br); bi = fmaf(d1.y, 0.9960498213768005f, bi);
-    ar = fmaf(s2.x, -0.9842305779457092f, ar); ai = fmaf(s2.y, -0.9842305779457092f, ai); br = fmaf(d2.x, -0.1768902689218521f, br); bi = fmaf(d2.y, -0.1768902689218521f, bi);
-    ar = fmaf(s3.x, 0.26358717679977417f, ar); ai = fmaf(s3.y, 0.26358717679977417f, ai); br = fmaf(d3.x, -0.9646356105804443f, br); bi = fmaf(d3.y, -0.9646356105804443f, bi);
-    ar = fmaf(s4.x, 0.9374196529388428f, ar); ai = fmaf(s4.y, 0.9374196529388428f, ai); br = fmaf(d4.x, 0.3482016324996948f, br); bi = fmaf(d4.y, 0.3482016324996948f, bi);
-    ar = fmaf(s5.x, -0.43006521463394165f, ar); ai = fmaf(s5.y, -0.43006521463394165f, ai); br = fmaf(d5.x, 0.9027978181838989f, br); bi = fmaf(d5.y, 0.9027978181838989f, bi);
-    ar = fmaf(s6.x, -0.8610436320304871f, ar); ai = fmaf(s6.y, -0.8610436320304871f, ai); br = fmaf(d6.x, -0.5085310935974121f, br); bi = fmaf(d6.y, -0.5085310935974121f, bi);
-    ar = fmaf(s7.x, 0.5829795002937317f, ar); ai = fmaf(s7.y, 0.5829795002937317f, ai); br = fmaf(d7.x, -0.8124868869781494f, br); bi = fmaf(d7.y, -0.8124868869781494f, bi);
-    ar = fmaf(s8.x, 0.7575112581253052f, ar); ai = fmaf(s8.y, 0.7575112581253052f, ai); br = fmaf(d8.x, 0.6528221368789673f, br); bi = fmaf(d8.y, 0.6528221368789673f, bi);
-    ar = fmaf(s9.x, -0.7175072431564331f, ar); ai = fmaf(s9.y, -0.7175072431564331f, ai); br = fmaf(d9.x, 0.6965510249137878f, br); bi = fmaf(d9.y, 0.6965510249137878f, bi);
-    ar = fmaf(s10.x, -0.6300878524780273f, ar); ai = fmaf(s10.y, -0.6300878524780273f, ai); br = fmaf(d10.x, -0.7765238881111145f, br); bi = fmaf(d10.y, -0.7765238881111145f, bi);
-    ar = fmaf(s11.x, 0.829405665397644f, ar); ai = fmaf(s11.y, 0.829405665397644f, ai); br = fmaf(d11.x, -0.5586467385292053f, br); bi = fmaf(d11.y, -0.5586467385292053f, bi);
-    ar = fmaf(s12.x, 0.4827921986579895f, ar); ai = fmaf(s12.y, 0.4827921986579895f, ai); br = fmaf(d12.x, 0.8757349252700806f, br); bi = fmaf(d12.y, 0.8757349252700806f, bi);
-    ar = fmaf(s13.x, -0.9151456356048584f, ar); ai = fmaf(s13.y, -0.9151456356048584f, ai); br = fmaf(d13.x, 0.4031234383583069f, br); bi = fmaf(d13.y, 0.4031234383583069f, bi);
-    ar = fmaf(s14.x, -0.3202698528766632f, ar); ai = fmaf(s14.y, -0.3202698528766632f, ai); br = fmaf(d14.x, -0.9473263621330261f, br); bi = fmaf(d14.y, -0.9473263621330261f, bi);
-    ar = fmaf(s15.x, 0.9720228910446167f, ar); ai = fmaf(s15.y, 0.9720228910446167f, ai); br = fmaf(d15.x, -0.2348860502243042f, br); bi = fmaf(d15.y, -0.2348860502243042f, bi);
-    ar = fmaf(s16.x, 0.14764656126499176f, ar); ai = fmaf(s16.y, 0.14764656126499176f, ai); br = fmaf(d16.x, 0.989040195941925f, br); bi = fmaf(d16.y, 0.989040195941925f, bi);
-    ar = fmaf(s17.x, -0.9982437491416931f, ar); ai = fmaf(s17.y, -0.9982437491416931f, ai); br = fmaf(d17.x, 0.05924062803387642f, br); bi = fmaf(d17.y, 0.05924062803387642f, bi);
-    ar = fmaf(s18.x, 0.029633328318595886f, ar); ai = fmaf(s18.y, 0.029633328318595886f, ai); br = fmaf(d18.x, -0.9995608329772949f, br); bi = fmaf(d18.y, -0.9995608329772949f, bi);
-    ar = fmaf(s19.x, 0.9929810762405396f, ar); ai = fmaf(s19.y, 0.9929810762405396f, ai); br = fmaf(d19.x, 0.11827316880226135f, br); bi = fmaf(d19.y, 0.11827316880226135f, bi);
-    ar = fmaf(s20.x, -0.2059786170721054f, ar); ai = fmaf(s20.y, -0.2059786170721054f, ai); br = fmaf(d20.x, 0.9785565137863159f, br); bi = fmaf(d20.y, 0.9785565137863159f, bi);
-    ar = fmaf(s21.x, -0.956400990486145f, ar); ai = fmaf(s21.y, -0.956400990486145f, ai); br = fmaf(d21.x, -0.29205676913261414f, br); bi = fmaf(d21.y, -0.29205676913261414f, bi);
-    ar = fmaf(s22.x, 0.3758275806903839f, ar); ai = fmaf(s22.y, 0.3758275806903839f, ai); br = fmaf(d22.x, -0.926689624786377f, br); bi = fmaf(d22.y, -0.926689624786377f, bi);
-    ar = fmaf(s23.x, 0.8896570801734924f, ar); ai = fmaf(s23.y, 0.8896570801734924f, ai); br = fmaf(d23.x, 0.4566292464733124f, br); bi = fmaf(d23.y, 0.4566292464733124f, bi);
-    ar = fmaf(s24.x, -0.5338233709335327f, ar); ai = fmaf(s24.y, -0.5338233709335327f, ai); br = fmaf(d24.x, 0.8455960154533386f, br); bi = fmaf(d24.y, 0.8455960154533386f, bi);
-    ar = fmaf(s25.x, -0.794854462146759f, ar); ai = fmaf(s25.y, -0.794854462146759f, ai); br = fmaf(d25.x, -0.6068001389503479f, br); bi = fmaf(d25.y, -0.6068001389503479f, bi);
-    ar = fmaf(s26.x, 0.674983024597168f, ar); ai = fmaf(s26.y, 0.674983024597168f, ai); br = fmaf(d26.x, -0.7378332614898682f, br); bi = fmaf(d26.y, -0.7378332614898682f, bi);
-    if (!INV) {
-      v[14] = make_float2(ar + bi, ai - br); v[39] = make_float2(ar - bi, ai + br);
-    } else {
-      v[14] = make_float2(ar - bi, ai + br); v[39] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.2059786170721054f, ar); ai = fmaf(s1.y, -0.2059786170721054f, ai); br = fmaf(d1.x, 0.9785565137863159f, br); bi = fmaf(d1.y, 0.9785565137863159f, bi);
-    ar = fmaf(s2.x, -0.9151456356048584f, ar); ai = fmaf(s2.y, -0.9151456356048584f, ai); br = fmaf(d2.x, -0.4031234383583069f, br); bi = fmaf(d2.y, -0.4031234383583069f, bi);
-    ar = fmaf(s3.x, 0.5829795002937317f, ar); ai = fmaf(s3.y, 0.5829795002937317f, ai); br = fmaf(d3.x, -0.8124868869781494f, br); bi = fmaf(d3.y, -0.8124868869781494f, bi);
-    ar = fmaf(s4.x, 0.674983024597168f, ar); ai = fmaf(s4.y, 0.674983024597168f, ai); br = fmaf(d4.x, 0.7378332614898682f, br); bi = fmaf(d4.y, 0.7378332614898682f, bi);
-    ar = fmaf(s5.x, -0.8610436320304871f, ar); ai = fmaf(s5.y, -0.8610436320304871f, ai); br = fmaf(d5.x, 0.5085310935974121f, br); bi = fmaf(d5.y, 0.5085310935974121f, bi);
-    ar = fmaf(s6.x, -0.3202698528766632f, ar); ai = fmaf(s6.y, -0.3202698528766632f, ai); br = fmaf(d6.x, -0.9473263621330261f, br); bi = fmaf(d6.y, -0.9473263621330261f, bi);
-    ar = fmaf(s7.x, 0.9929810762405396f, ar); ai = fmaf(s7.y, 0.9929810762405396f, ai); br = fmaf(d7.x, -0.11827316880226135f, br); bi = fmaf(d7.y, -0.11827316880226135f, bi);
-    ar = fmaf(s8.x, -0.08879589289426804f, ar); ai = fmaf(s8.y, -0.08879589289426804f, ai); br = fmaf(d8.x, 0.9960498213768005f, br); bi = fmaf(d8.y, 0.9960498213768005f, bi);
-    ar = fmaf(s9.x, -0.956400990486145f, ar); ai = fmaf(s9.y, -0.956400990486145f, ai); br = fmaf(d9.x, -0.29205676913261414f, br); bi = fmaf(d9.y, -0.29205676913261414f, bi);
-    ar = fmaf(s10.x, 0.4827921986579895f, ar); ai = fmaf(s10.y, 0.4827921986579895f, ai); br = fmaf(d10.x, -0.8757349252700806f, br); bi = fmaf(d10.y, -0.8757349252700806f, bi);
-    ar = fmaf(s11.x, 0.7575112581253052f, ar); ai = fmaf(s11.y, 0.7575112581253052f, ai); br = fmaf(d11.x, 0.6528221368789673f, br); bi = fmaf(d11.y, 0.6528221368789673f, bi);
-    ar = fmaf(s12.x, -0.794854462146759f, ar); ai = fmaf(s12.y, -0.794854462146759f, ai); br = fmaf(d12.x, 0.6068001389503479f, br); bi = fmaf(d12.y, 0.6068001389503479f, bi);
-    ar = fmaf(s13.x, -0.43006521463394165f, ar); ai = fmaf(s13.y, -0.43006521463394165f, ai); br = fmaf(d13.x, -0.9027978181838989f, br); bi = fmaf(d13.y, -0.9027978181838989f, bi);
-    ar = fmaf(s14.x, 0.9720228910446167f, ar); ai = fmaf(s14.y, 0.9720228910446167f, ai); br = fmaf(d14.x, -0.2348860502243042f, br); bi = fmaf(d14.y, -0.2348860502243042f, bi);
-    ar = fmaf(s15.x, 0.029633328318595886f, ar); ai = fmaf(s15.y, 0.029633328318595886f, ai); br = fmaf(d15.x, 0.9995608329772949f, br); bi = fmaf(d15.y, 0.9995608329772949f, bi);
-    ar = fmaf(s16.x, -0.9842305779457092f, ar); ai = fmaf(s16.y, -0.9842305779457092f, ai); br = fmaf(d16.x, -0.1768902689218521f, br); bi = fmaf(d16.y, -0.1768902689218521f, bi);
-    ar = fmaf(s17.x, 0.3758275806903839f, ar); ai = fmaf(s17.y, 0.3758275806903839f, ai); br = fmaf(d17.x, -0.926689624786377f, br); bi = fmaf(d17.y, -0.926689624786377f, bi);
-    ar = fmaf(s18.x, 0.829405665397644f, ar); ai = fmaf(s18.y, 0.829405665397644f, ai); br = fmaf(d18.x, 0.5586467385292053f, br); bi = fmaf(d18.y, 0.5586467385292053f, bi);
-    ar = fmaf(s19.x, -0.7175072431564331f, ar); ai = fmaf(s19.y, -0.7175072431564331f, ai); br = fmaf(d19.x, 0.6965510249137878f, br); bi = fmaf(d19.y, 0.6965510249137878f, bi);
-    ar = fmaf(s20.x, -0.5338233709335327f, ar); ai = fmaf(s20.y, -0.5338233709335327f, ai); br = fmaf(d20.x, -0.8455960154533386f, br); bi = fmaf(d20.y, -0.8455960154533386f, bi);
-    ar = fmaf(s21.x, 0.9374196529388428f, ar); ai = fmaf(s21.y, 0.9374196529388428f, ai); br = fmaf(d21.x, -0.3482016324996948f, br); bi = fmaf(d21.y, -0.3482016324996948f, bi);
-    ar = fmaf(s22.x, 0.14764656126499176f, ar); ai = fmaf(s22.y, 0.14764656126499176f, ai); br = fmaf(d22.x, 0.989040195941925f, br); bi = fmaf(d22.y, 0.989040195941925f, bi);
-    ar = fmaf(s23.x, -0.9982437491416931f, ar); ai = fmaf(s23.y, -0.9982437491416931f, ai); br = fmaf(d23.x, -0.05924062803387642f, br); bi = fmaf(d23.y, -0.05924062803387642f, bi);
-    ar = fmaf(s24.x, 0.26358717679977417f, ar); ai = fmaf(s24.y, 0.26358717679977417f, ai); br = fmaf(d24.x, -0.9646356105804443f, br); bi = fmaf(d24.y, -0.9646356105804443f, bi);
-    ar = fmaf(s25.x, 0.8896570801734924f, ar); ai = fmaf(s25.y, 0.8896570801734924f, ai); br = fmaf(d25.x, 0.4566292464733124f, br); bi = fmaf(d25.y, 0.4566292464733124f, bi);
-    ar = fmaf(s26.x, -0.6300878524780273f, ar); ai = fmaf(s26.y, -0.6300878524780273f, ai); br = fmaf(d26.x, 0.7765238881111145f, br); bi = fmaf(d26.y, 0.7765238881111145f, bi);
-    if (!INV) {
-      v[15] = make_float2(ar + bi, ai - br); v[38] = make_float2(ar - bi, ai + br);
-    } else {
-      v[15] = make_float2(ar - bi, ai + br); v[38] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.3202698528766632f, ar); ai = fmaf(s1.y, -0.3202698528766632f, ai); br = fmaf(d1.x, 0.9473263621330261f, br); bi = fmaf(d1.y, 0.9473263621330261f, bi);
-    ar = fmaf(s2.x, -0.794854462146759f, ar); ai = fmaf(s2.y, -0.794854462146759f, ai); br = fmaf(d2.x, -0.6068001389503479f, br); bi = fmaf(d2.y, -0.6068001389503479f, bi);
-    ar = fmaf(s3.x, 0.829405665397644f, ar); ai = fmaf(s3.y, 0.829405665397644f, ai); br = fmaf(d3.x, -0.5586467385292053f, br); bi = fmaf(d3.y, -0.5586467385292053f, bi);
-    ar = fmaf(s4.x, 0.26358717679977417f, ar); ai = fmaf(s4.y, 0.26358717679977417f, ai); br = fmaf(d4.x, 0.9646356105804443f, br); bi = fmaf(d4.y, 0.9646356105804443f, bi);
-    ar = fmaf(s5.x, -0.9982437491416931f, ar); ai = fmaf(s5.y, -0.9982437491416931f, ai); br = fmaf(d5.x, -0.05924062803387642f, br); bi = fmaf(d5.y, -0.05924062803387642f, bi);
-    ar = fmaf(s6.x, 0.3758275806903839f, ar); ai = fmaf(s6.y, 0.3758275806903839f, ai); br = fmaf(d6.x, -0.926689624786377f, br); bi = fmaf(d6.y, -0.926689624786377f, bi);
-    ar = fmaf(s7.x, 0.7575112581253052f, ar); ai = fmaf(s7.y, 0.7575112581253052f, ai); br = fmaf(d7.x, 0.6528221368789673f, br); bi = fmaf(d7.y, 0.6528221368789673f, bi);
-    ar = fmaf(s8.x, -0.8610436320304871f, ar); ai = fmaf(s8.y, -0.8610436320304871f, ai); br = fmaf(d8.x, 0.5085310935974121f, br); bi = fmaf(d8.y, 0.5085310935974121f, bi);
-    ar = fmaf(s9.x, -0.2059786170721054f, ar); ai = fmaf(s9.y, -0.2059786170721054f, ai); br = fmaf(d9.x, -0.9785565137863159f, br); bi = fmaf(d9.y, -0.9785565137863159f, bi);
-    ar = fmaf(s10.x, 0.9929810762405396f, ar); ai = fmaf(s10.y, 0.9929810762405396f, ai); br = fmaf(d10.x, 0.11827316880226135f, br); bi = fmaf(d10.y, 0.11827316880226135f, bi);
-    ar = fmaf(s11.x, -0.43006521463394165f, ar); ai = fmaf(s11.y, -0.43006521463394165f, ai); br = fmaf(d11.x, 0.9027978181838989f, br); bi = fmaf(d11.y, 0.9027978181838989f, bi);
-    ar = fmaf(s12.x, -0.7175072431564331f, ar); ai = fmaf(s12.y, -0.7175072431564331f, ai); br = fmaf(d12.x, -0.6965510249137878f, br); bi = fmaf(d12.y, -0.6965510249137878f, bi);
-    ar = fmaf(s13.x, 0.8896570801734924f, ar); ai = fmaf(s13.y, 0.8896570801734924f, ai); br = fmaf(d13.x, -0.4566292464733124f, br); bi = fmaf(d13.y, -0.4566292464733124f, bi);
-    ar = fmaf(s14.x, 0.14764656126499176f, ar); ai = fmaf(s14.y, 0.14764656126499176f, ai); br = fmaf(d14.x, 0.989040195941925f, br); bi = fmaf(d14.y, 0.989040195941925f, bi);
-    ar = fmaf(s15.x, -0.9842305779457092f, ar); ai = fmaf(s15.y, -0.9842305779457092f, ai); br = fmaf(d15.x, -0.1768902689218521f, br); bi = fmaf(d15.y, -0.1768902689218521f, bi);
-    ar = fmaf(s16.x, 0.4827921986579895f, ar); ai = fmaf(s16.y, 0.4827921986579895f, ai); br = fmaf(d16.x, -0.8757349252700806f, br); bi = fmaf(d16.y, -0.8757349252700806f, bi);
-    ar = fmaf(s17.x, 0.674983024597168f, ar); ai = fmaf(s17.y, 0.674983024597168f, ai); br = fmaf(d17.x, 0.7378332614898682f, br); bi = fmaf(d17.y, 0.7378332614898682f, bi);
-    ar = fmaf(s18.x, -0.9151456356048584f, ar); ai = fmaf(s18.y, -0.9151456356048584f, ai); br = fmaf(d18.x, 0.4031234383583069f, br); bi = fmaf(d18.y, 0.4031234383583069f, bi);
-    ar = fmaf(s19.x, -0.08879589289426804f, ar); ai = fmaf(s19.y, -0.08879589289426804f, ai); br = fmaf(d19.x, -0.9960498213768005f, br); bi = fmaf(d19.y, -0.9960498213768005f, bi);
-    ar = fmaf(s20.x, 0.9720228910446167f, ar); ai = fmaf(s20.y, 0.9720228910446167f, ai); br = fmaf(d20.x, 0.2348860502243042f, br); bi = fmaf(d20.y, 0.2348860502243042f, bi);
-    ar = fmaf(s21.x, -0.5338233709335327f, ar); ai = fmaf(s21.y, -0.5338233709335327f, ai); br = fmaf(d21.x, 0.8455960154533386f, br); bi = fmaf(d21.y, 0.8455960154533386f, bi);
-    ar = fmaf(s22.x, -0.6300878524780273f, ar); ai = fmaf(s22.y, -0.6300878524780273f, ai); br = fmaf(d22.x, -0.7765238881111145f, br); bi = fmaf(d22.y, -0.7765238881111145f, bi);
-    ar = fmaf(s23.x, 0.9374196529388428f, ar); ai = fmaf(s23.y, 0.9374196529388428f, ai); br = fmaf(d23.x, -0.3482016324996948f, br); bi = fmaf(d23.y, -0.3482016324996948f, bi);
-    ar = fmaf(s24.x, 0.029633328318595886f, ar); ai = fmaf(s24.y, 0.029633328318595886f, ai); br = fmaf(d24.x, 0.9995608329772949f, br); bi = fmaf(d24.y, 0.9995608329772949f, bi);
-    ar = fmaf(s25.x, -0.956400990486145f, ar); ai = fmaf(s25.y, -0.956400990486145f, ai); br = fmaf(d25.x, -0.29205676913261414f, br); bi = fmaf(d25.y, -0.29205676913261414f, bi);
-    ar = fmaf(s26.x, 0.5829795002937317f, ar); ai = fmaf(s26.y, 0.5829795002937317f, ai); br = fmaf(d26.x, -0.8124868869781494f, br); bi = fmaf(d26.y, -0.8124868869781494f, bi);
-    if (!INV) {
-      v[16] = make_float2(ar + bi, ai - br); v[37] = make_float2(ar - bi, ai + br);
-    } else {
-      v[16] = make_float2(ar - bi, ai + br); v[37] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.43006521463394165f, ar); ai = fmaf(s1.y, -0.43006521463394165f, ai); br = fmaf(d1.x, 0.9027978181838989f, br); bi = fmaf(d1.y, 0.9027978181838989f, bi);
-    ar = fmaf(s2.x, -0.6300878524780273f, ar); ai = fmaf(s2.y, -0.6300878524780273f, ai); br = fmaf(d2.x, -0.7765238881111145f, br); bi = fmaf(d2.y, -0.7765238881111145f, bi);
-    ar = fmaf(s3.x, 0.9720228910446167f, ar); ai = fmaf(s3.y, 0.9720228910446167f, ai); br = fmaf(d3.x, -0.2348860502243042f, br); bi = fmaf(d3.y, -0.2348860502243042f, bi);
-    ar = fmaf(s4.x, -0.2059786170721054f, ar); ai = fmaf(s4.y, -0.2059786170721054f, ai); br = fmaf(d4.x, 0.9785565137863159f, br); bi = fmaf(d4.y, 0.9785565137863159f, bi);
-    ar = fmaf(s5.x, -0.794854462146759f, ar); ai = fmaf(s5.y, -0.794854462146759f, ai); br = fmaf(d5.x, -0.6068001389503479f, br); bi = fmaf(d5.y, -0.6068001389503479f, bi);
-    ar = fmaf(s6.x, 0.8896570801734924f, ar); ai = fmaf(s6.y, 0.8896570801734924f, ai); br = fmaf(d6.x, -0.4566292464733124f, br); bi = fmaf(d6.y, -0.4566292464733124f, bi);
-    ar = fmaf(s7.x, 0.029633328318595886f, ar); ai = fmaf(s7.y, 0.029633328318595886f, ai); br = fmaf(d7.x, 0.9995608329772949f, br); bi = fmaf(d7.y, 0.9995608329772949f, bi);
-    ar = fmaf(s8.x, -0.9151456356048584f, ar); ai = fmaf(s8.y, -0.9151456356048584f, ai); br = fmaf(d8.x, -0.4031234383583069f, br); bi = fmaf(d8.y, -0.4031234383583069f, bi);
-    ar = fmaf(s9.x, 0.7575112581253052f, ar); ai = fmaf(s9.y, 0.7575112581253052f, ai); br = fmaf(d9.x, -0.6528221368789673f, br); bi = fmaf(d9.y, -0.6528221368789673f, bi);
-    ar = fmaf(s10.x, 0.26358717679977417f, ar); ai = fmaf(s10.y, 0.26358717679977417f, ai); br = fmaf(d10.x, 0.9646356105804443f, br); bi = fmaf(d10.y, 0.9646356105804443f, bi);
-    ar = fmaf(s11.x, -0.9842305779457092f, ar); ai = fmaf(s11.y, -0.9842305779457092f, ai); br = fmaf(d11.x, -0.1768902689218521f, br); bi = fmaf(d11.y, -0.1768902689218521f, bi);
-    ar = fmaf(s12.x, 0.5829795002937317f, ar); ai = fmaf(s12.y, 0.5829795002937317f, ai); br = fmaf(d12.x, -0.8124868869781494f, br); bi = fmaf(d12.y, -0.8124868869781494f, bi);
-    ar = fmaf(s13.x, 0.4827921986579895f, ar); ai = fmaf(s13.y, 0.4827921986579895f, ai); br = fmaf(d13.x, 0.8757349252700806f, br); bi = fmaf(d13.y, 0.8757349252700806f, bi);
-    ar = fmaf(s14.x, -0.9982437491416931f, ar); ai = fmaf(s14.y, -0.9982437491416931f, ai); br = fmaf(d14.x, 0.05924062803387642f, br); bi = fmaf(d14.y, 0.05924062803387642f, bi);
-    ar = fmaf(s15.x, 0.3758275806903839f, ar); ai = fmaf(s15.y, 0.3758275806903839f, ai); br = fmaf(d15.x, -0.926689624786377f, br); bi = fmaf(d15.y, -0.926689624786377f, bi);
-    ar = fmaf(s16.x, 0.674983024597168f, ar); ai = fmaf(s16.y, 0.674983024597168f, ai); br = fmaf(d16.x, 0.7378332614898682f, br); bi = fmaf(d16.y, 0.7378332614898682f, bi);
-    ar = fmaf(s17.x, -0.956400990486145f, ar); ai = fmaf(s17.y, -0.956400990486145f, ai); br = fmaf(d17.x, 0.29205676913261414f, br); bi = fmaf(d17.y, 0.29205676913261414f, bi);
-    ar = fmaf(s18.x, 0.14764656126499176f, ar); ai = fmaf(s18.y, 0.14764656126499176f, ai); br = fmaf(d18.x, -0.989040195941925f, br); bi = fmaf(d18.y, -0.989040195941925f, bi);
-    ar = fmaf(s19.x, 0.829405665397644f, ar); ai = fmaf(s19.y, 0.829405665397644f, ai); br = fmaf(d19.x, 0.5586467385292053f, br); bi = fmaf(d19.y, 0.5586467385292053f, bi);
-    ar = fmaf(s20.x, -0.8610436320304871f, ar); ai = fmaf(s20.y, -0.8610436320304871f, ai); br = fmaf(d20.x, 0.5085310935974121f, br); bi = fmaf(d20.y, 0.5085310935974121f, bi);
-    ar = fmaf(s21.x, -0.08879589289426804f, ar); ai = fmaf(s21.y, -0.08879589289426804f, ai); br = fmaf(d21.x, -0.9960498213768005f, br); bi = fmaf(d21.y, -0.9960498213768005f, bi);
-    ar = fmaf(s22.x, 0.9374196529388428f, ar); ai = fmaf(s22.y, 0.9374196529388428f, ai); br = fmaf(d22.x, 0.3482016324996948f, br); bi = fmaf(d22.y, 0.3482016324996948f, bi);
-    ar = fmaf(s23.x, -0.7175072431564331f, ar); ai = fmaf(s23.y, -0.7175072431564331f, ai); br = fmaf(d23.x, 0.6965510249137878f, br); bi = fmaf(d23.y, 0.6965510249137878f, bi);
-    ar = fmaf(s24.x, -0.3202698528766632f, ar); ai = fmaf(s24.y, -0.3202698528766632f, ai); br = fmaf(d24.x, -0.9473263621330261f, br); bi = fmaf(d24.y, -0.9473263621330261f, bi);
-    ar = fmaf(s25.x, 0.9929810762405396f, ar); ai = fmaf(s25.y, 0.9929810762405396f, ai); br = fmaf(d25.x, 0.11827316880226135f, br); bi = fmaf(d25.y, 0.11827316880226135f, bi);
-    ar = fmaf(s26.x, -0.5338233709335327f, ar); ai = fmaf(s26.y, -0.5338233709335327f, ai); br = fmaf(d26.x, 0.8455960154533386f, br); bi = fmaf(d26.y, 0.8455960154533386f, bi);
-    if (!INV) {
-      v[17] = make_float2(ar + bi, ai - br); v[36] = make_float2(ar - bi, ai + br);
-    } else {
-      v[17] = make_float2(ar - bi, ai + br); v[36] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.5338233709335327f, ar); ai = fmaf(s1.y, -0.5338233709335327f, ai); br = fmaf(d1.x, 0.8455960154533386f, br); bi = fmaf(d1.y, 0.8455960154533386f, bi);
-    ar = fmaf(s2.x, -0.43006521463394165f, ar); ai = fmaf(s2.y, -0.43006521463394165f, ai); br = fmaf(d2.x, -0.9027978181838989f, br); bi = fmaf(d2.y, -0.9027978181838989f, bi);
-    ar = fmaf(s3.x, 0.9929810762405396f, ar); ai = fmaf(s3.y, 0.9929810762405396f, ai); br = fmaf(d3.x, 0.11827316880226135f, br); bi = fmaf(d3.y, 0.11827316880226135f, bi);
-    ar = fmaf(s4.x, -0.6300878524780273f, ar); ai = fmaf(s4.y, -0.6300878524780273f, ai); br = fmaf(d4.x, 0.7765238881111145f, br); bi = fmaf(d4.y, 0.7765238881111145f, bi);
-    ar = fmaf(s5.x, -0.3202698528766632f, ar); ai = fmaf(s5.y, -0.3202698528766632f, ai); br = fmaf(d5.x, -0.9473263621330261f, br); bi = fmaf(d5.y, -0.9473263621330261f, bi);
-    ar = fmaf(s6.x, 0.9720228910446167f, ar); ai = fmaf(s6.y, 0.9720228910446167f, ai); br = fmaf(d6.x, 0.2348860502243042f, br); bi = fmaf(d6.y, 0.2348860502243042f, bi);
-    ar = fmaf(s7.x, -0.7175072431564331f, ar); ai = fmaf(s7.y, -0.7175072431564331f, ai); br = fmaf(d7.x, 0.6965510249137878f, br); bi = fmaf(d7.y, 0.6965510249137878f, bi);
-    ar = fmaf(s8.x, -0.2059786170721054f, ar); ai = fmaf(s8.y, -0.2059786170721054f, ai); br = fmaf(d8.x, -0.9785565137863159f, br); bi = fmaf(d8.y, -0.9785565137863159f, bi);
-    ar = fmaf(s9.x, 0.9374196529388428f, ar); ai = fmaf(s9.y, 0.9374196529388428f, ai); br = fmaf(d9.x, 0.3482016324996948f, br); bi = fmaf(d9.y, 0.3482016324996948f, bi);
-    ar = fmaf(s10.x, -0.794854462146759f, ar); ai = fmaf(s10.y, -0.794854462146759f, ai); br = fmaf(d10.x, 0.6068001389503479f, br); bi = fmaf(d10.y, 0.6068001389503479f, bi);
-    ar = fmaf(s11.x, -0.08879589289426804f, ar); ai = fmaf(s11.y, -0.08879589289426804f, ai); br = fmaf(d11.x, -0.9960498213768005f, br); bi = fmaf(d11.y, -0.9960498213768005f, bi);
-    ar = fmaf(s12.x, 0.8896570801734924f, ar); ai = fmaf(s12.y, 0.8896570801734924f, ai); br = fmaf(d12.x, 0.4566292464733124f, br); bi = fmaf(d12.y, 0.4566292464733124f, bi);
-    ar = fmaf(s13.x, -0.8610436320304871f, ar); ai = fmaf(s13.y, -0.8610436320304871f, ai); br = fmaf(d13.x, 0.5085310935974121f, br); bi = fmaf(d13.y, 0.5085310935974121f, bi);
-    ar = fmaf(s14.x, 0.029633328318595886f, ar); ai = fmaf(s14.y, 0.029633328318595886f, ai); br = fmaf(d14.x, -0.9995608329772949f, br); bi = fmaf(d14.y, -0.9995608329772949f, bi);
-    ar = fmaf(s15.x, 0.829405665397644f, ar); ai = fmaf(s15.y, 0.829405665397644f, ai); br = fmaf(d15.x, 0.5586467385292053f, br); bi = fmaf(d15.y, 0.5586467385292053f, bi);
-    ar = fmaf(s16.x, -0.9151456356048584f, ar); ai = fmaf(s16.y, -0.9151456356048584f, ai); br = fmaf(d16.x, 0.4031234383583069f, br); bi = fmaf(d16.y, 0.4031234383583069f, bi);
-    ar = fmaf(s17.x, 0.14764656126499176f, ar); ai = fmaf(s17.y, 0.14764656126499176f, ai); br = fmaf(d17.x, -0.989040195941925f, br); bi = fmaf(d17.y, -0.989040195941925f, bi);
-    ar = fmaf(s18.x, 0.7575112581253052f, ar); ai = fmaf(s18.y, 0.7575112581253052f, ai); br = fmaf(d18.x, 0.6528221368789673f, br); bi = fmaf(d18.y, 0.6528221368789673f, bi);
-    ar = fmaf(s19.x, -0.956400990486145f, ar); ai = fmaf(s19.y, -0.956400990486145f, ai); br = fmaf(d19.x, 0.29205676913261414f, br); bi = fmaf(d19.y, 0.29205676913261414f, bi);
-    ar = fmaf(s20.x, 0.26358717679977417f, ar); ai = fmaf(s20.y, 0.26358717679977417f, ai); br = fmaf(d20.x, -0.9646356105804443f, br); bi = fmaf(d20.y, -0.9646356105804443f, bi);
-    ar = fmaf(s21.x, 0.674983024597168f, ar); ai = fmaf(s21.y, 0.674983024597168f, ai); br = fmaf(d21.x, 0.7378332614898682f, br); bi = fmaf(d21.y, 0.7378332614898682f, bi);
-    ar = fmaf(s22.x, -0.9842305779457092f, ar); ai = fmaf(s22.y, -0.9842305779457092f, ai); br = fmaf(d22.x, 0.1768902689218521f, br); bi = fmaf(d22.y, 0.1768902689218521f, bi);
-    ar = fmaf(s23.x, 0.3758275806903839f, ar); ai = fmaf(s23.y, 0.3758275806903839f, ai); br = fmaf(d23.x, -0.926689624786377f, br); bi = fmaf(d23.y, -0.926689624786377f, bi);
-    ar = fmaf(s24.x, 0.5829795002937317f, ar); ai = fmaf(s24.y, 0.5829795002937317f, ai); br = fmaf(d24.x, 0.8124868869781494f, br); bi = fmaf(d24.y, 0.8124868869781494f, bi);
-    ar = fmaf(s25.x, -0.9982437491416931f, ar); ai = fmaf(s25.y, -0.9982437491416931f, ai); br = fmaf(d25.x, 0.05924062803387642f, br); bi = fmaf(d25.y, 0.05924062803387642f, bi);
-    ar = fmaf(s26.x, 0.4827921986579895f, ar); ai = fmaf(s26.y, 0.4827921986579895f, ai); br = fmaf(d26.x, -0.8757349252700806f, br); bi = fmaf(d26.y, -0.8757349252700806f, bi);
-    if (!INV) {
-      v[18] = make_float2(ar + bi, ai - br); v[35] = make_float2(ar - bi, ai + br);
-    } else {
-      v[18] = make_float2(ar - bi, ai + br); v[35] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.6300878524780273f, ar); ai = fmaf(s1.y, -0.6300878524780273f, ai); br = fmaf(d1.x, 0.7765238881111145f, br); bi = fmaf(d1.y, 0.7765238881111145f, bi);
-    ar = fmaf(s2.x, -0.2059786170721054f, ar); ai = fmaf(s2.y, -0.2059786170721054f, ai); br = fmaf(d2.x, -0.9785565137863159f, br); bi = fmaf(d2.y, -0.9785565137863159f, bi);
-    ar = fmaf(s3.x, 0.8896570801734924f, ar); ai = fmaf(s3.y, 0.8896570801734924f, ai); br = fmaf(d3.x, 0.4566292464733124f, br); bi = fmaf(d3.y, 0.4566292464733124f, bi);
-    ar = fmaf(s4.x, -0.9151456356048584f, ar); ai = fmaf(s4.y, -0.9151456356048584f, ai); br = fmaf(d4.x, 0.4031234383583069f, br); bi = fmaf(d4.y, 0.4031234383583069f, bi);
-    ar = fmaf(s5.x, 0.26358717679977417f, ar); ai = fmaf(s5.y, 0.26358717679977417f, ai); br = fmaf(d5.x, -0.9646356105804443f, br); bi = fmaf(d5.y, -0.9646356105804443f, bi);
-    ar = fmaf(s6.x, 0.5829795002937317f, ar); ai = fmaf(s6.y, 0.5829795002937317f, ai); br = fmaf(d6.x, 0.8124868869781494f, br); bi = fmaf(d6.y, 0.8124868869781494f, bi);
-    ar = fmaf(s7.x, -0.9982437491416931f, ar); ai = fmaf(s7.y, -0.9982437491416931f, ai); br = fmaf(d7.x, -0.05924062803387642f, br); bi = fmaf(d7.y, -0.05924062803387642f, bi);
-    ar = fmaf(s8.x, 0.674983024597168f, ar); ai = fmaf(s8.y, 0.674983024597168f, ai); br = fmaf(d8.x, -0.7378332614898682f, br); bi = fmaf(d8.y, -0.7378332614898682f, bi);
-    ar = fmaf(s9.x, 0.14764656126499176f, ar); ai = fmaf(s9.y, 0.14764656126499176f, ai); br = fmaf(d9.x, 0.989040195941925f, br); bi = fmaf(d9.y, 0.989040195941925f, bi);
-    ar = fmaf(s10.x, -0.8610436320304871f, ar); ai = fmaf(s10.y, -0.8610436320304871f, ai); br = fmaf(d10.x, -0.5085310935974121f, br); bi = fmaf(d10.y, -0.5085310935974121f, bi);
-    ar = fmaf(s11.x, 0.9374196529388428f, ar); ai = fmaf(s11.y, 0.9374196529388428f, ai); br = fmaf(d11.x, -0.3482016324996948f, br); bi = fmaf(d11.y, -0.3482016324996948f, bi);
-    ar = fmaf(s12.x, -0.3202698528766632f, ar); ai = fmaf(s12.y, -0.3202698528766632f, ai); br = fmaf(d12.x, 0.9473263621330261f, br); bi = fmaf(d12.y, 0.9473263621330261f, bi);
-    ar = fmaf(s13.x, -0.5338233709335327f, ar); ai = fmaf(s13.y, -0.5338233709335327f, ai); br = fmaf(d13.x, -0.8455960154533386f, br); bi = fmaf(d13.y, -0.8455960154533386f, bi);
-    ar = fmaf(s14.x, 0.9929810762405396f, ar); ai = fmaf(s14.y, 0.9929810762405396f, ai); br = fmaf(d14.x, 0.11827316880226135f, br); bi = fmaf(d14.y, 0.11827316880226135f, bi);
-    ar = fmaf(s15.x, -0.7175072431564331f, ar); ai = fmaf(s15.y, -0.7175072431564331f, ai); br = fmaf(d15.x, 0.6965510249137878f, br); bi = fmaf(d15.y, 0.6965510249137878f, bi);
-    ar = fmaf(s16.x, -0.08879589289426804f, ar); ai = fmaf(s16.y, -0.08879589289426804f, ai); br = fmaf(d16.x, -0.9960498213768005f, br); bi = fmaf(d16.y, -0.9960498213768005f, bi);
-    ar = fmaf(s17.x, 0.829405665397644f, ar); ai = fmaf(s17.y, 0.829405665397644f, ai); br = fmaf(d17.x, 0.5586467385292053f, br); bi = fmaf(d17.y, 0.5586467385292053f, bi);
-    ar = fmaf(s18.x, -0.956400990486145f, ar); ai = fmaf(s18.y, -0.956400990486145f, ai); br = fmaf(d18.x, 0.29205676913261414f, br); bi = fmaf(d18.y, 0.29205676913261414f, bi);
-    ar = fmaf(s19.x, 0.3758275806903839f, ar); ai = fmaf(s19.y, 0.3758275806903839f, ai); br = fmaf(d19.x, -0.926689624786377f, br); bi = fmaf(d19.y, -0.926689624786377f, bi);
-    ar = fmaf(s20.x, 0.4827921986579895f, ar); ai = fmaf(s20.y, 0.4827921986579895f, ai); br = fmaf(d20.x, 0.8757349252700806f, br); bi = fmaf(d20.y, 0.8757349252700806f, bi);
-    ar = fmaf(s21.x, -0.9842305779457092f, ar); ai = fmaf(s21.y, -0.9842305779457092f, ai); br = fmaf(d21.x, -0.1768902689218521f, br); bi = fmaf(d21.y, -0.1768902689218521f, bi);
-    ar = fmaf(s22.x, 0.7575112581253052f, ar); ai = fmaf(s22.y, 0.7575112581253052f, ai); br = fmaf(d22.x, -0.6528221368789673f, br); bi = fmaf(d22.y, -0.6528221368789673f, bi);
-    ar = fmaf(s23.x, 0.029633328318595886f, ar); ai = fmaf(s23.y, 0.029633328318595886f, ai); br = fmaf(d23.x, 0.9995608329772949f, br); bi = fmaf(d23.y, 0.9995608329772949f, bi);
-    ar = fmaf(s24.x, -0.794854462146759f, ar); ai = fmaf(s24.y, -0.794854462146759f, ai); br = fmaf(d24.x, -0.6068001389503479f, br); bi = fmaf(d24.y, -0.6068001389503479f, bi);
-    ar = fmaf(s25.x, 0.9720228910446167f, ar); ai = fmaf(s25.y, 0.9720228910446167f, ai); br = fmaf(d25.x, -0.2348860502243042f, br); bi = fmaf(d25.y, -0.2348860502243042f, bi);
-    ar = fmaf(s26.x, -0.43006521463394165f, ar); ai = fmaf(s26.y, -0.43006521463394165f, ai); br = fmaf(d26.x, 0.9027978181838989f, br); bi = fmaf(d26.y, 0.9027978181838989f, bi);
-    if (!INV) {
-      v[19] = make_float2(ar + bi, ai - br); v[34] = make_float2(ar - bi, ai + br);
-    } else {
-      v[19] = make_float2(ar - bi, ai + br); v[34] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.7175072431564331f, ar); ai = fmaf(s1.y, -0.7175072431564331f, ai); br = fmaf(d1.x, 0.6965510249137878f, br); bi = fmaf(d1.y, 0.6965510249137878f, bi);
-    ar = fmaf(s2.x, 0.029633328318595886f, ar); ai = fmaf(s2.y, 0.029633328318595886f, ai); br = fmaf(d2.x, -0.9995608329772949f, br); bi = fmaf(d2.y, -0.9995608329772949f, bi);
-    ar = fmaf(s3.x, 0.674983024597168f, ar); ai = fmaf(s3.y, 0.674983024597168f, ai); br = fmaf(d3.x, 0.7378332614898682f, br); bi = fmaf(d3.y, 0.7378332614898682f, bi);
-    ar = fmaf(s4.x, -0.9982437491416931f, ar); ai = fmaf(s4.y, -0.9982437491416931f, ai); br = fmaf(d4.x, -0.05924062803387642f, br); bi = fmaf(d4.y, -0.05924062803387642f, bi);
-    ar = fmaf(s5.x, 0.7575112581253052f, ar); ai = fmaf(s5.y, 0.7575112581253052f, ai); br = fmaf(d5.x, -0.6528221368789673f, br); bi = fmaf(d5.y, -0.6528221368789673f, bi);
-    ar = fmaf(s6.x, -0.08879589289426804f, ar); ai = fmaf(s6.y, -0.08879589289426804f, ai); br = fmaf(d6.x, 0.9960498213768005f, br); bi = fmaf(d6.y, 0.9960498213768005f, bi);
-    ar = fmaf(s7.x, -0.6300878524780273f, ar); ai = fmaf(s7.y, -0.6300878524780273f, ai); br = fmaf(d7.x, -0.7765238881111145f, br); bi = fmaf(d7.y, -0.7765238881111145f, bi);
-    ar = fmaf(s8.x, 0.9929810762405396f, ar); ai = fmaf(s8.y, 0.9929810762405396f, ai); br = fmaf(d8.x, 0.11827316880226135f, br); bi = fmaf(d8.y, 0.11827316880226135f, bi);
-    ar = fmaf(s9.x, -0.794854462146759f, ar); ai = fmaf(s9.y, -0.794854462146759f, ai); br = fmaf(d9.x, 0.6068001389503479f, br); bi = fmaf(d9.y, 0.6068001389503479f, bi);
-    ar = fmaf(s10.x, 0.14764656126499176f, ar); ai = fmaf(s10.y, 0.14764656126499176f, ai); br = fmaf(d10.x, -0.989040195941925f, br); bi = fmaf(d10.y, -0.989040195941925f, bi);
-    ar = fmaf(s11.x, 0.5829795002937317f, ar); ai = fmaf(s11.y, 0.5829795002937317f, ai); br = fmaf(d11.x, 0.8124868869781494f, br); bi = fmaf(d11.y, 0.8124868869781494f, bi);
-    ar = fmaf(s12.x, -0.9842305779457092f, ar); ai = fmaf(s12.y, -0.9842305779457092f, ai); br = fmaf(d12.x, -0.1768902689218521f, br); bi = fmaf(d12.y, -0.1768902689218521f, bi);
-    ar = fmaf(s13.x, 0.829405665397644f, ar); ai = fmaf(s13.y, 0.829405665397644f, ai); br = fmaf(d13.x, -0.5586467385292053f, br); bi = fmaf(d13.y, -0.5586467385292053f, bi);
-    ar = fmaf(s14.x, -0.2059786170721054f, ar); ai = fmaf(s14.y, -0.2059786170721054f, ai); br = fmaf(d14.x, 0.9785565137863159f, br); bi = fmaf(d14.y, 0.9785565137863159f, bi);
-    ar = fmaf(s15.x, -0.5338233709335327f, ar); ai = fmaf(s15.y, -0.5338233709335327f, ai); br = fmaf(d15.x, -0.8455960154533386f, br); bi = fmaf(d15.y, -0.8455960154533386f, bi);
-    ar = fmaf(s16.x, 0.9720228910446167f, ar); ai = fmaf(s16.y, 0.9720228910446167f, ai); br = fmaf(d16.x, 0.2348860502243042f, br); bi = fmaf(d16.y, 0.2348860502243042f, bi);
-    ar = fmaf(s17.x, -0.8610436320304871f, ar); ai = fmaf(s17.y, -0.8610436320304871f, ai); br = fmaf(d17.x, 0.5085310935974121f, br); bi = fmaf(d17.y, 0.5085310935974121f, bi);
-    ar = fmaf(s18.x, 0.26358717679977417f, ar); ai = fmaf(s18.y, 0.26358717679977417f, ai); br = fmaf(d18.x, -0.9646356105804443f, br); bi = fmaf(d18.y, -0.9646356105804443f, bi);
-    ar = fmaf(s19.x, 0.4827921986579895f, ar); ai = fmaf(s19.y, 0.4827921986579895f, ai); br = fmaf(d19.x, 0.8757349252700806f, br); bi = fmaf(d19.y, 0.8757349252700806f, bi);
-    ar = fmaf(s20.x, -0.956400990486145f, ar); ai = fmaf(s20.y, -0.956400990486145f, ai); br = fmaf(d20.x, -0.29205676913261414f, br); bi = fmaf(d20.y, -0.29205676913261414f, bi);
-    ar = fmaf(s21.x, 0.8896570801734924f, ar); ai = fmaf(s21.y, 0.8896570801734924f, ai); br = fmaf(d21.x, -0.4566292464733124f, br); bi = fmaf(d21.y, -0.4566292464733124f, bi);
-    ar = fmaf(s22.x, -0.3202698528766632f, ar); ai = fmaf(s22.y, -0.3202698528766632f, ai); br = fmaf(d22.x, 0.9473263621330261f, br); bi = fmaf(d22.y, 0.9473263621330261f, bi);
-    ar = fmaf(s23.x, -0.43006521463394165f, ar); ai = fmaf(s23.y, -0.43006521463394165f, ai); br = fmaf(d23.x, -0.9027978181838989f, br); bi = fmaf(d23.y, -0.9027978181838989f, bi);
-    ar = fmaf(s24.x, 0.9374196529388428f, ar); ai = fmaf(s24.y, 0.9374196529388428f, ai); br = fmaf(d24.x, 0.3482016324996948f, br); bi = fmaf(d24.y, 0.3482016324996948f, bi);
-    ar = fmaf(s25.x, -0.9151456356048584f, ar); ai = fmaf(s25.y, -0.9151456356048584f, ai); br = fmaf(d25.x, 0.4031234383583069f, br); bi = fmaf(d25.y, 0.4031234383583069f, bi);
-    ar = fmaf(s26.x, 0.3758275806903839f, ar); ai = fmaf(s26.y, 0.3758275806903839f, ai); br = fmaf(d26.x, -0.926689624786377f, br); bi = fmaf(d26.y, -0.926689624786377f, bi);
-    if (!INV) {
-      v[20] = make_float2(ar + bi, ai - br); v[33] = make_float2(ar - bi, ai + br);
-    } else {
-      v[20] = make_float2(ar - bi, ai + br); v[33] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.794854462146759f, ar); ai = fmaf(s1.y, -0.794854462146759f, ai); br = fmaf(d1.x, 0.6068001389503479f, br); bi = fmaf(d1.y, 0.6068001389503479f, bi);
-    ar = fmaf(s2.x, 0.26358717679977417f, ar); ai = fmaf(s2.y, 0.26358717679977417f, ai); br = fmaf(d2.x, -0.9646356105804443f, br); bi = fmaf(d2.y, -0.9646356105804443f, bi);
-    ar = fmaf(s3.x, 0.3758275806903839f, ar); ai = fmaf(s3.y, 0.3758275806903839f, ai); br = fmaf(d3.x, 0.926689624786377f, br); bi = fmaf(d3.y, 0.926689624786377f, bi);
-    ar = fmaf(s4.x, -0.8610436320304871f, ar); ai = fmaf(s4.y, -0.8610436320304871f, ai); br = fmaf(d4.x, -0.5085310935974121f, br); bi = fmaf(d4.y, -0.5085310935974121f, bi);
-    ar = fmaf(s5.x, 0.9929810762405396f, ar); ai = fmaf(s5.y, 0.9929810762405396f, ai); br = fmaf(d5.x, -0.11827316880226135f, br); bi = fmaf(d5.y, -0.11827316880226135f, bi);
-    ar = fmaf(s6.x, -0.7175072431564331f, ar); ai = fmaf(s6.y, -0.7175072431564331f, ai); br = fmaf(d6.x, 0.6965510249137878f, br); bi = fmaf(d6.y, 0.6965510249137878f, bi);
-    ar = fmaf(s7.x, 0.14764656126499176f, ar); ai = fmaf(s7.y, 0.14764656126499176f, ai); br = fmaf(d7.x, -0.989040195941925f, br); bi = fmaf(d7.y, -0.989040195941925f, bi);
-    ar = fmaf(s8.x, 0.4827921986579895f, ar); ai = fmaf(s8.y, 0.4827921986579895f, ai); br = fmaf(d8.x, 0.8757349252700806f, br); bi = fmaf(d8.y, 0.8757349252700806f, bi);
-    ar = fmaf(s9.x, -0.9151456356048584f, ar); ai = fmaf(s9.y, -0.9151456356048584f, ai); br = fmaf(d9.x, -0.4031234383583069f, br); bi = fmaf(d9.y, -0.4031234383583069f, bi);
-    ar = fmaf(s10.x, 0.9720228910446167f, ar); ai = fmaf(s10.y, 0.9720228910446167f, ai); br = fmaf(d10.x, -0.2348860502243042f, br); bi = fmaf(d10.y, -0.2348860502243042f, bi);
-    ar = fmaf(s11.x, -0.6300878524780273f, ar); ai = fmaf(s11.y, -0.6300878524780273f, ai); br = fmaf(d11.x, 0.7765238881111145f, br); bi = fmaf(d11.y, 0.7765238881111145f, bi);
-    ar = fmaf(s12.x, 0.029633328318595886f, ar); ai = fmaf(s12.y, 0.029633328318595886f, ai); br = fmaf(d12.x, -0.9995608329772949f, br); bi = fmaf(d12.y, -0.9995608329772949f, bi);
-    ar = fmaf(s13.x, 0.5829795002937317f, ar); ai = fmaf(s13.y, 0.5829795002937317f, ai); br = fmaf(d13.x, 0.8124868869781494f, br); bi = fmaf(d13.y, 0.8124868869781494f, bi);
-    ar = fmaf(s14.x, -0.956400990486145f, ar); ai = fmaf(s14.y, -0.956400990486145f, ai); br = fmaf(d14.x, -0.29205676913261414f, br); bi = fmaf(d14.y, -0.29205676913261414f, bi);
-    ar = fmaf(s15.x, 0.9374196529388428f, ar); ai = fmaf(s15.y, 0.9374196529388428f, ai); br = fmaf(d15.x, -0.3482016324996948f, br); bi = fmaf(d15.y, -0.3482016324996948f, bi);
-    ar = fmaf(s16.x, -0.5338233709335327f, ar); ai = fmaf(s16.y, -0.5338233709335327f, ai); br = fmaf(d16.x, 0.8455960154533386f, br); bi = fmaf(d16.y, 0.8455960154533386f, bi);
-    ar = fmaf(s17.x, -0.08879589289426804f, ar); ai = fmaf(s17.y, -0.08879589289426804f, ai); br = fmaf(d17.x, -0.9960498213768005f, br); bi = fmaf(d17.y, -0.9960498213768005f, bi);
-    ar = fmaf(s18.x, 0.674983024597168f, ar); ai = fmaf(s18.y, 0.674983024597168f, ai); br = fmaf(d18.x, 0.7378332614898682f, br); bi = fmaf(d18.y, 0.7378332614898682f, bi);
-    ar = fmaf(s19.x, -0.9842305779457092f, ar); ai = fmaf(s19.y, -0.9842305779457092f, ai); br = fmaf(d19.x, -0.1768902689218521f, br); bi = fmaf(d19.y, -0.1768902689218521f, bi);
-    ar = fmaf(s20.x, 0.8896570801734924f, ar); ai = fmaf(s20.y, 0.8896570801734924f, ai); br = fmaf(d20.x, -0.4566292464733124f, br); bi = fmaf(d20.y, -0.4566292464733124f, bi);
-    ar = fmaf(s21.x, -0.43006521463394165f, ar); ai = fmaf(s21.y, -0.43006521463394165f, ai); br = fmaf(d21.x, 0.9027978181838989f, br); bi = fmaf(d21.y, 0.9027978181838989f, bi);
-    ar = fmaf(s22.x, -0.2059786170721054f, ar); ai = fmaf(s22.y, -0.2059786170721054f, ai); br = fmaf(d22.x, -0.9785565137863159f, br); bi = fmaf(d22.y, -0.9785565137863159f, bi);
-    ar = fmaf(s23.x, 0.7575112581253052f, ar); ai = fmaf(s23.y, 0.7575112581253052f, ai); br = fmaf(d23.x, 0.6528221368789673f, br); bi = fmaf(d23.y, 0.6528221368789673f, bi);
-    ar = fmaf(s24.x, -0.9982437491416931f, ar); ai = fmaf(s24.y, -0.9982437491416931f, ai); br = fmaf(d24.x, -0.05924062803387642f, br); bi = fmaf(d24.y, -0.05924062803387642f, bi);
-    ar = fmaf(s25.x, 0.829405665397644f, ar); ai = fmaf(s25.y, 0.829405665397644f, ai); br = fmaf(d25.x, -0.5586467385292053f, br); bi = fmaf(d25.y, -0.5586467385292053f, bi);
-    ar = fmaf(s26.x, -0.3202698528766632f, ar); ai = fmaf(s26.y, -0.3202698528766632f, ai); br = fmaf(d26.x, 0.9473263621330261f, br); bi = fmaf(d26.y, 0.9473263621330261f, bi);
-    if (!INV) {
-      v[21] = make_float2(ar + bi, ai - br); v[32] = make_float2(ar - bi, ai + br);
-    } else {
-      v[21] = make_float2(ar - bi, ai + br); v[32] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.8610436320304871f, ar); ai = fmaf(s1.y, -0.8610436320304871f, ai); br = fmaf(d1.x, 0.5085310935974121f, br); bi = fmaf(d1.y, 0.5085310935974121f, bi);
-    ar = fmaf(s2.x, 0.4827921986579895f, ar); ai = fmaf(s2.y, 0.4827921986579895f, ai); br = fmaf(d2.x, -0.8757349252700806f, br); bi = fmaf(d2.y, -0.8757349252700806f, bi);
-    ar = fmaf(s3.x, 0.029633328318595886f, ar); ai = fmaf(s3.y, 0.029633328318595886f, ai); br = fmaf(d3.x, 0.9995608329772949f, br); bi = fmaf(d3.y, 0.9995608329772949f, bi);
-    ar = fmaf(s4.x, -0.5338233709335327f, ar); ai = fmaf(s4.y, -0.5338233709335327f, ai); br = fmaf(d4.x, -0.8455960154533386f, br); bi = fmaf(d4.y, -0.8455960154533386f, bi);
-    ar = fmaf(s5.x, 0.8896570801734924f, ar); ai = fmaf(s5.y, 0.8896570801734924f, ai); br = fmaf(d5.x, 0.4566292464733124f, br); bi = fmaf(d5.y, 0.4566292464733124f, bi);
-    ar = fmaf(s6.x, -0.9982437491416931f, ar); ai = fmaf(s6.y, -0.9982437491416931f, ai); br = fmaf(d6.x, 0.05924062803387642f, br); bi = fmaf(d6.y, 0.05924062803387642f, bi);
-    ar = fmaf(s7.x, 0.829405665397644f, ar); ai = fmaf(s7.y, 0.829405665397644f, ai); br = fmaf(d7.x, -0.5586467385292053f, br); bi = fmaf(d7.y, -0.5586467385292053f, bi);
-    ar = fmaf(s8.x, -0.43006521463394165f, ar); ai = fmaf(s8.y, -0.43006521463394165f, ai); br = fmaf(d8.x, 0.9027978181838989f, br); bi = fmaf(d8.y, 0.9027978181838989f, bi);
-    ar = fmaf(s9.x, -0.08879589289426804f, ar); ai = fmaf(s9.y, -0.08879589289426804f, ai); br = fmaf(d9.x, -0.9960498213768005f, br); bi = fmaf(d9.y, -0.9960498213768005f, bi);
-    ar = fmaf(s10.x, 0.5829795002937317f, ar); ai = fmaf(s10.y, 0.5829795002937317f, ai); br = fmaf(d10.x, 0.8124868869781494f, br); bi = fmaf(d10.y, 0.8124868869781494f, bi);
-    ar = fmaf(s11.x, -0.9151456356048584f, ar); ai = fmaf(s11.y, -0.9151456356048584f, ai); br = fmaf(d11.x, -0.4031234383583069f, br); bi = fmaf(d11.y, -0.4031234383583069f, bi);
-    ar = fmaf(s12.x, 0.9929810762405396f, ar); ai = fmaf(s12.y, 0.9929810762405396f, ai); br = fmaf(d12.x, -0.11827316880226135f, br); bi = fmaf(d12.y, -0.11827316880226135f, bi);
-    ar = fmaf(s13.x, -0.794854462146759f, ar); ai = fmaf(s13.y, -0.794854462146759f, ai); br = fmaf(d13.x, 0.6068001389503479f, br); bi = fmaf(d13.y, 0.6068001389503479f, bi);
-    ar = fmaf(s14.x, 0.3758275806903839f, ar); ai = fmaf(s14.y, 0.3758275806903839f, ai); br = fmaf(d14.x, -0.926689624786377f, br); bi = fmaf(d14.y, -0.926689624786377f, bi);
-    ar = fmaf(s15.x, 0.14764656126499176f, ar); ai = fmaf(s15.y, 0.14764656126499176f, ai); br = fmaf(d15.x, 0.989040195941925f, br); bi = fmaf(d15.y, 0.989040195941925f, bi);
-    ar = fmaf(s16.x, -0.6300878524780273f, ar); ai = fmaf(s16.y, -0.6300878524780273f, ai); br = fmaf(d16.x, -0.7765238881111145f, br); bi = fmaf(d16.y, -0.7765238881111145f, bi);
-    ar = fmaf(s17.x, 0.9374196529388428f, ar); ai = fmaf(s17.y, 0.9374196529388428f, ai); br = fmaf(d17.x, 0.3482016324996948f, br); bi = fmaf(d17.y, 0.3482016324996948f, bi);
-    ar = fmaf(s18.x, -0.9842305779457092f, ar); ai = fmaf(s18.y, -0.9842305779457092f, ai); br = fmaf(d18.x, 0.1768902689218521f, br); bi = fmaf(d18.y, 0.1768902689218521f, bi);
-    ar = fmaf(s19.x, 0.7575112581253052f, ar); ai = fmaf(s19.y, 0.7575112581253052f, ai); br = fmaf(d19.x, -0.6528221368789673f, br); bi = fmaf(d19.y, -0.6528221368789673f, bi);
-    ar = fmaf(s20.x, -0.3202698528766632f, ar); ai = fmaf(s20.y, -0.3202698528766632f, ai); br = fmaf(d20.x, 0.9473263621330261f, br); bi = fmaf(d20.y, 0.9473263621330261f, bi);
-    ar = fmaf(s21.x, -0.2059786170721054f, ar); ai = fmaf(s21.y, -0.2059786170721054f, ai); br = fmaf(d21.x, -0.9785565137863159f, br); bi = fmaf(d21.y, -0.9785565137863159f, bi);
-    ar = fmaf(s22.x, 0.674983024597168f, ar); ai = fmaf(s22.y, 0.674983024597168f, ai); br = fmaf(d22.x, 0.7378332614898682f, br); bi = fmaf(d22.y, 0.7378332614898682f, bi);
-    ar = fmaf(s23.x, -0.956400990486145f, ar); ai = fmaf(s23.y, -0.956400990486145f, ai); br = fmaf(d23.x, -0.29205676913261414f, br); bi = fmaf(d23.y, -0.29205676913261414f, bi);
-    ar = fmaf(s24.x, 0.9720228910446167f, ar); ai = fmaf(s24.y, 0.9720228910446167f, ai); br = fmaf(d24.x, -0.2348860502243042f, br); bi = fmaf(d24.y, -0.2348860502243042f, bi);
-    ar = fmaf(s25.x, -0.7175072431564331f, ar); ai = fmaf(s25.y, -0.7175072431564331f, ai); br = fmaf(d25.x, 0.6965510249137878f, br); bi = fmaf(d25.y, 0.6965510249137878f, bi);
-    ar = fmaf(s26.x, 0.26358717679977417f, ar); ai = fmaf(s26.y, 0.26358717679977417f, ai); br = fmaf(d26.x, -0.9646356105804443f, br); bi = fmaf(d26.y, -0.9646356105804443f, bi);
-    if (!INV) {
-      v[22] = make_float2(ar + bi, ai - br); v[31] = make_float2(ar - bi, ai + br);
-    } else {
-      v[22] = make_float2(ar - bi, ai + br); v[31] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.9151456356048584f, ar); ai = fmaf(s1.y, -0.9151456356048584f, ai); br = fmaf(d1.x, 0.4031234383583069f, br); bi = fmaf(d1.y, 0.4031234383583069f, bi);
-    ar = fmaf(s2.x, 0.674983024597168f, ar); ai = fmaf(s2.y, 0.674983024597168f, ai); br = fmaf(d2.x, -0.7378332614898682f, br); bi = fmaf(d2.y, -0.7378332614898682f, bi);
-    ar = fmaf(s3.x, -0.3202698528766632f, ar); ai = fmaf(s3.y, -0.3202698528766632f, ai); br = fmaf(d3.x, 0.9473263621330261f, br); bi = fmaf(d3.y, 0.9473263621330261f, bi);
-    ar = fmaf(s4.x, -0.08879589289426804f, ar); ai = fmaf(s4.y, -0.08879589289426804f, ai); br = fmaf(d4.x, -0.9960498213768005f, br); bi = fmaf(d4.y, -0.9960498213768005f, bi);
-    ar = fmaf(s5.x, 0.4827921986579895f, ar); ai = fmaf(s5.y, 0.4827921986579895f, ai); br = fmaf(d5.x, 0.8757349252700806f, br); bi = fmaf(d5.y, 0.8757349252700806f, bi);
-    ar = fmaf(s6.x, -0.794854462146759f, ar); ai = fmaf(s6.y, -0.794854462146759f, ai); br = fmaf(d6.x, -0.6068001389503479f, br); bi = fmaf(d6.y, -0.6068001389503479f, bi);
-    ar = fmaf(s7.x, 0.9720228910446167f, ar); ai = fmaf(s7.y, 0.9720228910446167f, ai); br = fmaf(d7.x, 0.2348860502243042f, br); bi = fmaf(d7.y, 0.2348860502243042f, bi);
-    ar = fmaf(s8.x, -0.9842305779457092f, ar); ai = fmaf(s8.y, -0.9842305779457092f, ai); br = fmaf(d8.x, 0.1768902689218521f, br); bi = fmaf(d8.y, 0.1768902689218521f, bi);
-    ar = fmaf(s9.x, 0.829405665397644f, ar); ai = fmaf(s9.y, 0.829405665397644f, ai); br = fmaf(d9.x, -0.5586467385292053f, br); bi = fmaf(d9.y, -0.5586467385292053f, bi);
-    ar = fmaf(s10.x, -0.5338233709335327f, ar); ai = fmaf(s10.y, -0.5338233709335327f, ai); br = fmaf(d10.x, 0.8455960154533386f, br); bi = fmaf(d10.y, 0.8455960154533386f, bi);
-    ar = fmaf(s11.x, 0.14764656126499176f, ar); ai = fmaf(s11.y, 0.14764656126499176f, ai); br = fmaf(d11.x, -0.989040195941925f, br); bi = fmaf(d11.y, -0.989040195941925f, bi);
-    ar = fmaf(s12.x, 0.26358717679977417f, ar); ai = fmaf(s12.y, 0.26358717679977417f, ai); br = fmaf(d12.x, 0.9646356105804443f, br); bi = fmaf(d12.y, 0.9646356105804443f, bi);
-    ar = fmaf(s13.x, -0.6300878524780273f, ar); ai = fmaf(s13.y, -0.6300878524780273f, ai); br = fmaf(d13.x, -0.7765238881111145f, br); bi = fmaf(d13.y, -0.7765238881111145f, bi);
-    ar = fmaf(s14.x, 0.8896570801734924f, ar); ai = fmaf(s14.y, 0.8896570801734924f, ai); br = fmaf(d14.x, 0.4566292464733124f, br); bi = fmaf(d14.y, 0.4566292464733124f, bi);
-    ar = fmaf(s15.x, -0.9982437491416931f, ar); ai = fmaf(s15.y, -0.9982437491416931f, ai); br = fmaf(d15.x, -0.05924062803387642f, br); bi = fmaf(d15.y, -0.05924062803387642f, bi);
-    ar = fmaf(s16.x, 0.9374196529388428f, ar); ai = fmaf(s16.y, 0.9374196529388428f, ai); br = fmaf(d16.x, -0.3482016324996948f, br); bi = fmaf(d16.y, -0.3482016324996948f, bi);
-    ar = fmaf(s17.x, -0.7175072431564331f, ar); ai = fmaf(s17.y, -0.7175072431564331f, ai); br = fmaf(d17.x, 0.6965510249137878f, br); bi = fmaf(d17.y, 0.6965510249137878f, bi);
-    ar = fmaf(s18.x, 0.3758275806903839f, ar); ai = fmaf(s18.y, 0.3758275806903839f, ai); br = fmaf(d18.x, -0.926689624786377f, br); bi = fmaf(d18.y, -0.926689624786377f, bi);
-    ar = fmaf(s19.x, 0.029633328318595886f, ar); ai = fmaf(s19.y, 0.029633328318595886f, ai); br = fmaf(d19.x, 0.9995608329772949f, br); bi = fmaf(d19.y, 0.9995608329772949f, bi);
-    ar = fmaf(s20.x, -0.43006521463394165f, ar); ai = fmaf(s20.y, -0.43006521463394165f, ai); br = fmaf(d20.x, -0.9027978181838989f, br); bi = fmaf(d20.y, -0.9027978181838989f, bi);
-    ar = fmaf(s21.x, 0.7575112581253052f, ar); ai = fmaf(s21.y, 0.7575112581253052f, ai); br = fmaf(d21.x, 0.6528221368789673f, br); bi = fmaf(d21.y, 0.6528221368789673f, bi);
-    ar = fmaf(s22.x, -0.956400990486145f, ar); ai = fmaf(s22.y, -0.956400990486145f, ai); br = fmaf(d22.x, -0.29205676913261414f, br); bi = fmaf(d22.y, -0.29205676913261414f, bi);
-    ar = fmaf(s23.x, 0.9929810762405396f, ar); ai = fmaf(s23.y, 0.9929810762405396f, ai); br = fmaf(d23.x, -0.11827316880226135f, br); bi = fmaf(d23.y, -0.11827316880226135f, bi);
-    ar = fmaf(s24.x, -0.8610436320304871f, ar); ai = fmaf(s24.y, -0.8610436320304871f, ai); br = fmaf(d24.x, 0.5085310935974121f, br); bi = fmaf(d24.y, 0.5085310935974121f, bi);
-    ar = fmaf(s25.x, 0.5829795002937317f, ar); ai = fmaf(s25.y, 0.5829795002937317f, ai); br = fmaf(d25.x, -0.8124868869781494f, br); bi = fmaf(d25.y, -0.8124868869781494f, bi);
-    ar = fmaf(s26.x, -0.2059786170721054f, ar); ai = fmaf(s26.y, -0.2059786170721054f, ai); br = fmaf(d26.x, 0.9785565137863159f, br); bi = fmaf(d26.y, 0.9785565137863159f, bi);
-    if (!INV) {
-      v[23] = make_float2(ar + bi, ai - br); v[30] = make_float2(ar - bi, ai + br);
-    } else {
-      v[23] = make_float2(ar - bi, ai + br); v[30] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.956400990486145f, ar); ai = fmaf(s1.y, -0.956400990486145f, ai); br = fmaf(d1.x, 0.29205676913261414f, br); bi = fmaf(d1.y, 0.29205676913261414f, bi);
-    ar = fmaf(s2.x, 0.829405665397644f, ar); ai = fmaf(s2.y, 0.829405665397644f, ai); br = fmaf(d2.x, -0.5586467385292053f, br); bi = fmaf(d2.y, -0.5586467385292053f, bi);
-    ar = fmaf(s3.x, -0.6300878524780273f, ar); ai = fmaf(s3.y, -0.6300878524780273f, ai); br = fmaf(d3.x, 0.7765238881111145f, br); bi = fmaf(d3.y, 0.7765238881111145f, bi);
-    ar = fmaf(s4.x, 0.3758275806903839f, ar); ai = fmaf(s4.y, 0.3758275806903839f, ai); br = fmaf(d4.x, -0.926689624786377f, br); bi = fmaf(d4.y, -0.926689624786377f, bi);
-    ar = fmaf(s5.x, -0.08879589289426804f, ar); ai = fmaf(s5.y, -0.08879589289426804f, ai); br = fmaf(d5.x, 0.9960498213768005f, br); bi = fmaf(d5.y, 0.9960498213768005f, bi);
-    ar = fmaf(s6.x, -0.2059786170721054f, ar); ai = fmaf(s6.y, -0.2059786170721054f, ai); br = fmaf(d6.x, -0.9785565137863159f, br); bi = fmaf(d6.y, -0.9785565137863159f, bi);
-    ar = fmaf(s7.x, 0.4827921986579895f, ar); ai = fmaf(s7.y, 0.4827921986579895f, ai); br = fmaf(d7.x, 0.8757349252700806f, br); bi = fmaf(d7.y, 0.8757349252700806f, bi);
-    ar = fmaf(s8.x, -0.7175072431564331f, ar); ai = fmaf(s8.y, -0.7175072431564331f, ai); br = fmaf(d8.x, -0.6965510249137878f, br); bi = fmaf(d8.y, -0.6965510249137878f, bi);
-    ar = fmaf(s9.x, 0.8896570801734924f, ar); ai = fmaf(s9.y, 0.8896570801734924f, ai); br = fmaf(d9.x, 0.4566292464733124f, br); bi = fmaf(d9.y, 0.4566292464733124f, bi);
-    ar = fmaf(s10.x, -0.9842305779457092f, ar); ai = fmaf(s10.y, -0.9842305779457092f, ai); br = fmaf(d10.x, -0.1768902689218521f, br); bi = fmaf(d10.y, -0.1768902689218521f, bi);
-    ar = fmaf(s11.x, 0.9929810762405396f, ar); ai = fmaf(s11.y, 0.9929810762405396f, ai); br = fmaf(d11.x, -0.11827316880226135f, br); bi = fmaf(d11.y, -0.11827316880226135f, bi);
-    ar = fmaf(s12.x, -0.9151456356048584f, ar); ai = fmaf(s12.y, -0.9151456356048584f, ai); br = fmaf(d12.x, 0.4031234383583069f, br); bi = fmaf(d12.y, 0.4031234383583069f, bi);
-    ar = fmaf(s13.x, 0.7575112581253052f, ar); ai = fmaf(s13.y, 0.7575112581253052f, ai); br = fmaf(d13.x, -0.6528221368789673f, br); bi = fmaf(d13.y, -0.6528221368789673f, bi);
-    ar = fmaf(s14.x, -0.5338233709335327f, ar); ai = fmaf(s14.y, -0.5338233709335327f, ai); br = fmaf(d14.x, 0.8455960154533386f, br); bi = fmaf(d14.y, 0.8455960154533386f, bi);
-    ar = fmaf(s15.x, 0.26358717679977417f, ar); ai = fmaf(s15.y, 0.26358717679977417f, ai); br = fmaf(d15.x, -0.9646356105804443f, br); bi = fmaf(d15.y, -0.9646356105804443f, bi);
-    ar = fmaf(s16.x, 0.029633328318595886f, ar); ai = fmaf(s16.y, 0.029633328318595886f, ai); br = fmaf(d16.x, 0.9995608329772949f, br); bi = fmaf(d16.y, 0.9995608329772949f, bi);
-    ar = fmaf(s17.x, -0.3202698528766632f, ar); ai = fmaf(s17.y, -0.3202698528766632f, ai); br = fmaf(d17.x, -0.9473263621330261f, br); bi = fmaf(d17.y, -0.9473263621330261f, bi);
-    ar = fmaf(s18.x, 0.5829795002937317f, ar); ai = fmaf(s18.y, 0.5829795002937317f, ai); br = fmaf(d18.x, 0.8124868869781494f, br); bi = fmaf(d18.y, 0.8124868869781494f, bi);
-    ar = fmaf(s19.x, -0.794854462146759f, ar); ai = fmaf(s19.y, -0.794854462146759f, ai); br = fmaf(d19.x, -0.6068001389503479f, br); bi = fmaf(d19.y, -0.6068001389503479f, bi);
-    ar = fmaf(s20.x, 0.9374196529388428f, ar); ai = fmaf(s20.y, 0.9374196529388428f, ai); br = fmaf(d20.x, 0.3482016324996948f, br); bi = fmaf(d20.y, 0.3482016324996948f, bi);
-    ar = fmaf(s21.x, -0.9982437491416931f, ar); ai = fmaf(s21.y, -0.9982437491416931f, ai); br = fmaf(d21.x, -0.05924062803387642f, br); bi = fmaf(d21.y, -0.05924062803387642f, bi);
-    ar = fmaf(s22.x, 0.9720228910446167f, ar); ai = fmaf(s22.y, 0.9720228910446167f, ai); br = fmaf(d22.x, -0.2348860502243042f, br); bi = fmaf(d22.y, -0.2348860502243042f, bi);
-    ar = fmaf(s23.x, -0.8610436320304871f, ar); ai = fmaf(s23.y, -0.8610436320304871f, ai); br = fmaf(d23.x, 0.5085310935974121f, br); bi = fmaf(d23.y, 0.5085310935974121f, bi);
-    ar = fmaf(s24.x, 0.674983024597168f, ar); ai = fmaf(s24.y, 0.674983024597168f, ai); br = fmaf(d24.x, -0.7378332614898682f, br); bi = fmaf(d24.y, -0.7378332614898682f, bi);
-    ar = fmaf(s25.x, -0.43006521463394165f, ar); ai = fmaf(s25.y, -0.43006521463394165f, ai); br = fmaf(d25.x, 0.9027978181838989f, br); bi = fmaf(d25.y, 0.9027978181838989f, bi);
-    ar = fmaf(s26.x, 0.14764656126499176f, ar); ai = fmaf(s26.y, 0.14764656126499176f, ai); br = fmaf(d26.x, -0.989040195941925f, br); bi = fmaf(d26.y, -0.989040195941925f, bi);
-    if (!INV) {
-      v[24] = make_float2(ar + bi, ai - br); v[29] = make_float2(ar - bi, ai + br);
-    } else {
-      v[24] = make_float2(ar - bi, ai + br); v[29] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.9842305779457092f, ar); ai = fmaf(s1.y, -0.9842305779457092f, ai); br = fmaf(d1.x, 0.1768902689218521f, br); bi = fmaf(d1.y, 0.1768902689218521f, bi);
-    ar = fmaf(s2.x, 0.9374196529388428f, ar); ai = fmaf(s2.y, 0.9374196529388428f, ai); br = fmaf(d2.x, -0.3482016324996948f, br); bi = fmaf(d2.y, -0.3482016324996948f, bi);
-    ar = fmaf(s3.x, -0.8610436320304871f, ar); ai = fmaf(s3.y, -0.8610436320304871f, ai); br = fmaf(d3.x, 0.5085310935974121f, br); bi = fmaf(d3.y, 0.5085310935974121f, bi);
-    ar = fmaf(s4.x, 0.7575112581253052f, ar); ai = fmaf(s4.y, 0.7575112581253052f, ai); br = fmaf(d4.x, -0.6528221368789673f, br); bi = fmaf(d4.y, -0.6528221368789673f, bi);
-    ar = fmaf(s5.x, -0.6300878524780273f, ar); ai = fmaf(s5.y, -0.6300878524780273f, ai); br = fmaf(d5.x, 0.7765238881111145f, br); bi = fmaf(d5.y, 0.7765238881111145f, bi);
-    ar = fmaf(s6.x, 0.4827921986579895f, ar); ai = fmaf(s6.y, 0.4827921986579895f, ai); br = fmaf(d6.x, -0.8757349252700806f, br); bi = fmaf(d6.y, -0.8757349252700806f, bi);
-    ar = fmaf(s7.x, -0.3202698528766632f, ar); ai = fmaf(s7.y, -0.3202698528766632f, ai); br = fmaf(d7.x, 0.9473263621330261f, br); bi = fmaf(d7.y, 0.9473263621330261f, bi);
-    ar = fmaf(s8.x, 0.14764656126499176f, ar); ai = fmaf(s8.y, 0.14764656126499176f, ai); br = fmaf(d8.x, -0.989040195941925f, br); bi = fmaf(d8.y, -0.989040195941925f, bi);
-    ar = fmaf(s9.x, 0.029633328318595886f, ar); ai = fmaf(s9.y, 0.029633328318595886f, ai); br = fmaf(d9.x, 0.9995608329772949f, br); bi = fmaf(d9.y, 0.9995608329772949f, bi);
-    ar = fmaf(s10.x, -0.2059786170721054f, ar); ai = fmaf(s10.y, -0.2059786170721054f, ai); br = fmaf(d10.x, -0.9785565137863159f, br); bi = fmaf(d10.y, -0.9785565137863159f, bi);
-    ar = fmaf(s11.x, 0.3758275806903839f, ar); ai = fmaf(s11.y, 0.3758275806903839f, ai); br = fmaf(d11.x, 0.926689624786377f, br); bi = fmaf(d11.y, 0.926689624786377f, bi);
-    ar = fmaf(s12.x, -0.5338233709335327f, ar); ai = fmaf(s12.y, -0.5338233709335327f, ai); br = fmaf(d12.x, -0.8455960154533386f, br); bi = fmaf(d12.y, -0.8455960154533386f, bi);
-    ar = fmaf(s13.x, 0.674983024597168f, ar); ai = fmaf(s13.y, 0.674983024597168f, ai); br = fmaf(d13.x, 0.7378332614898682f, br); bi = fmaf(d13.y, 0.7378332614898682f, bi);
-    ar = fmaf(s14.x, -0.794854462146759f, ar); ai = fmaf(s14.y, -0.794854462146759f, ai); br = fmaf(d14.x, -0.6068001389503479f, br); bi = fmaf(d14.y, -0.6068001389503479f, bi);
-    ar = fmaf(s15.x, 0.8896570801734924f, ar); ai = fmaf(s15.y, 0.8896570801734924f, ai); br = fmaf(d15.x, 0.4566292464733124f, br); bi = fmaf(d15.y, 0.4566292464733124f, bi);
-    ar = fmaf(s16.x, -0.956400990486145f, ar); ai = fmaf(s16.y, -0.956400990486145f, ai); br = fmaf(d16.x, -0.29205676913261414f, br); bi = fmaf(d16.y, -0.29205676913261414f, bi);
-    ar = fmaf(s17.x, 0.9929810762405396f, ar); ai = fmaf(s17.y, 0.9929810762405396f, ai); br = fmaf(d17.x, 0.11827316880226135f, br); bi = fmaf(d17.y, 0.11827316880226135f, bi);
-    ar = fmaf(s18.x, -0.9982437491416931f, ar); ai = fmaf(s18.y, -0.9982437491416931f, ai); br = fmaf(d18.x, 0.05924062803387642f, br); bi = fmaf(d18.y, 0.05924062803387642f, bi);
-    ar = fmaf(s19.x, 0.9720228910446167f, ar); ai = fmaf(s19.y, 0.9720228910446167f, ai); br = fmaf(d19.x, -0.2348860502243042f, br); bi = fmaf(d19.y, -0.2348860502243042f, bi);
-    ar = fmaf(s20.x, -0.9151456356048584f, ar); ai = fmaf(s20.y, -0.9151456356048584f, ai); br = fmaf(d20.x, 0.4031234383583069f, br); bi = fmaf(d20.y, 0.4031234383583069f, bi);
-    ar = fmaf(s21.x, 0.829405665397644f, ar); ai = fmaf(s21.y, 0.829405665397644f, ai); br = fmaf(d21.x, -0.5586467385292053f, br); bi = fmaf(d21.y, -0.5586467385292053f, bi);
-    ar = fmaf(s22.x, -0.7175072431564331f, ar); ai = fmaf(s22.y, -0.7175072431564331f, ai); br = fmaf(d22.x, 0.6965510249137878f, br); bi = fmaf(d22.y, 0.6965510249137878f, bi);
-    ar = fmaf(s23.x, 0.5829795002937317f, ar); ai = fmaf(s23.y, 0.5829795002937317f, ai); br = fmaf(d23.x, -0.8124868869781494f, br); bi = fmaf(d23.y, -0.8124868869781494f, bi);
-    ar = fmaf(s24.x, -0.43006521463394165f, ar); ai = fmaf(s24.y, -0.43006521463394165f, ai); br = fmaf(d24.x, 0.9027978181838989f, br); bi = fmaf(d24.y, 0.9027978181838989f, bi);
-    ar = fmaf(s25.x, 0.26358717679977417f, ar); ai = fmaf(s25.y, 0.26358717679977417f, ai); br = fmaf(d25.x, -0.9646356105804443f, br); bi = fmaf(d25.y, -0.9646356105804443f, bi);
-    ar = fmaf(s26.x, -0.08879589289426804f, ar); ai = fmaf(s26.y, -0.08879589289426804f, ai); br = fmaf(d26.x, 0.9960498213768005f, br); bi = fmaf(d26.y, 0.9960498213768005f, bi);
-    if (!INV) {
-      v[25] = make_float2(ar + bi, ai - br); v[28] = make_float2(ar - bi, ai + br);
-    } else {
-      v[25] = make_float2(ar - bi, ai + br); v[28] = make_float2(ar + bi, ai - br);
-    }
-  }
-  {
-    float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-    ar = fmaf(s1.x, -0.9982437491416931f, ar); ai = fmaf(s1.y, -0.9982437491416931f, ai); br = fmaf(d1.x, 0.05924062803387642f, br); bi = fmaf(d1.y, 0.05924062803387642f, bi);
-    ar = fmaf(s2.x, 0.9929810762405396f, ar); ai = fmaf(s2.y, 0.9929810762405396f, ai); br = fmaf(d2.x, -0.11827316880226135f, br); bi = fmaf(d2.y, -0.11827316880226135f, bi);
-    ar = fmaf(s3.x, -0.9842305779457092f, ar); ai = fmaf(s3.y, -0.9842305779457092f, ai); br = fmaf(d3.x, 0.1768902689218521f, br); bi = fmaf(d3.y, 0.1768902689218521f, bi);
-    ar = fmaf(s4.x, 0.9720228910446167f, ar); ai = fmaf(s4.y, 0.9720228910446167f, ai); br = fmaf(d4.x, -0.2348860502243042f, br); bi = fmaf(d4.y, -0.2348860502243042f, bi);
-    ar = fmaf(s5.x, -0.956400990486145f, ar); ai = fmaf(s5.y, -0.956400990486145f, ai); br = fmaf(d5.x, 0.29205676913261414f, br); bi = fmaf(d5.y, 0.29205676913261414f, bi);
-    ar = fmaf(s6.x, 0.9374196529388428f, ar); ai = fmaf(s6.y, 0.9374196529388428f, ai); br = fmaf(d6.x, -0.3482016324996948f, br); bi = fmaf(d6.y, -0.3482016324996948f, bi);
-    ar = fmaf(s7.x, -0.9151456356048584f, ar); ai = fmaf(s7.y, -0.9151456356048584f, ai); br = fmaf(d7.x, 0.4031234383583069f, br); bi = fmaf(d7.y, 0.4031234383583069f, bi);
-    ar = fmaf(s8.x, 0.8896570801734924f, ar); ai = fmaf(s8.y, 0.8896570801734924f, ai); br = fmaf(d8.x, -0.4566292464733124f, br); bi = fmaf(d8.y, -0.4566292464733124f, bi);
-    ar = fmaf(s9.x, -0.8610436320304871f, ar); ai = fmaf(s9.y, -0.8610436320304871f, ai); br = fmaf(d9.x, 0.5085310935974121f, br); bi = fmaf(d9.y, 0.5085310935974121f, bi);
-    ar = fmaf(s10.x, 0.829405665397644f, ar); ai = fmaf(s10.y, 0.829405665397644f, ai); br = fmaf(d10.x, -0.5586467385292053f, br); bi = fmaf(d10.y, -0.5586467385292053f, bi);
-    ar = fmaf(s11.x, -0.794854462146759f, ar); ai = fmaf(s11.y, -0.794854462146759f, ai); br = fmaf(d11.x, 0.6068001389503479f, br); bi = fmaf(d11.y, 0.6068001389503479f, bi);
-    ar = fmaf(s12.x, 0.7575112581253052f, ar); ai = fmaf(s12.y, 0.7575112581253052f, ai); br = fmaf(d12.x, -0.6528221368789673f, br); bi = fmaf(d12.y, -0.6528221368789673f, bi);
-    ar = fmaf(s13.x, -0.7175072431564331f, ar); ai = fmaf(s13.y, -0.7175072431564331f, ai); br = fmaf(d13.x, 0.6965510249137878f, br); bi = fmaf(d13.y, 0.6965510249137878f, bi);
-    ar = fmaf(s14.x, 0.674983024597168f, ar); ai = fmaf(s14.y, 0.674983024597168f, ai); br = fmaf(d14.x, -0.7378332614898682f, br); bi = fmaf(d14.y, -0.7378332614898682f, bi);
-    ar = fmaf(s15.x, -0.6300878524780273f, ar); ai = fmaf(s15.y, -0.6300878524780273f, ai); br = fmaf(d15.x, 0.7765238881111145f, br); bi = fmaf(d15.y, 0.7765238881111145f, bi);
-    ar = fmaf(s16.x, 0.5829795002937317f, ar); ai = fmaf(s16.y, 0.5829795002937317f, ai); br = fmaf(d16.x, -0.8124868869781494f, br); bi = fmaf(d16.y, -0.8124868869781494f, bi);
-    ar = fmaf(s17.x, -0.5338233709335327f, ar); ai = fmaf(s17.y, -0.5338233709335327f, ai); br = fmaf(d17.x, 0.8455960154533386f, br); bi = fmaf(d17.y, 0.8455960154533386f, bi);
-    ar = fmaf(s18.x, 0.4827921986579895f, ar); ai = fmaf(s18.y, 0.4827921986579895f, ai); br = fmaf(d18.x, -0.8757349252700806f, br); bi = fmaf(d18.y, -0.8757349252700806f, bi);
-    ar = fmaf(s19.x, -0.43006521463394165f, ar); ai = fmaf(s19.y, -0.43006521463394165f, ai); br = fmaf(d19.x, 0.9027978181838989f, br); bi = fmaf(d19.y, 0.9027978181838989f, bi);
-    ar = fmaf(s20.x, 0.3758275806903839f, ar); ai = fmaf(s20.y, 0.3758275806903839f, ai); br = fmaf(d20.x, -0.926689624786377f, br); bi = fmaf(d20.y, -0.926689624786377f, bi);
-    ar = fmaf(s21.x, -0.3202698528766632f, ar); ai = fmaf(s21.y, -0.3202698528766632f, ai); br = fmaf(d21.x, 0.9473263621330261f, br); bi = fmaf(d21.y, 0.9473263621330261f, bi);
-    ar = fmaf(s22.x, 0.26358717679977417f, ar); ai = fmaf(s22.y, 0.26358717679977417f, ai); br = fmaf(d22.x, -0.9646356105804443f, br); bi = fmaf(d22.y, -0.9646356105804443f, bi);
-    ar = fmaf(s23.x, -0.2059786170721054f, ar); ai = fmaf(s23.y, -0.2059786170721054f, ai); br = fmaf(d23.x, 0.9785565137863159f, br); bi = fmaf(d23.y, 0.9785565137863159f, bi);
-    ar = fmaf(s24.x, 0.14764656126499176f, ar); ai = fmaf(s24.y, 0.14764656126499176f, ai); br = fmaf(d24.x, -0.989040195941925f, br); bi = fmaf(d24.y, -0.989040195941925f, bi);
-    ar = fmaf(s25.x, -0.08879589289426804f, ar); ai = fmaf(s25.y, -0.08879589289426804f, ai); br = fmaf(d25.x, 0.9960498213768005f, br); bi = fmaf(d25.y, 0.9960498213768005f, bi);
-    ar = fmaf(s26.x, 0.029633328318595886f, ar); ai = fmaf(s26.y, 0.029633328318595886f, ai); br = fmaf(d26.x, -0.9995608329772949f, br); bi = fmaf(d26.y, -0.9995608329772949f, bi);
-    if (!INV) {
-      v[26] = make_float2(ar + bi, ai - br); v[27] = make_float2(ar - bi, ai + br);
-    } else {
-      v[26] = make_float2(ar - bi, ai + br); v[27] = make_float2(ar + bi, ai - br);
-    }
-  }
-}
-constexpr int kSplit53 = 3;
-template <bool INV, typename St>
-__device__ __forceinline__ void dft_r53_part(const float2* v, int part, St&& st) {
-  const float2 x0 = v[0];
-  const float2 s1 = padd(v[1], v[52]);
-  const float2 d1 = psub(v[1], v[52]);
-  const float2 s2 = padd(v[2], v[51]);
-  const float2 d2 = psub(v[2], v[51]);
-  const float2 s3 = padd(v[3], v[50]);
-  const float2 d3 = psub(v[3], v[50]);
-  const float2 s4 = padd(v[4], v[49]);
-  const float2 d4 = psub(v[4], v[49]);
-  const float2 s5 = padd(v[5], v[48]);
-  const float2 d5 = psub(v[5], v[48]);
-  const float2 s6 = padd(v[6], v[47]);
-  const float2 d6 = psub(v[6], v[47]);
-  const float2 s7 = padd(v[7], v[46]);
-  const float2 d7 = psub(v[7], v[46]);
-  const float2 s8 = padd(v[8], v[45]);
-  const float2 d8 = psub(v[8], v[45]);
-  const float2 s9 = padd(v[9], v[44]);
-  const float2 d9 = psub(v[9], v[44]);
-  const float2 s10 = padd(v[10], v[43]);
-  const float2 d10 = psub(v[10], v[43]);
-  const float2 s11 = padd(v[11], v[42]);
-  const float2 d11 = psub(v[11], v[42]);
-  const float2 s12 = padd(v[12], v[41]);
-  const float2 d12 = psub(v[12], v[41]);
-  const float2 s13 = padd(v[13], v[40]);
-  const float2 d13 = psub(v[13], v[40]);
-  const float2 s14 = padd(v[14], v[39]);
-  const float2 d14 = psub(v[14], v[39]);
-  const float2 s15 = padd(v[15], v[38]);
-  const float2 d15 = psub(v[15], v[38]);
-  const float2 s16 = padd(v[16], v[37]);
-  const float2 d16 = psub(v[16], v[37]);
-  const float2 s17 = padd(v[17], v[36]);
-  const float2 d17 = psub(v[17], v[36]);
-  const float2 s18 = padd(v[18], v[35]);
-  const float2 d18 = psub(v[18], v[35]);
-  const float2 s19 = padd(v[19], v[34]);
-  const float2 d19 = psub(v[19], v[34]);
-  const float2 s20 = padd(v[20], v[33]);
-  const float2 d20 = psub(v[20], v[33]);
-  const float2 s21 = padd(v[21], v[32]);
-  const float2 d21 = psub(v[21], v[32]);
-  const float2 s22 = padd(v[22], v[31]);
-  const float2 d22 = psub(v[22], v[31]);
-  const float2 s23 = padd(v[23], v[30]);
-  const float2 d23 = psub(v[23], v[30]);
-  const float2 s24 = padd(v[24], v[29]);
-  const float2 d24 = psub(v[24], v[29]);
-  const float2 s25 = padd(v[25], v[28]);
-  const float2 d25 = psub(v[25], v[28]);
-  const float2 s26 = padd(v[26], v[27]);
-  const float2 d26 = psub(v[26], v[27]);
-  if (part == 0) st(0, make_float2(x0.x + (s1.x + s2.x + s3.x + s4.x + s5.x + s6.x + s7.x + s8.x + s9.x + s10.x + s11.x + s12.x + s13.x + s14.x + s15.x + s16.x + s17.x + s18.x + s19.x + s20.x + s21.x + s22.x + s23.x + s24.x + s25.x + s26.x), x0.y + (s1.y + s2.y + s3.y + s4.y + s5.y + s6.y + s7.y + s8.y + s9.y + s10.y + s11.y + s12.y + s13.y + s14.y + s15.y + s16.y + s17.y + s18.y + s19.y + s20.y + s21.y + s22.y + s23.y + s24.y + s25.y + s26.y)));
-  switch (part) {
-  case 0: {
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.9929810762405396f, ar); ai = fmaf(s1.y, 0.9929810762405396f, ai); br = fmaf(d1.x, 0.11827316880226135f, br); bi = fmaf(d1.y, 0.11827316880226135f, bi);
-      ar = fmaf(s2.x, 0.9720228910446167f, ar); ai = fmaf(s2.y, 0.9720228910446167f, ai); br = fmaf(d2.x, 0.2348860502243042f, br); bi = fmaf(d2.y, 0.2348860502243042f, bi);
-      ar = fmaf(s3.x, 0.9374196529388428f, ar); ai = fmaf(s3.y, 0.9374196529388428f, ai); br = fmaf(d3.x, 0.3482016324996948f, br); bi = fmaf(d3.y, 0.3482016324996948f, bi);
-      ar = fmaf(s4.x, 0.8896570801734924f, ar); ai = fmaf(s4.y, 0.8896570801734924f, ai); br = fmaf(d4.x, 0.4566292464733124f, br); bi = fmaf(d4.y, 0.4566292464733124f, bi);
-      ar = fmaf(s5.x, 0.829405665397644f, ar); ai = fmaf(s5.y, 0.829405665397644f, ai); br = fmaf(d5.x, 0.5586467385292053f, br); bi = fmaf(d5.y, 0.5586467385292053f, bi);
-      ar = fmaf(s6.x, 0.7575112581253052f, ar); ai = fmaf(s6.y, 0.7575112581253052f, ai); br = fmaf(d6.x, 0.6528221368789673f, br); bi = fmaf(d6.y, 0.6528221368789673f, bi);
-      ar = fmaf(s7.x, 0.674983024597168f, ar); ai = fmaf(s7.y, 0.674983024597168f, ai); br = fmaf(d7.x, 0.7378332614898682f, br); bi = fmaf(d7.y, 0.7378332614898682f, bi);
-      ar = fmaf(s8.x, 0.5829795002937317f, ar); ai = fmaf(s8.y, 0.5829795002937317f, ai); br = fmaf(d8.x, 0.8124868869781494f, br); bi = fmaf(d8.y, 0.8124868869781494f, bi);
-      ar = fmaf(s9.x, 0.4827921986579895f, ar); ai = fmaf(s9.y, 0.4827921986579895f, ai); br = fmaf(d9.x, 0.8757349252700806f, br); bi = fmaf(d9.y, 0.8757349252700806f, bi);
-      ar = fmaf(s10.x, 0.3758275806903839f, ar); ai = fmaf(s10.y, 0.3758275806903839f, ai); br = fmaf(d10.x, 0.926689624786377f, br); bi = fmaf(d10.y, 0.926689624786377f, bi);
-      ar = fmaf(s11.x, 0.26358717679977417f, ar); ai = fmaf(s11.y, 0.26358717679977417f, ai); br = fmaf(d11.x, 0.9646356105804443f, br); bi = fmaf(d11.y, 0.9646356105804443f, bi);
-      ar = fmaf(s12.x, 0.14764656126499176f, ar); ai = fmaf(s12.y, 0.14764656126499176f, ai); br = fmaf(d12.x, 0.989040195941925f, br); bi = fmaf(d12.y, 0.989040195941925f, bi);
-      ar = fmaf(s13.x, 0.029633328318595886f, ar); ai = fmaf(s13.y, 0.029633328318595886f, ai); br = fmaf(d13.x, 0.9995608329772949f, br); bi = fmaf(d13.y, 0.9995608329772949f, bi);
-      ar = fmaf(s14.x, -0.08879589289426804f, ar); ai = fmaf(s14.y, -0.08879589289426804f, ai); br = fmaf(d14.x, 0.9960498213768005f, br); bi = fmaf(d14.y, 0.9960498213768005f, bi);
-      ar = fmaf(s15.x, -0.2059786170721054f, ar); ai = fmaf(s15.y, -0.2059786170721054f, ai); br = fmaf(d15.x, 0.9785565137863159f, br); bi = fmaf(d15.y, 0.9785565137863159f, bi);
-      ar = fmaf(s16.x, -0.3202698528766632f, ar); ai = fmaf(s16.y, -0.3202698528766632f, ai); br = fmaf(d16.x, 0.9473263621330261f, br); bi = fmaf(d16.y, 0.9473263621330261f, bi);
-      ar = fmaf(s17.x, -0.43006521463394165f, ar); ai = fmaf(s17.y, -0.43006521463394165f, ai); br = fmaf(d17.x, 0.9027978181838989f, br); bi = fmaf(d17.y, 0.9027978181838989f, bi);
-      ar = fmaf(s18.x, -0.5338233709335327f, ar); ai = fmaf(s18.y, -0.5338233709335327f, ai); br = fmaf(d18.x, 0.8455960154533386f, br); bi = fmaf(d18.y, 0.8455960154533386f, bi);
-      ar = fmaf(s19.x, -0.6300878524780273f, ar); ai = fmaf(s19.y, -0.6300878524780273f, ai); br = fmaf(d19.x, 0.7765238881111145f, br); bi = fmaf(d19.y, 0.7765238881111145f, bi);
-      ar = fmaf(s20.x, -0.7175072431564331f, ar); ai = fmaf(s20.y, -0.7175072431564331f, ai); br = fmaf(d20.x, 0.6965510249137878f, br); bi = fmaf(d20.y, 0.6965510249137878f, bi);
-      ar = fmaf(s21.x, -0.794854462146759f, ar); ai = fmaf(s21.y, -0.794854462146759f, ai); br = fmaf(d21.x, 0.6068001389503479f, br); bi = fmaf(d21.y, 0.6068001389503479f, bi);
-      ar = fmaf(s22.x, -0.8610436320304871f, ar); ai = fmaf(s22.y, -0.8610436320304871f, ai); br = fmaf(d22.x, 0.5085310935974121f, br); bi = fmaf(d22.y, 0.5085310935974121f, bi);
-      ar = fmaf(s23.x, -0.9151456356048584f, ar); ai = fmaf(s23.y, -0.9151456356048584f, ai); br = fmaf(d23.x, 0.4031234383583069f, br); bi = fmaf(d23.y, 0.4031234383583069f, bi);
-      ar = fmaf(s24.x, -0.956400990486145f, ar); ai = fmaf(s24.y, -0.956400990486145f, ai); br = fmaf(d24.x, 0.29205676913261414f, br); bi = fmaf(d24.y, 0.29205676913261414f, bi);
-      ar = fmaf(s25.x, -0.9842305779457092f, ar); ai = fmaf(s25.y, -0.9842305779457092f, ai); br = fmaf(d25.x, 0.1768902689218521f, br); bi = fmaf(d25.y, 0.1768902689218521f, bi);
-      ar = fmaf(s26.x, -0.9982437491416931f, ar); ai = fmaf(s26.y, -0.9982437491416931f, ai); br = fmaf(d26.x, 0.05924062803387642f, br); bi = fmaf(d26.y, 0.05924062803387642f, bi);
-      if (!INV) { st(1, make_float2(ar + bi, ai - br)); st(52, make_float2(ar - bi, ai + br)); }
-      else { st(1, make_float2(ar - bi, ai + br)); st(52, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.9720228910446167f, ar); ai = fmaf(s1.y, 0.9720228910446167f, ai); br = fmaf(d1.x, 0.2348860502243042f, br); bi = fmaf(d1.y, 0.2348860502243042f, bi);
-      ar = fmaf(s2.x, 0.8896570801734924f, ar); ai = fmaf(s2.y, 0.8896570801734924f, ai); br = fmaf(d2.x, 0.4566292464733124f, br); bi = fmaf(d2.y, 0.4566292464733124f, bi);
-      ar = fmaf(s3.x, 0.7575112581253052f, ar); ai = fmaf(s3.y, 0.7575112581253052f, ai); br = fmaf(d3.x, 0.6528221368789673f, br); bi = fmaf(d3.y, 0.6528221368789673f, bi);
-      ar = fmaf(s4.x, 0.5829795002937317f, ar); ai = fmaf(s4.y, 0.5829795002937317f, ai); br = fmaf(d4.x, 0.8124868869781494f, br); bi = fmaf(d4.y, 0.8124868869781494f, bi);
-      ar = fmaf(s5.x, 0.3758275806903839f, ar); ai = fmaf(s5.y, 0.3758275806903839f, ai); br = fmaf(d5.x, 0.926689624786377f, br); bi = fmaf(d5.y, 0.926689624786377f, bi);
-      ar = fmaf(s6.x, 0.14764656126499176f, ar); ai = fmaf(s6.y, 0.14764656126499176f, ai); br = fmaf(d6.x, 0.989040195941925f, br); bi = fmaf(d6.y, 0.989040195941925f, bi);
-      ar = fmaf(s7.x, -0.08879589289426804f, ar); ai = fmaf(s7.y, -0.08879589289426804f, ai); br = fmaf(d7.x, 0.9960498213768005f, br); bi = fmaf(d7.y, 0.9960498213768005f, bi);
-      ar = fmaf(s8.x, -0.3202698528766632f, ar); ai = fmaf(s8.y, -0.3202698528766632f, ai); br = fmaf(d8.x, 0.9473263621330261f, br); bi = fmaf(d8.y, 0.9473263621330261f, bi);
-      ar = fmaf(s9.x, -0.5338233709335327f, ar); ai = fmaf(s9.y, -0.5338233709335327f, ai); br = fmaf(d9.x, 0.8455960154533386f, br); bi = fmaf(d9.y, 0.8455960154533386f, bi);
-      ar = fmaf(s10.x, -0.7175072431564331f, ar); ai = fmaf(s10.y, -0.7175072431564331f, ai); br = fmaf(d10.x, 0.6965510249137878f, br); bi = fmaf(d10.y, 0.6965510249137878f, bi);
-      ar = fmaf(s11.x, -0.8610436320304871f, ar); ai = fmaf(s11.y, -0.8610436320304871f, ai); br = fmaf(d11.x, 0.5085310935974121f, br); bi = fmaf(d11.y, 0.5085310935974121f, bi);
-      ar = fmaf(s12.x, -0.956400990486145f, ar); ai = fmaf(s12.y, -0.956400990486145f, ai); br = fmaf(d12.x, 0.29205676913261414f, br); bi = fmaf(d12.y, 0.29205676913261414f, bi);
-      ar = fmaf(s13.x, -0.9982437491416931f, ar); ai = fmaf(s13.y, -0.9982437491416931f, ai); br = fmaf(d13.x, 0.05924062803387642f, br); bi = fmaf(d13.y, 0.05924062803387642f, bi);
-      ar = fmaf(s14.x, -0.9842305779457092f, ar); ai = fmaf(s14.y, -0.9842305779457092f, ai); br = fmaf(d14.x, -0.1768902689218521f, br); bi = fmaf(d14.y, -0.1768902689218521f, bi);
-      ar = fmaf(s15.x, -0.9151456356048584f, ar); ai = fmaf(s15.y, -0.9151456356048584f, ai); br = fmaf(d15.x, -0.4031234383583069f, br); bi = fmaf(d15.y, -0.4031234383583069f, bi);
-      ar = fmaf(s16.x, -0.794854462146759f, ar); ai = fmaf(s16.y, -0.794854462146759f, ai); br = fmaf(d16.x, -0.6068001389503479f, br); bi = fmaf(d16.y, -0.6068001389503479f, bi);
-      ar = fmaf(s17.x, -0.6300878524780273f, ar); ai = fmaf(s17.y, -0.6300878524780273f, ai); br = fmaf(d17.x, -0.7765238881111145f, br); bi = fmaf(d17.y, -0.7765238881111145f, bi);
-      ar = fmaf(s18.x, -0.43006521463394165f, ar); ai = fmaf(s18.y, -0.43006521463394165f, ai); br = fmaf(d18.x, -0.9027978181838989f, br); bi = fmaf(d18.y, -0.9027978181838989f, bi);
-      ar = fmaf(s19.x, -0.2059786170721054f, ar); ai = fmaf(s19.y, -0.2059786170721054f, ai); br = fmaf(d19.x, -0.9785565137863159f, br); bi = fmaf(d19.y, -0.9785565137863159f, bi);
-      ar = fmaf(s20.x, 0.029633328318595886f, ar); ai = fmaf(s20.y, 0.029633328318595886f, ai); br = fmaf(d20.x, -0.9995608329772949f, br); bi = fmaf(d20.y, -0.9995608329772949f, bi);
-      ar = fmaf(s21.x, 0.26358717679977417f, ar); ai = fmaf(s21.y, 0.26358717679977417f, ai); br = fmaf(d21.x, -0.9646356105804443f, br); bi = fmaf(d21.y, -0.9646356105804443f, bi);
-      ar = fmaf(s22.x, 0.4827921986579895f, ar); ai = fmaf(s22.y, 0.4827921986579895f, ai); br = fmaf(d22.x, -0.8757349252700806f, br); bi = fmaf(d22.y, -0.8757349252700806f, bi);
-      ar = fmaf(s23.x, 0.674983024597168f, ar); ai = fmaf(s23.y, 0.674983024597168f, ai); br = fmaf(d23.x, -0.7378332614898682f, br); bi = fmaf(d23.y, -0.7378332614898682f, bi);
-      ar = fmaf(s24.x, 0.829405665397644f, ar); ai = fmaf(s24.y, 0.829405665397644f, ai); br = fmaf(d24.x, -0.5586467385292053f, br); bi = fmaf(d24.y, -0.5586467385292053f, bi);
-      ar = fmaf(s25.x, 0.9374196529388428f, ar); ai = fmaf(s25.y, 0.9374196529388428f, ai); br = fmaf(d25.x, -0.3482016324996948f, br); bi = fmaf(d25.y, -0.3482016324996948f, bi);
-      ar = fmaf(s26.x, 0.9929810762405396f, ar); ai = fmaf(s26.y, 0.9929810762405396f, ai); br = fmaf(d26.x, -0.11827316880226135f, br); bi = fmaf(d26.y, -0.11827316880226135f, bi);
-      if (!INV) { st(2, make_float2(ar + bi, ai - br)); st(51, make_float2(ar - bi, ai + br)); }
-      else { st(2, make_float2(ar - bi, ai + br)); st(51, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.9374196529388428f, ar); ai = fmaf(s1.y, 0.9374196529388428f, ai); br = fmaf(d1.x, 0.3482016324996948f, br); bi = fmaf(d1.y, 0.3482016324996948f, bi);
-      ar = fmaf(s2.x, 0.7575112581253052f, ar); ai = fmaf(s2.y, 0.7575112581253052f, ai); br = fmaf(d2.x, 0.6528221368789673f, br); bi = fmaf(d2.y, 0.6528221368789673f, bi);
-      ar = fmaf(s3.x, 0.4827921986579895f, ar); ai = fmaf(s3.y, 0.4827921986579895f, ai); br = fmaf(d3.x, 0.8757349252700806f, br); bi = fmaf(d3.y, 0.8757349252700806f, bi);
-      ar = fmaf(s4.x, 0.14764656126499176f, ar); ai = fmaf(s4.y, 0.14764656126499176f, ai); br = fmaf(d4.x, 0.989040195941925f, br); bi = fmaf(d4.y, 0.989040195941925f, bi);
-      ar = fmaf(s5.x, -0.2059786170721054f, ar); ai = fmaf(s5.y, -0.2059786170721054f, ai); br = fmaf(d5.x, 0.9785565137863159f, br); bi = fmaf(d5.y, 0.9785565137863159f, bi);
-      ar = fmaf(s6.x, -0.5338233709335327f, ar); ai = fmaf(s6.y, -0.5338233709335327f, ai); br = fmaf(d6.x, 0.8455960154533386f, br); bi = fmaf(d6.y, 0.8455960154533386f, bi);
-      ar = fmaf(s7.x, -0.794854462146759f, ar); ai = fmaf(s7.y, -0.794854462146759f, ai); br = fmaf(d7.x, 0.6068001389503479f, br); bi = fmaf(d7.y, 0.6068001389503479f, bi);
-      ar = fmaf(s8.x, -0.956400990486145f, ar); ai = fmaf(s8.y, -0.956400990486145f, ai); br = fmaf(d8.x, 0.29205676913261414f, br); bi = fmaf(d8.y, 0.29205676913261414f, bi);
-      ar = fmaf(s9.x, -0.9982437491416931f, ar); ai = fmaf(s9.y, -0.9982437491416931f, ai); br = fmaf(d9.x, -0.05924062803387642f, br); bi = fmaf(d9.y, -0.05924062803387642f, bi);
-      ar = fmaf(s10.x, -0.9151456356048584f, ar); ai = fmaf(s10.y, -0.9151456356048584f, ai); br = fmaf(d10.x, -0.4031234383583069f, br); bi = fmaf(d10.y, -0.4031234383583069f, bi);
-      ar = fmaf(s11.x, -0.7175072431564331f, ar); ai = fmaf(s11.y, -0.7175072431564331f, ai); br = fmaf(d11.x, -0.6965510249137878f, br); bi = fmaf(d11.y, -0.6965510249137878f, bi);
-      ar = fmaf(s12.x, -0.43006521463394165f, ar); ai = fmaf(s12.y, -0.43006521463394165f, ai); br = fmaf(d12.x, -0.9027978181838989f, br); bi = fmaf(d12.y, -0.9027978181838989f, bi);
-      ar = fmaf(s13.x, -0.08879589289426804f, ar); ai = fmaf(s13.y, -0.08879589289426804f, ai); br = fmaf(d13.x, -0.9960498213768005f, br); bi = fmaf(d13.y, -0.9960498213768005f, bi);
-      ar = fmaf(s14.x, 0.26358717679977417f, ar); ai = fmaf(s14.y, 0.26358717679977417f, ai); br = fmaf(d14.x, -0.9646356105804443f, br); bi = fmaf(d14.y, -0.9646356105804443f, bi);
-      ar = fmaf(s15.x, 0.5829795002937317f, ar); ai = fmaf(s15.y, 0.5829795002937317f, ai); br = fmaf(d15.x, -0.8124868869781494f, br); bi = fmaf(d15.y, -0.8124868869781494f, bi);
-      ar = fmaf(s16.x, 0.829405665397644f, ar); ai = fmaf(s16.y, 0.829405665397644f, ai); br = fmaf(d16.x, -0.5586467385292053f, br); bi = fmaf(d16.y, -0.5586467385292053f, bi);
-      ar = fmaf(s17.x, 0.9720228910446167f, ar); ai = fmaf(s17.y, 0.9720228910446167f, ai); br = fmaf(d17.x, -0.2348860502243042f, br); bi = fmaf(d17.y, -0.2348860502243042f, bi);
-      ar = fmaf(s18.x, 0.9929810762405396f, ar); ai = fmaf(s18.y, 0.9929810762405396f, ai); br = fmaf(d18.x, 0.11827316880226135f, br); bi = fmaf(d18.y, 0.11827316880226135f, bi);
-      ar = fmaf(s19.x, 0.8896570801734924f, ar); ai = fmaf(s19.y, 0.8896570801734924f, ai); br = fmaf(d19.x, 0.4566292464733124f, br); bi = fmaf(d19.y, 0.4566292464733124f, bi);
-      ar = fmaf(s20.x, 0.674983024597168f, ar); ai = fmaf(s20.y, 0.674983024597168f, ai); br = fmaf(d20.x, 0.7378332614898682f, br); bi = fmaf(d20.y, 0.7378332614898682f, bi);
-      ar = fmaf(s21.x, 0.3758275806903839f, ar); ai = fmaf(s21.y, 0.3758275806903839f, ai); br = fmaf(d21.x, 0.926689624786377f, br); bi = fmaf(d21.y, 0.926689624786377f, bi);
-      ar = fmaf(s22.x, 0.029633328318595886f, ar); ai = fmaf(s22.y, 0.029633328318595886f, ai); br = fmaf(d22.x, 0.9995608329772949f, br); bi = fmaf(d22.y, 0.9995608329772949f, bi);
-      ar = fmaf(s23.x, -0.3202698528766632f, ar); ai = fmaf(s23.y, -0.3202698528766632f, ai); br = fmaf(d23.x, 0.9473263621330261f, br); bi = fmaf(d23.y, 0.9473263621330261f, bi);
-      ar = fmaf(s24.x, -0.6300878524780273f, ar); ai = fmaf(s24.y, -0.6300878524780273f, ai); br = fmaf(d24.x, 0.7765238881111145f, br); bi = fmaf(d24.y, 0.7765238881111145f, bi);
-      ar = fmaf(s25.x, -0.8610436320304871f, ar); ai = fmaf(s25.y, -0.8610436320304871f, ai); br = fmaf(d25.x, 0.5085310935974121f, br); bi = fmaf(d25.y, 0.5085310935974121f, bi);
-      ar = fmaf(s26.x, -0.9842305779457092f, ar); ai = fmaf(s26.y, -0.9842305779457092f, ai); br = fmaf(d26.x, 0.1768902689218521f, br); bi = fmaf(d26.y, 0.1768902689218521f, bi);
-      if (!INV) { st(3, make_float2(ar + bi, ai - br)); st(50, make_float2(ar - bi, ai + br)); }
-      else { st(3, make_float2(ar - bi, ai + br)); st(50, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.8896570801734924f, ar); ai = fmaf(s1.y, 0.8896570801734924f, ai); br = fmaf(d1.x, 0.4566292464733124f, br); bi = fmaf(d1.y, 0.4566292464733124f, bi);
-      ar = fmaf(s2.x, 0.5829795002937317f, ar); ai = fmaf(s2.y, 0.5829795002937317f, ai); br = fmaf(d2.x, 0.8124868869781494f, br); bi = fmaf(d2.y, 0.8124868869781494f, bi);
-      ar = fmaf(s3.x, 0.14764656126499176f, ar); ai = fmaf(s3.y, 0.14764656126499176f, ai); br = fmaf(d3.x, 0.989040195941925f, br); bi = fmaf(d3.y, 0.989040195941925f, bi);
-      ar = fmaf(s4.x, -0.3202698528766632f, ar); ai = fmaf(s4.y, -0.3202698528766632f, ai); br = fmaf(d4.x, 0.9473263621330261f, br); bi = fmaf(d4.y, 0.9473263621330261f, bi);
-      ar = fmaf(s5.x, -0.7175072431564331f, ar); ai = fmaf(s5.y, -0.7175072431564331f, ai); br = fmaf(d5.x, 0.6965510249137878f, br); bi = fmaf(d5.y, 0.6965510249137878f, bi);
-      ar = fmaf(s6.x, -0.956400990486145f, ar); ai = fmaf(s6.y, -0.956400990486145f, ai); br = fmaf(d6.x, 0.29205676913261414f, br); bi = fmaf(d6.y, 0.29205676913261414f, bi);
-      ar = fmaf(s7.x, -0.9842305779457092f, ar); ai = fmaf(s7.y, -0.9842305779457092f, ai); br = fmaf(d7.x, -0.1768902689218521f, br); bi = fmaf(d7.y, -0.1768902689218521f, bi);
-      ar = fmaf(s8.x, -0.794854462146759f, ar); ai = fmaf(s8.y, -0.794854462146759f, ai); br = fmaf(d8.x, -0.6068001389503479f, br); bi = fmaf(d8.y, -0.6068001389503479f, bi);
-      ar = fmaf(s9.x, -0.43006521463394165f, ar); ai = fmaf(s9.y, -0.43006521463394165f, ai); br = fmaf(d9.x, -0.9027978181838989f, br); bi = fmaf(d9.y, -0.9027978181838989f, bi);
-      ar = fmaf(s10.x, 0.029633328318595886f, ar); ai = fmaf(s10.y, 0.029633328318595886f, ai); br = fmaf(d10.x, -0.9995608329772949f, br); bi = fmaf(d10.y, -0.9995608329772949f, bi);
-      ar = fmaf(s11.x, 0.4827921986579895f, ar); ai = fmaf(s11.y, 0.4827921986579895f, ai); br = fmaf(d11.x, -0.8757349252700806f, br); bi = fmaf(d11.y, -0.8757349252700806f, bi);
-      ar = fmaf(s12.x, 0.829405665397644f, ar); ai = fmaf(s12.y, 0.829405665397644f, ai); br = fmaf(d12.x, -0.5586467385292053f, br); bi = fmaf(d12.y, -0.5586467385292053f, bi);
-      ar = fmaf(s13.x, 0.9929810762405396f, ar); ai = fmaf(s13.y, 0.9929810762405396f, ai); br = fmaf(d13.x, -0.11827316880226135f, br); bi = fmaf(d13.y, -0.11827316880226135f, bi);
-      ar = fmaf(s14.x, 0.9374196529388428f, ar); ai = fmaf(s14.y, 0.9374196529388428f, ai); br = fmaf(d14.x, 0.3482016324996948f, br); bi = fmaf(d14.y, 0.3482016324996948f, bi);
-      ar = fmaf(s15.x, 0.674983024597168f, ar); ai = fmaf(s15.y, 0.674983024597168f, ai); br = fmaf(d15.x, 0.7378332614898682f, br); bi = fmaf(d15.y, 0.7378332614898682f, bi);
-      ar = fmaf(s16.x, 0.26358717679977417f, ar); ai = fmaf(s16.y, 0.26358717679977417f, ai); br = fmaf(d16.x, 0.9646356105804443f, br); bi = fmaf(d16.y, 0.9646356105804443f, bi);
-      ar = fmaf(s17.x, -0.2059786170721054f, ar); ai = fmaf(s17.y, -0.2059786170721054f, ai); br = fmaf(d17.x, 0.9785565137863159f, br); bi = fmaf(d17.y, 0.9785565137863159f, bi);
-      ar = fmaf(s18.x, -0.6300878524780273f, ar); ai = fmaf(s18.y, -0.6300878524780273f, ai); br = fmaf(d18.x, 0.7765238881111145f, br); bi = fmaf(d18.y, 0.7765238881111145f, bi);
-      ar = fmaf(s19.x, -0.9151456356048584f, ar); ai = fmaf(s19.y, -0.9151456356048584f, ai); br = fmaf(d19.x, 0.4031234383583069f, br); bi = fmaf(d19.y, 0.4031234383583069f, bi);
-      ar = fmaf(s20.x, -0.9982437491416931f, ar); ai = fmaf(s20.y, -0.9982437491416931f, ai); br = fmaf(d20.x, -0.05924062803387642f, br); bi = fmaf(d20.y, -0.05924062803387642f, bi);
-      ar = fmaf(s21.x, -0.8610436320304871f, ar); ai = fmaf(s21.y, -0.8610436320304871f, ai); br = fmaf(d21.x, -0.5085310935974121f, br); bi = fmaf(d21.y, -0.5085310935974121f, bi);
-      ar = fmaf(s22.x, -0.5338233709335327f, ar); ai = fmaf(s22.y, -0.5338233709335327f, ai); br = fmaf(d22.x, -0.8455960154533386f, br); bi = fmaf(d22.y, -0.8455960154533386f, bi);
-      ar = fmaf(s23.x, -0.08879589289426804f, ar); ai = fmaf(s23.y, -0.08879589289426804f, ai); br = fmaf(d23.x, -0.9960498213768005f, br); bi = fmaf(d23.y, -0.9960498213768005f, bi);
-      ar = fmaf(s24.x, 0.3758275806903839f, ar); ai = fmaf(s24.y, 0.3758275806903839f, ai); br = fmaf(d24.x, -0.926689624786377f, br); bi = fmaf(d24.y, -0.926689624786377f, bi);
-      ar = fmaf(s25.x, 0.7575112581253052f, ar); ai = fmaf(s25.y, 0.7575112581253052f, ai); br = fmaf(d25.x, -0.6528221368789673f, br); bi = fmaf(d25.y, -0.6528221368789673f, bi);
-      ar = fmaf(s26.x, 0.9720228910446167f, ar); ai = fmaf(s26.y, 0.9720228910446167f, ai); br = fmaf(d26.x, -0.2348860502243042f, br); bi = fmaf(d26.y, -0.2348860502243042f, bi);
-      if (!INV) { st(4, make_float2(ar + bi, ai - br)); st(49, make_float2(ar - bi, ai + br)); }
-      else { st(4, make_float2(ar - bi, ai + br)); st(49, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.829405665397644f, ar); ai = fmaf(s1.y, 0.829405665397644f, ai); br = fmaf(d1.x, 0.5586467385292053f, br); bi = fmaf(d1.y, 0.5586467385292053f, bi);
-      ar = fmaf(s2.x, 0.3758275806903839f, ar); ai = fmaf(s2.y, 0.3758275806903839f, ai); br = fmaf(d2.x, 0.926689624786377f, br); bi = fmaf(d2.y, 0.926689624786377f, bi);
-      ar = fmaf(s3.x, -0.2059786170721054f, ar); ai = fmaf(s3.y, -0.2059786170721054f, ai); br = fmaf(d3.x, 0.9785565137863159f, br); bi = fmaf(d3.y, 0.9785565137863159f, bi);
-      ar = fmaf(s4.x, -0.7175072431564331f, ar); ai = fmaf(s4.y, -0.7175072431564331f, ai); br = fmaf(d4.x, 0.6965510249137878f, br); bi = fmaf(d4.y, 0.6965510249137878f, bi);
-      ar = fmaf(s5.x, -0.9842305779457092f, ar); ai = fmaf(s5.y, -0.9842305779457092f, ai); br = fmaf(d5.x, 0.1768902689218521f, br); bi = fmaf(d5.y, 0.1768902689218521f, bi);
-      ar = fmaf(s6.x, -0.9151456356048584f, ar); ai = fmaf(s6.y, -0.9151456356048584f, ai); br = fmaf(d6.x, -0.4031234383583069f, br); bi = fmaf(d6.y, -0.4031234383583069f, bi);
-      ar = fmaf(s7.x, -0.5338233709335327f, ar); ai = fmaf(s7.y, -0.5338233709335327f, ai); br = fmaf(d7.x, -0.8455960154533386f, br); bi = fmaf(d7.y, -0.8455960154533386f, bi);
-      ar = fmaf(s8.x, 0.029633328318595886f, ar); ai = fmaf(s8.y, 0.029633328318595886f, ai); br = fmaf(d8.x, -0.9995608329772949f, br); bi = fmaf(d8.y, -0.9995608329772949f, bi);
-      ar = fmaf(s9.x, 0.5829795002937317f, ar); ai = fmaf(s9.y, 0.5829795002937317f, ai); br = fmaf(d9.x, -0.8124868869781494f, br); bi = fmaf(d9.y, -0.8124868869781494f, bi);
-      ar = fmaf(s10.x, 0.9374196529388428f, ar); ai = fmaf(s10.y, 0.9374196529388428f, ai); br = fmaf(d10.x, -0.3482016324996948f, br); bi = fmaf(d10.y, -0.3482016324996948f, bi);
-      ar = fmaf(s11.x, 0.9720228910446167f, ar); ai = fmaf(s11.y, 0.9720228910446167f, ai); br = fmaf(d11.x, 0.2348860502243042f, br); bi = fmaf(d11.y, 0.2348860502243042f, bi);
-      ar = fmaf(s12.x, 0.674983024597168f, ar); ai = fmaf(s12.y, 0.674983024597168f, ai); br = fmaf(d12.x, 0.7378332614898682f, br); bi = fmaf(d12.y, 0.7378332614898682f, bi);
-      ar = fmaf(s13.x, 0.14764656126499176f, ar); ai = fmaf(s13.y, 0.14764656126499176f, ai); br = fmaf(d13.x, 0.989040195941925f, br); bi = fmaf(d13.y, 0.989040195941925f, bi);
-      ar = fmaf(s14.x, -0.43006521463394165f, ar); ai = fmaf(s14.y, -0.43006521463394165f, ai); br = fmaf(d14.x, 0.9027978181838989f, br); bi = fmaf(d14.y, 0.9027978181838989f, bi);
-      ar = fmaf(s15.x, -0.8610436320304871f, ar); ai = fmaf(s15.y, -0.8610436320304871f, ai); br = fmaf(d15.x, 0.5085310935974121f, br); bi = fmaf(d15.y, 0.5085310935974121f, bi);
-      ar = fmaf(s16.x, -0.9982437491416931f, ar); ai = fmaf(s16.y, -0.9982437491416931f, ai); br = fmaf(d16.x, -0.05924062803387642f, br); bi = fmaf(d16.y, -0.05924062803387642f, bi);
-      ar = fmaf(s17.x, -0.794854462146759f, ar); ai = fmaf(s17.y, -0.794854462146759f, ai); br = fmaf(d17.x, -0.6068001389503479f, br); bi = fmaf(d17.y, -0.6068001389503479f, bi);
-      ar = fmaf(s18.x, -0.3202698528766632f, ar); ai = fmaf(s18.y, -0.3202698528766632f, ai); br = fmaf(d18.x, -0.9473263621330261f, br); bi = fmaf(d18.y, -0.9473263621330261f, bi);
-      ar = fmaf(s19.x, 0.26358717679977417f, ar); ai = fmaf(s19.y, 0.26358717679977417f, ai); br = fmaf(d19.x, -0.9646356105804443f, br); bi = fmaf(d19.y, -0.9646356105804443f, bi);
-      ar = fmaf(s20.x, 0.7575112581253052f, ar); ai = fmaf(s20.y, 0.7575112581253052f, ai); br = fmaf(d20.x, -0.6528221368789673f, br); bi = fmaf(d20.y, -0.6528221368789673f, bi);
-      ar = fmaf(s21.x, 0.9929810762405396f, ar); ai = fmaf(s21.y, 0.9929810762405396f, ai); br = fmaf(d21.x, -0.11827316880226135f, br); bi = fmaf(d21.y, -0.11827316880226135f, bi);
-      ar = fmaf(s22.x, 0.8896570801734924f, ar); ai = fmaf(s22.y, 0.8896570801734924f, ai); br = fmaf(d22.x, 0.4566292464733124f, br); bi = fmaf(d22.y, 0.4566292464733124f, bi);
-      ar = fmaf(s23.x, 0.4827921986579895f, ar); ai = fmaf(s23.y, 0.4827921986579895f, ai); br = fmaf(d23.x, 0.8757349252700806f, br); bi = fmaf(d23.y, 0.8757349252700806f, bi);
-      ar = fmaf(s24.x, -0.08879589289426804f, ar); ai = fmaf(s24.y, -0.08879589289426804f, ai); br = fmaf(d24.x, 0.9960498213768005f, br); bi = fmaf(d24.y, 0.9960498213768005f, bi);
-      ar = fmaf(s25.x, -0.6300878524780273f, ar); ai = fmaf(s25.y, -0.6300878524780273f, ai); br = fmaf(d25.x, 0.7765238881111145f, br); bi = fmaf(d25.y, 0.7765238881111145f, bi);
-      ar = fmaf(s26.x, -0.956400990486145f, ar); ai = fmaf(s26.y, -0.956400990486145f, ai); br = fmaf(d26.x, 0.29205676913261414f, br); bi = fmaf(d26.y, 0.29205676913261414f, bi);
-      if (!INV) { st(5, make_float2(ar + bi, ai - br)); st(48, make_float2(ar - bi, ai + br)); }
-      else { st(5, make_float2(ar - bi, ai + br)); st(48, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.7575112581253052f, ar); ai = fmaf(s1.y, 0.7575112581253052f, ai); br = fmaf(d1.x, 0.6528221368789673f, br); bi = fmaf(d1.y, 0.6528221368789673f, bi);
-      ar = fmaf(s2.x, 0.14764656126499176f, ar); ai = fmaf(s2.y, 0.14764656126499176f, ai); br = fmaf(d2.x, 0.989040195941925f, br); bi = fmaf(d2.y, 0.989040195941925f, bi);
-      ar = fmaf(s3.x, -0.5338233709335327f, ar); ai = fmaf(s3.y, -0.5338233709335327f, ai); br = fmaf(d3.x, 0.8455960154533386f, br); bi = fmaf(d3.y, 0.8455960154533386f, bi);
-      ar = fmaf(s4.x, -0.956400990486145f, ar); ai = fmaf(s4.y, -0.956400990486145f, ai); br = fmaf(d4.x, 0.29205676913261414f, br); bi = fmaf(d4.y, 0.29205676913261414f, bi);
-      ar = fmaf(s5.x, -0.9151456356048584f, ar); ai = fmaf(s5.y, -0.9151456356048584f, ai); br = fmaf(d5.x, -0.4031234383583069f, br); bi = fmaf(d5.y, -0.4031234383583069f, bi);
-      ar = fmaf(s6.x, -0.43006521463394165f, ar); ai = fmaf(s6.y, -0.43006521463394165f, ai); br = fmaf(d6.x, -0.9027978181838989f, br); bi = fmaf(d6.y, -0.9027978181838989f, bi);
-      ar = fmaf(s7.x, 0.26358717679977417f, ar); ai = fmaf(s7.y, 0.26358717679977417f, ai); br = fmaf(d7.x, -0.9646356105804443f, br); bi = fmaf(d7.y, -0.9646356105804443f, bi);
-      ar = fmaf(s8.x, 0.829405665397644f, ar); ai = fmaf(s8.y, 0.829405665397644f, ai); br = fmaf(d8.x, -0.5586467385292053f, br); bi = fmaf(d8.y, -0.5586467385292053f, bi);
-      ar = fmaf(s9.x, 0.9929810762405396f, ar); ai = fmaf(s9.y, 0.9929810762405396f, ai); br = fmaf(d9.x, 0.11827316880226135f, br); bi = fmaf(d9.y, 0.11827316880226135f, bi);
-      ar = fmaf(s10.x, 0.674983024597168f, ar); ai = fmaf(s10.y, 0.674983024597168f, ai); br = fmaf(d10.x, 0.7378332614898682f, br); bi = fmaf(d10.y, 0.7378332614898682f, bi);
-      ar = fmaf(s11.x, 0.029633328318595886f, ar); ai = fmaf(s11.y, 0.029633328318595886f, ai); br = fmaf(d11.x, 0.9995608329772949f, br); bi = fmaf(d11.y, 0.9995608329772949f, bi);
-      ar = fmaf(s12.x, -0.6300878524780273f, ar); ai = fmaf(s12.y, -0.6300878524780273f, ai); br = fmaf(d12.x, 0.7765238881111145f, br); bi = fmaf(d12.y, 0.7765238881111145f, bi);
-      ar = fmaf(s13.x, -0.9842305779457092f, ar); ai = fmaf(s13.y, -0.9842305779457092f, ai); br = fmaf(d13.x, 0.1768902689218521f, br); bi = fmaf(d13.y, 0.1768902689218521f, bi);
-      ar = fmaf(s14.x, -0.8610436320304871f, ar); ai = fmaf(s14.y, -0.8610436320304871f, ai); br = fmaf(d14.x, -0.5085310935974121f, br); bi = fmaf(d14.y, -0.5085310935974121f, bi);
-      ar = fmaf(s15.x, -0.3202698528766632f, ar); ai = fmaf(s15.y, -0.3202698528766632f, ai); br = fmaf(d15.x, -0.9473263621330261f, br); bi = fmaf(d15.y, -0.9473263621330261f, bi);
-      ar = fmaf(s16.x, 0.3758275806903839f, ar); ai = fmaf(s16.y, 0.3758275806903839f, ai); br = fmaf(d16.x, -0.926689624786377f, br); bi = fmaf(d16.y, -0.926689624786377f, bi);
-      ar = fmaf(s17.x, 0.8896570801734924f, ar); ai = fmaf(s17.y, 0.8896570801734924f, ai); br = fmaf(d17.x, -0.4566292464733124f, br); bi = fmaf(d17.y, -0.4566292464733124f, bi);
-      ar = fmaf(s18.x, 0.9720228910446167f, ar); ai = fmaf(s18.y, 0.9720228910446167f, ai); br = fmaf(d18.x, 0.2348860502243042f, br); bi = fmaf(d18.y, 0.2348860502243042f, bi);
-      ar = fmaf(s19.x, 0.5829795002937317f, ar); ai = fmaf(s19.y, 0.5829795002937317f, ai); br = fmaf(d19.x, 0.8124868869781494f, br); bi = fmaf(d19.y, 0.8124868869781494f, bi);
-      ar = fmaf(s20.x, -0.08879589289426804f, ar); ai = fmaf(s20.y, -0.08879589289426804f, ai); br = fmaf(d20.x, 0.9960498213768005f, br); bi = fmaf(d20.y, 0.9960498213768005f, bi);
-      ar = fmaf(s21.x, -0.7175072431564331f, ar); ai = fmaf(s21.y, -0.7175072431564331f, ai); br = fmaf(d21.x, 0.6965510249137878f, br); bi = fmaf(d21.y, 0.6965510249137878f, bi);
-      ar = fmaf(s22.x, -0.9982437491416931f, ar); ai = fmaf(s22.y, -0.9982437491416931f, ai); br = fmaf(d22.x, 0.05924062803387642f, br); bi = fmaf(d22.y, 0.05924062803387642f, bi);
-      ar = fmaf(s23.x, -0.794854462146759f, ar); ai = fmaf(s23.y, -0.794854462146759f, ai); br = fmaf(d23.x, -0.6068001389503479f, br); bi = fmaf(d23.y, -0.6068001389503479f, bi);
-      ar = fmaf(s24.x, -0.2059786170721054f, ar); ai = fmaf(s24.y, -0.2059786170721054f, ai); br = fmaf(d24.x, -0.9785565137863159f, br); bi = fmaf(d24.y, -0.9785565137863159f, bi);
-      ar = fmaf(s25.x, 0.4827921986579895f, ar); ai = fmaf(s25.y, 0.4827921986579895f, ai); br = fmaf(d25.x, -0.8757349252700806f, br); bi = fmaf(d25.y, -0.8757349252700806f, bi);
-      ar = fmaf(s26.x, 0.9374196529388428f, ar); ai = fmaf(s26.y, 0.9374196529388428f, ai); br = fmaf(d26.x, -0.3482016324996948f, br); bi = fmaf(d26.y, -0.3482016324996948f, bi);
-      if (!INV) { st(6, make_float2(ar + bi, ai - br)); st(47, make_float2(ar - bi, ai + br)); }
-      else { st(6, make_float2(ar - bi, ai + br)); st(47, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.674983024597168f, ar); ai = fmaf(s1.y, 0.674983024597168f, ai); br = fmaf(d1.x, 0.7378332614898682f, br); bi = fmaf(d1.y, 0.7378332614898682f, bi);
-      ar = fmaf(s2.x, -0.08879589289426804f, ar); ai = fmaf(s2.y, -0.08879589289426804f, ai); br = fmaf(d2.x, 0.9960498213768005f, br); bi = fmaf(d2.y, 0.9960498213768005f, bi);
-      ar = fmaf(s3.x, -0.794854462146759f, ar); ai = fmaf(s3.y, -0.794854462146759f, ai); br = fmaf(d3.x, 0.6068001389503479f, br); bi = fmaf(d3.y, 0.6068001389503479f, bi);
-      ar = fmaf(s4.x, -0.9842305779457092f, ar); ai = fmaf(s4.y, -0.9842305779457092f, ai); br = fmaf(d4.x, -0.1768902689218521f, br); bi = fmaf(d4.y, -0.1768902689218521f, bi);
-      ar = fmaf(s5.x, -0.5338233709335327f, ar); ai = fmaf(s5.y, -0.5338233709335327f, ai); br = fmaf(d5.x, -0.8455960154533386f, br); bi = fmaf(d5.y, -0.8455960154533386f, bi);
-      ar = fmaf(s6.x, 0.26358717679977417f, ar); ai = fmaf(s6.y, 0.26358717679977417f, ai); br = fmaf(d6.x, -0.9646356105804443f, br); bi = fmaf(d6.y, -0.9646356105804443f, bi);
-      ar = fmaf(s7.x, 0.8896570801734924f, ar); ai = fmaf(s7.y, 0.8896570801734924f, ai); br = fmaf(d7.x, -0.4566292464733124f, br); bi = fmaf(d7.y, -0.4566292464733124f, bi);
-      ar = fmaf(s8.x, 0.9374196529388428f, ar); ai = fmaf(s8.y, 0.9374196529388428f, ai); br = fmaf(d8.x, 0.3482016324996948f, br); bi = fmaf(d8.y, 0.3482016324996948f, bi);
-      ar = fmaf(s9.x, 0.3758275806903839f, ar); ai = fmaf(s9.y, 0.3758275806903839f, ai); br = fmaf(d9.x, 0.926689624786377f, br); bi = fmaf(d9.y, 0.926689624786377f, bi);
-      ar = fmaf(s10.x, -0.43006521463394165f, ar); ai = fmaf(s10.y, -0.43006521463394165f, ai); br = fmaf(d10.x, 0.9027978181838989f, br); bi = fmaf(d10.y, 0.9027978181838989f, bi);
-      ar = fmaf(s11.x, -0.956400990486145f, ar); ai = fmaf(s11.y, -0.956400990486145f, ai); br = fmaf(d11.x, 0.29205676913261414f, br); bi = fmaf(d11.y, 0.29205676913261414f, bi);
-      ar = fmaf(s12.x, -0.8610436320304871f, ar); ai = fmaf(s12.y, -0.8610436320304871f, ai); br = fmaf(d12.x, -0.5085310935974121f, br); bi = fmaf(d12.y, -0.5085310935974121f, bi);
-      ar = fmaf(s13.x, -0.2059786170721054f, ar); ai = fmaf(s13.y, -0.2059786170721054f, ai); br = fmaf(d13.x, -0.9785565137863159f, br); bi = fmaf(d13.y, -0.9785565137863159f, bi);
-      ar = fmaf(s14.x, 0.5829795002937317f, ar); ai = fmaf(s14.y, 0.5829795002937317f, ai); br = fmaf(d14.x, -0.8124868869781494f, br); bi = fmaf(d14.y, -0.8124868869781494f, bi);
-      ar = fmaf(s15.x, 0.9929810762405396f, ar); ai = fmaf(s15.y, 0.9929810762405396f, ai); br = fmaf(d15.x, -0.11827316880226135f, br); bi = fmaf(d15.y, -0.11827316880226135f, bi);
-      ar = fmaf(s16.x, 0.7575112581253052f, ar); ai = fmaf(s16.y, 0.7575112581253052f, ai); br = fmaf(d16.x, 0.6528221368789673f, br); bi = fmaf(d16.y, 0.6528221368789673f, bi);
-      ar = fmaf(s17.x, 0.029633328318595886f, ar); ai = fmaf(s17.y, 0.029633328318595886f, ai); br = fmaf(d17.x, 0.9995608329772949f, br); bi = fmaf(d17.y, 0.9995608329772949f, bi);
-      ar = fmaf(s18.x, -0.7175072431564331f, ar); ai = fmaf(s18.y, -0.7175072431564331f, ai); br = fmaf(d18.x, 0.6965510249137878f, br); bi = fmaf(d18.y, 0.6965510249137878f, bi);
-      ar = fmaf(s19.x, -0.9982437491416931f, ar); ai = fmaf(s19.y, -0.9982437491416931f, ai); br = fmaf(d19.x, -0.05924062803387642f, br); bi = fmaf(d19.y, -0.05924062803387642f, bi);
-      ar = fmaf(s20.x, -0.6300878524780273f, ar); ai = fmaf(s20.y, -0.6300878524780273f, ai); br = fmaf(d20.x, -0.7765238881111145f, br); bi = fmaf(d20.y, -0.7765238881111145f, bi);
-      ar = fmaf(s21.x, 0.14764656126499176f, ar); ai = fmaf(s21.y, 0.14764656126499176f, ai); br = fmaf(d21.x, -0.989040195941925f, br); bi = fmaf(d21.y, -0.989040195941925f, bi);
-      ar = fmaf(s22.x, 0.829405665397644f, ar); ai = fmaf(s22.y, 0.829405665397644f, ai); br = fmaf(d22.x, -0.5586467385292053f, br); bi = fmaf(d22.y, -0.5586467385292053f, bi);
-      ar = fmaf(s23.x, 0.9720228910446167f, ar); ai = fmaf(s23.y, 0.9720228910446167f, ai); br = fmaf(d23.x, 0.2348860502243042f, br); bi = fmaf(d23.y, 0.2348860502243042f, bi);
-      ar = fmaf(s24.x, 0.4827921986579895f, ar); ai = fmaf(s24.y, 0.4827921986579895f, ai); br = fmaf(d24.x, 0.8757349252700806f, br); bi = fmaf(d24.y, 0.8757349252700806f, bi);
-      ar = fmaf(s25.x, -0.3202698528766632f, ar); ai = fmaf(s25.y, -0.3202698528766632f, ai); br = fmaf(d25.x, 0.9473263621330261f, br); bi = fmaf(d25.y, 0.9473263621330261f, bi);
-      ar = fmaf(s26.x, -0.9151456356048584f, ar); ai = fmaf(s26.y, -0.9151456356048584f, ai); br = fmaf(d26.x, 0.4031234383583069f, br); bi = fmaf(d26.y, 0.4031234383583069f, bi);
-      if (!INV) { st(7, make_float2(ar + bi, ai - br)); st(46, make_float2(ar - bi, ai + br)); }
-      else { st(7, make_float2(ar - bi, ai + br)); st(46, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.5829795002937317f, ar); ai = fmaf(s1.y, 0.5829795002937317f, ai); br = fmaf(d1.x, 0.8124868869781494f, br); bi = fmaf(d1.y, 0.8124868869781494f, bi);
-      ar = fmaf(s2.x, -0.3202698528766632f, ar); ai = fmaf(s2.y, -0.3202698528766632f, ai); br = fmaf(d2.x, 0.9473263621330261f, br); bi = fmaf(d2.y, 0.9473263621330261f, bi);
-      ar = fmaf(s3.x, -0.956400990486145f, ar); ai = fmaf(s3.y, -0.956400990486145f, ai); br = fmaf(d3.x, 0.29205676913261414f, br); bi = fmaf(d3.y, 0.29205676913261414f, bi);
-      ar = fmaf(s4.x, -0.794854462146759f, ar); ai = fmaf(s4.y, -0.794854462146759f, ai); br = fmaf(d4.x, -0.6068001389503479f, br); bi = fmaf(d4.y, -0.6068001389503479f, bi);
-      ar = fmaf(s5.x, 0.029633328318595886f, ar); ai = fmaf(s5.y, 0.029633328318595886f, ai); br = fmaf(d5.x, -0.9995608329772949f, br); bi = fmaf(d5.y, -0.9995608329772949f, bi);
-      ar = fmaf(s6.x, 0.829405665397644f, ar); ai = fmaf(s6.y, 0.829405665397644f, ai); br = fmaf(d6.x, -0.5586467385292053f, br); bi = fmaf(d6.y, -0.5586467385292053f, bi);
-      ar = fmaf(s7.x, 0.9374196529388428f, ar); ai = fmaf(s7.y, 0.9374196529388428f, ai); br = fmaf(d7.x, 0.3482016324996948f, br); bi = fmaf(d7.y, 0.3482016324996948f, bi);
-      ar = fmaf(s8.x, 0.26358717679977417f, ar); ai = fmaf(s8.y, 0.26358717679977417f, ai); br = fmaf(d8.x, 0.9646356105804443f, br); bi = fmaf(d8.y, 0.9646356105804443f, bi);
-      ar = fmaf(s9.x, -0.6300878524780273f, ar); ai = fmaf(s9.y, -0.6300878524780273f, ai); br = fmaf(d9.x, 0.7765238881111145f, br); bi = fmaf(d9.y, 0.7765238881111145f, bi);
-      ar = fmaf(s10.x, -0.9982437491416931f, ar); ai = fmaf(s10.y, -0.9982437491416931f, ai); br = fmaf(d10.x, -0.05924062803387642f, br); bi = fmaf(d10.y, -0.05924062803387642f, bi);
-      ar = fmaf(s11.x, -0.5338233709335327f, ar); ai = fmaf(s11.y, -0.5338233709335327f, ai); br = fmaf(d11.x, -0.8455960154533386f, br); bi = fmaf(d11.y, -0.8455960154533386f, bi);
-      ar = fmaf(s12.x, 0.3758275806903839f, ar); ai = fmaf(s12.y, 0.3758275806903839f, ai); br = fmaf(d12.x, -0.926689624786377f, br); bi = fmaf(d12.y, -0.926689624786377f, bi);
-      ar = fmaf(s13.x, 0.9720228910446167f, ar); ai = fmaf(s13.y, 0.9720228910446167f, ai); br = fmaf(d13.x, -0.2348860502243042f, br); bi = fmaf(d13.y, -0.2348860502243042f, bi);
-      ar = fmaf(s14.x, 0.7575112581253052f, ar); ai = fmaf(s14.y, 0.7575112581253052f, ai); br = fmaf(d14.x, 0.6528221368789673f, br); bi = fmaf(d14.y, 0.6528221368789673f, bi);
-      ar = fmaf(s15.x, -0.08879589289426804f, ar); ai = fmaf(s15.y, -0.08879589289426804f, ai); br = fmaf(d15.x, 0.9960498213768005f, br); bi = fmaf(d15.y, 0.9960498213768005f, bi);
-      ar = fmaf(s16.x, -0.8610436320304871f, ar); ai = fmaf(s16.y, -0.8610436320304871f, ai); br = fmaf(d16.x, 0.5085310935974121f, br); bi = fmaf(d16.y, 0.5085310935974121f, bi);
-      ar = fmaf(s17.x, -0.9151456356048584f, ar); ai = fmaf(s17.y, -0.9151456356048584f, ai); br = fmaf(d17.x, -0.4031234383583069f, br); bi = fmaf(d17.y, -0.4031234383583069f, bi);
-      ar = fmaf(s18.x, -0.2059786170721054f, ar); ai = fmaf(s18.y, -0.2059786170721054f, ai); br = fmaf(d18.x, -0.9785565137863159f, br); bi = fmaf(d18.y, -0.9785565137863159f, bi);
-      ar = fmaf(s19.x, 0.674983024597168f, ar); ai = fmaf(s19.y, 0.674983024597168f, ai); br = fmaf(d19.x, -0.7378332614898682f, br); bi = fmaf(d19.y, -0.7378332614898682f, bi);
-      ar = fmaf(s20.x, 0.9929810762405396f, ar); ai = fmaf(s20.y, 0.9929810762405396f, ai); br = fmaf(d20.x, 0.11827316880226135f, br); bi = fmaf(d20.y, 0.11827316880226135f, bi);
-      ar = fmaf(s21.x, 0.4827921986579895f, ar); ai = fmaf(s21.y, 0.4827921986579895f, ai); br = fmaf(d21.x, 0.8757349252700806f, br); bi = fmaf(d21.y, 0.8757349252700806f, bi);
-      ar = fmaf(s22.x, -0.43006521463394165f, ar); ai = fmaf(s22.y, -0.43006521463394165f, ai); br = fmaf(d22.x, 0.9027978181838989f, br); bi = fmaf(d22.y, 0.9027978181838989f, bi);
-      ar = fmaf(s23.x, -0.9842305779457092f, ar); ai = fmaf(s23.y, -0.9842305779457092f, ai); br = fmaf(d23.x, 0.1768902689218521f, br); bi = fmaf(d23.y, 0.1768902689218521f, bi);
-      ar = fmaf(s24.x, -0.7175072431564331f, ar); ai = fmaf(s24.y, -0.7175072431564331f, ai); br = fmaf(d24.x, -0.6965510249137878f, br); bi = fmaf(d24.y, -0.6965510249137878f, bi);
-      ar = fmaf(s25.x, 0.14764656126499176f, ar); ai = fmaf(s25.y, 0.14764656126499176f, ai); br = fmaf(d25.x, -0.989040195941925f, br); bi = fmaf(d25.y, -0.989040195941925f, bi);
-      ar = fmaf(s26.x, 0.8896570801734924f, ar); ai = fmaf(s26.y, 0.8896570801734924f, ai); br = fmaf(d26.x, -0.4566292464733124f, br); bi = fmaf(d26.y, -0.4566292464733124f, bi);
-      if (!INV) { st(8, make_float2(ar + bi, ai - br)); st(45, make_float2(ar - bi, ai + br)); }
-      else { st(8, make_float2(ar - bi, ai + br)); st(45, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.4827921986579895f, ar); ai = fmaf(s1.y, 0.4827921986579895f, ai); br = fmaf(d1.x, 0.8757349252700806f, br); bi = fmaf(d1.y, 0.8757349252700806f, bi);
-      ar = fmaf(s2.x, -0.5338233709335327f, ar); ai = fmaf(s2.y, -0.5338233709335327f, ai); br = fmaf(d2.x, 0.8455960154533386f, br); bi = fmaf(d2.y, 0.8455960154533386f, bi);
-      ar = fmaf(s3.x, -0.9982437491416931f, ar); ai = fmaf(s3.y, -0.9982437491416931f, ai); br = fmaf(d3.x, -0.05924062803387642f, br); bi = fmaf(d3.y, -0.05924062803387642f, bi);
-      ar = fmaf(s4.x, -0.43006521463394165f, ar); ai = fmaf(s4.y, -0.43006521463394165f, ai); br = fmaf(d4.x, -0.9027978181838989f, br); bi = fmaf(d4.y, -0.9027978181838989f, bi);
-      ar = fmaf(s5.x, 0.5829795002937317f, ar); ai = fmaf(s5.y, 0.5829795002937317f, ai); br = fmaf(d5.x, -0.8124868869781494f, br); bi = fmaf(d5.y, -0.8124868869781494f, bi);
-      ar = fmaf(s6.x, 0.9929810762405396f, ar); ai = fmaf(s6.y, 0.9929810762405396f, ai); br = fmaf(d6.x, 0.11827316880226135f, br); bi = fmaf(d6.y, 0.11827316880226135f, bi);
-      ar = fmaf(s7.x, 0.3758275806903839f, ar); ai = fmaf(s7.y, 0.3758275806903839f, ai); br = fmaf(d7.x, 0.926689624786377f, br); bi = fmaf(d7.y, 0.926689624786377f, bi);
-      ar = fmaf(s8.x, -0.6300878524780273f, ar); ai = fmaf(s8.y, -0.6300878524780273f, ai); br = fmaf(d8.x, 0.7765238881111145f, br); bi = fmaf(d8.y, 0.7765238881111145f, bi);
-      ar = fmaf(s9.x, -0.9842305779457092f, ar); ai = fmaf(s9.y, -0.9842305779457092f, ai); br = fmaf(d9.x, -0.1768902689218521f, br); bi = fmaf(d9.y, -0.1768902689218521f, bi);
-      ar = fmaf(s10.x, -0.3202698528766632f, ar); ai = fmaf(s10.y, -0.3202698528766632f, ai); br = fmaf(d10.x, -0.9473263621330261f, br); bi = fmaf(d10.y, -0.9473263621330261f, bi);
-      ar = fmaf(s11.x, 0.674983024597168f, ar); ai = fmaf(s11.y, 0.674983024597168f, ai); br = fmaf(d11.x, -0.7378332614898682f, br); bi = fmaf(d11.y, -0.7378332614898682f, bi);
-      ar = fmaf(s12.x, 0.9720228910446167f, ar); ai = fmaf(s12.y, 0.9720228910446167f, ai); br = fmaf(d12.x, 0.2348860502243042f, br); bi = fmaf(d12.y, 0.2348860502243042f, bi);
-      ar = fmaf(s13.x, 0.26358717679977417f, ar); ai = fmaf(s13.y, 0.26358717679977417f, ai); br = fmaf(d13.x, 0.9646356105804443f, br); bi = fmaf(d13.y, 0.9646356105804443f, bi);
-      ar = fmaf(s14.x, -0.7175072431564331f, ar); ai = fmaf(s14.y, -0.7175072431564331f, ai); br = fmaf(d14.x, 0.6965510249137878f, br); bi = fmaf(d14.y, 0.6965510249137878f, bi);
-      ar = fmaf(s15.x, -0.956400990486145f, ar); ai = fmaf(s15.y, -0.956400990486145f, ai); br = fmaf(d15.x, -0.29205676913261414f, br); bi = fmaf(d15.y, -0.29205676913261414f, bi);
-      ar = fmaf(s16.x, -0.2059786170721054f, ar); ai = fmaf(s16.y, -0.2059786170721054f, ai); br = fmaf(d16.x, -0.9785565137863159f, br); bi = fmaf(d16.y, -0.9785565137863159f, bi);
-      ar = fmaf(s17.x, 0.7575112581253052f, ar); ai = fmaf(s17.y, 0.7575112581253052f, ai); br = fmaf(d17.x, -0.6528221368789673f, br); bi = fmaf(d17.y, -0.6528221368789673f, bi);
-      ar = fmaf(s18.x, 0.9374196529388428f, ar); ai = fmaf(s18.y, 0.9374196529388428f, ai); br = fmaf(d18.x, 0.3482016324996948f, br); bi = fmaf(d18.y, 0.3482016324996948f, bi);
-      ar = fmaf(s19.x, 0.14764656126499176f, ar); ai = fmaf(s19.y, 0.14764656126499176f, ai); br = fmaf(d19.x, 0.989040195941925f, br); bi = fmaf(d19.y, 0.989040195941925f, bi);
-      ar = fmaf(s20.x, -0.794854462146759f, ar); ai = fmaf(s20.y, -0.794854462146759f, ai); br = fmaf(d20.x, 0.6068001389503479f, br); bi = fmaf(d20.y, 0.6068001389503479f, bi);
-      ar = fmaf(s21.x, -0.9151456356048584f, ar); ai = fmaf(s21.y, -0.9151456356048584f, ai); br = fmaf(d21.x, -0.4031234383583069f, br); bi = fmaf(d21.y, -0.4031234383583069f, bi);
-      ar = fmaf(s22.x, -0.08879589289426804f, ar); ai = fmaf(s22.y, -0.08879589289426804f, ai); br = fmaf(d22.x, -0.9960498213768005f, br); bi = fmaf(d22.y, -0.9960498213768005f, bi);
-      ar = fmaf(s23.x, 0.829405665397644f, ar); ai = fmaf(s23.y, 0.829405665397644f, ai); br = fmaf(d23.x, -0.5586467385292053f, br); bi = fmaf(d23.y, -0.5586467385292053f, bi);
-      ar = fmaf(s24.x, 0.8896570801734924f, ar); ai = fmaf(s24.y, 0.8896570801734924f, ai); br = fmaf(d24.x, 0.4566292464733124f, br); bi = fmaf(d24.y, 0.4566292464733124f, bi);
-      ar = fmaf(s25.x, 0.029633328318595886f, ar); ai = fmaf(s25.y, 0.029633328318595886f, ai); br = fmaf(d25.x, 0.9995608329772949f, br); bi = fmaf(d25.y, 0.9995608329772949f, bi);
-      ar = fmaf(s26.x, -0.8610436320304871f, ar); ai = fmaf(s26.y, -0.8610436320304871f, ai); br = fmaf(d26.x, 0.5085310935974121f, br); bi = fmaf(d26.y, 0.5085310935974121f, bi);
-      if (!INV) { st(9, make_float2(ar + bi, ai - br)); st(44, make_float2(ar - bi, ai + br)); }
-      else { st(9, make_float2(ar - bi, ai + br)); st(44, make_float2(ar + bi, ai - br)); }
-    }
-    break;
-  }
-  case 1: {
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.3758275806903839f, ar); ai = fmaf(s1.y, 0.3758275806903839f, ai); br = fmaf(d1.x, 0.926689624786377f, br); bi = fmaf(d1.y, 0.926689624786377f, bi);
-      ar = fmaf(s2.x, -0.7175072431564331f, ar); ai = fmaf(s2.y, -0.7175072431564331f, ai); br = fmaf(d2.x, 0.6965510249137878f, br); bi = fmaf(d2.y, 0.6965510249137878f, bi);
-      ar = fmaf(s3.x, -0.9151456356048584f, ar); ai = fmaf(s3.y, -0.9151456356048584f, ai); br = fmaf(d3.x, -0.4031234383583069f, br); bi = fmaf(d3.y, -0.4031234383583069f, bi);
-      ar = fmaf(s4.x, 0.029633328318595886f, ar); ai = fmaf(s4.y, 0.029633328318595886f, ai); br = fmaf(d4.x, -0.9995608329772949f, br); bi = fmaf(d4.y, -0.9995608329772949f, bi);
-      ar = fmaf(s5.x, 0.9374196529388428f, ar); ai = fmaf(s5.y, 0.9374196529388428f, ai); br = fmaf(d5.x, -0.3482016324996948f, br); bi = fmaf(d5.y, -0.3482016324996948f, bi);
-      ar = fmaf(s6.x, 0.674983024597168f, ar); ai = fmaf(s6.y, 0.674983024597168f, ai); br = fmaf(d6.x, 0.7378332614898682f, br); bi = fmaf(d6.y, 0.7378332614898682f, bi);
-      ar = fmaf(s7.x, -0.43006521463394165f, ar); ai = fmaf(s7.y, -0.43006521463394165f, ai); br = fmaf(d7.x, 0.9027978181838989f, br); bi = fmaf(d7.y, 0.9027978181838989f, bi);
-      ar = fmaf(s8.x, -0.9982437491416931f, ar); ai = fmaf(s8.y, -0.9982437491416931f, ai); br = fmaf(d8.x, -0.05924062803387642f, br); bi = fmaf(d8.y, -0.05924062803387642f, bi);
-      ar = fmaf(s9.x, -0.3202698528766632f, ar); ai = fmaf(s9.y, -0.3202698528766632f, ai); br = fmaf(d9.x, -0.9473263621330261f, br); bi = fmaf(d9.y, -0.9473263621330261f, bi);
-      ar = fmaf(s10.x, 0.7575112581253052f, ar); ai = fmaf(s10.y, 0.7575112581253052f, ai); br = fmaf(d10.x, -0.6528221368789673f, br); bi = fmaf(d10.y, -0.6528221368789673f, bi);
-      ar = fmaf(s11.x, 0.8896570801734924f, ar); ai = fmaf(s11.y, 0.8896570801734924f, ai); br = fmaf(d11.x, 0.4566292464733124f, br); bi = fmaf(d11.y, 0.4566292464733124f, bi);
-      ar = fmaf(s12.x, -0.08879589289426804f, ar); ai = fmaf(s12.y, -0.08879589289426804f, ai); br = fmaf(d12.x, 0.9960498213768005f, br); bi = fmaf(d12.y, 0.9960498213768005f, bi);
-      ar = fmaf(s13.x, -0.956400990486145f, ar); ai = fmaf(s13.y, -0.956400990486145f, ai); br = fmaf(d13.x, 0.29205676913261414f, br); bi = fmaf(d13.y, 0.29205676913261414f, bi);
-      ar = fmaf(s14.x, -0.6300878524780273f, ar); ai = fmaf(s14.y, -0.6300878524780273f, ai); br = fmaf(d14.x, -0.7765238881111145f, br); bi = fmaf(d14.y, -0.7765238881111145f, bi);
-      ar = fmaf(s15.x, 0.4827921986579895f, ar); ai = fmaf(s15.y, 0.4827921986579895f, ai); br = fmaf(d15.x, -0.8757349252700806f, br); bi = fmaf(d15.y, -0.8757349252700806f, bi);
-      ar = fmaf(s16.x, 0.9929810762405396f, ar); ai = fmaf(s16.y, 0.9929810762405396f, ai); br = fmaf(d16.x, 0.11827316880226135f, br); bi = fmaf(d16.y, 0.11827316880226135f, bi);
-      ar = fmaf(s17.x, 0.26358717679977417f, ar); ai = fmaf(s17.y, 0.26358717679977417f, ai); br = fmaf(d17.x, 0.9646356105804443f, br); bi = fmaf(d17.y, 0.9646356105804443f, bi);
-      ar = fmaf(s18.x, -0.794854462146759f, ar); ai = fmaf(s18.y, -0.794854462146759f, ai); br = fmaf(d18.x, 0.6068001389503479f, br); bi = fmaf(d18.y, 0.6068001389503479f, bi);
-      ar = fmaf(s19.x, -0.8610436320304871f, ar); ai = fmaf(s19.y, -0.8610436320304871f, ai); br = fmaf(d19.x, -0.5085310935974121f, br); bi = fmaf(d19.y, -0.5085310935974121f, bi);
-      ar = fmaf(s20.x, 0.14764656126499176f, ar); ai = fmaf(s20.y, 0.14764656126499176f, ai); br = fmaf(d20.x, -0.989040195941925f, br); bi = fmaf(d20.y, -0.989040195941925f, bi);
-      ar = fmaf(s21.x, 0.9720228910446167f, ar); ai = fmaf(s21.y, 0.9720228910446167f, ai); br = fmaf(d21.x, -0.2348860502243042f, br); bi = fmaf(d21.y, -0.2348860502243042f, bi);
-      ar = fmaf(s22.x, 0.5829795002937317f, ar); ai = fmaf(s22.y, 0.5829795002937317f, ai); br = fmaf(d22.x, 0.8124868869781494f, br); bi = fmaf(d22.y, 0.8124868869781494f, bi);
-      ar = fmaf(s23.x, -0.5338233709335327f, ar); ai = fmaf(s23.y, -0.5338233709335327f, ai); br = fmaf(d23.x, 0.8455960154533386f, br); bi = fmaf(d23.y, 0.8455960154533386f, bi);
-      ar = fmaf(s24.x, -0.9842305779457092f, ar); ai = fmaf(s24.y, -0.9842305779457092f, ai); br = fmaf(d24.x, -0.1768902689218521f, br); bi = fmaf(d24.y, -0.1768902689218521f, bi);
-      ar = fmaf(s25.x, -0.2059786170721054f, ar); ai = fmaf(s25.y, -0.2059786170721054f, ai); br = fmaf(d25.x, -0.9785565137863159f, br); bi = fmaf(d25.y, -0.9785565137863159f, bi);
-      ar = fmaf(s26.x, 0.829405665397644f, ar); ai = fmaf(s26.y, 0.829405665397644f, ai); br = fmaf(d26.x, -0.5586467385292053f, br); bi = fmaf(d26.y, -0.5586467385292053f, bi);
-      if (!INV) { st(10, make_float2(ar + bi, ai - br)); st(43, make_float2(ar - bi, ai + br)); }
-      else { st(10, make_float2(ar - bi, ai + br)); st(43, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.26358717679977417f, ar); ai = fmaf(s1.y, 0.26358717679977417f, ai); br = fmaf(d1.x, 0.9646356105804443f, br); bi = fmaf(d1.y, 0.9646356105804443f, bi);
-      ar = fmaf(s2.x, -0.8610436320304871f, ar); ai = fmaf(s2.y, -0.8610436320304871f, ai); br = fmaf(d2.x, 0.5085310935974121f, br); bi = fmaf(d2.y, 0.5085310935974121f, bi);
-      ar = fmaf(s3.x, -0.7175072431564331f, ar); ai = fmaf(s3.y, -0.7175072431564331f, ai); br = fmaf(d3.x, -0.6965510249137878f, br); bi = fmaf(d3.y, -0.6965510249137878f, bi);
-      ar = fmaf(s4.x, 0.4827921986579895f, ar); ai = fmaf(s4.y, 0.4827921986579895f, ai); br = fmaf(d4.x, -0.8757349252700806f, br); bi = fmaf(d4.y, -0.8757349252700806f, bi);
-      ar = fmaf(s5.x, 0.9720228910446167f, ar); ai = fmaf(s5.y, 0.9720228910446167f, ai); br = fmaf(d5.x, 0.2348860502243042f, br); bi = fmaf(d5.y, 0.2348860502243042f, bi);
-      ar = fmaf(s6.x, 0.029633328318595886f, ar); ai = fmaf(s6.y, 0.029633328318595886f, ai); br = fmaf(d6.x, 0.9995608329772949f, br); bi = fmaf(d6.y, 0.9995608329772949f, bi);
-      ar = fmaf(s7.x, -0.956400990486145f, ar); ai = fmaf(s7.y, -0.956400990486145f, ai); br = fmaf(d7.x, 0.29205676913261414f, br); bi = fmaf(d7.y, 0.29205676913261414f, bi);
-      ar = fmaf(s8.x, -0.5338233709335327f, ar); ai = fmaf(s8.y, -0.5338233709335327f, ai); br = fmaf(d8.x, -0.8455960154533386f, br); bi = fmaf(d8.y, -0.8455960154533386f, bi);
-      ar = fmaf(s9.x, 0.674983024597168f, ar); ai = fmaf(s9.y, 0.674983024597168f, ai); br = fmaf(d9.x, -0.7378332614898682f, br); bi = fmaf(d9.y, -0.7378332614898682f, bi);
-      ar = fmaf(s10.x, 0.8896570801734924f, ar); ai = fmaf(s10.y, 0.8896570801734924f, ai); br = fmaf(d10.x, 0.4566292464733124f, br); bi = fmaf(d10.y, 0.4566292464733124f, bi);
-      ar = fmaf(s11.x, -0.2059786170721054f, ar); ai = fmaf(s11.y, -0.2059786170721054f, ai); br = fmaf(d11.x, 0.9785565137863159f, br); bi = fmaf(d11.y, 0.9785565137863159f, bi);
-      ar = fmaf(s12.x, -0.9982437491416931f, ar); ai = fmaf(s12.y, -0.9982437491416931f, ai); br = fmaf(d12.x, 0.05924062803387642f, br); bi = fmaf(d12.y, 0.05924062803387642f, bi);
-      ar = fmaf(s13.x, -0.3202698528766632f, ar); ai = fmaf(s13.y, -0.3202698528766632f, ai); br = fmaf(d13.x, -0.9473263621330261f, br); bi = fmaf(d13.y, -0.9473263621330261f, bi);
-      ar = fmaf(s14.x, 0.829405665397644f, ar); ai = fmaf(s14.y, 0.829405665397644f, ai); br = fmaf(d14.x, -0.5586467385292053f, br); bi = fmaf(d14.y, -0.5586467385292053f, bi);
-      ar = fmaf(s15.x, 0.7575112581253052f, ar); ai = fmaf(s15.y, 0.7575112581253052f, ai); br = fmaf(d15.x, 0.6528221368789673f, br); bi = fmaf(d15.y, 0.6528221368789673f, bi);
-      ar = fmaf(s16.x, -0.43006521463394165f, ar); ai = fmaf(s16.y, -0.43006521463394165f, ai); br = fmaf(d16.x, 0.9027978181838989f, br); bi = fmaf(d16.y, 0.9027978181838989f, bi);
-      ar = fmaf(s17.x, -0.9842305779457092f, ar); ai = fmaf(s17.y, -0.9842305779457092f, ai); br = fmaf(d17.x, -0.1768902689218521f, br); bi = fmaf(d17.y, -0.1768902689218521f, bi);
-      ar = fmaf(s18.x, -0.08879589289426804f, ar); ai = fmaf(s18.y, -0.08879589289426804f, ai); br = fmaf(d18.x, -0.9960498213768005f, br); bi = fmaf(d18.y, -0.9960498213768005f, bi);
-      ar = fmaf(s19.x, 0.9374196529388428f, ar); ai = fmaf(s19.y, 0.9374196529388428f, ai); br = fmaf(d19.x, -0.3482016324996948f, br); bi = fmaf(d19.y, -0.3482016324996948f, bi);
-      ar = fmaf(s20.x, 0.5829795002937317f, ar); ai = fmaf(s20.y, 0.5829795002937317f, ai); br = fmaf(d20.x, 0.8124868869781494f, br); bi = fmaf(d20.y, 0.8124868869781494f, bi);
-      ar = fmaf(s21.x, -0.6300878524780273f, ar); ai = fmaf(s21.y, -0.6300878524780273f, ai); br = fmaf(d21.x, 0.7765238881111145f, br); bi = fmaf(d21.y, 0.7765238881111145f, bi);
-      ar = fmaf(s22.x, -0.9151456356048584f, ar); ai = fmaf(s22.y, -0.9151456356048584f, ai); br = fmaf(d22.x, -0.4031234383583069f, br); bi = fmaf(d22.y, -0.4031234383583069f, bi);
-      ar = fmaf(s23.x, 0.14764656126499176f, ar); ai = fmaf(s23.y, 0.14764656126499176f, ai); br = fmaf(d23.x, -0.989040195941925f, br); bi = fmaf(d23.y, -0.989040195941925f, bi);
-      ar = fmaf(s24.x, 0.9929810762405396f, ar); ai = fmaf(s24.y, 0.9929810762405396f, ai); br = fmaf(d24.x, -0.11827316880226135f, br); bi = fmaf(d24.y, -0.11827316880226135f, bi);
-      ar = fmaf(s25.x, 0.3758275806903839f, ar); ai = fmaf(s25.y, 0.3758275806903839f, ai); br = fmaf(d25.x, 0.926689624786377f, br); bi = fmaf(d25.y, 0.926689624786377f, bi);
-      ar = fmaf(s26.x, -0.794854462146759f, ar); ai = fmaf(s26.y, -0.794854462146759f, ai); br = fmaf(d26.x, 0.6068001389503479f, br); bi = fmaf(d26.y, 0.6068001389503479f, bi);
-      if (!INV) { st(11, make_float2(ar + bi, ai - br)); st(42, make_float2(ar - bi, ai + br)); }
-      else { st(11, make_float2(ar - bi, ai + br)); st(42, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.14764656126499176f, ar); ai = fmaf(s1.y, 0.14764656126499176f, ai); br = fmaf(d1.x, 0.989040195941925f, br); bi = fmaf(d1.y, 0.989040195941925f, bi);
-      ar = fmaf(s2.x, -0.956400990486145f, ar); ai = fmaf(s2.y, -0.956400990486145f, ai); br = fmaf(d2.x, 0.29205676913261414f, br); bi = fmaf(d2.y, 0.29205676913261414f, bi);
-      ar = fmaf(s3.x, -0.43006521463394165f, ar); ai = fmaf(s3.y, -0.43006521463394165f, ai); br = fmaf(d3.x, -0.9027978181838989f, br); bi = fmaf(d3.y, -0.9027978181838989f, bi);
-      ar = fmaf(s4.x, 0.829405665397644f, ar); ai = fmaf(s4.y, 0.829405665397644f, ai); br = fmaf(d4.x, -0.5586467385292053f, br); bi = fmaf(d4.y, -0.5586467385292053f, bi);
-      ar = fmaf(s5.x, 0.674983024597168f, ar); ai = fmaf(s5.y, 0.674983024597168f, ai); br = fmaf(d5.x, 0.7378332614898682f, br); bi = fmaf(d5.y, 0.7378332614898682f, bi);
-      ar = fmaf(s6.x, -0.6300878524780273f, ar); ai = fmaf(s6.y, -0.6300878524780273f, ai); br = fmaf(d6.x, 0.7765238881111145f, br); bi = fmaf(d6.y, 0.7765238881111145f, bi);
-      ar = fmaf(s7.x, -0.8610436320304871f, ar); ai = fmaf(s7.y, -0.8610436320304871f, ai); br = fmaf(d7.x, -0.5085310935974121f, br); bi = fmaf(d7.y, -0.5085310935974121f, bi);
-      ar = fmaf(s8.x, 0.3758275806903839f, ar); ai = fmaf(s8.y, 0.3758275806903839f, ai); br = fmaf(d8.x, -0.926689624786377f, br); bi = fmaf(d8.y, -0.926689624786377f, bi);
-      ar = fmaf(s9.x, 0.9720228910446167f, ar); ai = fmaf(s9.y, 0.9720228910446167f, ai); br = fmaf(d9.x, 0.2348860502243042f, br); bi = fmaf(d9.y, 0.2348860502243042f, bi);
-      ar = fmaf(s10.x, -0.08879589289426804f, ar); ai = fmaf(s10.y, -0.08879589289426804f, ai); br = fmaf(d10.x, 0.9960498213768005f, br); bi = fmaf(d10.y, 0.9960498213768005f, bi);
-      ar = fmaf(s11.x, -0.9982437491416931f, ar); ai = fmaf(s11.y, -0.9982437491416931f, ai); br = fmaf(d11.x, 0.05924062803387642f, br); bi = fmaf(d11.y, 0.05924062803387642f, bi);
-      ar = fmaf(s12.x, -0.2059786170721054f, ar); ai = fmaf(s12.y, -0.2059786170721054f, ai); br = fmaf(d12.x, -0.9785565137863159f, br); bi = fmaf(d12.y, -0.9785565137863159f, bi);
-      ar = fmaf(s13.x, 0.9374196529388428f, ar); ai = fmaf(s13.y, 0.9374196529388428f, ai); br = fmaf(d13.x, -0.3482016324996948f, br); bi = fmaf(d13.y, -0.3482016324996948f, bi);
-      ar = fmaf(s14.x, 0.4827921986579895f, ar); ai = fmaf(s14.y, 0.4827921986579895f, ai); br = fmaf(d14.x, 0.8757349252700806f, br); bi = fmaf(d14.y, 0.8757349252700806f, bi);
-      ar = fmaf(s15.x, -0.794854462146759f, ar); ai = fmaf(s15.y, -0.794854462146759f, ai); br = fmaf(d15.x, 0.6068001389503479f, br); bi = fmaf(d15.y, 0.6068001389503479f, bi);
-      ar = fmaf(s16.x, -0.7175072431564331f, ar); ai = fmaf(s16.y, -0.7175072431564331f, ai); br = fmaf(d16.x, -0.6965510249137878f, br); bi = fmaf(d16.y, -0.6965510249137878f, bi);
-      ar = fmaf(s17.x, 0.5829795002937317f, ar); ai = fmaf(s17.y, 0.5829795002937317f, ai); br = fmaf(d17.x, -0.8124868869781494f, br); bi = fmaf(d17.y, -0.8124868869781494f, bi);
-      ar = fmaf(s18.x, 0.8896570801734924f, ar); ai = fmaf(s18.y, 0.8896570801734924f, ai); br = fmaf(d18.x, 0.4566292464733124f, br); bi = fmaf(d18.y, 0.4566292464733124f, bi);
-      ar = fmaf(s19.x, -0.3202698528766632f, ar); ai = fmaf(s19.y, -0.3202698528766632f, ai); br = fmaf(d19.x, 0.9473263621330261f, br); bi = fmaf(d19.y, 0.9473263621330261f, bi);
-      ar = fmaf(s20.x, -0.9842305779457092f, ar); ai = fmaf(s20.y, -0.9842305779457092f, ai); br = fmaf(d20.x, -0.1768902689218521f, br); bi = fmaf(d20.y, -0.1768902689218521f, bi);
-      ar = fmaf(s21.x, 0.029633328318595886f, ar); ai = fmaf(s21.y, 0.029633328318595886f, ai); br = fmaf(d21.x, -0.9995608329772949f, br); bi = fmaf(d21.y, -0.9995608329772949f, bi);
-      ar = fmaf(s22.x, 0.9929810762405396f, ar); ai = fmaf(s22.y, 0.9929810762405396f, ai); br = fmaf(d22.x, -0.11827316880226135f, br); bi = fmaf(d22.y, -0.11827316880226135f, bi);
-      ar = fmaf(s23.x, 0.26358717679977417f, ar); ai = fmaf(s23.y, 0.26358717679977417f, ai); br = fmaf(d23.x, 0.9646356105804443f, br); bi = fmaf(d23.y, 0.9646356105804443f, bi);
-      ar = fmaf(s24.x, -0.9151456356048584f, ar); ai = fmaf(s24.y, -0.9151456356048584f, ai); br = fmaf(d24.x, 0.4031234383583069f, br); bi = fmaf(d24.y, 0.4031234383583069f, bi);
-      ar = fmaf(s25.x, -0.5338233709335327f, ar); ai = fmaf(s25.y, -0.5338233709335327f, ai); br = fmaf(d25.x, -0.8455960154533386f, br); bi = fmaf(d25.y, -0.8455960154533386f, bi);
-      ar = fmaf(s26.x, 0.7575112581253052f, ar); ai = fmaf(s26.y, 0.7575112581253052f, ai); br = fmaf(d26.x, -0.6528221368789673f, br); bi = fmaf(d26.y, -0.6528221368789673f, bi);
-      if (!INV) { st(12, make_float2(ar + bi, ai - br)); st(41, make_float2(ar - bi, ai + br)); }
-      else { st(12, make_float2(ar - bi, ai + br)); st(41, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, 0.029633328318595886f, ar); ai = fmaf(s1.y, 0.029633328318595886f, ai); br = fmaf(d1.x, 0.9995608329772949f, br); bi = fmaf(d1.y, 0.9995608329772949f, bi);
-      ar = fmaf(s2.x, -0.9982437491416931f, ar); ai = fmaf(s2.y, -0.9982437491416931f, ai); br = fmaf(d2.x, 0.05924062803387642f, br); bi = fmaf(d2.y, 0.05924062803387642f, bi);
-      ar = fmaf(s3.x, -0.08879589289426804f, ar); ai = fmaf(s3.y, -0.08879589289426804f, ai); br = fmaf(d3.x, -0.9960498213768005f, br); bi = fmaf(d3.y, -0.9960498213768005f, bi);
-      ar = fmaf(s4.x, 0.9929810762405396f, ar); ai = fmaf(s4.y, 0.9929810762405396f, ai); br = fmaf(d4.x, -0.11827316880226135f, br); bi = fmaf(d4.y, -0.11827316880226135f, bi);
-      ar = fmaf(s5.x, 0.14764656126499176f, ar); ai = fmaf(s5.y, 0.14764656126499176f, ai); br = fmaf(d5.x, 0.989040195941925f, br); bi = fmaf(d5.y, 0.989040195941925f, bi);
-      ar = fmaf(s6.x, -0.9842305779457092f, ar); ai = fmaf(s6.y, -0.9842305779457092f, ai); br = fmaf(d6.x, 0.1768902689218521f, br); bi = fmaf(d6.y, 0.1768902689218521f, bi);
-      ar = fmaf(s7.x, -0.2059786170721054f, ar); ai = fmaf(s7.y, -0.2059786170721054f, ai); br = fmaf(d7.x, -0.9785565137863159f, br); bi = fmaf(d7.y, -0.9785565137863159f, bi);
-      ar = fmaf(s8.x, 0.9720228910446167f, ar); ai = fmaf(s8.y, 0.9720228910446167f, ai); br = fmaf(d8.x, -0.2348860502243042f, br); bi = fmaf(d8.y, -0.2348860502243042f, bi);
-      ar = fmaf(s9.x, 0.26358717679977417f, ar); ai = fmaf(s9.y, 0.26358717679977417f, ai); br = fmaf(d9.x, 0.9646356105804443f, br); bi = fmaf(d9.y, 0.9646356105804443f, bi);
-      ar = fmaf(s10.x, -0.956400990486145f, ar); ai = fmaf(s10.y, -0.956400990486145f, ai); br = fmaf(d10.x, 0.29205676913261414f, br); bi = fmaf(d10.y, 0.29205676913261414f, bi);
-      ar = fmaf(s11.x, -0.3202698528766632f, ar); ai = fmaf(s11.y, -0.3202698528766632f, ai); br = fmaf(d11.x, -0.9473263621330261f, br); bi = fmaf(d11.y, -0.9473263621330261f, bi);
-      ar = fmaf(s12.x, 0.9374196529388428f, ar); ai = fmaf(s12.y, 0.9374196529388428f, ai); br = fmaf(d12.x, -0.3482016324996948f, br); bi = fmaf(d12.y, -0.3482016324996948f, bi);
-      ar = fmaf(s13.x, 0.3758275806903839f, ar); ai = fmaf(s13.y, 0.3758275806903839f, ai); br = fmaf(d13.x, 0.926689624786377f, br); bi = fmaf(d13.y, 0.926689624786377f, bi);
-      ar = fmaf(s14.x, -0.9151456356048584f, ar); ai = fmaf(s14.y, -0.9151456356048584f, ai); br = fmaf(d14.x, 0.4031234383583069f, br); bi = fmaf(d14.y, 0.4031234383583069f, bi);
-      ar = fmaf(s15.x, -0.43006521463394165f, ar); ai = fmaf(s15.y, -0.43006521463394165f, ai); br = fmaf(d15.x, -0.9027978181838989f, br); bi = fmaf(d15.y, -0.9027978181838989f, bi);
-      ar = fmaf(s16.x, 0.8896570801734924f, ar); ai = fmaf(s16.y, 0.8896570801734924f, ai); br = fmaf(d16.x, -0.4566292464733124f, br); bi = fmaf(d16.y, -0.4566292464733124f, bi);
-      ar = fmaf(s17.x, 0.4827921986579895f, ar); ai = fmaf(s17.y, 0.4827921986579895f, ai); br = fmaf(d17.x, 0.8757349252700806f, br); bi = fmaf(d17.y, 0.8757349252700806f, bi);
-      ar = fmaf(s18.x, -0.8610436320304871f, ar); ai = fmaf(s18.y, -0.8610436320304871f, ai); br = fmaf(d18.x, 0.5085310935974121f, br); bi = fmaf(d18.y, 0.5085310935974121f, bi);
-      ar = fmaf(s19.x, -0.5338233709335327f, ar); ai = fmaf(s19.y, -0.5338233709335327f, ai); br = fmaf(d19.x, -0.8455960154533386f, br); bi = fmaf(d19.y, -0.8455960154533386f, bi);
-      ar = fmaf(s20.x, 0.829405665397644f, ar); ai = fmaf(s20.y, 0.829405665397644f, ai); br = fmaf(d20.x, -0.5586467385292053f, br); bi = fmaf(d20.y, -0.5586467385292053f, bi);
-      ar = fmaf(s21.x, 0.5829795002937317f, ar); ai = fmaf(s21.y, 0.5829795002937317f, ai); br = fmaf(d21.x, 0.8124868869781494f, br); bi = fmaf(d21.y, 0.8124868869781494f, bi);
-      ar = fmaf(s22.x, -0.794854462146759f, ar); ai = fmaf(s22.y, -0.794854462146759f, ai); br = fmaf(d22.x, 0.6068001389503479f, br); bi = fmaf(d22.y, 0.6068001389503479f, bi);
-      ar = fmaf(s23.x, -0.6300878524780273f, ar); ai = fmaf(s23.y, -0.6300878524780273f, ai); br = fmaf(d23.x, -0.7765238881111145f, br); bi = fmaf(d23.y, -0.7765238881111145f, bi);
-      ar = fmaf(s24.x, 0.7575112581253052f, ar); ai = fmaf(s24.y, 0.7575112581253052f, ai); br = fmaf(d24.x, -0.6528221368789673f, br); bi = fmaf(d24.y, -0.6528221368789673f, bi);
-      ar = fmaf(s25.x, 0.674983024597168f, ar); ai = fmaf(s25.y, 0.674983024597168f, ai); br = fmaf(d25.x, 0.7378332614898682f, br); bi = fmaf(d25.y, 0.7378332614898682f, bi);
-      ar = fmaf(s26.x, -0.7175072431564331f, ar); ai = fmaf(s26.y, -0.7175072431564331f, ai); br = fmaf(d26.x, 0.6965510249137878f, br); bi = fmaf(d26.y, 0.6965510249137878f, bi);
-      if (!INV) { st(13, make_float2(ar + bi, ai - br)); st(40, make_float2(ar - bi, ai + br)); }
-      else { st(13, make_float2(ar - bi, ai + br)); st(40, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.08879589289426804f, ar); ai = fmaf(s1.y, -0.08879589289426804f, ai); br = fmaf(d1.x, 0.9960498213768005f, br); bi = fmaf(d1.y, 0.9960498213768005f, bi);
-      ar = fmaf(s2.x, -0.9842305779457092f, ar); ai = fmaf(s2.y, -0.9842305779457092f, ai); br = fmaf(d2.x, -0.1768902689218521f, br); bi = fmaf(d2.y, -0.1768902689218521f, bi);
-      ar = fmaf(s3.x, 0.26358717679977417f, ar); ai = fmaf(s3.y, 0.26358717679977417f, ai); br = fmaf(d3.x, -0.9646356105804443f, br); bi = fmaf(d3.y, -0.9646356105804443f, bi);
-      ar = fmaf(s4.x, 0.9374196529388428f, ar); ai = fmaf(s4.y, 0.9374196529388428f, ai); br = fmaf(d4.x, 0.3482016324996948f, br); bi = fmaf(d4.y, 0.3482016324996948f, bi);
-      ar = fmaf(s5.x, -0.43006521463394165f, ar); ai = fmaf(s5.y, -0.43006521463394165f, ai); br = fmaf(d5.x, 0.9027978181838989f, br); bi = fmaf(d5.y, 0.9027978181838989f, bi);
-      ar = fmaf(s6.x, -0.8610436320304871f, ar); ai = fmaf(s6.y, -0.8610436320304871f, ai); br = fmaf(d6.x, -0.5085310935974121f, br); bi = fmaf(d6.y, -0.5085310935974121f, bi);
-      ar = fmaf(s7.x, 0.5829795002937317f, ar); ai = fmaf(s7.y, 0.5829795002937317f, ai); br = fmaf(d7.x, -0.8124868869781494f, br); bi = fmaf(d7.y, -0.8124868869781494f, bi);
-      ar = fmaf(s8.x, 0.7575112581253052f, ar); ai = fmaf(s8.y, 0.7575112581253052f, ai); br = fmaf(d8.x, 0.6528221368789673f, br); bi = fmaf(d8.y, 0.6528221368789673f, bi);
-      ar = fmaf(s9.x, -0.7175072431564331f, ar); ai = fmaf(s9.y, -0.7175072431564331f, ai); br = fmaf(d9.x, 0.6965510249137878f, br); bi = fmaf(d9.y, 0.6965510249137878f, bi);
-      ar = fmaf(s10.x, -0.6300878524780273f, ar); ai = fmaf(s10.y, -0.6300878524780273f, ai); br = fmaf(d10.x, -0.7765238881111145f, br); bi = fmaf(d10.y, -0.7765238881111145f, bi);
-      ar = fmaf(s11.x, 0.829405665397644f, ar); ai = fmaf(s11.y, 0.829405665397644f, ai); br = fmaf(d11.x, -0.5586467385292053f, br); bi = fmaf(d11.y, -0.5586467385292053f, bi);
-      ar = fmaf(s12.x, 0.4827921986579895f, ar); ai = fmaf(s12.y, 0.4827921986579895f, ai); br = fmaf(d12.x, 0.8757349252700806f, br); bi = fmaf(d12.y, 0.8757349252700806f, bi);
-      ar = fmaf(s13.x, -0.9151456356048584f, ar); ai = fmaf(s13.y, -0.9151456356048584f, ai); br = fmaf(d13.x, 0.4031234383583069f, br); bi = fmaf(d13.y, 0.4031234383583069f, bi);
-      ar = fmaf(s14.x, -0.3202698528766632f, ar); ai = fmaf(s14.y, -0.3202698528766632f, ai); br = fmaf(d14.x, -0.9473263621330261f, br); bi = fmaf(d14.y, -0.9473263621330261f, bi);
-      ar = fmaf(s15.x, 0.9720228910446167f, ar); ai = fmaf(s15.y, 0.9720228910446167f, ai); br = fmaf(d15.x, -0.2348860502243042f, br); bi = fmaf(d15.y, -0.2348860502243042f, bi);
-      ar = fmaf(s16.x, 0.14764656126499176f, ar); ai = fmaf(s16.y, 0.14764656126499176f, ai); br = fmaf(d16.x, 0.989040195941925f, br); bi = fmaf(d16.y, 0.989040195941925f, bi);
-      ar = fmaf(s17.x, -0.9982437491416931f, ar); ai = fmaf(s17.y, -0.9982437491416931f, ai); br = fmaf(d17.x, 0.05924062803387642f, br); bi = fmaf(d17.y, 0.05924062803387642f, bi);
-      ar = fmaf(s18.x, 0.029633328318595886f, ar); ai = fmaf(s18.y, 0.029633328318595886f, ai); br = fmaf(d18.x, -0.9995608329772949f, br); bi = fmaf(d18.y, -0.9995608329772949f, bi);
-      ar = fmaf(s19.x, 0.9929810762405396f, ar); ai = fmaf(s19.y, 0.9929810762405396f, ai); br = fmaf(d19.x, 0.11827316880226135f, br); bi = fmaf(d19.y, 0.11827316880226135f, bi);
-      ar = fmaf(s20.x, -0.2059786170721054f, ar); ai = fmaf(s20.y, -0.2059786170721054f, ai); br = fmaf(d20.x, 0.9785565137863159f, br); bi = fmaf(d20.y, 0.9785565137863159f, bi);
-      ar = fmaf(s21.x, -0.956400990486145f, ar); ai = fmaf(s21.y, -0.956400990486145f, ai); br = fmaf(d21.x, -0.29205676913261414f, br); bi = fmaf(d21.y, -0.29205676913261414f, bi);
-      ar = fmaf(s22.x, 0.3758275806903839f, ar); ai = fmaf(s22.y, 0.3758275806903839f, ai); br = fmaf(d22.x, -0.926689624786377f, br); bi = fmaf(d22.y, -0.926689624786377f, bi);
-      ar = fmaf(s23.x, 0.8896570801734924f, ar); ai = fmaf(s23.y, 0.8896570801734924f, ai); br = fmaf(d23.x, 0.4566292464733124f, br); bi = fmaf(d23.y, 0.4566292464733124f, bi);
-      ar = fmaf(s24.x, -0.5338233709335327f, ar); ai = fmaf(s24.y, -0.5338233709335327f, ai); br = fmaf(d24.x, 0.8455960154533386f, br); bi = fmaf(d24.y, 0.8455960154533386f, bi);
-      ar = fmaf(s25.x, -0.794854462146759f, ar); ai = fmaf(s25.y, -0.794854462146759f, ai); br = fmaf(d25.x, -0.6068001389503479f, br); bi = fmaf(d25.y, -0.6068001389503479f, bi);
-      ar = fmaf(s26.x, 0.674983024597168f, ar); ai = fmaf(s26.y, 0.674983024597168f, ai); br = fmaf(d26.x, -0.7378332614898682f, br); bi = fmaf(d26.y, -0.7378332614898682f, bi);
-      if (!INV) { st(14, make_float2(ar + bi, ai - br)); st(39, make_float2(ar - bi, ai + br)); }
-      else { st(14, make_float2(ar - bi, ai + br)); st(39, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.2059786170721054f, ar); ai = fmaf(s1.y, -0.2059786170721054f, ai); br = fmaf(d1.x, 0.9785565137863159f, br); bi = fmaf(d1.y, 0.9785565137863159f, bi);
-      ar = fmaf(s2.x, -0.9151456356048584f, ar); ai = fmaf(s2.y, -0.9151456356048584f, ai); br = fmaf(d2.x, -0.4031234383583069f, br); bi = fmaf(d2.y, -0.4031234383583069f, bi);
-      ar = fmaf(s3.x, 0.5829795002937317f, ar); ai = fmaf(s3.y, 0.5829795002937317f, ai); br = fmaf(d3.x, -0.8124868869781494f, br); bi = fmaf(d3.y, -0.8124868869781494f, bi);
-      ar = fmaf(s4.x, 0.674983024597168f, ar); ai = fmaf(s4.y, 0.674983024597168f, ai); br = fmaf(d4.x, 0.7378332614898682f, br); bi = fmaf(d4.y, 0.7378332614898682f, bi);
-      ar = fmaf(s5.x, -0.8610436320304871f, ar); ai = fmaf(s5.y, -0.8610436320304871f, ai); br = fmaf(d5.x, 0.5085310935974121f, br); bi = fmaf(d5.y, 0.5085310935974121f, bi);
-      ar = fmaf(s6.x, -0.3202698528766632f, ar); ai = fmaf(s6.y, -0.3202698528766632f, ai); br = fmaf(d6.x, -0.9473263621330261f, br); bi = fmaf(d6.y, -0.9473263621330261f, bi);
-      ar = fmaf(s7.x, 0.9929810762405396f, ar); ai = fmaf(s7.y, 0.9929810762405396f, ai); br = fmaf(d7.x, -0.11827316880226135f, br); bi = fmaf(d7.y, -0.11827316880226135f, bi);
-      ar = fmaf(s8.x, -0.08879589289426804f, ar); ai = fmaf(s8.y, -0.08879589289426804f, ai); br = fmaf(d8.x, 0.9960498213768005f, br); bi = fmaf(d8.y, 0.9960498213768005f, bi);
-      ar = fmaf(s9.x, -0.956400990486145f, ar); ai = fmaf(s9.y, -0.956400990486145f, ai); br = fmaf(d9.x, -0.29205676913261414f, br); bi = fmaf(d9.y, -0.29205676913261414f, bi);
-      ar = fmaf(s10.x, 0.4827921986579895f, ar); ai = fmaf(s10.y, 0.4827921986579895f, ai); br = fmaf(d10.x, -0.8757349252700806f, br); bi = fmaf(d10.y, -0.8757349252700806f, bi);
-      ar = fmaf(s11.x, 0.7575112581253052f, ar); ai = fmaf(s11.y, 0.7575112581253052f, ai); br = fmaf(d11.x, 0.6528221368789673f, br); bi = fmaf(d11.y, 0.6528221368789673f, bi);
-      ar = fmaf(s12.x, -0.794854462146759f, ar); ai = fmaf(s12.y, -0.794854462146759f, ai); br = fmaf(d12.x, 0.6068001389503479f, br); bi = fmaf(d12.y, 0.6068001389503479f, bi);
-      ar = fmaf(s13.x, -0.43006521463394165f, ar); ai = fmaf(s13.y, -0.43006521463394165f, ai); br = fmaf(d13.x, -0.9027978181838989f, br); bi = fmaf(d13.y, -0.9027978181838989f, bi);
-      ar = fmaf(s14.x, 0.9720228910446167f, ar); ai = fmaf(s14.y, 0.9720228910446167f, ai); br = fmaf(d14.x, -0.2348860502243042f, br); bi = fmaf(d14.y, -0.2348860502243042f, bi);
-      ar = fmaf(s15.x, 0.029633328318595886f, ar); ai = fmaf(s15.y, 0.029633328318595886f, ai); br = fmaf(d15.x, 0.9995608329772949f, br); bi = fmaf(d15.y, 0.9995608329772949f, bi);
-      ar = fmaf(s16.x, -0.9842305779457092f, ar); ai = fmaf(s16.y, -0.9842305779457092f, ai); br = fmaf(d16.x, -0.1768902689218521f, br); bi = fmaf(d16.y, -0.1768902689218521f, bi);
-      ar = fmaf(s17.x, 0.3758275806903839f, ar); ai = fmaf(s17.y, 0.3758275806903839f, ai); br = fmaf(d17.x, -0.926689624786377f, br); bi = fmaf(d17.y, -0.926689624786377f, bi);
-      ar = fmaf(s18.x, 0.829405665397644f, ar); ai = fmaf(s18.y, 0.829405665397644f, ai); br = fmaf(d18.x, 0.5586467385292053f, br); bi = fmaf(d18.y, 0.5586467385292053f, bi);
-      ar = fmaf(s19.x, -0.7175072431564331f, ar); ai = fmaf(s19.y, -0.7175072431564331f, ai); br = fmaf(d19.x, 0.6965510249137878f, br); bi = fmaf(d19.y, 0.6965510249137878f, bi);
-      ar = fmaf(s20.x, -0.5338233709335327f, ar); ai = fmaf(s20.y, -0.5338233709335327f, ai); br = fmaf(d20.x, -0.8455960154533386f, br); bi = fmaf(d20.y, -0.8455960154533386f, bi);
-      ar = fmaf(s21.x, 0.9374196529388428f, ar); ai = fmaf(s21.y, 0.9374196529388428f, ai); br = fmaf(d21.x, -0.3482016324996948f, br); bi = fmaf(d21.y, -0.3482016324996948f, bi);
-      ar = fmaf(s22.x, 0.14764656126499176f, ar); ai = fmaf(s22.y, 0.14764656126499176f, ai); br = fmaf(d22.x, 0.989040195941925f, br); bi = fmaf(d22.y, 0.989040195941925f, bi);
-      ar = fmaf(s23.x, -0.9982437491416931f, ar); ai = fmaf(s23.y, -0.9982437491416931f, ai); br = fmaf(d23.x, -0.05924062803387642f, br); bi = fmaf(d23.y, -0.05924062803387642f, bi);
-      ar = fmaf(s24.x, 0.26358717679977417f, ar); ai = fmaf(s24.y, 0.26358717679977417f, ai); br = fmaf(d24.x, -0.9646356105804443f, br); bi = fmaf(d24.y, -0.9646356105804443f, bi);
-      ar = fmaf(s25.x, 0.8896570801734924f, ar); ai = fmaf(s25.y, 0.8896570801734924f, ai); br = fmaf(d25.x, 0.4566292464733124f, br); bi = fmaf(d25.y, 0.4566292464733124f, bi);
-      ar = fmaf(s26.x, -0.6300878524780273f, ar); ai = fmaf(s26.y, -0.6300878524780273f, ai); br = fmaf(d26.x, 0.7765238881111145f, br); bi = fmaf(d26.y, 0.7765238881111145f, bi);
-      if (!INV) { st(15, make_float2(ar + bi, ai - br)); st(38, make_float2(ar - bi, ai + br)); }
-      else { st(15, make_float2(ar - bi, ai + br)); st(38, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.3202698528766632f, ar); ai = fmaf(s1.y, -0.3202698528766632f, ai); br = fmaf(d1.x, 0.9473263621330261f, br); bi = fmaf(d1.y, 0.9473263621330261f, bi);
-      ar = fmaf(s2.x, -0.794854462146759f, ar); ai = fmaf(s2.y, -0.794854462146759f, ai); br = fmaf(d2.x, -0.6068001389503479f, br); bi = fmaf(d2.y, -0.6068001389503479f, bi);
-      ar = fmaf(s3.x, 0.829405665397644f, ar); ai = fmaf(s3.y, 0.829405665397644f, ai); br = fmaf(d3.x, -0.5586467385292053f, br); bi = fmaf(d3.y, -0.5586467385292053f, bi);
-      ar = fmaf(s4.x, 0.26358717679977417f, ar); ai = fmaf(s4.y, 0.26358717679977417f, ai); br = fmaf(d4.x, 0.9646356105804443f, br); bi = fmaf(d4.y, 0.9646356105804443f, bi);
-      ar = fmaf(s5.x, -0.9982437491416931f, ar); ai = fmaf(s5.y, -0.9982437491416931f, ai); br = fmaf(d5.x, -0.05924062803387642f, br); bi = fmaf(d5.y, -0.05924062803387642f, bi);
-      ar = fmaf(s6.x, 0.3758275806903839f, ar); ai = fmaf(s6.y, 0.3758275806903839f, ai); br = fmaf(d6.x, -0.926689624786377f, br); bi = fmaf(d6.y, -0.926689624786377f, bi);
-      ar = fmaf(s7.x, 0.7575112581253052f, ar); ai = fmaf(s7.y, 0.7575112581253052f, ai); br = fmaf(d7.x, 0.6528221368789673f, br); bi = fmaf(d7.y, 0.6528221368789673f, bi);
-      ar = fmaf(s8.x, -0.8610436320304871f, ar); ai = fmaf(s8.y, -0.8610436320304871f, ai); br = fmaf(d8.x, 0.5085310935974121f, br); bi = fmaf(d8.y, 0.5085310935974121f, bi);
-      ar = fmaf(s9.x, -0.2059786170721054f, ar); ai = fmaf(s9.y, -0.2059786170721054f, ai); br = fmaf(d9.x, -0.9785565137863159f, br); bi = fmaf(d9.y, -0.9785565137863159f, bi);
-      ar = fmaf(s10.x, 0.9929810762405396f, ar); ai = fmaf(s10.y, 0.9929810762405396f, ai); br = fmaf(d10.x, 0.11827316880226135f, br); bi = fmaf(d10.y, 0.11827316880226135f, bi);
-      ar = fmaf(s11.x, -0.43006521463394165f, ar); ai = fmaf(s11.y, -0.43006521463394165f, ai); br = fmaf(d11.x, 0.9027978181838989f, br); bi = fmaf(d11.y, 0.9027978181838989f, bi);
-      ar = fmaf(s12.x, -0.7175072431564331f, ar); ai = fmaf(s12.y, -0.7175072431564331f, ai); br = fmaf(d12.x, -0.6965510249137878f, br); bi = fmaf(d12.y, -0.6965510249137878f, bi);
-      ar = fmaf(s13.x, 0.8896570801734924f, ar); ai = fmaf(s13.y, 0.8896570801734924f, ai); br = fmaf(d13.x, -0.4566292464733124f, br); bi = fmaf(d13.y, -0.4566292464733124f, bi);
-      ar = fmaf(s14.x, 0.14764656126499176f, ar); ai = fmaf(s14.y, 0.14764656126499176f, ai); br = fmaf(d14.x, 0.989040195941925f, br); bi = fmaf(d14.y, 0.989040195941925f, bi);
-      ar = fmaf(s15.x, -0.9842305779457092f, ar); ai = fmaf(s15.y, -0.9842305779457092f, ai); br = fmaf(d15.x, -0.1768902689218521f, br); bi = fmaf(d15.y, -0.1768902689218521f, bi);
-      ar = fmaf(s16.x, 0.4827921986579895f, ar); ai = fmaf(s16.y, 0.4827921986579895f, ai); br = fmaf(d16.x, -0.8757349252700806f, br); bi = fmaf(d16.y, -0.8757349252700806f, bi);
-      ar = fmaf(s17.x, 0.674983024597168f, ar); ai = fmaf(s17.y, 0.674983024597168f, ai); br = fmaf(d17.x, 0.7378332614898682f, br); bi = fmaf(d17.y, 0.7378332614898682f, bi);
-      ar = fmaf(s18.x, -0.9151456356048584f, ar); ai = fmaf(s18.y, -0.9151456356048584f, ai); br = fmaf(d18.x, 0.4031234383583069f, br); bi = fmaf(d18.y, 0.4031234383583069f, bi);
-      ar = fmaf(s19.x, -0.08879589289426804f, ar); ai = fmaf(s19.y, -0.08879589289426804f, ai); br = fmaf(d19.x, -0.9960498213768005f, br); bi = fmaf(d19.y, -0.9960498213768005f, bi);
-      ar = fmaf(s20.x, 0.9720228910446167f, ar); ai = fmaf(s20.y, 0.9720228910446167f, ai); br = fmaf(d20.x, 0.2348860502243042f, br); bi = fmaf(d20.y, 0.2348860502243042f, bi);
-      ar = fmaf(s21.x, -0.5338233709335327f, ar); ai = fmaf(s21.y, -0.5338233709335327f, ai); br = fmaf(d21.x, 0.8455960154533386f, br); bi = fmaf(d21.y, 0.8455960154533386f, bi);
-      ar = fmaf(s22.x, -0.6300878524780273f, ar); ai = fmaf(s22.y, -0.6300878524780273f, ai); br = fmaf(d22.x, -0.7765238881111145f, br); bi = fmaf(d22.y, -0.7765238881111145f, bi);
-      ar = fmaf(s23.x, 0.9374196529388428f, ar); ai = fmaf(s23.y, 0.9374196529388428f, ai); br = fmaf(d23.x, -0.3482016324996948f, br); bi = fmaf(d23.y, -0.3482016324996948f, bi);
-      ar = fmaf(s24.x, 0.029633328318595886f, ar); ai = fmaf(s24.y, 0.029633328318595886f, ai); br = fmaf(d24.x, 0.9995608329772949f, br); bi = fmaf(d24.y, 0.9995608329772949f, bi);
-      ar = fmaf(s25.x, -0.956400990486145f, ar); ai = fmaf(s25.y, -0.956400990486145f, ai); br = fmaf(d25.x, -0.29205676913261414f, br); bi = fmaf(d25.y, -0.29205676913261414f, bi);
-      ar = fmaf(s26.x, 0.5829795002937317f, ar); ai = fmaf(s26.y, 0.5829795002937317f, ai); br = fmaf(d26.x, -0.8124868869781494f, br); bi = fmaf(d26.y, -0.8124868869781494f, bi);
-      if (!INV) { st(16, make_float2(ar + bi, ai - br)); st(37, make_float2(ar - bi, ai + br)); }
-      else { st(16, make_float2(ar - bi, ai + br)); st(37, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.43006521463394165f, ar); ai = fmaf(s1.y, -0.43006521463394165f, ai); br = fmaf(d1.x, 0.9027978181838989f, br); bi = fmaf(d1.y, 0.9027978181838989f, bi);
-      ar = fmaf(s2.x, -0.6300878524780273f, ar); ai = fmaf(s2.y, -0.6300878524780273f, ai); br = fmaf(d2.x, -0.7765238881111145f, br); bi = fmaf(d2.y, -0.7765238881111145f, bi);
-      ar = fmaf(s3.x, 0.9720228910446167f, ar); ai = fmaf(s3.y, 0.9720228910446167f, ai); br = fmaf(d3.x, -0.2348860502243042f, br); bi = fmaf(d3.y, -0.2348860502243042f, bi);
-      ar = fmaf(s4.x, -0.2059786170721054f, ar); ai = fmaf(s4.y, -0.2059786170721054f, ai); br = fmaf(d4.x, 0.9785565137863159f, br); bi = fmaf(d4.y, 0.9785565137863159f, bi);
-      ar = fmaf(s5.x, -0.794854462146759f, ar); ai = fmaf(s5.y, -0.794854462146759f, ai); br = fmaf(d5.x, -0.6068001389503479f, br); bi = fmaf(d5.y, -0.6068001389503479f, bi);
-      ar = fmaf(s6.x, 0.8896570801734924f, ar); ai = fmaf(s6.y, 0.8896570801734924f, ai); br = fmaf(d6.x, -0.4566292464733124f, br); bi = fmaf(d6.y, -0.4566292464733124f, bi);
-      ar = fmaf(s7.x, 0.029633328318595886f, ar); ai = fmaf(s7.y, 0.029633328318595886f, ai); br = fmaf(d7.x, 0.9995608329772949f, br); bi = fmaf(d7.y, 0.9995608329772949f, bi);
-      ar = fmaf(s8.x, -0.9151456356048584f, ar); ai = fmaf(s8.y, -0.9151456356048584f, ai); br = fmaf(d8.x, -0.4031234383583069f, br); bi = fmaf(d8.y, -0.4031234383583069f, bi);
-      ar = fmaf(s9.x, 0.7575112581253052f, ar); ai = fmaf(s9.y, 0.7575112581253052f, ai); br = fmaf(d9.x, -0.6528221368789673f, br); bi = fmaf(d9.y, -0.6528221368789673f, bi);
-      ar = fmaf(s10.x, 0.26358717679977417f, ar); ai = fmaf(s10.y, 0.26358717679977417f, ai); br = fmaf(d10.x, 0.9646356105804443f, br); bi = fmaf(d10.y, 0.9646356105804443f, bi);
-      ar = fmaf(s11.x, -0.9842305779457092f, ar); ai = fmaf(s11.y, -0.9842305779457092f, ai); br = fmaf(d11.x, -0.1768902689218521f, br); bi = fmaf(d11.y, -0.1768902689218521f, bi);
-      ar = fmaf(s12.x, 0.5829795002937317f, ar); ai = fmaf(s12.y, 0.5829795002937317f, ai); br = fmaf(d12.x, -0.8124868869781494f, br); bi = fmaf(d12.y, -0.8124868869781494f, bi);
-      ar = fmaf(s13.x, 0.4827921986579895f, ar); ai = fmaf(s13.y, 0.4827921986579895f, ai); br = fmaf(d13.x, 0.8757349252700806f, br); bi = fmaf(d13.y, 0.8757349252700806f, bi);
-      ar = fmaf(s14.x, -0.9982437491416931f, ar); ai = fmaf(s14.y, -0.9982437491416931f, ai); br = fmaf(d14.x, 0.05924062803387642f, br); bi = fmaf(d14.y, 0.05924062803387642f, bi);
-      ar = fmaf(s15.x, 0.3758275806903839f, ar); ai = fmaf(s15.y, 0.3758275806903839f, ai); br = fmaf(d15.x, -0.926689624786377f, br); bi = fmaf(d15.y, -0.926689624786377f, bi);
-      ar = fmaf(s16.x, 0.674983024597168f, ar); ai = fmaf(s16.y, 0.674983024597168f, ai); br = fmaf(d16.x, 0.7378332614898682f, br); bi = fmaf(d16.y, 0.7378332614898682f, bi);
-      ar = fmaf(s17.x, -0.956400990486145f, ar); ai = fmaf(s17.y, -0.956400990486145f, ai); br = fmaf(d17.x, 0.29205676913261414f, br); bi = fmaf(d17.y, 0.29205676913261414f, bi);
-      ar = fmaf(s18.x, 0.14764656126499176f, ar); ai = fmaf(s18.y, 0.14764656126499176f, ai); br = fmaf(d18.x, -0.989040195941925f, br); bi = fmaf(d18.y, -0.989040195941925f, bi);
-      ar = fmaf(s19.x, 0.829405665397644f, ar); ai = fmaf(s19.y, 0.829405665397644f, ai); br = fmaf(d19.x, 0.5586467385292053f, br); bi = fmaf(d19.y, 0.5586467385292053f, bi);
-      ar = fmaf(s20.x, -0.8610436320304871f, ar); ai = fmaf(s20.y, -0.8610436320304871f, ai); br = fmaf(d20.x, 0.5085310935974121f, br); bi = fmaf(d20.y, 0.5085310935974121f, bi);
-      ar = fmaf(s21.x, -0.08879589289426804f, ar); ai = fmaf(s21.y, -0.08879589289426804f, ai); br = fmaf(d21.x, -0.9960498213768005f, br); bi = fmaf(d21.y, -0.9960498213768005f, bi);
-      ar = fmaf(s22.x, 0.9374196529388428f, ar); ai = fmaf(s22.y, 0.9374196529388428f, ai); br = fmaf(d22.x, 0.3482016324996948f, br); bi = fmaf(d22.y, 0.3482016324996948f, bi);
-      ar = fmaf(s23.x, -0.7175072431564331f, ar); ai = fmaf(s23.y, -0.7175072431564331f, ai); br = fmaf(d23.x, 0.6965510249137878f, br); bi = fmaf(d23.y, 0.6965510249137878f, bi);
-      ar = fmaf(s24.x, -0.3202698528766632f, ar); ai = fmaf(s24.y, -0.3202698528766632f, ai); br = fmaf(d24.x, -0.9473263621330261f, br); bi = fmaf(d24.y, -0.9473263621330261f, bi);
-      ar = fmaf(s25.x, 0.9929810762405396f, ar); ai = fmaf(s25.y, 0.9929810762405396f, ai); br = fmaf(d25.x, 0.11827316880226135f, br); bi = fmaf(d25.y, 0.11827316880226135f, bi);
-      ar = fmaf(s26.x, -0.5338233709335327f, ar); ai = fmaf(s26.y, -0.5338233709335327f, ai); br = fmaf(d26.x, 0.8455960154533386f, br); bi = fmaf(d26.y, 0.8455960154533386f, bi);
-      if (!INV) { st(17, make_float2(ar + bi, ai - br)); st(36, make_float2(ar - bi, ai + br)); }
-      else { st(17, make_float2(ar - bi, ai + br)); st(36, make_float2(ar + bi, ai - br)); }
-    }
-    break;
-  }
-  case 2: {
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.5338233709335327f, ar); ai = fmaf(s1.y, -0.5338233709335327f, ai); br = fmaf(d1.x, 0.8455960154533386f, br); bi = fmaf(d1.y, 0.8455960154533386f, bi);
-      ar = fmaf(s2.x, -0.43006521463394165f, ar); ai = fmaf(s2.y, -0.43006521463394165f, ai); br = fmaf(d2.x, -0.9027978181838989f, br); bi = fmaf(d2.y, -0.9027978181838989f, bi);
-      ar = fmaf(s3.x, 0.9929810762405396f, ar); ai = fmaf(s3.y, 0.9929810762405396f, ai); br = fmaf(d3.x, 0.11827316880226135f, br); bi = fmaf(d3.y, 0.11827316880226135f, bi);
-      ar = fmaf(s4.x, -0.6300878524780273f, ar); ai = fmaf(s4.y, -0.6300878524780273f, ai); br = fmaf(d4.x, 0.7765238881111145f, br); bi = fmaf(d4.y, 0.7765238881111145f, bi);
-      ar = fmaf(s5.x, -0.3202698528766632f, ar); ai = fmaf(s5.y, -0.3202698528766632f, ai); br = fmaf(d5.x, -0.9473263621330261f, br); bi = fmaf(d5.y, -0.9473263621330261f, bi);
-      ar = fmaf(s6.x, 0.9720228910446167f, ar); ai = fmaf(s6.y, 0.9720228910446167f, ai); br = fmaf(d6.x, 0.2348860502243042f, br); bi = fmaf(d6.y, 0.2348860502243042f, bi);
-      ar = fmaf(s7.x, -0.7175072431564331f, ar); ai = fmaf(s7.y, -0.7175072431564331f, ai); br = fmaf(d7.x, 0.6965510249137878f, br); bi = fmaf(d7.y, 0.6965510249137878f, bi);
-      ar = fmaf(s8.x, -0.2059786170721054f, ar); ai = fmaf(s8.y, -0.2059786170721054f, ai); br = fmaf(d8.x, -0.9785565137863159f, br); bi = fmaf(d8.y, -0.9785565137863159f, bi);
-      ar = fmaf(s9.x, 0.9374196529388428f, ar); ai = fmaf(s9.y, 0.9374196529388428f, ai); br = fmaf(d9.x, 0.3482016324996948f, br); bi = fmaf(d9.y, 0.3482016324996948f, bi);
-      ar = fmaf(s10.x, -0.794854462146759f, ar); ai = fmaf(s10.y, -0.794854462146759f, ai); br = fmaf(d10.x, 0.6068001389503479f, br); bi = fmaf(d10.y, 0.6068001389503479f, bi);
-      ar = fmaf(s11.x, -0.08879589289426804f, ar); ai = fmaf(s11.y, -0.08879589289426804f, ai); br = fmaf(d11.x, -0.9960498213768005f, br); bi = fmaf(d11.y, -0.9960498213768005f, bi);
-      ar = fmaf(s12.x, 0.8896570801734924f, ar); ai = fmaf(s12.y, 0.8896570801734924f, ai); br = fmaf(d12.x, 0.4566292464733124f, br); bi = fmaf(d12.y, 0.4566292464733124f, bi);
-      ar = fmaf(s13.x, -0.8610436320304871f, ar); ai = fmaf(s13.y, -0.8610436320304871f, ai); br = fmaf(d13.x, 0.5085310935974121f, br); bi = fmaf(d13.y, 0.5085310935974121f, bi);
-      ar = fmaf(s14.x, 0.029633328318595886f, ar); ai = fmaf(s14.y, 0.029633328318595886f, ai); br = fmaf(d14.x, -0.9995608329772949f, br); bi = fmaf(d14.y, -0.9995608329772949f, bi);
-      ar = fmaf(s15.x, 0.829405665397644f, ar); ai = fmaf(s15.y, 0.829405665397644f, ai); br = fmaf(d15.x, 0.5586467385292053f, br); bi = fmaf(d15.y, 0.5586467385292053f, bi);
-      ar = fmaf(s16.x, -0.9151456356048584f, ar); ai = fmaf(s16.y, -0.9151456356048584f, ai); br = fmaf(d16.x, 0.4031234383583069f, br); bi = fmaf(d16.y, 0.4031234383583069f, bi);
-      ar = fmaf(s17.x, 0.14764656126499176f, ar); ai = fmaf(s17.y, 0.14764656126499176f, ai); br = fmaf(d17.x, -0.989040195941925f, br); bi = fmaf(d17.y, -0.989040195941925f, bi);
-      ar = fmaf(s18.x, 0.7575112581253052f, ar); ai = fmaf(s18.y, 0.7575112581253052f, ai); br = fmaf(d18.x, 0.6528221368789673f, br); bi = fmaf(d18.y, 0.6528221368789673f, bi);
-      ar = fmaf(s19.x, -0.956400990486145f, ar); ai = fmaf(s19.y, -0.956400990486145f, ai); br = fmaf(d19.x, 0.29205676913261414f, br); bi = fmaf(d19.y, 0.29205676913261414f, bi);
-      ar = fmaf(s20.x, 0.26358717679977417f, ar); ai = fmaf(s20.y, 0.26358717679977417f, ai); br = fmaf(d20.x, -0.9646356105804443f, br); bi = fmaf(d20.y, -0.9646356105804443f, bi);
-      ar = fmaf(s21.x, 0.674983024597168f, ar); ai = fmaf(s21.y, 0.674983024597168f, ai); br = fmaf(d21.x, 0.7378332614898682f, br); bi = fmaf(d21.y, 0.7378332614898682f, bi);
-      ar = fmaf(s22.x, -0.9842305779457092f, ar); ai = fmaf(s22.y, -0.9842305779457092f, ai); br = fmaf(d22.x, 0.1768902689218521f, br); bi = fmaf(d22.y, 0.1768902689218521f, bi);
-      ar = fmaf(s23.x, 0.3758275806903839f, ar); ai = fmaf(s23.y, 0.3758275806903839f, ai); br = fmaf(d23.x, -0.926689624786377f, br); bi = fmaf(d23.y, -0.926689624786377f, bi);
-      ar = fmaf(s24.x, 0.5829795002937317f, ar); ai = fmaf(s24.y, 0.5829795002937317f, ai); br = fmaf(d24.x, 0.8124868869781494f, br); bi = fmaf(d24.y, 0.8124868869781494f, bi);
-      ar = fmaf(s25.x, -0.9982437491416931f, ar); ai = fmaf(s25.y, -0.9982437491416931f, ai); br = fmaf(d25.x, 0.05924062803387642f, br); bi = fmaf(d25.y, 0.05924062803387642f, bi);
-      ar = fmaf(s26.x, 0.4827921986579895f, ar); ai = fmaf(s26.y, 0.4827921986579895f, ai); br = fmaf(d26.x, -0.8757349252700806f, br); bi = fmaf(d26.y, -0.8757349252700806f, bi);
-      if (!INV) { st(18, make_float2(ar + bi, ai - br)); st(35, make_float2(ar - bi, ai + br)); }
-      else { st(18, make_float2(ar - bi, ai + br)); st(35, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.6300878524780273f, ar); ai = fmaf(s1.y, -0.6300878524780273f, ai); br = fmaf(d1.x, 0.7765238881111145f, br); bi = fmaf(d1.y, 0.7765238881111145f, bi);
-      ar = fmaf(s2.x, -0.2059786170721054f, ar); ai = fmaf(s2.y, -0.2059786170721054f, ai); br = fmaf(d2.x, -0.9785565137863159f, br); bi = fmaf(d2.y, -0.9785565137863159f, bi);
-      ar = fmaf(s3.x, 0.8896570801734924f, ar); ai = fmaf(s3.y, 0.8896570801734924f, ai); br = fmaf(d3.x, 0.4566292464733124f, br); bi = fmaf(d3.y, 0.4566292464733124f, bi);
-      ar = fmaf(s4.x, -0.9151456356048584f, ar); ai = fmaf(s4.y, -0.9151456356048584f, ai); br = fmaf(d4.x, 0.4031234383583069f, br); bi = fmaf(d4.y, 0.4031234383583069f, bi);
-      ar = fmaf(s5.x, 0.26358717679977417f, ar); ai = fmaf(s5.y, 0.26358717679977417f, ai); br = fmaf(d5.x, -0.9646356105804443f, br); bi = fmaf(d5.y, -0.9646356105804443f, bi);
-      ar = fmaf(s6.x, 0.5829795002937317f, ar); ai = fmaf(s6.y, 0.5829795002937317f, ai); br = fmaf(d6.x, 0.8124868869781494f, br); bi = fmaf(d6.y, 0.8124868869781494f, bi);
-      ar = fmaf(s7.x, -0.9982437491416931f, ar); ai = fmaf(s7.y, -0.9982437491416931f, ai); br = fmaf(d7.x, -0.05924062803387642f, br); bi = fmaf(d7.y, -0.05924062803387642f, bi);
-      ar = fmaf(s8.x, 0.674983024597168f, ar); ai = fmaf(s8.y, 0.674983024597168f, ai); br = fmaf(d8.x, -0.7378332614898682f, br); bi = fmaf(d8.y, -0.7378332614898682f, bi);
-      ar = fmaf(s9.x, 0.14764656126499176f, ar); ai = fmaf(s9.y, 0.14764656126499176f, ai); br = fmaf(d9.x, 0.989040195941925f, br); bi = fmaf(d9.y, 0.989040195941925f, bi);
-      ar = fmaf(s10.x, -0.8610436320304871f, ar); ai = fmaf(s10.y, -0.8610436320304871f, ai); br = fmaf(d10.x, -0.5085310935974121f, br); bi = fmaf(d10.y, -0.5085310935974121f, bi);
-      ar = fmaf(s11.x, 0.9374196529388428f, ar); ai = fmaf(s11.y, 0.9374196529388428f, ai); br = fmaf(d11.x, -0.3482016324996948f, br); bi = fmaf(d11.y, -0.3482016324996948f, bi);
-      ar = fmaf(s12.x, -0.3202698528766632f, ar); ai = fmaf(s12.y, -0.3202698528766632f, ai); br = fmaf(d12.x, 0.9473263621330261f, br); bi = fmaf(d12.y, 0.9473263621330261f, bi);
-      ar = fmaf(s13.x, -0.5338233709335327f, ar); ai = fmaf(s13.y, -0.5338233709335327f, ai); br = fmaf(d13.x, -0.8455960154533386f, br); bi = fmaf(d13.y, -0.8455960154533386f, bi);
-      ar = fmaf(s14.x, 0.9929810762405396f, ar); ai = fmaf(s14.y, 0.9929810762405396f, ai); br = fmaf(d14.x, 0.11827316880226135f, br); bi = fmaf(d14.y, 0.11827316880226135f, bi);
-      ar = fmaf(s15.x, -0.7175072431564331f, ar); ai = fmaf(s15.y, -0.7175072431564331f, ai); br = fmaf(d15.x, 0.6965510249137878f, br); bi = fmaf(d15.y, 0.6965510249137878f, bi);
-      ar = fmaf(s16.x, -0.08879589289426804f, ar); ai = fmaf(s16.y, -0.08879589289426804f, ai); br = fmaf(d16.x, -0.9960498213768005f, br); bi = fmaf(d16.y, -0.9960498213768005f, bi);
-      ar = fmaf(s17.x, 0.829405665397644f, ar); ai = fmaf(s17.y, 0.829405665397644f, ai); br = fmaf(d17.x, 0.5586467385292053f, br); bi = fmaf(d17.y, 0.5586467385292053f, bi);
-      ar = fmaf(s18.x, -0.956400990486145f, ar); ai = fmaf(s18.y, -0.956400990486145f, ai); br = fmaf(d18.x, 0.29205676913261414f, br); bi = fmaf(d18.y, 0.29205676913261414f, bi);
-      ar = fmaf(s19.x, 0.3758275806903839f, ar); ai = fmaf(s19.y, 0.3758275806903839f, ai); br = fmaf(d19.x, -0.926689624786377f, br); bi = fmaf(d19.y, -0.926689624786377f, bi);
-      ar = fmaf(s20.x, 0.4827921986579895f, ar); ai = fmaf(s20.y, 0.4827921986579895f, ai); br = fmaf(d20.x, 0.8757349252700806f, br); bi = fmaf(d20.y, 0.8757349252700806f, bi);
-      ar = fmaf(s21.x, -0.9842305779457092f, ar); ai = fmaf(s21.y, -0.9842305779457092f, ai); br = fmaf(d21.x, -0.1768902689218521f, br); bi = fmaf(d21.y, -0.1768902689218521f, bi);
-      ar = fmaf(s22.x, 0.7575112581253052f, ar); ai = fmaf(s22.y, 0.7575112581253052f, ai); br = fmaf(d22.x, -0.6528221368789673f, br); bi = fmaf(d22.y, -0.6528221368789673f, bi);
-      ar = fmaf(s23.x, 0.029633328318595886f, ar); ai = fmaf(s23.y, 0.029633328318595886f, ai); br = fmaf(d23.x, 0.9995608329772949f, br); bi = fmaf(d23.y, 0.9995608329772949f, bi);
-      ar = fmaf(s24.x, -0.794854462146759f, ar); ai = fmaf(s24.y, -0.794854462146759f, ai); br = fmaf(d24.x, -0.6068001389503479f, br); bi = fmaf(d24.y, -0.6068001389503479f, bi);
-      ar = fmaf(s25.x, 0.9720228910446167f, ar); ai = fmaf(s25.y, 0.9720228910446167f, ai); br = fmaf(d25.x, -0.2348860502243042f, br); bi = fmaf(d25.y, -0.2348860502243042f, bi);
-      ar = fmaf(s26.x, -0.43006521463394165f, ar); ai = fmaf(s26.y, -0.43006521463394165f, ai); br = fmaf(d26.x, 0.9027978181838989f, br); bi = fmaf(d26.y, 0.9027978181838989f, bi);
-      if (!INV) { st(19, make_float2(ar + bi, ai - br)); st(34, make_float2(ar - bi, ai + br)); }
-      else { st(19, make_float2(ar - bi, ai + br)); st(34, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.7175072431564331f, ar); ai = fmaf(s1.y, -0.7175072431564331f, ai); br = fmaf(d1.x, 0.6965510249137878f, br); bi = fmaf(d1.y, 0.6965510249137878f, bi);
-      ar = fmaf(s2.x, 0.029633328318595886f, ar); ai = fmaf(s2.y, 0.029633328318595886f, ai); br = fmaf(d2.x, -0.9995608329772949f, br); bi = fmaf(d2.y, -0.9995608329772949f, bi);
-      ar = fmaf(s3.x, 0.674983024597168f, ar); ai = fmaf(s3.y, 0.674983024597168f, ai); br = fmaf(d3.x, 0.7378332614898682f, br); bi = fmaf(d3.y, 0.7378332614898682f, bi);
-      ar = fmaf(s4.x, -0.9982437491416931f, ar); ai = fmaf(s4.y, -0.9982437491416931f, ai); br = fmaf(d4.x, -0.05924062803387642f, br); bi = fmaf(d4.y, -0.05924062803387642f, bi);
-      ar = fmaf(s5.x, 0.7575112581253052f, ar); ai = fmaf(s5.y, 0.7575112581253052f, ai); br = fmaf(d5.x, -0.6528221368789673f, br); bi = fmaf(d5.y, -0.6528221368789673f, bi);
-      ar = fmaf(s6.x, -0.08879589289426804f, ar); ai = fmaf(s6.y, -0.08879589289426804f, ai); br = fmaf(d6.x, 0.9960498213768005f, br); bi = fmaf(d6.y, 0.9960498213768005f, bi);
-      ar = fmaf(s7.x, -0.6300878524780273f, ar); ai = fmaf(s7.y, -0.6300878524780273f, ai); br = fmaf(d7.x, -0.7765238881111145f, br); bi = fmaf(d7.y, -0.7765238881111145f, bi);
-      ar = fmaf(s8.x, 0.9929810762405396f, ar); ai = fmaf(s8.y, 0.9929810762405396f, ai); br = fmaf(d8.x, 0.11827316880226135f, br); bi = fmaf(d8.y, 0.11827316880226135f, bi);
-      ar = fmaf(s9.x, -0.794854462146759f, ar); ai = fmaf(s9.y, -0.794854462146759f, ai); br = fmaf(d9.x, 0.6068001389503479f, br); bi = fmaf(d9.y, 0.6068001389503479f, bi);
-      ar = fmaf(s10.x, 0.14764656126499176f, ar); ai = fmaf(s10.y, 0.14764656126499176f, ai); br = fmaf(d10.x, -0.989040195941925f, br); bi = fmaf(d10.y, -0.989040195941925f, bi);
-      ar = fmaf(s11.x, 0.5829795002937317f, ar); ai = fmaf(s11.y, 0.5829795002937317f, ai); br = fmaf(d11.x, 0.8124868869781494f, br); bi = fmaf(d11.y, 0.8124868869781494f, bi);
-      ar = fmaf(s12.x, -0.9842305779457092f, ar); ai = fmaf(s12.y, -0.9842305779457092f, ai); br = fmaf(d12.x, -0.1768902689218521f, br); bi = fmaf(d12.y, -0.1768902689218521f, bi);
-      ar = fmaf(s13.x, 0.829405665397644f, ar); ai = fmaf(s13.y, 0.829405665397644f, ai); br = fmaf(d13.x, -0.5586467385292053f, br); bi = fmaf(d13.y, -0.5586467385292053f, bi);
-      ar = fmaf(s14.x, -0.2059786170721054f, ar); ai = fmaf(s14.y, -0.2059786170721054f, ai); br = fmaf(d14.x, 0.9785565137863159f, br); bi = fmaf(d14.y, 0.9785565137863159f, bi);
-      ar = fmaf(s15.x, -0.5338233709335327f, ar); ai = fmaf(s15.y, -0.5338233709335327f, ai); br = fmaf(d15.x, -0.8455960154533386f, br); bi = fmaf(d15.y, -0.8455960154533386f, bi);
-      ar = fmaf(s16.x, 0.9720228910446167f, ar); ai = fmaf(s16.y, 0.9720228910446167f, ai); br = fmaf(d16.x, 0.2348860502243042f, br); bi = fmaf(d16.y, 0.2348860502243042f, bi);
-      ar = fmaf(s17.x, -0.8610436320304871f, ar); ai = fmaf(s17.y, -0.8610436320304871f, ai); br = fmaf(d17.x, 0.5085310935974121f, br); bi = fmaf(d17.y, 0.5085310935974121f, bi);
-      ar = fmaf(s18.x, 0.26358717679977417f, ar); ai = fmaf(s18.y, 0.26358717679977417f, ai); br = fmaf(d18.x, -0.9646356105804443f, br); bi = fmaf(d18.y, -0.9646356105804443f, bi);
-      ar = fmaf(s19.x, 0.4827921986579895f, ar); ai = fmaf(s19.y, 0.4827921986579895f, ai); br = fmaf(d19.x, 0.8757349252700806f, br); bi = fmaf(d19.y, 0.8757349252700806f, bi);
-      ar = fmaf(s20.x, -0.956400990486145f, ar); ai = fmaf(s20.y, -0.956400990486145f, ai); br = fmaf(d20.x, -0.29205676913261414f, br); bi = fmaf(d20.y, -0.29205676913261414f, bi);
-      ar = fmaf(s21.x, 0.8896570801734924f, ar); ai = fmaf(s21.y, 0.8896570801734924f, ai); br = fmaf(d21.x, -0.4566292464733124f, br); bi = fmaf(d21.y, -0.4566292464733124f, bi);
-      ar = fmaf(s22.x, -0.3202698528766632f, ar); ai = fmaf(s22.y, -0.3202698528766632f, ai); br = fmaf(d22.x, 0.9473263621330261f, br); bi = fmaf(d22.y, 0.9473263621330261f, bi);
-      ar = fmaf(s23.x, -0.43006521463394165f, ar); ai = fmaf(s23.y, -0.43006521463394165f, ai); br = fmaf(d23.x, -0.9027978181838989f, br); bi = fmaf(d23.y, -0.9027978181838989f, bi);
-      ar = fmaf(s24.x, 0.9374196529388428f, ar); ai = fmaf(s24.y, 0.9374196529388428f, ai); br = fmaf(d24.x, 0.3482016324996948f, br); bi = fmaf(d24.y, 0.3482016324996948f, bi);
-      ar = fmaf(s25.x, -0.9151456356048584f, ar); ai = fmaf(s25.y, -0.9151456356048584f, ai); br = fmaf(d25.x, 0.4031234383583069f, br); bi = fmaf(d25.y, 0.4031234383583069f, bi);
-      ar = fmaf(s26.x, 0.3758275806903839f, ar); ai = fmaf(s26.y, 0.3758275806903839f, ai); br = fmaf(d26.x, -0.926689624786377f, br); bi = fmaf(d26.y, -0.926689624786377f, bi);
-      if (!INV) { st(20, make_float2(ar + bi, ai - br)); st(33, make_float2(ar - bi, ai + br)); }
-      else { st(20, make_float2(ar - bi, ai + br)); st(33, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.794854462146759f, ar); ai = fmaf(s1.y, -0.794854462146759f, ai); br = fmaf(d1.x, 0.6068001389503479f, br); bi = fmaf(d1.y, 0.6068001389503479f, bi);
-      ar = fmaf(s2.x, 0.26358717679977417f, ar); ai = fmaf(s2.y, 0.26358717679977417f, ai); br = fmaf(d2.x, -0.9646356105804443f, br); bi = fmaf(d2.y, -0.9646356105804443f, bi);
-      ar = fmaf(s3.x, 0.3758275806903839f, ar); ai = fmaf(s3.y, 0.3758275806903839f, ai); br = fmaf(d3.x, 0.926689624786377f, br); bi = fmaf(d3.y, 0.926689624786377f, bi);
-      ar = fmaf(s4.x, -0.8610436320304871f, ar); ai = fmaf(s4.y, -0.8610436320304871f, ai); br = fmaf(d4.x, -0.5085310935974121f, br); bi = fmaf(d4.y, -0.5085310935974121f, bi);
-      ar = fmaf(s5.x, 0.9929810762405396f, ar); ai = fmaf(s5.y, 0.9929810762405396f, ai); br = fmaf(d5.x, -0.11827316880226135f, br); bi = fmaf(d5.y, -0.11827316880226135f, bi);
-      ar = fmaf(s6.x, -0.7175072431564331f, ar); ai = fmaf(s6.y, -0.7175072431564331f, ai); br = fmaf(d6.x, 0.6965510249137878f, br); bi = fmaf(d6.y, 0.6965510249137878f, bi);
-      ar = fmaf(s7.x, 0.14764656126499176f, ar); ai = fmaf(s7.y, 0.14764656126499176f, ai); br = fmaf(d7.x, -0.989040195941925f, br); bi = fmaf(d7.y, -0.989040195941925f, bi);
-      ar = fmaf(s8.x, 0.4827921986579895f, ar); ai = fmaf(s8.y, 0.4827921986579895f, ai); br = fmaf(d8.x, 0.8757349252700806f, br); bi = fmaf(d8.y, 0.8757349252700806f, bi);
-      ar = fmaf(s9.x, -0.9151456356048584f, ar); ai = fmaf(s9.y, -0.9151456356048584f, ai); br = fmaf(d9.x, -0.4031234383583069f, br); bi = fmaf(d9.y, -0.4031234383583069f, bi);
-      ar = fmaf(s10.x, 0.9720228910446167f, ar); ai = fmaf(s10.y, 0.9720228910446167f, ai); br = fmaf(d10.x, -0.2348860502243042f, br); bi = fmaf(d10.y, -0.2348860502243042f, bi);
-      ar = fmaf(s11.x, -0.6300878524780273f, ar); ai = fmaf(s11.y, -0.6300878524780273f, ai); br = fmaf(d11.x, 0.7765238881111145f, br); bi = fmaf(d11.y, 0.7765238881111145f, bi);
-      ar = fmaf(s12.x, 0.029633328318595886f, ar); ai = fmaf(s12.y, 0.029633328318595886f, ai); br = fmaf(d12.x, -0.9995608329772949f, br); bi = fmaf(d12.y, -0.9995608329772949f, bi);
-      ar = fmaf(s13.x, 0.5829795002937317f, ar); ai = fmaf(s13.y, 0.5829795002937317f, ai); br = fmaf(d13.x, 0.8124868869781494f, br); bi = fmaf(d13.y, 0.8124868869781494f, bi);
-      ar = fmaf(s14.x, -0.956400990486145f, ar); ai = fmaf(s14.y, -0.956400990486145f, ai); br = fmaf(d14.x, -0.29205676913261414f, br); bi = fmaf(d14.y, -0.29205676913261414f, bi);
-      ar = fmaf(s15.x, 0.9374196529388428f, ar); ai = fmaf(s15.y, 0.9374196529388428f, ai); br = fmaf(d15.x, -0.3482016324996948f, br); bi = fmaf(d15.y, -0.3482016324996948f, bi);
-      ar = fmaf(s16.x, -0.5338233709335327f, ar); ai = fmaf(s16.y, -0.5338233709335327f, ai); br = fmaf(d16.x, 0.8455960154533386f, br); bi = fmaf(d16.y, 0.8455960154533386f, bi);
-      ar = fmaf(s17.x, -0.08879589289426804f, ar); ai = fmaf(s17.y, -0.08879589289426804f, ai); br = fmaf(d17.x, -0.9960498213768005f, br); bi = fmaf(d17.y, -0.9960498213768005f, bi);
-      ar = fmaf(s18.x, 0.674983024597168f, ar); ai = fmaf(s18.y, 0.674983024597168f, ai); br = fmaf(d18.x, 0.7378332614898682f, br); bi = fmaf(d18.y, 0.7378332614898682f, bi);
-      ar = fmaf(s19.x, -0.9842305779457092f, ar); ai = fmaf(s19.y, -0.9842305779457092f, ai); br = fmaf(d19.x, -0.1768902689218521f, br); bi = fmaf(d19.y, -0.1768902689218521f, bi);
-      ar = fmaf(s20.x, 0.8896570801734924f, ar); ai = fmaf(s20.y, 0.8896570801734924f, ai); br = fmaf(d20.x, -0.4566292464733124f, br); bi = fmaf(d20.y, -0.4566292464733124f, bi);
-      ar = fmaf(s21.x, -0.43006521463394165f, ar); ai = fmaf(s21.y, -0.43006521463394165f, ai); br = fmaf(d21.x, 0.9027978181838989f, br); bi = fmaf(d21.y, 0.9027978181838989f, bi);
-      ar = fmaf(s22.x, -0.2059786170721054f, ar); ai = fmaf(s22.y, -0.2059786170721054f, ai); br = fmaf(d22.x, -0.9785565137863159f, br); bi = fmaf(d22.y, -0.9785565137863159f, bi);
-      ar = fmaf(s23.x, 0.7575112581253052f, ar); ai = fmaf(s23.y, 0.7575112581253052f, ai); br = fmaf(d23.x, 0.6528221368789673f, br); bi = fmaf(d23.y, 0.6528221368789673f, bi);
-      ar = fmaf(s24.x, -0.9982437491416931f, ar); ai = fmaf(s24.y, -0.9982437491416931f, ai); br = fmaf(d24.x, -0.05924062803387642f, br); bi = fmaf(d24.y, -0.05924062803387642f, bi);
-      ar = fmaf(s25.x, 0.829405665397644f, ar); ai = fmaf(s25.y, 0.829405665397644f, ai); br = fmaf(d25.x, -0.5586467385292053f, br); bi = fmaf(d25.y, -0.5586467385292053f, bi);
-      ar = fmaf(s26.x, -0.3202698528766632f, ar); ai = fmaf(s26.y, -0.3202698528766632f, ai); br = fmaf(d26.x, 0.9473263621330261f, br); bi = fmaf(d26.y, 0.9473263621330261f, bi);
-      if (!INV) { st(21, make_float2(ar + bi, ai - br)); st(32, make_float2(ar - bi, ai + br)); }
-      else { st(21, make_float2(ar - bi, ai + br)); st(32, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.8610436320304871f, ar); ai = fmaf(s1.y, -0.8610436320304871f, ai); br = fmaf(d1.x, 0.5085310935974121f, br); bi = fmaf(d1.y, 0.5085310935974121f, bi);
-      ar = fmaf(s2.x, 0.4827921986579895f, ar); ai = fmaf(s2.y, 0.4827921986579895f, ai); br = fmaf(d2.x, -0.8757349252700806f, br); bi = fmaf(d2.y, -0.8757349252700806f, bi);
-      ar = fmaf(s3.x, 0.029633328318595886f, ar); ai = fmaf(s3.y, 0.029633328318595886f, ai); br = fmaf(d3.x, 0.9995608329772949f, br); bi = fmaf(d3.y, 0.9995608329772949f, bi);
-      ar = fmaf(s4.x, -0.5338233709335327f, ar); ai = fmaf(s4.y, -0.5338233709335327f, ai); br = fmaf(d4.x, -0.8455960154533386f, br); bi = fmaf(d4.y, -0.8455960154533386f, bi);
-      ar = fmaf(s5.x, 0.8896570801734924f, ar); ai = fmaf(s5.y, 0.8896570801734924f, ai); br = fmaf(d5.x, 0.4566292464733124f, br); bi = fmaf(d5.y, 0.4566292464733124f, bi);
-      ar = fmaf(s6.x, -0.9982437491416931f, ar); ai = fmaf(s6.y, -0.9982437491416931f, ai); br = fmaf(d6.x, 0.05924062803387642f, br); bi = fmaf(d6.y, 0.05924062803387642f, bi);
-      ar = fmaf(s7.x, 0.829405665397644f, ar); ai = fmaf(s7.y, 0.829405665397644f, ai); br = fmaf(d7.x, -0.5586467385292053f, br); bi = fmaf(d7.y, -0.5586467385292053f, bi);
-      ar = fmaf(s8.x, -0.43006521463394165f, ar); ai = fmaf(s8.y, -0.43006521463394165f, ai); br = fmaf(d8.x, 0.9027978181838989f, br); bi = fmaf(d8.y, 0.9027978181838989f, bi);
-      ar = fmaf(s9.x, -0.08879589289426804f, ar); ai = fmaf(s9.y, -0.08879589289426804f, ai); br = fmaf(d9.x, -0.9960498213768005f, br); bi = fmaf(d9.y, -0.9960498213768005f, bi);
-      ar = fmaf(s10.x, 0.5829795002937317f, ar); ai = fmaf(s10.y, 0.5829795002937317f, ai); br = fmaf(d10.x, 0.8124868869781494f, br); bi = fmaf(d10.y, 0.8124868869781494f, bi);
-      ar = fmaf(s11.x, -0.9151456356048584f, ar); ai = fmaf(s11.y, -0.9151456356048584f, ai); br = fmaf(d11.x, -0.4031234383583069f, br); bi = fmaf(d11.y, -0.4031234383583069f, bi);
-      ar = fmaf(s12.x, 0.9929810762405396f, ar); ai = fmaf(s12.y, 0.9929810762405396f, ai); br = fmaf(d12.x, -0.11827316880226135f, br); bi = fmaf(d12.y, -0.11827316880226135f, bi);
-      ar = fmaf(s13.x, -0.794854462146759f, ar); ai = fmaf(s13.y, -0.794854462146759f, ai); br = fmaf(d13.x, 0.6068001389503479f, br); bi = fmaf(d13.y, 0.6068001389503479f, bi);
-      ar = fmaf(s14.x, 0.3758275806903839f, ar); ai = fmaf(s14.y, 0.3758275806903839f, ai); br = fmaf(d14.x, -0.926689624786377f, br); bi = fmaf(d14.y, -0.926689624786377f, bi);
-      ar = fmaf(s15.x, 0.14764656126499176f, ar); ai = fmaf(s15.y, 0.14764656126499176f, ai); br = fmaf(d15.x, 0.989040195941925f, br); bi = fmaf(d15.y, 0.989040195941925f, bi);
-      ar = fmaf(s16.x, -0.6300878524780273f, ar); ai = fmaf(s16.y, -0.6300878524780273f, ai); br = fmaf(d16.x, -0.7765238881111145f, br); bi = fmaf(d16.y, -0.7765238881111145f, bi);
-      ar = fmaf(s17.x, 0.9374196529388428f, ar); ai = fmaf(s17.y, 0.9374196529388428f, ai); br = fmaf(d17.x, 0.3482016324996948f, br); bi = fmaf(d17.y, 0.3482016324996948f, bi);
-      ar = fmaf(s18.x, -0.9842305779457092f, ar); ai = fmaf(s18.y, -0.9842305779457092f, ai); br = fmaf(d18.x, 0.1768902689218521f, br); bi = fmaf(d18.y, 0.1768902689218521f, bi);
-      ar = fmaf(s19.x, 0.7575112581253052f, ar); ai = fmaf(s19.y, 0.7575112581253052f, ai); br = fmaf(d19.x, -0.6528221368789673f, br); bi = fmaf(d19.y, -0.6528221368789673f, bi);
-      ar = fmaf(s20.x, -0.3202698528766632f, ar); ai = fmaf(s20.y, -0.3202698528766632f, ai); br = fmaf(d20.x, 0.9473263621330261f, br); bi = fmaf(d20.y, 0.9473263621330261f, bi);
-      ar = fmaf(s21.x, -0.2059786170721054f, ar); ai = fmaf(s21.y, -0.2059786170721054f, ai); br = fmaf(d21.x, -0.9785565137863159f, br); bi = fmaf(d21.y, -0.9785565137863159f, bi);
-      ar = fmaf(s22.x, 0.674983024597168f, ar); ai = fmaf(s22.y, 0.674983024597168f, ai); br = fmaf(d22.x, 0.7378332614898682f, br); bi = fmaf(d22.y, 0.7378332614898682f, bi);
-      ar = fmaf(s23.x, -0.956400990486145f, ar); ai = fmaf(s23.y, -0.956400990486145f, ai); br = fmaf(d23.x, -0.29205676913261414f, br); bi = fmaf(d23.y, -0.29205676913261414f, bi);
-      ar = fmaf(s24.x, 0.9720228910446167f, ar); ai = fmaf(s24.y, 0.9720228910446167f, ai); br = fmaf(d24.x, -0.2348860502243042f, br); bi = fmaf(d24.y, -0.2348860502243042f, bi);
-      ar = fmaf(s25.x, -0.7175072431564331f, ar); ai = fmaf(s25.y, -0.7175072431564331f, ai); br = fmaf(d25.x, 0.6965510249137878f, br); bi = fmaf(d25.y, 0.6965510249137878f, bi);
-      ar = fmaf(s26.x, 0.26358717679977417f, ar); ai = fmaf(s26.y, 0.26358717679977417f, ai); br = fmaf(d26.x, -0.9646356105804443f, br); bi = fmaf(d26.y, -0.9646356105804443f, bi);
-      if (!INV) { st(22, make_float2(ar + bi, ai - br)); st(31, make_float2(ar - bi, ai + br)); }
-      else { st(22, make_float2(ar - bi, ai + br)); st(31, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.9151456356048584f, ar); ai = fmaf(s1.y, -0.9151456356048584f, ai); br = fmaf(d1.x, 0.4031234383583069f, br); bi = fmaf(d1.y, 0.4031234383583069f, bi);
-      ar = fmaf(s2.x, 0.674983024597168f, ar); ai = fmaf(s2.y, 0.674983024597168f, ai); br = fmaf(d2.x, -0.7378332614898682f, br); bi = fmaf(d2.y, -0.7378332614898682f, bi);
-      ar = fmaf(s3.x, -0.3202698528766632f, ar); ai = fmaf(s3.y, -0.3202698528766632f, ai); br = fmaf(d3.x, 0.9473263621330261f, br); bi = fmaf(d3.y, 0.9473263621330261f, bi);
-      ar = fmaf(s4.x, -0.08879589289426804f, ar); ai = fmaf(s4.y, -0.08879589289426804f, ai); br = fmaf(d4.x, -0.9960498213768005f, br); bi = fmaf(d4.y, -0.9960498213768005f, bi);
-      ar = fmaf(s5.x, 0.4827921986579895f, ar); ai = fmaf(s5.y, 0.4827921986579895f, ai); br = fmaf(d5.x, 0.8757349252700806f, br); bi = fmaf(d5.y, 0.8757349252700806f, bi);
-      ar = fmaf(s6.x, -0.794854462146759f, ar); ai = fmaf(s6.y, -0.794854462146759f, ai); br = fmaf(d6.x, -0.6068001389503479f, br); bi = fmaf(d6.y, -0.6068001389503479f, bi);
-      ar = fmaf(s7.x, 0.9720228910446167f, ar); ai = fmaf(s7.y, 0.9720228910446167f, ai); br = fmaf(d7.x, 0.2348860502243042f, br); bi = fmaf(d7.y, 0.2348860502243042f, bi);
-      ar = fmaf(s8.x, -0.9842305779457092f, ar); ai = fmaf(s8.y, -0.9842305779457092f, ai); br = fmaf(d8.x, 0.1768902689218521f, br); bi = fmaf(d8.y, 0.1768902689218521f, bi);
-      ar = fmaf(s9.x, 0.829405665397644f, ar); ai = fmaf(s9.y, 0.829405665397644f, ai); br = fmaf(d9.x, -0.5586467385292053f, br); bi = fmaf(d9.y, -0.5586467385292053f, bi);
-      ar = fmaf(s10.x, -0.5338233709335327f, ar); ai = fmaf(s10.y, -0.5338233709335327f, ai); br = fmaf(d10.x, 0.8455960154533386f, br); bi = fmaf(d10.y, 0.8455960154533386f, bi);
-      ar = fmaf(s11.x, 0.14764656126499176f, ar); ai = fmaf(s11.y, 0.14764656126499176f, ai); br = fmaf(d11.x, -0.989040195941925f, br); bi = fmaf(d11.y, -0.989040195941925f, bi);
-      ar = fmaf(s12.x, 0.26358717679977417f, ar); ai = fmaf(s12.y, 0.26358717679977417f, ai); br = fmaf(d12.x, 0.9646356105804443f, br); bi = fmaf(d12.y, 0.9646356105804443f, bi);
-      ar = fmaf(s13.x, -0.6300878524780273f, ar); ai = fmaf(s13.y, -0.6300878524780273f, ai); br = fmaf(d13.x, -0.7765238881111145f, br); bi = fmaf(d13.y, -0.7765238881111145f, bi);
-      ar = fmaf(s14.x, 0.8896570801734924f, ar); ai = fmaf(s14.y, 0.8896570801734924f, ai); br = fmaf(d14.x, 0.4566292464733124f, br); bi = fmaf(d14.y, 0.4566292464733124f, bi);
-      ar = fmaf(s15.x, -0.9982437491416931f, ar); ai = fmaf(s15.y, -0.9982437491416931f, ai); br = fmaf(d15.x, -0.05924062803387642f, br); bi = fmaf(d15.y, -0.05924062803387642f, bi);
-      ar = fmaf(s16.x, 0.9374196529388428f, ar); ai = fmaf(s16.y, 0.9374196529388428f, ai); br = fmaf(d16.x, -0.3482016324996948f, br); bi = fmaf(d16.y, -0.3482016324996948f, bi);
-      ar = fmaf(s17.x, -0.7175072431564331f, ar); ai = fmaf(s17.y, -0.7175072431564331f, ai); br = fmaf(d17.x, 0.6965510249137878f, br); bi = fmaf(d17.y, 0.6965510249137878f, bi);
-      ar = fmaf(s18.x, 0.3758275806903839f, ar); ai = fmaf(s18.y, 0.3758275806903839f, ai); br = fmaf(d18.x, -0.926689624786377f, br); bi = fmaf(d18.y, -0.926689624786377f, bi);
-      ar = fmaf(s19.x, 0.029633328318595886f, ar); ai = fmaf(s19.y, 0.029633328318595886f, ai); br = fmaf(d19.x, 0.9995608329772949f, br); bi = fmaf(d19.y, 0.9995608329772949f, bi);
-      ar = fmaf(s20.x, -0.43006521463394165f, ar); ai = fmaf(s20.y, -0.43006521463394165f, ai); br = fmaf(d20.x, -0.9027978181838989f, br); bi = fmaf(d20.y, -0.9027978181838989f, bi);
-      ar = fmaf(s21.x, 0.7575112581253052f, ar); ai = fmaf(s21.y, 0.7575112581253052f, ai); br = fmaf(d21.x, 0.6528221368789673f, br); bi = fmaf(d21.y, 0.6528221368789673f, bi);
-      ar = fmaf(s22.x, -0.956400990486145f, ar); ai = fmaf(s22.y, -0.956400990486145f, ai); br = fmaf(d22.x, -0.29205676913261414f, br); bi = fmaf(d22.y, -0.29205676913261414f, bi);
-      ar = fmaf(s23.x, 0.9929810762405396f, ar); ai = fmaf(s23.y, 0.9929810762405396f, ai); br = fmaf(d23.x, -0.11827316880226135f, br); bi = fmaf(d23.y, -0.11827316880226135f, bi);
-      ar = fmaf(s24.x, -0.8610436320304871f, ar); ai = fmaf(s24.y, -0.8610436320304871f, ai); br = fmaf(d24.x, 0.5085310935974121f, br); bi = fmaf(d24.y, 0.5085310935974121f, bi);
-      ar = fmaf(s25.x, 0.5829795002937317f, ar); ai = fmaf(s25.y, 0.5829795002937317f, ai); br = fmaf(d25.x, -0.8124868869781494f, br); bi = fmaf(d25.y, -0.8124868869781494f, bi);
-      ar = fmaf(s26.x, -0.2059786170721054f, ar); ai = fmaf(s26.y, -0.2059786170721054f, ai); br = fmaf(d26.x, 0.9785565137863159f, br); bi = fmaf(d26.y, 0.9785565137863159f, bi);
-      if (!INV) { st(23, make_float2(ar + bi, ai - br)); st(30, make_float2(ar - bi, ai + br)); }
-      else { st(23, make_float2(ar - bi, ai + br)); st(30, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.956400990486145f, ar); ai = fmaf(s1.y, -0.956400990486145f, ai); br = fmaf(d1.x, 0.29205676913261414f, br); bi = fmaf(d1.y, 0.29205676913261414f, bi);
-      ar = fmaf(s2.x, 0.829405665397644f, ar); ai = fmaf(s2.y, 0.829405665397644f, ai); br = fmaf(d2.x, -0.5586467385292053f, br); bi = fmaf(d2.y, -0.5586467385292053f, bi);
-      ar = fmaf(s3.x, -0.6300878524780273f, ar); ai = fmaf(s3.y, -0.6300878524780273f, ai); br = fmaf(d3.x, 0.7765238881111145f, br); bi = fmaf(d3.y, 0.7765238881111145f, bi);
-      ar = fmaf(s4.x, 0.3758275806903839f, ar); ai = fmaf(s4.y, 0.3758275806903839f, ai); br = fmaf(d4.x, -0.926689624786377f, br); bi = fmaf(d4.y, -0.926689624786377f, bi);
-      ar = fmaf(s5.x, -0.08879589289426804f, ar); ai = fmaf(s5.y, -0.08879589289426804f, ai); br = fmaf(d5.x, 0.9960498213768005f, br); bi = fmaf(d5.y, 0.9960498213768005f, bi);
-      ar = fmaf(s6.x, -0.2059786170721054f, ar); ai = fmaf(s6.y, -0.2059786170721054f, ai); br = fmaf(d6.x, -0.9785565137863159f, br); bi = fmaf(d6.y, -0.9785565137863159f, bi);
-      ar = fmaf(s7.x, 0.4827921986579895f, ar); ai = fmaf(s7.y, 0.4827921986579895f, ai); br = fmaf(d7.x, 0.8757349252700806f, br); bi = fmaf(d7.y, 0.8757349252700806f, bi);
-      ar = fmaf(s8.x, -0.7175072431564331f, ar); ai = fmaf(s8.y, -0.7175072431564331f, ai); br = fmaf(d8.x, -0.6965510249137878f, br); bi = fmaf(d8.y, -0.6965510249137878f, bi);
-      ar = fmaf(s9.x, 0.8896570801734924f, ar); ai = fmaf(s9.y, 0.8896570801734924f, ai); br = fmaf(d9.x, 0.4566292464733124f, br); bi = fmaf(d9.y, 0.4566292464733124f, bi);
-      ar = fmaf(s10.x, -0.9842305779457092f, ar); ai = fmaf(s10.y, -0.9842305779457092f, ai); br = fmaf(d10.x, -0.1768902689218521f, br); bi = fmaf(d10.y, -0.1768902689218521f, bi);
-      ar = fmaf(s11.x, 0.9929810762405396f, ar); ai = fmaf(s11.y, 0.9929810762405396f, ai); br = fmaf(d11.x, -0.11827316880226135f, br); bi = fmaf(d11.y, -0.11827316880226135f, bi);
-      ar = fmaf(s12.x, -0.9151456356048584f, ar); ai = fmaf(s12.y, -0.9151456356048584f, ai); br = fmaf(d12.x, 0.4031234383583069f, br); bi = fmaf(d12.y, 0.4031234383583069f, bi);
-      ar = fmaf(s13.x, 0.7575112581253052f, ar); ai = fmaf(s13.y, 0.7575112581253052f, ai); br = fmaf(d13.x, -0.6528221368789673f, br); bi = fmaf(d13.y, -0.6528221368789673f, bi);
-      ar = fmaf(s14.x, -0.5338233709335327f, ar); ai = fmaf(s14.y, -0.5338233709335327f, ai); br = fmaf(d14.x, 0.8455960154533386f, br); bi = fmaf(d14.y, 0.8455960154533386f, bi);
-      ar = fmaf(s15.x, 0.26358717679977417f, ar); ai = fmaf(s15.y, 0.26358717679977417f, ai); br = fmaf(d15.x, -0.9646356105804443f, br); bi = fmaf(d15.y, -0.9646356105804443f, bi);
-      ar = fmaf(s16.x, 0.029633328318595886f, ar); ai = fmaf(s16.y, 0.029633328318595886f, ai); br = fmaf(d16.x, 0.9995608329772949f, br); bi = fmaf(d16.y, 0.9995608329772949f, bi);
-      ar = fmaf(s17.x, -0.3202698528766632f, ar); ai = fmaf(s17.y, -0.3202698528766632f, ai); br = fmaf(d17.x, -0.9473263621330261f, br); bi = fmaf(d17.y, -0.9473263621330261f, bi);
-      ar = fmaf(s18.x, 0.5829795002937317f, ar); ai = fmaf(s18.y, 0.5829795002937317f, ai); br = fmaf(d18.x, 0.8124868869781494f, br); bi = fmaf(d18.y, 0.8124868869781494f, bi);
-      ar = fmaf(s19.x, -0.794854462146759f, ar); ai = fmaf(s19.y, -0.794854462146759f, ai); br = fmaf(d19.x, -0.6068001389503479f, br); bi = fmaf(d19.y, -0.6068001389503479f, bi);
-      ar = fmaf(s20.x, 0.9374196529388428f, ar); ai = fmaf(s20.y, 0.9374196529388428f, ai); br = fmaf(d20.x, 0.3482016324996948f, br); bi = fmaf(d20.y, 0.3482016324996948f, bi);
-      ar = fmaf(s21.x, -0.9982437491416931f, ar); ai = fmaf(s21.y, -0.9982437491416931f, ai); br = fmaf(d21.x, -0.05924062803387642f, br); bi = fmaf(d21.y, -0.05924062803387642f, bi);
-      ar = fmaf(s22.x, 0.9720228910446167f, ar); ai = fmaf(s22.y, 0.9720228910446167f, ai); br = fmaf(d22.x, -0.2348860502243042f, br); bi = fmaf(d22.y, -0.2348860502243042f, bi);
-      ar = fmaf(s23.x, -0.8610436320304871f, ar); ai = fmaf(s23.y, -0.8610436320304871f, ai); br = fmaf(d23.x, 0.5085310935974121f, br); bi = fmaf(d23.y, 0.5085310935974121f, bi);
-      ar = fmaf(s24.x, 0.674983024597168f, ar); ai = fmaf(s24.y, 0.674983024597168f, ai); br = fmaf(d24.x, -0.7378332614898682f, br); bi = fmaf(d24.y, -0.7378332614898682f, bi);
-      ar = fmaf(s25.x, -0.43006521463394165f, ar); ai = fmaf(s25.y, -0.43006521463394165f, ai); br = fmaf(d25.x, 0.9027978181838989f, br); bi = fmaf(d25.y, 0.9027978181838989f, bi);
-      ar = fmaf(s26.x, 0.14764656126499176f, ar); ai = fmaf(s26.y, 0.14764656126499176f, ai); br = fmaf(d26.x, -0.989040195941925f, br); bi = fmaf(d26.y, -0.989040195941925f, bi);
-      if (!INV) { st(24, make_float2(ar + bi, ai - br)); st(29, make_float2(ar - bi, ai + br)); }
-      else { st(24, make_float2(ar - bi, ai + br)); st(29, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.9842305779457092f, ar); ai = fmaf(s1.y, -0.9842305779457092f, ai); br = fmaf(d1.x, 0.1768902689218521f, br); bi = fmaf(d1.y, 0.1768902689218521f, bi);
-      ar = fmaf(s2.x, 0.9374196529388428f, ar); ai = fmaf(s2.y, 0.9374196529388428f, ai); br = fmaf(d2.x, -0.3482016324996948f, br); bi = fmaf(d2.y, -0.3482016324996948f, bi);
-      ar = fmaf(s3.x, -0.8610436320304871f, ar); ai = fmaf(s3.y, -0.8610436320304871f, ai); br = fmaf(d3.x, 0.5085310935974121f, br); bi = fmaf(d3.y, 0.5085310935974121f, bi);
-      ar = fmaf(s4.x, 0.7575112581253052f, ar); ai = fmaf(s4.y, 0.7575112581253052f, ai); br = fmaf(d4.x, -0.6528221368789673f, br); bi = fmaf(d4.y, -0.6528221368789673f, bi);
-      ar = fmaf(s5.x, -0.6300878524780273f, ar); ai = fmaf(s5.y, -0.6300878524780273f, ai); br = fmaf(d5.x, 0.7765238881111145f, br); bi = fmaf(d5.y, 0.7765238881111145f, bi);
-      ar = fmaf(s6.x, 0.4827921986579895f, ar); ai = fmaf(s6.y, 0.4827921986579895f, ai); br = fmaf(d6.x, -0.8757349252700806f, br); bi = fmaf(d6.y, -0.8757349252700806f, bi);
-      ar = fmaf(s7.x, -0.3202698528766632f, ar); ai = fmaf(s7.y, -0.3202698528766632f, ai); br = fmaf(d7.x, 0.9473263621330261f, br); bi = fmaf(d7.y, 0.9473263621330261f, bi);
-      ar = fmaf(s8.x, 0.14764656126499176f, ar); ai = fmaf(s8.y, 0.14764656126499176f, ai); br = fmaf(d8.x, -0.989040195941925f, br); bi = fmaf(d8.y, -0.989040195941925f, bi);
-      ar = fmaf(s9.x, 0.029633328318595886f, ar); ai = fmaf(s9.y, 0.029633328318595886f, ai); br = fmaf(d9.x, 0.9995608329772949f, br); bi = fmaf(d9.y, 0.9995608329772949f, bi);
-      ar = fmaf(s10.x, -0.2059786170721054f, ar); ai = fmaf(s10.y, -0.2059786170721054f, ai); br = fmaf(d10.x, -0.9785565137863159f, br); bi = fmaf(d10.y, -0.9785565137863159f, bi);
-      ar = fmaf(s11.x, 0.3758275806903839f, ar); ai = fmaf(s11.y, 0.3758275806903839f, ai); br = fmaf(d11.x, 0.926689624786377f, br); bi = fmaf(d11.y, 0.926689624786377f, bi);
-      ar = fmaf(s12.x, -0.5338233709335327f, ar); ai = fmaf(s12.y, -0.5338233709335327f, ai); br = fmaf(d12.x, -0.8455960154533386f, br); bi = fmaf(d12.y, -0.8455960154533386f, bi);
-      ar = fmaf(s13.x, 0.674983024597168f, ar); ai = fmaf(s13.y, 0.674983024597168f, ai); br = fmaf(d13.x, 0.7378332614898682f, br); bi = fmaf(d13.y, 0.7378332614898682f, bi);
-      ar = fmaf(s14.x, -0.794854462146759f, ar); ai = fmaf(s14.y, -0.794854462146759f, ai); br = fmaf(d14.x, -0.6068001389503479f, br); bi = fmaf(d14.y, -0.6068001389503479f, bi);
-      ar = fmaf(s15.x, 0.8896570801734924f, ar); ai = fmaf(s15.y, 0.8896570801734924f, ai); br = fmaf(d15.x, 0.4566292464733124f, br); bi = fmaf(d15.y, 0.4566292464733124f, bi);
-      ar = fmaf(s16.x, -0.956400990486145f, ar); ai = fmaf(s16.y, -0.956400990486145f, ai); br = fmaf(d16.x, -0.29205676913261414f, br); bi = fmaf(d16.y, -0.29205676913261414f, bi);
-      ar = fmaf(s17.x, 0.9929810762405396f, ar); ai = fmaf(s17.y, 0.9929810762405396f, ai); br = fmaf(d17.x, 0.11827316880226135f, br); bi = fmaf(d17.y, 0.11827316880226135f, bi);
-      ar = fmaf(s18.x, -0.9982437491416931f, ar); ai = fmaf(s18.y, -0.9982437491416931f, ai); br = fmaf(d18.x, 0.05924062803387642f, br); bi = fmaf(d18.y, 0.05924062803387642f, bi);
-      ar = fmaf(s19.x, 0.9720228910446167f, ar); ai = fmaf(s19.y, 0.9720228910446167f, ai); br = fmaf(d19.x, -0.2348860502243042f, br); bi = fmaf(d19.y, -0.2348860502243042f, bi);
-      ar = fmaf(s20.x, -0.9151456356048584f, ar); ai = fmaf(s20.y, -0.9151456356048584f, ai); br = fmaf(d20.x, 0.4031234383583069f, br); bi = fmaf(d20.y, 0.4031234383583069f, bi);
-      ar = fmaf(s21.x, 0.829405665397644f, ar); ai = fmaf(s21.y, 0.829405665397644f, ai); br = fmaf(d21.x, -0.5586467385292053f, br); bi = fmaf(d21.y, -0.5586467385292053f, bi);
-      ar = fmaf(s22.x, -0.7175072431564331f, ar); ai = fmaf(s22.y, -0.7175072431564331f, ai); br = fmaf(d22.x, 0.6965510249137878f, br); bi = fmaf(d22.y, 0.6965510249137878f, bi);
-      ar = fmaf(s23.x, 0.5829795002937317f, ar); ai = fmaf(s23.y, 0.5829795002937317f, ai); br = fmaf(d23.x, -0.8124868869781494f, br); bi = fmaf(d23.y, -0.8124868869781494f, bi);
-      ar = fmaf(s24.x, -0.43006521463394165f, ar); ai = fmaf(s24.y, -0.43006521463394165f, ai); br = fmaf(d24.x, 0.9027978181838989f, br); bi = fmaf(d24.y, 0.9027978181838989f, bi);
-      ar = fmaf(s25.x, 0.26358717679977417f, ar); ai = fmaf(s25.y, 0.26358717679977417f, ai); br = fmaf(d25.x, -0.9646356105804443f, br); bi = fmaf(d25.y, -0.9646356105804443f, bi);
-      ar = fmaf(s26.x, -0.08879589289426804f, ar); ai = fmaf(s26.y, -0.08879589289426804f, ai); br = fmaf(d26.x, 0.9960498213768005f, br); bi = fmaf(d26.y, 0.9960498213768005f, bi);
-      if (!INV) { st(25, make_float2(ar + bi, ai - br)); st(28, make_float2(ar - bi, ai + br)); }
-      else { st(25, make_float2(ar - bi, ai + br)); st(28, make_float2(ar + bi, ai - br)); }
-    }
-    {
-      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;
-      ar = fmaf(s1.x, -0.9982437491416931f, ar); ai = fmaf(s1.y, -0.9982437491416931f, ai); br = fmaf(d1.x, 0.05924062803387642f, br); bi = fmaf(d1.y, 0.05924062803387642f, bi);
-      ar = fmaf(s2.x, 0.9929810762405396f, ar); ai = fmaf(s2.y, 0.9929810762405396f, ai); br = fmaf(d2.x, -0.11827316880226135f, br); bi = fmaf(d2.y, -0.11827316880226135f, bi);
-      ar = fmaf(s3.x, -0.9842305779457092f, ar); ai = fmaf(s3.y, -0.9842305779457092f, ai); br = fmaf(d3.x, 0.1768902689218521f, br); bi = fmaf(d3.y, 0.1768902689218521f, bi);
-      ar = fmaf(s4.x, 0.9720228910446167f, ar); ai = fmaf(s4.y, 0.9720228910446167f, ai); br = fmaf(d4.x, -0.2348860502243042f, br); bi = fmaf(d4.y, -0.2348860502243042f, bi);
-      ar = fmaf(s5.x, -0.956400990486145f, ar); ai = fmaf(s5.y, -0.956400990486145f, ai); br = fmaf(d5.x, 0.29205676913261414f, br); bi = fmaf(d5.y, 0.29205676913261414f, bi);
-      ar = fmaf(s6.x, 0.9374196529388428f, ar); ai = fmaf(s6.y, 0.9374196529388428f, ai); br = fmaf(d6.x, -0.3482016324996948f, br); bi = fmaf(d6.y, -0.3482016324996948f, bi);
-      ar = fmaf(s7.x, -0.9151456356048584f, ar); ai = fmaf(s7.y, -0.9151456356048584f, ai); br = fmaf(d7.x, 0.4031234383583069f, br); bi = fmaf(d7.y, 0.4031234383583069f, bi);
-      ar = fmaf(s8.x, 0.8896570801734924f, ar); ai = fmaf(s8.y, 0.8896570801734924f, ai); br = fmaf(d8.x, -0.4566292464733124f, br); bi = fmaf(d8.y, -0.4566292464733124f, bi);
-      ar = fmaf(s9.x, -0.8610436320304871f, ar); ai = fmaf(s9.y, -0.8610436320304871f, ai); br = fmaf(d9.x, 0.5085310935974121f, br); bi = fmaf(d9.y, 0.5085310935974121f, bi);
-      ar = fmaf(s10.x, 0.829405665397644f, ar); ai = fmaf(s10.y, 0.829405665397644f, ai); br = fmaf(d10.x, -0.5586467385292053f, br); bi = fmaf(d10.y, -0.5586467385292053f, bi);
-      ar = fmaf(s11.x, -0.794854462146759f, ar); ai = fmaf(s11.y, -0.794854462146759f, ai); br = fmaf(d11.x, 0.6068001389503479f, br); bi = fmaf(d11.y, 0.6068001389503479f, bi);
-      ar = fmaf(s12.x, 0.7575112581253052f, ar); ai = fmaf(s12.y, 0.7575112581253052f, ai); br = fmaf(d12.x, -0.6528221368789673f, br); bi = fmaf(d12.y, -0.6528221368789673f, bi);
-      ar = fmaf(s13.x, -0.7175072431564331f, ar); ai = fmaf(s13.y, -0.7175072431564331f, ai); br = fmaf(d13.x, 0.6965510249137878f, br); bi = fmaf(d13.y, 0.6965510249137878f, bi);
-      ar = fmaf(s14.x, 0.674983024597168f, ar); ai = fmaf(s14.y, 0.674983024597168f, ai); br = fmaf(d14.x, -0.7378332614898682f, br); bi = fmaf(d14.y, -0.7378332614898682f, bi);
-      ar = fmaf(s15.x, -0.6300878524780273f, ar); ai = fmaf(s15.y, -0.6300878524780273f, ai); br = fmaf(d15.x, 0.7765238881111145f, br); bi = fmaf(d15.y, 0.7765238881111145f, bi);
-      ar = fmaf(s16.x, 0.5829795002937317f, ar); ai = fmaf(s16.y, 0.5829795002937317f, ai); br = fmaf(d16.x, -0.8124868869781494f, br); bi = fmaf(d16.y, -0.8124868869781494f, bi);
-      ar = fmaf(s17.x, -0.5338233709335327f, ar); ai = fmaf(s17.y, -0.5338233709335327f, ai); br = fmaf(d17.x, 0.8455960154533386f, br); bi = fmaf(d17.y, 0.8455960154533386f, bi);
-      ar = fmaf(s18.x, 0.4827921986579895f, ar); ai = fmaf(s18.y, 0.4827921986579895f, ai); br = fmaf(d18.x, -0.8757349252700806f, br); bi = fmaf(d18.y, -0.8757349252700806f, bi);
-      ar = fmaf(s19.x, -0.43006521463394165f, ar); ai = fmaf(s19.y, -0.43006521463394165f, ai); br = fmaf(d19.x, 0.9027978181838989f, br); bi = fmaf(d19.y, 0.9027978181838989f, bi);
-      ar = fmaf(s20.x, 0.3758275806903839f, ar); ai = fmaf(s20.y, 0.3758275806903839f, ai); br = fmaf(d20.x, -0.926689624786377f, br); bi = fmaf(d20.y, -0.926689624786377f, bi);
-      ar = fmaf(s21.x, -0.3202698528766632f, ar); ai = fmaf(s21.y, -0.3202698528766632f, ai); br = fmaf(d21.x, 0.9473263621330261f, br); bi = fmaf(d21.y, 0.9473263621330261f, bi);
-      ar = fmaf(s22.x, 0.26358717679977417f, ar); ai = fmaf(s22.y, 0.26358717679977417f, ai); br = fmaf(d22.x, -0.9646356105804443f, br); bi = fmaf(d22.y, -0.9646356105804443f, bi);
-      ar = fmaf(s23.x, -0.2059786170721054f, ar); ai = fmaf(s23.y, -0.2059786170721054f, ai); br = fmaf(d23.x, 0.9785565137863159f, br); bi = fmaf(d23.y, 0.9785565137863159f, bi);
-      ar = fmaf(s24.x, 0.14764656126499176f, ar); ai = fmaf(s24.y, 0.14764656126499176f, ai); br = fmaf(d24.x, -0.989040195941925f, br); bi = fmaf(d24.y, -0.989040195941925f, bi);
-      ar = fmaf(s25.x, -0.08879589289426804f, ar); ai = fmaf(s25.y, -0.08879589289426804f, ai); br = fmaf(d25.x, 0.9960498213768005f, br); bi = fmaf(d25.y, 0.9960498213768005f, bi);
-      ar = fmaf(s26.x, 0.029633328318595886f, ar); ai = fmaf(s26.y, 0.029633328318595886f, ai); br = fmaf(d26.x, -0.9995608329772949f, br); bi = fmaf(d26.y, -0.9995608329772949f, bi);
-      if (!INV) { st(26, make_float2(ar + bi, ai - br)); st(27, make_float2(ar - bi, ai + br)); }
-      else { st(26, make_float2(ar - bi, ai + br)); st(27, make_float2(ar + bi, ai - br)); }
-    }
-    break;
-  }
-  default: break;
-  }
 }
 __constant__ float2 c_tw53[27][27] = {{{1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}, {1.0f, 0.0f}},
   {{1.0f, 0.0f}, {0.9929810762405396f, 0.11827316880226135f}, {0.9720228910446167f, 0.2348860502243042f}, {0.9374196529388428f, 0.3482016324996948f}, {0.8896570801734924f, 0.4566292464733124f}, {0.829405665397644f, 0.5586467385292053f}, {0.7575112581253052f, 0.6528221368789673f}, {0.674983024597168f, 0.7378332614898682f}, {0.5829795002937317f, 0.8124868869781494f}, {0.4827921986579895f, 0.8757349252700806f}, {0.3758275806903839f, 0.926689624786377f}, {0.26358717679977417f, 0.9646356105804443f}, {0.14764656126499176f, 0.989040195941925f}, {0.029633328318595886f, 0.9995608329772949f}, {-0.08879589289426804f, 0.9960498213768005f}, {-0.2059786170721054f, 0.9785565137863159f}, {-0.3202698528766632f, 0.9473263621330261f}, {-0.43006521463394165f, 0.9027978181838989f}, {-0.5338233709335327f, 0.8455960154533386f}, {-0.6300878524780273f, 0.7765238881111145f}, {-0.7175072431564331f, 0.6965510249137878f}, {-0.794854462146759f, 0.6068001389503479f}, {-0.8610436320304871f, 0.5085310935974121f}, {-0.9151456356048584f, 0.4031234383583069f}, {-0.956400990486145f, 0.29205676913261414f}, {-0.9842305779457092f, 0.1768902689218521f}, {-0.9982437491416931f, 0.05924062803387642f}},

@@ -1,19 +1,5 @@
-// Mixed-radix Stockham FFT over shared memory.
-//
-// A transform of length n runs as a list of stages with radices R_0..R_{s-1}
-// (product n).  Stage s with span Ns = R_0*..*R_{s-1} does, for every
-// butterfly j in [0, n/R):
-//     v[r]  = src[j + r*n/R] * W_n^(r * (j mod Ns) * n/(Ns*R))      (r >= 1)
-//     v     = DFT_R(v)
-//     dst[(j div Ns)*Ns*R + (j mod Ns) + r*Ns] = v[r]
-// which leaves the result in natural order (autosort) after the last stage.
-// W_n = exp(-2 pi i / n) for the forward transform, its conjugate for the
-// inverse; both transforms are un-normalised (cuFFT / FFTW convention).
-//
-// A batch of B transforms shares the stages.  Two element layouts exist:
-//   rows        element (b, i) at b*ld + i   (thread index: i fastest)
-//   interleaved element (b, i) at b + B*i    (thread index: b fastest)
-// Both keep consecutive threads on consecutive shared-memory words.
+// Complex helpers, small butterflies and the plan of a mixed-radix transform
+// (mixed_fft.cuh runs it).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -54,7 +40,9 @@ __device__ __forceinline__ void fdivmod(uint32_t x, FastDiv f, uint32_t& q, uint
 struct FftStage {
   int R;          // radix
   int Ns;         // span before this stage
-  int tws;        // twiddle index step n/(Ns*R)
+  int tw;         // offset of the stage's factors W_(Ns R)^(r jm), [(r - 1) * Ns + jm], in the table memory
+  int G;          // prime radix with a cosine/sine table: output pairs a thread forms (0: none)
+  int ct, ctp;    // offset of that table (float2) and its row pitch (float4), [r - 1][k - 1] = (cos, sin)(2 pi r k / R)
   FastDiv nsdiv;  // divide by Ns
   FastDiv nqdiv;  // divide by n/R
 };
@@ -62,6 +50,7 @@ struct FftStage {
 struct FftPlan1D {
   int n;
   int nst;
+  int ntab;       // float2 entries of the table memory (fft_tables)
   FftStage st[kMaxStages];
 };
 
@@ -128,156 +117,6 @@ __device__ __forceinline__ void dft_any(float2* v) {
   else if constexpr (R == 7) dft_r7<INV>(v);
   else if constexpr (R == 11) dft_r11<INV>(v);
   else if constexpr (R == 13) dft_r13<INV>(v);
-  else if constexpr (R == 53) dft_r53<INV>(v);
-}
-
-// One Stockham stage with compile-time radix R over B transforms.
-// INTERLEAVED=false: element (b, i) at b*ld + i.  true: at b + B*i.
-template <int R, bool INV, bool INTERLEAVED>
-__device__ __forceinline__ void stage_fixed(const float2* __restrict__ src, float2* __restrict__ dst,
-                                            const FftStage& s, int B, FastDiv bdiv, int ld,
-                                            const float2* __restrict__ tw, int tid, int nth) {
-  const int nq = (int)s.nqdiv.d;
-  const int total = nq * B;
-  for (int t = tid; t < total; t += nth) {
-    uint32_t j, b;
-    if (INTERLEAVED) fdivmod((uint32_t)t, bdiv, j, b);
-    else fdivmod((uint32_t)t, s.nqdiv, b, j);
-    uint32_t jq, jm;
-    fdivmod(j, s.nsdiv, jq, jm);
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      const int i = (int)j + r * nq;
-      v[r] = INTERLEAVED ? src[b + B * i] : src[b * ld + i];
-    }
-    if (s.Ns > 1) {
-      const int step = (int)jm * s.tws;
-#pragma unroll
-      for (int r = 1; r < R; r++) {
-        float2 w = tw[r * step];
-        if (INV) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    dft_any<R, INV>(v);
-    const int base = (int)jq * s.Ns * R + (int)jm;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      const int i = base + r * s.Ns;
-      if (INTERLEAVED) dst[b + B * i] = v[r];
-      else dst[b * ld + i] = v[r];
-    }
-  }
-}
-
-// Radix-53 stage with every butterfly spread over kSplit53 threads: each
-// thread loads the 53 inputs and produces its share of the outputs.  The
-// stage has only n/53 butterflies per transform, so this keeps the CTA busy.
-template <bool INV, bool INTERLEAVED>
-__device__ __forceinline__ void stage_r53_split(const float2* __restrict__ src, float2* __restrict__ dst,
-                                                const FftStage& s, int B, FastDiv bdiv, int ld,
-                                                const float2* __restrict__ tw, int tid, int nth) {
-  constexpr int R = 53;
-  const int nq = (int)s.nqdiv.d;
-  const int total = nq * B * kSplit53;
-  const FastDiv sdiv = make_fastdiv((uint32_t)kSplit53);
-  for (int t = tid; t < total; t += nth) {
-    uint32_t jb, part;
-    fdivmod((uint32_t)t, sdiv, jb, part);
-    uint32_t j, b;
-    if (INTERLEAVED) fdivmod(jb, bdiv, j, b);
-    else fdivmod(jb, s.nqdiv, b, j);
-    uint32_t jq, jm;
-    fdivmod(j, s.nsdiv, jq, jm);
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      const int i = (int)j + r * nq;
-      v[r] = INTERLEAVED ? src[b + B * i] : src[b * ld + i];
-    }
-    if (s.Ns > 1) {
-      const int step = (int)jm * s.tws;
-#pragma unroll
-      for (int r = 1; r < R; r++) {
-        float2 w = tw[r * step];
-        if (INV) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    const int base = (int)jq * s.Ns * R + (int)jm;
-    dft_r53_part<INV>(v, (int)part, [&](int r, float2 x) {
-      const int i = base + r * s.Ns;
-      if (INTERLEAVED) dst[b + B * i] = x;
-      else dst[b * ld + i] = x;
-    });
-  }
-}
-
-// Runtime-radix fallback: every output of every butterfly as a direct sum,
-//   X_k = sum_r src[j + r*n/R] * W_n^(r*((j mod Ns)*tws + k*n/R)).
-template <bool INV, bool INTERLEAVED>
-__device__ void stage_generic(const float2* __restrict__ src, float2* __restrict__ dst, const FftStage& s,
-                              int n, int B, FastDiv bdiv, int ld, const float2* __restrict__ tw, int tid,
-                              int nth) {
-  const int R = s.R;
-  const int nq = (int)s.nqdiv.d;
-  const int total = nq * B * R;
-  const FastDiv rdiv = make_fastdiv((uint32_t)R);
-  for (int t = tid; t < total; t += nth) {
-    uint32_t jb, k;
-    fdivmod((uint32_t)t, rdiv, jb, k);
-    uint32_t j, b;
-    if (INTERLEAVED) fdivmod(jb, bdiv, j, b);
-    else fdivmod(jb, s.nqdiv, b, j);
-    uint32_t jq, jm;
-    fdivmod(j, s.nsdiv, jq, jm);
-    const int step = ((int)jm * s.tws + (int)k * nq) % n;
-    int e = 0;
-    float2 acc = make_float2(0.f, 0.f);
-    for (int r = 0; r < R; r++) {
-      const int i = (int)j + r * nq;
-      const float2 x = INTERLEAVED ? src[b + B * i] : src[b * ld + i];
-      float2 w = tw[e];
-      if (INV) w.y = -w.y;
-      const float2 p = cmul(x, w);
-      acc.x += p.x;
-      acc.y += p.y;
-      e += step;
-      if (e >= n) e -= n;
-    }
-    const int i = (int)jq * s.Ns * R + (int)jm + (int)k * s.Ns;
-    if (INTERLEAVED) dst[b + B * i] = acc;
-    else dst[b * ld + i] = acc;
-  }
-}
-
-// Runs all stages; a and b are the two shared-memory buffers.  Returns the
-// buffer holding the result.  Ends with a __syncthreads().
-template <bool INV, bool INTERLEAVED>
-__device__ float2* fft_run(float2* a, float2* b, const FftPlan1D& p, int B, int ld,
-                           const float2* __restrict__ tw, int tid, int nth) {
-  const FastDiv bdiv = make_fastdiv((uint32_t)B);
-  for (int si = 0; si < p.nst; si++) {
-    const FftStage& s = p.st[si];
-    switch (s.R) {
-      case 2: stage_fixed<2, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 3: stage_fixed<3, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 4: stage_fixed<4, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 5: stage_fixed<5, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 7: stage_fixed<7, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 8: stage_fixed<8, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 11: stage_fixed<11, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 13: stage_fixed<13, INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      case 53: stage_r53_split<INV, INTERLEAVED>(a, b, s, B, bdiv, ld, tw, tid, nth); break;
-      default: stage_generic<INV, INTERLEAVED>(a, b, s, p.n, B, bdiv, ld, tw, tid, nth); break;
-    }
-    __syncthreads();
-    float2* t = a;
-    a = b;
-    b = t;
-  }
-  return a;
 }
 
 }  // namespace mc

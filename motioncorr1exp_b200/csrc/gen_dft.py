@@ -15,7 +15,7 @@ the FMA instructions.  Run:  python gen_dft.py > dft_gen.cuh
 import math
 import sys
 
-ODD_RADICES = [3, 5, 7, 11, 13, 53]
+ODD_RADICES = [3, 5, 7, 11, 13]
 
 
 def flit(x: float) -> str:
@@ -30,35 +30,34 @@ def emit_odd(R: int) -> str:
     L = []
     L.append(f"template <bool INV> __device__ __forceinline__ void dft_r{R}(float2* v) {{")
     L.append("  const float2 x0 = v[0];")
-    if R < 53:
-        # MC_PACKED_FMA=1: the cosine and sine sums on packed FP32 pairs, one
-        # fma.f32x2 per term for the real and imaginary halves
-        L.append("#if MC_PACKED_FMA")
+    # MC_PACKED_FMA=1: the cosine and sine sums on packed FP32 pairs, one
+    # fma.f32x2 per term for the real and imaginary halves
+    L.append("#if MC_PACKED_FMA")
+    for n in range(1, h + 1):
+        L.append(f"  const f2reg S{n} = f2pk(padd(v[{n}], v[{R-n}]));")
+        L.append(f"  const f2reg D{n} = f2pk(psub(v[{n}], v[{R-n}]));")
+    sx = " + ".join([f"v[{n}].x + v[{R-n}].x" for n in range(1, h + 1)])
+    sy = " + ".join([f"v[{n}].y + v[{R-n}].y" for n in range(1, h + 1)])
+    L.append(f"  {{ float2 t = f2up(S1);")
+    for n in range(2, h + 1):
+        L.append(f"    {{ const float2 u = f2up(S{n}); t.x += u.x; t.y += u.y; }}")
+    L.append("    v[0] = make_float2(x0.x + t.x, x0.y + t.y); }")
+    for k in range(1, h + 1):
+        L.append("  {")
+        L.append("    f2reg A = f2pk(x0), B = 0ull;")
         for n in range(1, h + 1):
-            L.append(f"  const f2reg S{n} = f2pk(padd(v[{n}], v[{R-n}]));")
-            L.append(f"  const f2reg D{n} = f2pk(psub(v[{n}], v[{R-n}]));")
-        sx = " + ".join([f"v[{n}].x + v[{R-n}].x" for n in range(1, h + 1)])
-        sy = " + ".join([f"v[{n}].y + v[{R-n}].y" for n in range(1, h + 1)])
-        L.append(f"  {{ float2 t = f2up(S1);")
-        for n in range(2, h + 1):
-            L.append(f"    {{ const float2 u = f2up(S{n}); t.x += u.x; t.y += u.y; }}")
-        L.append("    v[0] = make_float2(x0.x + t.x, x0.y + t.y); }")
-        for k in range(1, h + 1):
-            L.append("  {")
-            L.append("    f2reg A = f2pk(x0), B = 0ull;")
-            for n in range(1, h + 1):
-                m = (n * k) % R
-                c = flit(math.cos(2.0 * math.pi * m / R))
-                s = flit(math.sin(2.0 * math.pi * m / R))
-                L.append(f"    A = f2fma(S{n}, f2splat({c}), A); B = f2fma(D{n}, f2splat({s}), B);")
-            L.append("    const float2 a = f2up(A), b = f2up(B);")
-            L.append("    if (!INV) {")
-            L.append(f"      v[{k}] = make_float2(a.x + b.y, a.y - b.x); v[{R-k}] = make_float2(a.x - b.y, a.y + b.x);")
-            L.append("    } else {")
-            L.append(f"      v[{k}] = make_float2(a.x - b.y, a.y + b.x); v[{R-k}] = make_float2(a.x + b.y, a.y - b.x);")
-            L.append("    }")
-            L.append("  }")
-        L.append("#else")
+            m = (n * k) % R
+            c = flit(math.cos(2.0 * math.pi * m / R))
+            s = flit(math.sin(2.0 * math.pi * m / R))
+            L.append(f"    A = f2fma(S{n}, f2splat({c}), A); B = f2fma(D{n}, f2splat({s}), B);")
+        L.append("    const float2 a = f2up(A), b = f2up(B);")
+        L.append("    if (!INV) {")
+        L.append(f"      v[{k}] = make_float2(a.x + b.y, a.y - b.x); v[{R-k}] = make_float2(a.x - b.y, a.y + b.x);")
+        L.append("    } else {")
+        L.append(f"      v[{k}] = make_float2(a.x - b.y, a.y + b.x); v[{R-k}] = make_float2(a.x + b.y, a.y - b.x);")
+        L.append("    }")
+        L.append("  }")
+    L.append("#else")
     for n in range(1, h + 1):
         L.append(f"  const float2 s{n} = padd(v[{n}], v[{R-n}]);")
         L.append(f"  const float2 d{n} = psub(v[{n}], v[{R-n}]);")
@@ -81,46 +80,7 @@ def emit_odd(R: int) -> str:
         L.append(f"      v[{k}] = make_float2(ar - bi, ai + br); v[{R-k}] = make_float2(ar + bi, ai - br);")
         L.append("    }")
         L.append("  }")
-    if R < 53:
-        L.append("#endif")
-    L.append("}")
-    return "\n".join(L)
-
-
-def emit_odd_split(R: int, S: int) -> str:
-    """Radix-R butterfly whose outputs are split over S threads: part p
-    computes X_0 (p == 0) and the pairs (X_k, X_{R-k}) of its k-range, and
-    hands each output to st(index, value)."""
-    h = (R - 1) // 2
-    bounds = [round(i * h / S) for i in range(S + 1)]
-    L = [f"template <bool INV, typename St>",
-         f"__device__ __forceinline__ void dft_r{R}_part(const float2* v, int part, St&& st) {{",
-         "  const float2 x0 = v[0];"]
-    for n in range(1, h + 1):
-        L.append(f"  const float2 s{n} = padd(v[{n}], v[{R-n}]);")
-        L.append(f"  const float2 d{n} = psub(v[{n}], v[{R-n}]);")
-    sx = " + ".join([f"s{n}.x" for n in range(1, h + 1)])
-    sy = " + ".join([f"s{n}.y" for n in range(1, h + 1)])
-    L.append(f"  if (part == 0) st(0, make_float2(x0.x + ({sx}), x0.y + ({sy})));")
-    L.append("  switch (part) {")
-    for p in range(S):
-        L.append(f"  case {p}: {{")
-        for k in range(bounds[p] + 1, bounds[p + 1] + 1):
-            L.append("    {")
-            L.append("      float ar = x0.x, ai = x0.y, br = 0.0f, bi = 0.0f;")
-            for n in range(1, h + 1):
-                m = (n * k) % R
-                c = flit(math.cos(2.0 * math.pi * m / R))
-                s = flit(math.sin(2.0 * math.pi * m / R))
-                L.append(f"      ar = fmaf(s{n}.x, {c}, ar); ai = fmaf(s{n}.y, {c}, ai);"
-                         f" br = fmaf(d{n}.x, {s}, br); bi = fmaf(d{n}.y, {s}, bi);")
-            L.append(f"      if (!INV) {{ st({k}, make_float2(ar + bi, ai - br)); st({R-k}, make_float2(ar - bi, ai + br)); }}")
-            L.append(f"      else {{ st({k}, make_float2(ar - bi, ai + br)); st({R-k}, make_float2(ar + bi, ai - br)); }}")
-            L.append("    }")
-        L.append("    break;")
-        L.append("  }")
-    L.append("  default: break;")
-    L.append("  }")
+    L.append("#endif")
     L.append("}")
     return "\n".join(L)
 
@@ -350,7 +310,8 @@ def emit_codelet(q: int) -> str:
 
 
 CODELETS = [4, 8, 10, 12, 14, 16, 20, 24, 28, 30, 32, 35, 40, 48, 56, 60, 64, 70]
-SPLIT53 = 3
+# further register radices of the mixed-radix engine (not pair-stage splits)
+RADIX_CODELETS = [6, 9, 15]
 
 
 def main() -> None:
@@ -371,8 +332,6 @@ def main() -> None:
         out.append(f"constexpr int kGeneratedOddRadices[] = {{{', '.join(map(str, ODD_RADICES))}}};")
         for R in ODD_RADICES:
             out.append(emit_odd(R))
-        out.append(f"constexpr int kSplit53 = {SPLIT53};")
-        out.append(emit_odd_split(53, SPLIT53))
         out.append(emit_odd_compact(53))
         out.append("}  // namespace mc")
     else:
@@ -382,22 +341,22 @@ def main() -> None:
         out.append("namespace mc {")
         out.append(f"constexpr int kCodelets[] = {{{', '.join(map(str, CODELETS))}}};")
         out.append(f"constexpr int kNumCodelets = {len(CODELETS)};")
-        for q in CODELETS:
+        for q in sorted(CODELETS + RADIX_CODELETS):
             out.append(emit_codelet(q))
         out.append("template <int Q, bool INV> __device__ __forceinline__ void fft_reg(float2* a) {")
-        for i, q in enumerate(CODELETS):
+        for i, q in enumerate(sorted(CODELETS + RADIX_CODELETS)):
             kw = "if" if i == 0 else "else if"
             out.append(f"  {kw} constexpr (Q == {q}) fft_reg_{q}<INV>(a);")
         out.append("}")
         # prime-factor (Good-Thomas) forms of the lengths with coprime factors:
         # the pair kernels use them (measured faster there; the forward
         # transforms keep the Stockham forms, which measured faster in them)
-        for q in CODELETS:
+        for q in sorted(CODELETS + RADIX_CODELETS):
             if pfa_plan(q):
                 out.append(emit_codelet_pfa(q))
         out.append("template <int Q, bool INV> __device__ __forceinline__ void fft_reg_pf(float2* a) {")
         first = True
-        for q in CODELETS:
+        for q in sorted(CODELETS + RADIX_CODELETS):
             if pfa_plan(q):
                 out.append(f"  {'if' if first else 'else if'} constexpr (Q == {q}) fft_pfa_{q}<INV>(a);")
                 first = False

@@ -7,7 +7,7 @@
 #include <stdint.h>
 
 #include "kernels.cuh"
-#include "codelets_gen.cuh"
+#include "mixed_fft.cuh"
 
 namespace mc {
 
@@ -24,11 +24,6 @@ __device__ __forceinline__ float load_pixel(const void* frame, int mode, long lo
     case MC_MODE_F16: return __half2float(((const __half*)frame)[idx]);
     default: return ((const float*)frame)[idx];
   }
-}
-
-// exp(+/-2 pi i m / len) tables live in shared memory for the whole kernel.
-__device__ __forceinline__ void copy_table(float2* dst, const float2* __restrict__ src, int cnt) {
-  for (int i = threadIdx.x; i < cnt; i += blockDim.x) dst[i] = src[i];
 }
 
 }  // namespace
@@ -49,12 +44,6 @@ __device__ __forceinline__ const void* fwd_frame(const FwdRowsArgs& a) {
 // generated radix-53 butterfly.  One CTA (a team of `T2L` threads) per
 // transform; step A's factors W_N^(n1 k2) come from a global table laid out
 // [k2][n1] (fft_tables), so the threads n1 of a warp read consecutive words.
-template <int N1, bool INV>
-__device__ __forceinline__ void fft_n1(float2* v) {
-  if constexpr (N1 == 53) dft_r53<INV>(v);
-  else fft_reg<N1, INV>(v);
-}
-
 // Built-in radix-53 schedules of the forward row / column transforms: two
 // output pairs per loop pass in both (measured on c2: the row pass 9 %
 // faster paired; the column pass 12 % faster paired once its stores lost
@@ -109,7 +98,7 @@ struct TwoLevel {
       // compact radix-53 DFT: small code, outputs stored as they are formed
       if (act) dft_r53_compact<INV, PAIRED>(v, [&](int k1, float2 x) { store(lt + N2 * k1, x); }, kmax);
     } else {
-      if (act) fft_n1<N1, INV>(v);
+      if (act) fft_reg<N1, INV>(v);
       if (act) {
 #pragma unroll
         for (int k1 = 0; k1 < N1; k1++) store(lt + N2 * k1, v[k1]);
@@ -118,7 +107,8 @@ struct TwoLevel {
   }
 };
 
-// Stage the two packed input rows of k_fwd_rows2l in shared memory: every
+// Stage the two packed input rows of k_fwd_rows2l or of one transform of
+// k_fwd_rows in shared memory: every
 // thread of the CTA issues independent typed loads of the raw pixels.
 template <typename Px>
 __device__ __forceinline__ void stage_rows(float2* xin, const FwdRowsArgs& a, long long r0, long long r1, int n,

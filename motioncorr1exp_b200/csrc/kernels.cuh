@@ -131,8 +131,7 @@ struct ShiftSumArgs {
   long long ld_out;
   FftPlan1D plan;        // length n (mode 1)
   const float2* tw;
-  float2* acc;           // mode 1: H x ldn scratch for the sum spectrum (split
-                         // accumulate / transform); null = fused kernel
+  float2* acc;           // mode 1: H x ldn scratch for the sum spectrum
   int accumulate;        // mode 0: 1 = add the listed frames onto out's contents
                          // (a sum over several launches), 0 = overwrite
 };
@@ -238,7 +237,7 @@ struct CountSumArgs {
 cudaError_t launch_count_sum(const CountSumArgs& a, cudaStream_t st);
 
 cudaError_t launch_fwd_rows(const FwdRowsArgs& a, cudaStream_t st);
-cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, int rows_per_cta, cudaStream_t st);
+cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, cudaStream_t st);
 cudaError_t launch_pair_cols(const PairColsArgs& a, cudaStream_t st);
 cudaError_t launch_pair_rows(const PairRowsArgs& a, cudaStream_t st);
 cudaError_t launch_peak(const PeakArgs& a, cudaStream_t st);
@@ -275,6 +274,17 @@ cudaError_t launch_ql_crop(const float2* spec, int ldn, int n, int d, float2* ou
 // h = 1 at kx = 0, d/2, else 2; tmp holds (d/2+1) x d complex.
 cudaError_t launch_ql_c2r(const float2* in, int d, float scale, float2* tmp, float* img, cudaStream_t st);
 
+// Launch shape of a mixed-radix kernel over `count` transforms: B per CTA,
+// threads, dynamic shared memory (two buffers of B rows).  `gather`: the
+// kernel's stores gain from two or more transforms side by side.
+struct MixedShape {
+  int B, threads;
+  size_t smem;
+};
+constexpr int kMixedMaxThreads = 512;
+constexpr int kMixedMinBlocks = 2;
+MixedShape mixed_shape(const FftPlan1D& p, int count, bool gather);
+
 // Sets the calling thread's mc_last_error() text; returns `code`.
 int record_error(int code, const char* text);
 
@@ -291,12 +301,8 @@ size_t pair_cols_reg_smem(int n, int team);
 // dynamic shared memory launch_pair_cols asks for with this split
 size_t pair_cols_launch_smem(int n, int P, int Q, int box);
 
-size_t fwd_rows_smem(int nu);
-size_t rows_fft_smem(int n, int rows_per_cta);
 size_t pair_cols_smem(int n, int P, int Q, int box);
 // the generic column kernel keeps a length-n twiddle table instead of P x box
 inline bool pair_cols_tabn(int n, int P, int box) { return (long long)P * box > n; }
-size_t shift_sum_smem(int n, int nsum);
-size_t c2r_rows_smem(int n);
 
 }  // namespace mc

@@ -10,70 +10,60 @@
 namespace mc {
 
 // =========================================================== forward rows ==
-__global__ void __launch_bounds__(kThreads) k_fwd_rows(FwdRowsArgs a) {
-  const void* frame = fwd_frame(a);
+// Lengths without a compiled split: B packed transforms (two rows each, or
+// the two reference sets of one row) per CTA on the mixed-radix engine.  With
+// B >= 2 the CTA's half spectra of one kx fill 32-byte sectors of the
+// transposed store.
+__global__ void __launch_bounds__(kMixedMaxThreads, kMixedMinBlocks) k_fwd_rows(FwdRowsArgs a, int B) {
   extern __shared__ float2 sm[];
   const int nu = a.nu;
-  float2* b0 = sm;
-  float2* b1 = sm + nu;
-  float2* tw = sm + 2 * nu;
-  copy_table(tw, a.tw, nu);
+  float2* s0 = sm;
+  float2* s1 = sm + (size_t)B * nu;
   const int tid = threadIdx.x, nth = blockDim.x;
-  // rows handled by this CTA
-  int y0, y1;
-  if (a.two_outputs) {
-    y0 = blockIdx.x;
-    y1 = y0;
-  } else {
-    y0 = 2 * blockIdx.x;
-    y1 = y0 + 1;
-  }
-  const bool hasd = a.dark != nullptr, hasn = a.norm != nullptr;
-  const long long r0 = (long long)(a.offy + y0) * a.nx + a.offx;
-  const long long r1 = (long long)(a.offy + y1) * a.nx + a.offx;
-  for (int x = tid; x < nu; x += nth) {
-    float re, im;
-    if (a.two_outputs) {
-      const long long i0 = r0 + x;
-      const float raw = load_pixel(frame, a.mode, i0);
-      const float d1 = hasd ? a.dark[i0] : 0.f;
-      const float d2 = hasd ? (a.dark2 ? a.dark2[i0] : 0.f) : 0.f;
-      const float g1 = hasn ? a.norm[i0] : 1.f;
-      const float g2 = hasn ? (a.norm2 ? a.norm2[i0] : 1.f) : 1.f;
-      re = (raw - d1) * g1;  // hbuf   (DFAlign.cu:725)
-      im = (raw - d2) * g2;  // hbuf2  (DFAlign.cu:724)
-    } else {
-      re = load_pixel(frame, a.mode, r0 + x);
-      im = load_pixel(frame, a.mode, r1 + x);
-      if (hasd || hasn) {  // identical references: one spectrum per frame
-        const long long i0 = r0 + x, i1 = r1 + x;
-        re = (re - (hasd ? a.dark[i0] : 0.f)) * (hasn ? a.norm[i0] : 1.f);
-        im = (im - (hasd ? a.dark[i1] : 0.f)) * (hasn ? a.norm[i1] : 1.f);
-      }
+  const int q0 = blockIdx.x * B, npair = a.two_outputs ? nu : nu / 2;
+  const int nb = min(B, npair - q0);
+  for (int b = 0; b < B; b++) {
+    float2* xin = s1 + (size_t)b * nu;
+    if (b >= nb) {
+      for (int x = tid; x < nu; x += nth) xin[x] = make_float2(0.f, 0.f);
+      continue;
     }
-    b0[x] = make_float2(re, im);
+    const int y0 = a.two_outputs ? q0 + b : 2 * (q0 + b);
+    const long long r0 = (long long)(a.offy + y0) * a.nx + a.offx, r1 = a.two_outputs ? r0 : r0 + a.nx;
+    switch (a.mode) {
+      case 0: stage_rows<int8_t>(xin, a, r0, r1, nu, nth); break;
+      case MC_MODE_U8: stage_rows<uint8_t>(xin, a, r0, r1, nu, nth); break;
+      case 1: stage_rows<int16_t>(xin, a, r0, r1, nu, nth); break;
+      case 6: stage_rows<uint16_t>(xin, a, r0, r1, nu, nth); break;
+      case MC_MODE_F16: stage_rows<__half>(xin, a, r0, r1, nu, nth); break;
+      default: stage_rows<float>(xin, a, r0, r1, nu, nth); break;
+    }
   }
   __syncthreads();
-  float2* Z = fft_run<false, false>(b0, b1, a.plan, 1, nu, tw, tid, nth);
+  fft_exec<false, false>(
+      s0, s1, a.plan, B, nu, a.tw, tid, nth, [&](int b, int i) { return s1[b * nu + i]; },
+      [&](float2* dst, int b, int i, float2 v) { dst[b * nu + i] = v; });
+  __syncthreads();
+  const float2* Z = (a.plan.nst & 1) ? s0 : s1;
   float2* outA = a.outA + blockIdx.y * a.out_stride;
   float2* outB = a.two_outputs ? a.outB + blockIdx.y * a.out_stride : nullptr;
   // split the two real transforms: X = (Z(k) + conj Z(-k))/2, Y = -i (Z(k) - conj Z(-k))/2
-  for (int k = tid; k < a.hk; k += nth) {
-    const float2 z = Z[k];
-    const float2 zc = Z[k == 0 ? 0 : nu - k];
+  for (int t = tid; t < a.hk * B; t += nth) {
+    const int k = t / B, b = t - k * B;
+    if (b >= nb) continue;
+    const float2* z0 = Z + b * nu;
+    const float2 z = z0[k];
+    const float2 zc = z0[k == 0 ? 0 : nu - k];
     const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
     const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
     if (a.two_outputs) {
-      outA[(long long)k * a.ldt + y0] = X;
-      outB[(long long)k * a.ldt + y0] = Y;
+      outA[(long long)k * a.ldt + q0 + b] = X;
+      outB[(long long)k * a.ldt + q0 + b] = Y;
     } else {
-      float4* dst = reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0);
-      *dst = make_float4(X.x, X.y, Y.x, Y.y);
+      *reinterpret_cast<float4*>(outA + (long long)k * a.ldt + 2 * (q0 + b)) = make_float4(X.x, X.y, Y.x, Y.y);
     }
   }
 }
-
-size_t fwd_rows_smem(int nu) { return (size_t)3 * nu * sizeof(float2); }
 
 bool two_level_split(int n, int& n1, int& n2);
 cudaError_t launch_fwd_rows2l(const FwdRowsArgs& a, cudaStream_t st);
@@ -88,63 +78,55 @@ cudaError_t launch_fwd_rows(const FwdRowsArgs& a, cudaStream_t st) {
   if (two_level_split(a.nu, n1, n2)) return launch_fwd_rows2l(a, st);
   const bool raw = !a.two_outputs && !a.dark && !a.dark2 && !a.norm && !a.norm2;
   if (raw && dif_supported(a.nu)) return launch_fwd_rows_dif(a, st);
-  const size_t smem = fwd_rows_smem(a.nu);
-  cudaError_t e = allow_smem((const void*)k_fwd_rows, smem);
+  const int npair = a.two_outputs ? a.nu : a.nu / 2;
+  const MixedShape sh = mixed_shape(a.plan, npair * std::max(a.nfr, 1), true);
+  cudaError_t e = allow_smem((const void*)k_fwd_rows, sh.smem);
   if (e != cudaSuccess) return e;
-  const int grid = a.two_outputs ? a.nu : a.nu / 2;
-  k_fwd_rows<<<dim3(grid, std::max(a.nfr, 1)), kThreads, smem, st>>>(a);
+  const dim3 grid((npair + sh.B - 1) / sh.B, std::max(a.nfr, 1));
+  k_fwd_rows<<<grid, sh.threads, sh.smem, st>>>(a, sh.B);
   return cudaGetLastError();
 }
 
 // ========================================================= row transforms ==
 template <bool INV>
-__global__ void __launch_bounds__(kThreads) k_rows_fft(RowsFftArgs a, int rows_per_cta) {
+__global__ void __launch_bounds__(kMixedMaxThreads, kMixedMinBlocks) k_rows_fft(RowsFftArgs a, int B) {
   extern __shared__ float2 sm[];
   const int n = a.plan.n;
-  const int B = rows_per_cta;
-  float2* b0 = sm;
-  float2* b1 = sm + (size_t)B * n;
-  float2* tw = sm + (size_t)2 * B * n;
-  copy_table(tw, a.tw, n);
-  const int tid = threadIdx.x, nth = blockDim.x;
   const int row0 = blockIdx.x * B;
-  const float2* in = a.in + blockIdx.y * a.in_stride;
-  float2* out = a.out + blockIdx.y * a.out_stride;
   const int nb = min(B, a.nrows - row0);
-  for (int t = tid; t < B * n; t += nth) {
-    const int b = t / n, i = t - b * n;
-    b0[t] = (b < nb) ? in[(long long)(row0 + b) * a.ld_in + i] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  float2* X = fft_run<INV, false>(b0, b1, a.plan, B, n, tw, tid, nth);
+  const float2* in = a.in + blockIdx.y * a.in_stride + (long long)row0 * a.ld_in;
+  float2* out = a.out + blockIdx.y * a.out_stride + (long long)row0 * a.ld_out;
   const int shift = n - a.n_out;
-  for (int t = tid; t < nb * a.n_out; t += nth) {
-    const int b = t / a.n_out, i = t - b * a.n_out;
-    const int src = (i < a.keep_lo) ? i : i + shift;
-    const float2 v = X[b * n + src];
-    out[(long long)(row0 + b) * a.ld_out + i] = make_float2(v.x * a.scale, v.y * a.scale);
-  }
+  // in place: every stage but the last one leaves `out` alone, and a barrier
+  // (or, for a single stage, the thread's own order) precedes the last
+  fft_exec<INV, false>(
+      sm, sm + (size_t)B * n, a.plan, B, n, a.tw, threadIdx.x, blockDim.x,
+      [&](int b, int i) { return b < nb ? in[(long long)b * a.ld_in + i] : make_float2(0.f, 0.f); },
+      [&](float2*, int b, int i, float2 v) {
+        int o = i;
+        if (i >= a.keep_lo) {
+          if (i < a.keep_lo + shift) return;
+          o = i - shift;
+        }
+        if (b < nb) out[(long long)b * a.ld_out + o] = make_float2(v.x * a.scale, v.y * a.scale);
+      });
 }
 
-size_t rows_fft_smem(int n, int rows_per_cta) {
-  return (size_t)(2 * rows_per_cta + 1) * n * sizeof(float2);
-}
-
-cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, int rows_per_cta, cudaStream_t st) {
+cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, cudaStream_t st) {
   int n1, n2;
   if (two_level_split(a.plan.n, n1, n2)) return launch_rows_fft2l(a, inverse, st);
   if (!inverse && dif_supported(a.plan.n)) return launch_rows_fft_dif(a, st);
-  const size_t smem = rows_fft_smem(a.plan.n, rows_per_cta);
-  const dim3 grid((a.nrows + rows_per_cta - 1) / rows_per_cta, std::max(a.nfr, 1));
+  const MixedShape sh = mixed_shape(a.plan, a.nrows * std::max(a.nfr, 1), false);
+  const dim3 grid((a.nrows + sh.B - 1) / sh.B, std::max(a.nfr, 1));
   cudaError_t e;
   if (inverse) {
-    e = allow_smem((const void*)k_rows_fft<true>, smem);
+    e = allow_smem((const void*)k_rows_fft<true>, sh.smem);
     if (e != cudaSuccess) return e;
-    k_rows_fft<true><<<grid, kThreads, smem, st>>>(a, rows_per_cta);
+    k_rows_fft<true><<<grid, sh.threads, sh.smem, st>>>(a, sh.B);
   } else {
-    e = allow_smem((const void*)k_rows_fft<false>, smem);
+    e = allow_smem((const void*)k_rows_fft<false>, sh.smem);
     if (e != cudaSuccess) return e;
-    k_rows_fft<false><<<grid, kThreads, smem, st>>>(a, rows_per_cta);
+    k_rows_fft<false><<<grid, sh.threads, sh.smem, st>>>(a, sh.B);
   }
   return cudaGetLastError();
 }

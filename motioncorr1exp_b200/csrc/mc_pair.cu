@@ -13,10 +13,10 @@ namespace mc {
 
 // ============================================================ pair columns ==
 size_t pair_cols_smem(int n, int P, int Q, int box) {
+  (void)Q;
   const size_t outer = pair_cols_tabn(n, P, box) ? (size_t)n : (size_t)P * box;
   return (size_t)2 * n * sizeof(float2)     // ping-pong
          + (size_t)n * sizeof(float)        // B-factor column
-         + (size_t)Q * sizeof(float2)       // inner twiddles
          + outer * sizeof(float2);          // outer twiddles
 }
 
@@ -26,14 +26,12 @@ __global__ void __launch_bounds__(kThreads) k_pair_cols(PairColsArgs a) {
   float2* x0 = sm;
   float2* x1 = sm + n;
   float* wcol = reinterpret_cast<float*>(sm + 2 * n);
-  float2* twQ = reinterpret_cast<float2*>(wcol + n + (n & 1));  // keep 8-byte alignment
-  float2* twO = twQ + Q;
+  float2* twO = reinterpret_cast<float2*>(wcol + n + (n & 1));  // keep 8-byte alignment
   const int tid = threadIdx.x, nth = blockDim.x;
   const int kx = blockIdx.y;
   const bool tabn = a.twN != nullptr;
-  copy_table(twQ, a.twQ, Q);
-  if (tabn) copy_table(twO, a.twN, n);
-  else copy_table(twO, a.twO, P * box);
+  const float2* outer = tabn ? a.twN : a.twO;
+  for (int i = tid; i < (tabn ? n : P * box); i += nth) twO[i] = outer[i];
   const int half = n / 2;
   for (int ky = tid; ky < n; ky += nth) {
     const int y = ky < half ? ky : ky - n;
@@ -49,12 +47,17 @@ __global__ void __launch_bounds__(kThreads) k_pair_cols(PairColsArgs a) {
     const int2 pr = a.pairs[p];
     const float2* ca = a.specA + (long long)pr.x * a.strideA + (long long)kx * a.ldn;
     const float2* cb = a.specB + (long long)pr.y * a.strideB + (long long)kx * a.ldn;
-    for (int ky = tid; ky < n; ky += nth) {
-      const float2 u = ca[ky], v = cb[ky];
-      x0[ky] = cscale(cmulc(u, v), wcol[ky]);
+    // subsequence b holds ky = b + P i: the interleaved layout is ky's own order
+    auto product = [&](int ky) { return cscale(cmulc(__ldg(ca + ky), __ldg(cb + ky)), wcol[ky]); };
+    if (Q > 1) {
+      fft_exec<true, true>(
+          x0, x1, a.qplan, P, 0, a.twQ, tid, nth, [&](int b, int i) { return product(b + P * i); },
+          [&](float2* dst, int b, int i, float2 v) { dst[b + P * i] = v; });
+    } else {
+      for (int ky = tid; ky < n; ky += nth) x0[ky] = product(ky);
     }
     __syncthreads();
-    const float2* Y = fft_run<true, true>(x0, x1, a.qplan, P, 0, twQ, tid, nth);
+    const float2* Y = Q == 1 || (a.qplan.nst & 1) ? x0 : x1;
     for (int base = 0; base < nout; base += nth) {
       const int o = base + tid;
       const bool ok = o < nout;

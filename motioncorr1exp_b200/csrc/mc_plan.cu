@@ -80,6 +80,7 @@ namespace {
 
 constexpr double kPi = 3.14159265358979323846;
 constexpr int kPairBatch = 512;
+constexpr int kTablePrime = 127;  // largest prime radix with a cosine/sine table (mixed_fft.cuh)
 constexpr int kPairsPerCta = 32;
 constexpr int kForwardCtas = 148 * 16;  // row CTAs (of four rows) a forward launch is filled to
 // spectrum slots: the fewest a plan works with (two blocks of two frames in
@@ -91,46 +92,61 @@ constexpr size_t kKeepFree = (size_t)256 << 20;
 inline long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 
 // ----------------------------------------------------------- FFT planning --
-const int kFixedRadices[] = {53, 13, 11, 7, 5, 3};
+// Instructions per point of a radix' butterfly (mixed_fft.cuh): its
+// arithmetic; a stage adds its shared-memory and twiddle traffic.
+double radix_arith(int r) {
+  static const double a[17] = {0, 0, 2, 5.3, 4, 7.2, 7.3, 9.4, 7.5, 13, 9.2, 13.6, 9.3, 15.7, 11.4, 12.5, 11};
+  return r <= 16 ? a[r] : (r <= kTablePrime ? 6.0 + 1.3 * r : 8.0 * r);
+}
+constexpr double kStageCost = 14.0;
+
+double radices_cost(const std::vector<int>& rad) {
+  double c = 0.0;
+  for (int r : rad) c += radix_arith(r) + kStageCost;
+  return c;
+}
+
+// The radices of length n that cost least: primes above 13 are stages of
+// their own, the rest splits into radices up to 16.
+void split_radices(int m, int top, std::vector<int>& cur, std::vector<int>& best) {
+  if (m == 1) {
+    if (best.empty() || radices_cost(cur) < radices_cost(best)) best = cur;
+    return;
+  }
+  for (int r = std::min(top, m); r >= 2; r--) {
+    if (m % r) continue;
+    cur.push_back(r);
+    split_radices(m / r, r, cur, best);
+    cur.pop_back();
+  }
+}
 
 std::vector<int> factor_radices(int n) {
-  std::vector<int> r;
+  std::vector<int> primes, cur, rad;
   int m = n;
-  for (int p : kFixedRadices)
+  for (int p = 2; p <= 13; p++)
+    while (m % p == 0) m /= p;
+  int smooth = n / m;
+  for (int p = 17; (long long)p * p <= m; p += 2)
     while (m % p == 0) {
-      r.push_back(p);
+      primes.push_back(p);
       m /= p;
     }
-  int twos = 0;
-  while (m % 2 == 0) {
-    twos++;
-    m /= 2;
-  }
-  // remaining primes -> runtime-radix stages (placed first: no twiddles)
-  std::vector<int> generic;
-  for (int p = 3; (long long)p * p <= m; p += 2)
-    while (m % p == 0) {
-      generic.push_back(p);
-      m /= p;
-    }
-  if (m > 1) generic.push_back(m);
-  std::vector<int> pw;
-  while (twos >= 3) {
-    if (twos == 4) {
-      pw.push_back(4);
-      pw.push_back(4);
-      twos = 0;
-      break;
-    }
-    pw.push_back(8);
-    twos -= 3;
-  }
-  if (twos == 2) pw.push_back(4);
-  if (twos == 1) pw.push_back(2);
-  std::vector<int> out = generic;
-  out.insert(out.end(), r.begin(), r.end());
-  out.insert(out.end(), pw.begin(), pw.end());
-  return out;
+  if (m > 1) primes.push_back(m);
+  if (smooth > 1) split_radices(smooth, 16, cur, rad);
+  // odd radices before even ones (mixed_fft.cuh), the primes first of all
+  std::sort(rad.begin(), rad.end(), [](int a, int b) { return a % 2 != b % 2 ? a % 2 > b % 2 : a > b; });
+  primes.insert(primes.end(), rad.begin(), rad.end());
+  return primes;
+}
+
+// Compiled two-level length the tables of n hold step A's factors for: n, or
+// n / 2 of the radix-2 split; 0 when there is none.
+int two_level_part(int n) {
+  int n1, n2;
+  if (mc::two_level_split(n, n1, n2)) return n;
+  if (n % 2 == 0 && mc::two_level_split(n / 2, n1, n2)) return n / 2;
+  return 0;
 }
 
 bool make_plan(int n, FftPlan1D& p) {
@@ -138,42 +154,47 @@ bool make_plan(int n, FftPlan1D& p) {
   if ((int)rad.size() > mc::kMaxStages) return false;
   p.n = n;
   p.nst = (int)rad.size();
-  int ns = 1;
+  int ns = 1, off = n + two_level_part(n);
   for (int s = 0; s < p.nst; s++) {
     mc::FftStage& st = p.st[s];
     st.R = rad[s];
     st.Ns = ns;
-    st.tws = n / (ns * rad[s]);
+    st.tw = off;
+    if (ns > 1) off += (rad[s] - 1) * ns;
+    st.G = 0;
+    if (rad[s] > 16 && rad[s] <= kTablePrime) {
+      // six or eight output pairs a thread, whichever leaves fewer of them idle
+      const int h = (rad[s] - 1) / 2;
+      st.G = (h + 5) / 6 * 6 < (h + 7) / 8 * 8 ? 6 : 8;
+      st.ctp = (h + st.G - 1) / st.G * (st.G / 2);
+      off = (off + 1) / 2 * 2;
+      st.ct = off;
+      off += h * st.ctp * 2;
+    }
     st.nsdiv = mc::make_fastdiv((uint32_t)ns);
     st.nqdiv = mc::make_fastdiv((uint32_t)(n / rad[s]));
     ns *= rad[s];
   }
+  p.ntab = off;
   return ns == n || n == 1;
 }
 
-// largest prime factor of n
-int max_prime(int n) {
-  int best = 1, m = n;
-  for (int p = 2; (long long)p * p <= m; p++)
-    while (m % p == 0) {
-      best = p;
-      m /= p;
-    }
-  return std::max(best, m);
-}
-
-double radix_cost(int r) {
-  switch (r) {
-    case 2: return 2.0;
-    case 4: return 2.5;
-    case 8: return 3.0;
-    case 3: return 3.0;
-    case 5: return 4.0;
-    case 7: return 5.0;
-    case 11: return 7.0;
-    case 13: return 8.0;
-    default: return (double)r;
+// Cost of a codelet length's radices 7, 5, 3, 8, 4, 2 per point.
+double codelet_cost(int q) {
+  static const int rad[] = {7, 5, 3};
+  static const double cost[] = {5.0, 4.0, 3.0};
+  double c = 0.0;
+  int stages = 0;
+  for (int i = 0; i < 3; i++)
+    for (; q % rad[i] == 0; q /= rad[i]) c += cost[i] + (stages++ ? 2.0 : 0.0);
+  int twos = 0;
+  for (; q % 2 == 0; q /= 2) twos++;
+  for (; twos > 0; stages++) {
+    const int t = twos == 4 ? 2 : std::min(twos, 3);
+    c += (t == 3 ? 3.0 : t == 2 ? 2.5 : 2.0) + (stages ? 2.0 : 0.0);
+    twos -= t;
   }
+  return c;
 }
 
 // Pair-stage schedules by binned side n (mc_schedule_set): the autotuner's
@@ -208,10 +229,7 @@ bool mc::reg_pair_split(int n, int box, int* Pout, int* Qout) {
   int P = 0, Q = 0;
   for (int q = 2; q <= n; q++) {
     if (n % q || !mc::pair_cols_reg_supported(n / q, q)) continue;
-    std::vector<int> rad = factor_radices(q);
-    double c = 0.0;
-    for (size_t s = 0; s < rad.size(); s++) c += radix_cost(rad[s]) + (s ? 2.0 : 0.0);
-    const double cost = (double)n * c + 4.0 * box * (n / q);
+    const double cost = (double)n * codelet_cost(q) + 4.0 * box * (n / q);
     if (cost < best) {
       best = cost;
       P = n / q;
@@ -226,6 +244,24 @@ bool mc::reg_pair_split(int n, int box, int* Pout, int* Qout) {
 
 namespace {
 
+// Sides the pair stage takes (others are MC_E_SIZE): those with a register
+// split, or with a split n = P*Q, Q of primes up to 13, whose column of
+// products, ping-pong buffer, weights and tables fit shared memory.
+bool pair_stage_takes(int n, int box) {
+  int P, Q;
+  if (mc::reg_pair_split(n, box, &P, &Q)) return true;
+  for (int q = 1; q <= n; q++) {
+    if (n % q) continue;
+    int m = q;
+    for (int p = 2; p <= 13; p++)
+      while (m % p == 0) m /= p;
+    if (m > 1) continue;
+    const size_t outer = mc::pair_cols_tabn(n, n / q, box) ? (size_t)n : (size_t)(n / q) * box;
+    if ((size_t)20 * n + 8 * (q + outer) + 16 <= 227 * 1024) return true;
+  }
+  return false;
+}
+
 // n = P*Q for the pruned inverse: Q-point FFTs + P-term output sums.
 void choose_prune(int n, int box, int& P, int& Q) {
   double best = 1e300;
@@ -237,12 +273,9 @@ void choose_prune(int n, int box, int& P, int& Q) {
     if (n % q) continue;
     const int p = n / q;
     if (mc::pair_cols_smem(n, p, q, box) + 16 > 227 * 1024) continue;  // must fit shared memory
-    if (q > 1 && max_prime(q) > 13) continue;
-    double c = 0.0;
-    if (q > 1) {
-      std::vector<int> rad = factor_radices(q);
-      for (size_t s = 0; s < rad.size(); s++) c += radix_cost(rad[s]) + (s ? 2.0 : 0.0);
-    }
+    const std::vector<int> rad = factor_radices(q);
+    if (q > 1 && *std::max_element(rad.begin(), rad.end()) > kTablePrime) continue;
+    const double c = radices_cost(rad);
     const double cost = (double)n * c + 4.0 * box * p;
     if (cost < best) {
       best = cost;
@@ -261,23 +294,39 @@ std::vector<float2> twiddles(int n, int sign) {
   return t;
 }
 
-// Twiddle memory of one transform length: exp(-2 pi i j / n), j < n, then
-// for a two-level length N1*N2 (or 2*N1*N2, the radix-2 split) step A's
-// factors exp(-2 pi i n1 k2 / (N1*N2)) laid out [k2][n1].  The threads n1 of
-// a warp read one k2 row each step: consecutive words, where the plain table
-// at n1*k2 made every load a gather of up to 32 lines (3710^2 x 40: row
-// pass 3.09 -> 2.98 ms, column pass 1.91 -> 1.79 ms; 7420^2 x 24 binned by 2:
-// 7.90 -> 7.00 and 3.34 -> 2.84 ms; the same floats, bitwise equal results).
-std::vector<float2> fft_tables(int n) {
+// Twiddle memory of one transform: exp(-2 pi i j / n), j < n; for a two-level
+// length N1*N2 (or 2*N1*N2, the radix-2 split) step A's factors
+// exp(-2 pi i n1 k2 / (N1*N2)) laid out [k2][n1]; then the mixed-radix
+// stages' factors and prime tables at the plan's offsets.  Each part lies in
+// the order its threads read it: consecutive words, where the plain table
+// made every load a gather of up to 32 lines (3710^2 x 40: row pass 3.09 ->
+// 2.98 ms, column pass 1.91 -> 1.79 ms; 7420^2 x 24 binned by 2: 7.90 -> 7.00
+// and 3.34 -> 2.84 ms; the same floats, bitwise equal results).
+std::vector<float2> fft_tables(const FftPlan1D& p) {
+  const int n = p.n;
   std::vector<float2> t = twiddles(n, -1);
-  int n1, n2, len = n;
-  if (!mc::two_level_split(len, n1, n2)) {
-    len = n / 2;
-    if (n % 2 || !mc::two_level_split(len, n1, n2)) return t;
+  t.resize(p.ntab, make_float2(0.f, 0.f));
+  int n1, n2;
+  const int len = two_level_part(n);
+  if (len) {
+    mc::two_level_split(len, n1, n2);
+    for (int k2 = 0; k2 < n2; k2++)
+      for (int i = 0; i < n1; i++) t[n + k2 * n1 + i] = t[(size_t)(n / len) * i * k2];
   }
-  t.reserve((size_t)n + len);
-  for (int k2 = 0; k2 < n2; k2++)
-    for (int i = 0; i < n1; i++) t.push_back(t[(size_t)(n / len) * i * k2]);
+  for (int s = 0; s < p.nst; s++) {
+    const mc::FftStage& st = p.st[s];
+    if (st.Ns > 1)
+      for (int r = 1; r < st.R; r++)
+        for (int m = 0; m < st.Ns; m++) t[st.tw + (r - 1) * st.Ns + m] = t[(size_t)r * m * (n / (st.Ns * st.R))];
+    if (st.G) {
+      const int h = (st.R - 1) / 2;
+      for (int r = 1; r <= h; r++)
+        for (int k = 1; k <= h; k++) {
+          const double a = 2.0 * kPi * ((r * k) % st.R) / st.R;
+          t[st.ct + (r - 1) * st.ctp * 2 + k - 1] = make_float2((float)std::cos(a), (float)std::sin(a));
+        }
+    }
+  }
   return t;
 }
 
@@ -364,7 +413,7 @@ struct mc_plan {
   float *d_pshift = nullptr, *d_pcc = nullptr;
   int* d_ppeak = nullptr;
   float2 *d_sum = nullptr, *d_T2 = nullptr, *d_ey = nullptr;
-  float2* d_sumacc = nullptr;  // sum spectrum of the split image sum (two-level n)
+  float2* d_sumacc = nullptr;  // sum spectrum of an image sum
   float* d_image = nullptr;
   int *d_sumframes = nullptr, *d_apply = nullptr;
   double2* d_sumshift = nullptr;
@@ -1111,7 +1160,8 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
     const int team = pl->P <= 32 ? 32 : (pl->P <= 64 ? 64 : 128);
     const size_t need = std::max(mc::pair_cols_launch_smem(pl->n, pl->P, pl->Q, pl->box),
                                  reg ? mc::pair_cols_reg_smem(pl->n, team) : (size_t)0);
-    if (need > 227 * 1024) return set_err(MC_E_SIZE, "pair stage does not fit shared memory for n=%d", pl->n);
+    if (need > 227 * 1024 || !pair_stage_takes(pl->n, pl->box))
+      return set_err(MC_E_SIZE, "pair stage does not fit shared memory for n=%d", pl->n);
     mc_schedule sc{};
     const bool have_sc = find_schedule(pl->n, &sc);
     pl->ppc = (have_sc && sc.pairs_per_cta > 0) ? std::min(sc.pairs_per_cta, 512) : kPairsPerCta;
@@ -1144,13 +1194,7 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
   CKR(pl->alloc(&pl->d_ppeak, sizeof(int) * 2 * pl->maxp));
   CKR(pl->alloc(&pl->d_sum, sizeof(float2) * pl->fstride));
   CKR(pl->alloc(&pl->d_T2, sizeof(float2) * (size_t)pl->n * pl->ldt2));
-  {
-    // image sums of two-level sizes accumulate into d_sumacc, then transform
-    // (other sizes run the single fused kernel)
-    int n1, n2;
-    if (mc::two_level_split(pl->n, n1, n2))
-      CKR(pl->alloc(&pl->d_sumacc, sizeof(float2) * pl->fstride));
-  }
+  CKR(pl->alloc(&pl->d_sumacc, sizeof(float2) * pl->fstride));
   CKR(pl->alloc(&pl->d_ey, sizeof(float2) * (size_t)capf * pl->n));
   CKR(pl->alloc(&pl->d_image, sizeof(float) * (size_t)pl->n * pl->n));
   CKR(pl->alloc(&pl->d_sumframes, sizeof(int) * capf));
@@ -1203,19 +1247,22 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
 
   // tables
   {
-    const std::vector<float2> t = fft_tables(pl->nu);
+    const std::vector<float2> t = fft_tables(pl->plan_nu);
     CKR(pl->alloc(&pl->d_tw_nu, sizeof(float2) * t.size()));
     CKR(upload(pl, pl->d_tw_nu, t));
   }
   if (pl->nu == pl->n) {
     pl->d_tw_n = pl->d_tw_nu;
   } else {
-    const std::vector<float2> t = fft_tables(pl->n);
+    const std::vector<float2> t = fft_tables(pl->plan_n);
     CKR(pl->alloc(&pl->d_tw_n, sizeof(float2) * t.size()));
     CKR(upload(pl, pl->d_tw_n, t));
   }
-  CKR(pl->alloc(&pl->d_twQ, sizeof(float2) * pl->Q));
-  CKR(upload(pl, pl->d_twQ, twiddles(pl->Q, -1)));
+  {
+    const std::vector<float2> t = fft_tables(pl->plan_q);
+    CKR(pl->alloc(&pl->d_twQ, sizeof(float2) * t.size()));
+    CKR(upload(pl, pl->d_twQ, t));
+  }
   if (!mc::pair_cols_reg_supported(pl->P, pl->Q) && mc::pair_cols_tabn(pl->n, pl->P, pl->box)) {
     // generic column kernel with a length-n outer table: exp(+2 pi i e / n)
     std::vector<float2> tn(pl->n);
@@ -1566,7 +1613,7 @@ static int enqueue_forward(mc_plan* pl, const std::vector<cudaEvent_t>* waits, i
         c.plan = pl->plan_nu;
         c.tw = pl->d_tw_nu;
         c.paired = pl->fwd_cols_pairing;
-        LAUNCH(pl, MC_K_FWD_COLS, t_bytes + s_bytes, mc::launch_rows_fft(c, false, 1, fs));
+        LAUNCH(pl, MC_K_FWD_COLS, t_bytes + s_bytes, mc::launch_rows_fft(c, false, fs));
       }
       continue;
     }
@@ -1588,7 +1635,7 @@ static int enqueue_forward(mc_plan* pl, const std::vector<cudaEvent_t>* waits, i
       c.paired = pl->fwd_cols_pairing;
       c.nfr = cnt;
       c.in_stride = c.out_stride = pl->fstride;
-      LAUNCH(pl, MC_K_FWD_COLS, t_bytes + s_bytes, mc::launch_rows_fft(c, false, 1, fs));
+      LAUNCH(pl, MC_K_FWD_COLS, t_bytes + s_bytes, mc::launch_rows_fft(c, false, fs));
     }
   }
   if (multi)
@@ -2182,7 +2229,7 @@ int mc_plan_quicklook(mc_plan* pl, int which, int16_t* out) {
     c.scale = 1.f;
     c.plan = pl->plan_n;
     c.tw = pl->d_tw_n;
-    CK(mc::launch_rows_fft(c, false, 1, pl->st));
+    CK(mc::launch_rows_fft(c, false, pl->st));
     scale = 1.0f / ((float)D * D);
   }
   CK(mc::launch_ql_c2r(spec, D, scale, tmp, pl->d_qlimg, pl->st));
@@ -2720,7 +2767,7 @@ int mc_fft1d(int n, int batch, int inverse, const void* d_in, void* d_out, void*
   FftPlan1D p{};
   if (!make_plan(n, p)) return set_err(MC_E_SIZE, "no FFT plan for %d", n);
   float2* tw = nullptr;
-  const std::vector<float2> t = fft_tables(n);
+  const std::vector<float2> t = fft_tables(p);
   CK(cudaMalloc(&tw, sizeof(float2) * t.size()));
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemcpyAsync(tw, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice, st);
@@ -2736,7 +2783,7 @@ int mc_fft1d(int n, int batch, int inverse, const void* d_in, void* d_out, void*
     a.scale = 1.f;
     a.plan = p;
     a.tw = tw;
-    e = mc::launch_rows_fft(a, inverse != 0, 1, st);
+    e = mc::launch_rows_fft(a, inverse != 0, st);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(tw);

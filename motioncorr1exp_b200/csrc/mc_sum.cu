@@ -331,50 +331,6 @@ cudaError_t launch_peak(const PeakArgs& a, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, k_peak, a, C);
 }
 
-// ============================================================== shift-sum ==
-size_t shift_sum_smem(int n, int nsum) {
-  return (size_t)3 * n * sizeof(float2) + (size_t)nsum * sizeof(float2);
-}
-
-__global__ void __launch_bounds__(kThreads) k_shift_sum(ShiftSumArgs a, const float2* __restrict__ ey) {
-  extern __shared__ float2 sm[];
-  const int n = a.n;
-  float2* acc = sm;
-  float2* b1 = sm + n;
-  float2* tw = sm + 2 * n;
-  float2* ex = sm + 3 * n;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int kx = blockIdx.x;
-  if (a.mode == 1) copy_table(tw, a.tw, n);
-  for (int f = tid; f < a.nsum; f += nth) {
-    double sn, cn;
-    // exp(+2 pi i sx kx / n), argument reduced in double
-    const double t = a.shifts[f].x * (double)kx / (double)n;
-    sincospi(2.0 * (t - rint(t)), &sn, &cn);
-    ex[f] = make_float2((float)cn, (float)sn);
-  }
-  for (int ky = tid; ky < n; ky += nth) acc[ky] = make_float2(0.f, 0.f);
-  __syncthreads();
-  for (int f = 0; f < a.nsum; f++) {
-    const float2* col = a.spec + (long long)a.frames[f] * a.stride + (long long)kx * a.ldn;
-    const float2 e = ex[f];
-    const float2* eyf = ey + (long long)f * n;
-    const bool ap = a.apply[f] != 0;
-    for (int ky = tid; ky < n; ky += nth) {
-      float2 v = col[ky];
-      if (ap) v = cmul(v, cmul(e, eyf[ky]));
-      acc[ky] = cadd(acc[ky], v);
-    }
-  }
-  __syncthreads();
-  if (a.mode == 0) {
-    for (int ky = tid; ky < n; ky += nth) a.out[(long long)kx * a.ld_out + ky] = acc[ky];
-    return;
-  }
-  float2* X = fft_run<true, false>(acc, b1, a.plan, 1, n, tw, tid, nth);
-  for (int y = tid; y < n; y += nth) a.out[(long long)y * a.ld_out + kx] = X[y];
-}
-
 // ============================================================ count sums ==
 // One thread per 4 consecutive crop pixels of a row; frames summed in int32
 // registers (exact: |pixel| <= 65535 and at most 2^15 frames).
@@ -427,73 +383,11 @@ __global__ void k_ramp(RampArgs a) {
   }
 }
 
-// Two-level variant for columns of length N1*N2: each thread keeps the
-// running sums of its E = ceil(n/256) column elements in registers, so a
-// frame's column is requested with E independent loads per thread; the final
-// inverse along ky is the two-level transform.
-template <int N1, int N2>
-__global__ void __launch_bounds__(kThreads) k_shift_sum2l(ShiftSumArgs a, const float2* __restrict__ ey) {
-  using TL = TwoLevel<N1, N2>;
-  constexpr int N = TL::N;
-  constexpr int E = (N + kThreads - 1) / kThreads;
-  extern __shared__ float2 sm2l[];
-  float2* col = sm2l;         // accumulated column, then the step-A input
-  float2* ysm = sm2l + N;     // exchange buffer
-  float2* ex = sm2l + 2 * N;  // per-frame exp(+2 pi i sx kx / n)
-  const int tid = threadIdx.x;
-  const int kx = blockIdx.x;
-  for (int f = tid; f < a.nsum; f += kThreads) {
-    double sn, cn;
-    const double t = a.shifts[f].x * (double)kx / (double)N;
-    sincospi(2.0 * (t - rint(t)), &sn, &cn);
-    ex[f] = make_float2((float)cn, (float)sn);
-  }
-  __syncthreads();
-  float2 acc[E];
-#pragma unroll
-  for (int j = 0; j < E; j++) acc[j] = make_float2(0.f, 0.f);
-  for (int f = 0; f < a.nsum; f++) {
-    const float2* c = a.spec + (long long)a.frames[f] * a.stride + (long long)kx * a.ldn;
-    const float2* eyf = ey + (long long)f * N;
-    const float2 e = ex[f];
-    const bool ap = a.apply[f] != 0;
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-      const int ky = tid + kThreads * j;
-      if (ky < N) {
-        float2 v = __ldg(c + ky);
-        if (ap) v = cmul(v, cmul(e, __ldg(eyf + ky)));
-        acc[j] = cadd(acc[j], v);
-      }
-    }
-  }
-  if (a.mode == 0) {
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-      const int ky = tid + kThreads * j;
-      if (ky < N) a.out[(long long)kx * a.ld_out + ky] = acc[j];
-    }
-    return;
-  }
-#pragma unroll
-  for (int j = 0; j < E; j++) {
-    const int ky = tid + kThreads * j;
-    if (ky < N) col[ky] = acc[j];
-  }
-  __syncthreads();
-  float2* out = a.out;
-  const long long ld = a.ld_out;
-  TL::template run<true, false>(ysm, a.tw + N, [&](int i) { return col[i]; },
-                                [&](int k, float2 v) { out[(long long)k * ld + kx] = v; });
-}
-
-// Accumulation alone (no transform): each CTA covers kSumChunk consecutive ky
-// of one kx column, kSumE per thread, with the operations and frame order of
-// the fused kernels, so the sum spectrum is bitwise the same.  The loads of
+// ============================================================== shift-sum ==
+// Accumulation (no transform): each CTA covers kSumChunk consecutive ky of
+// one kx column, kSumE per thread, frames added in list order.  The loads of
 // kSumG frames are issued before their products are added: 64 registers,
-// four CTAs per SM and 2 * kSumE * kSumG loads per thread in flight, where
-// the fused two-level kernel (its transform needs most of the register file)
-// runs one CTA per SM.  Measured on 3710^2 x 40 frames: 0.38 ms against a
+// four CTAs per SM and 2 * kSumE * kSumG loads per thread in flight.  Measured on 3710^2 x 40 frames: 0.38 ms against a
 // 0.34 ms HBM floor (kSumG = 1: 0.56 ms; kSumE = 2 or 8: slower).
 constexpr int kSumE = 4;
 constexpr int kSumG = 2;
@@ -560,8 +454,7 @@ __global__ void __launch_bounds__(kThreads) k_shift_acc(ShiftSumArgs a, const fl
 }
 
 // The inverse along ky of each accumulated column, written transposed
-// (out[y * ld_out + kx]) for the C2R row pass: the transform of the fused
-// two-level kernel, here at TwoLevel's own CTA size.
+// (out[y * ld_out + kx]) for the C2R row pass.
 template <int N1, int N2>
 __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS)
     k_sum_cols2l(const float2* __restrict__ in, long long ld_in, const float2* __restrict__ tw, float2* out,
@@ -574,6 +467,22 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS)
                                 [&](int k, float2 v) { out[(long long)k * ld_out + kx] = v; });
 }
 
+// The same for lengths without a compiled split, B columns per CTA on the
+// mixed-radix engine.
+__global__ void __launch_bounds__(kMixedMaxThreads, kMixedMinBlocks)
+    k_sum_cols(const float2* __restrict__ in, long long ld_in, FftPlan1D plan, const float2* __restrict__ tw,
+               float2* out, long long ld_out, int H, int B) {
+  extern __shared__ float2 sm[];
+  const int n = plan.n, kx0 = blockIdx.x * B, nb = min(B, H - kx0);
+  const float2* col = in + (long long)kx0 * ld_in;
+  fft_exec<true, false>(
+      sm, sm + (size_t)B * n, plan, B, n, tw, threadIdx.x, blockDim.x,
+      [&](int b, int i) { return b < nb ? __ldg(col + (long long)b * ld_in + i) : make_float2(0.f, 0.f); },
+      [&](float2*, int b, int i, float2 v) {
+        if (b < nb) out[(long long)i * ld_out + kx0 + b] = v;
+      });
+}
+
 cudaError_t launch_shift_acc(const ShiftSumArgs& a, const float2* ey, float2* out, long long ld_out,
                              cudaStream_t st) {
   const size_t smem = (size_t)a.nsum * sizeof(float2);
@@ -584,10 +493,7 @@ cudaError_t launch_shift_acc(const ShiftSumArgs& a, const float2* ey, float2* ou
   return cudaGetLastError();
 }
 
-int shift_sum_kernels(const ShiftSumArgs& a) {
-  int n1, n2;
-  return (a.mode == 1 && a.acc && two_level_split(a.n, n1, n2)) ? 3 : 2;  // k_ramp first
-}
+int shift_sum_kernels(const ShiftSumArgs& a) { return a.mode == 1 ? 3 : 2; }  // k_ramp first
 
 cudaError_t launch_shift_sum(const ShiftSumArgs& a, float2* ey, cudaStream_t st) {
   RampArgs r;
@@ -600,10 +506,10 @@ cudaError_t launch_shift_sum(const ShiftSumArgs& a, float2* ey, cudaStream_t st)
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (a.mode == 0) return launch_shift_acc(a, ey, a.out, a.ld_out, st);
+  e = launch_shift_acc(a, ey, a.acc, a.ldn, st);
+  if (e != cudaSuccess) return e;
   int n1 = 0, n2 = 0;
-  if (a.acc && two_level_split(a.n, n1, n2)) {
-    e = launch_shift_acc(a, ey, a.acc, a.ldn, st);
-    if (e != cudaSuccess) return e;
+  if (two_level_split(a.n, n1, n2)) {
 #define MC_TL_COLS(A, B)                                                                     \
   if (n1 == (A) && n2 == (B)) {                                                              \
     k_sum_cols2l<A, B><<<a.H, TwoLevel<A, B>::T, 0, st>>>(a.acc, a.ldn, a.tw, a.out, a.ld_out); \
@@ -612,64 +518,50 @@ cudaError_t launch_shift_sum(const ShiftSumArgs& a, float2* ey, cudaStream_t st)
     MC_TWO_LEVEL_LIST(MC_TL_COLS)
 #undef MC_TL_COLS
   }
-  if (two_level_split(a.n, n1, n2)) {
-    const size_t smem2 = (size_t)(2 * a.n + a.nsum) * sizeof(float2);
-#define MC_TL_SUM(A, B)                                                                                       \
-  if (n1 == (A) && n2 == (B)) {                                                                               \
-    e = allow_smem((const void*)k_shift_sum2l<A, B>, smem2);                                                \
-    if (e != cudaSuccess) return e;                                                                           \
-    k_shift_sum2l<A, B><<<a.H, kThreads, smem2, st>>>(a, ey);                                                 \
-    return cudaGetLastError();                                                                                \
-  }
-    MC_TWO_LEVEL_LIST(MC_TL_SUM)
-#undef MC_TL_SUM
-  }
-  const size_t smem = shift_sum_smem(a.n, a.nsum);
-  e = allow_smem((const void*)k_shift_sum, smem);
+  const MixedShape sh = mixed_shape(a.plan, a.H, true);
+  e = allow_smem((const void*)k_sum_cols, sh.smem);
   if (e != cudaSuccess) return e;
-  k_shift_sum<<<a.H, kThreads, smem, st>>>(a, ey);
+  k_sum_cols<<<(a.H + sh.B - 1) / sh.B, sh.threads, sh.smem, st>>>(a.acc, a.ldn, a.plan, a.tw, a.out, a.ld_out,
+                                                                   a.H, sh.B);
   return cudaGetLastError();
 }
 
 // ================================================================ C2R rows ==
-size_t c2r_rows_smem(int n) { return (size_t)3 * n * sizeof(float2); }
-
-__global__ void __launch_bounds__(kThreads) k_c2r_rows(C2rRowsArgs a) {
+// Row pairs y, y+1 packed as one complex inverse transform, B pairs per CTA.
+__global__ void __launch_bounds__(kMixedMaxThreads, kMixedMinBlocks) k_c2r_rows(C2rRowsArgs a, int B) {
   extern __shared__ float2 sm[];
-  const int n = a.n, H = a.H, half = n / 2;
-  float2* b0 = sm;
-  float2* b1 = sm + n;
-  float2* tw = sm + 2 * n;
-  copy_table(tw, a.tw, n);
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int y0 = 2 * blockIdx.x, y1 = y0 + 1;
-  const float2* g0 = a.t2 + (long long)y0 * a.ld_t2;
-  const float2* g1 = a.t2 + (long long)y1 * a.ld_t2;
-  for (int k = tid; k < n; k += nth) {
-    float2 u, v;
-    if (k <= half) {
-      u = g0[k];
-      v = g1[k];
-      if (k == 0 || k == half) {  // C2R uses only the real part of DC and Nyquist
-        u.y = 0.f;
-        v.y = 0.f;
-      }
-    } else {
-      u = g0[n - k];
-      v = g1[n - k];
-      u.y = -u.y;
-      v.y = -v.y;
-    }
-    b0[k] = make_float2(u.x - v.y, u.y + v.x);  // u + i v
-  }
-  (void)H;
-  __syncthreads();
-  float2* X = fft_run<true, false>(b0, b1, a.plan, 1, n, tw, tid, nth);
-  for (int x = tid; x < n; x += nth) {
-    const float2 z = X[x];
-    a.image[(long long)y0 * n + x] = z.x * a.scale;
-    a.image[(long long)y1 * n + x] = z.y * a.scale;
-  }
+  const int n = a.n, half = n / 2;
+  const int q0 = blockIdx.x * B, nb = min(B, half - q0);
+  const float2* g = a.t2 + (long long)(2 * q0) * a.ld_t2;
+  float* img = a.image + (long long)(2 * q0) * n;
+  fft_exec<true, false>(
+      sm, sm + (size_t)B * n, a.plan, B, n, a.tw, threadIdx.x, blockDim.x,
+      [&](int b, int k) {
+        if (b >= nb) return make_float2(0.f, 0.f);
+        const float2* g0 = g + (long long)(2 * b) * a.ld_t2;
+        const float2* g1 = g0 + a.ld_t2;
+        float2 u, v;
+        if (k <= half) {
+          u = g0[k];
+          v = g1[k];
+          if (k == 0 || k == half) {  // C2R uses only the real part of DC and Nyquist
+            u.y = 0.f;
+            v.y = 0.f;
+          }
+        } else {
+          u = g0[n - k];
+          v = g1[n - k];
+          u.y = -u.y;
+          v.y = -v.y;
+        }
+        return make_float2(u.x - v.y, u.y + v.x);  // u + i v
+      },
+      [&](float2*, int b, int x, float2 z) {
+        if (b >= nb) return;
+        float* i0 = img + (long long)(2 * b) * n;
+        i0[x] = z.x * a.scale;
+        i0[x + n] = z.y * a.scale;
+      });
 }
 
 // =============================================================== adjoint ==
@@ -1011,10 +903,10 @@ cudaError_t launch_c2r_rows(const C2rRowsArgs& a, cudaStream_t st) {
     MC_TWO_LEVEL_LIST(MC_TL_C2R)
 #undef MC_TL_C2R
   }
-  const size_t smem = c2r_rows_smem(a.n);
-  cudaError_t e = allow_smem((const void*)k_c2r_rows, smem);
+  const MixedShape sh = mixed_shape(a.plan, a.n / 2, false);
+  cudaError_t e = allow_smem((const void*)k_c2r_rows, sh.smem);
   if (e != cudaSuccess) return e;
-  k_c2r_rows<<<a.n / 2, kThreads, smem, st>>>(a);
+  k_c2r_rows<<<(a.n / 2 + sh.B - 1) / sh.B, sh.threads, sh.smem, st>>>(a, sh.B);
   return cudaGetLastError();
 }
 
