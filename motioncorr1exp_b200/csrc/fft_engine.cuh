@@ -37,12 +37,21 @@ __device__ __forceinline__ void fdivmod(uint32_t x, FastDiv f, uint32_t& q, uint
   r = (uint32_t)rr;
 }
 
+// One pass of a mixed-radix transform: two neighbouring stages of radix R1, R2
+// held in registers (kind R1 * 16 + R2, R2 = 1 for one stage), or one stage of
+// a prime above 13.
+constexpr int kStageDirect = 1, kStageSymmetric = 2, kStageGeneric = 3;
+constexpr int kPrimePairs = 6;  // output pairs a thread forms in the symmetric stage
+#define MC_FUSED_LIST(X) \
+  X(5, 5) X(7, 3) X(5, 3) X(3, 3) X(11, 2) X(7, 2) X(5, 2) X(3, 2) X(5, 4) X(3, 4) X(3, 8) X(4, 4) X(8, 2)
 struct FftStage {
-  int R;          // radix
-  int Ns;         // span before this stage
-  int tw;         // offset of the stage's factors W_(Ns R)^(r jm), [(r - 1) * Ns + jm], in the table memory
-  int G;          // prime radix with a cosine/sine table: output pairs a thread forms (0: none)
-  int ct, ctp;    // offset of that table (float2) and its row pitch (float4), [r - 1][k - 1] = (cos, sin)(2 pi r k / R)
+  int kind;
+  int R;          // radix (R1 * R2)
+  int Ns;         // span before this pass
+  int tw, tw2;    // offsets of the factors in the table memory: W_(Ns R1)^(r jm), [(r - 1) * Ns + jm], and the
+                  // second stage's W_(Ns R)^(r m), [(r - 1) * Ns * R1 + m]
+  int ct, ctp;    // prime stages: offset of the table (float2) and its row pitch (float4): direct
+                  // [r][k] = W_p^(r k), symmetric [r - 1][k - 1] = (cos, sin)(2 pi r k / p)
   FastDiv nsdiv;  // divide by Ns
   FastDiv nqdiv;  // divide by n/R
 };

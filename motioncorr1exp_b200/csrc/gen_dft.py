@@ -310,8 +310,6 @@ def emit_codelet(q: int) -> str:
 
 
 CODELETS = [4, 8, 10, 12, 14, 16, 20, 24, 28, 30, 32, 35, 40, 48, 56, 60, 64, 70]
-# further register radices of the mixed-radix engine (not pair-stage splits)
-RADIX_CODELETS = [6, 9, 15]
 
 
 def main() -> None:
@@ -341,22 +339,22 @@ def main() -> None:
         out.append("namespace mc {")
         out.append(f"constexpr int kCodelets[] = {{{', '.join(map(str, CODELETS))}}};")
         out.append(f"constexpr int kNumCodelets = {len(CODELETS)};")
-        for q in sorted(CODELETS + RADIX_CODELETS):
+        for q in CODELETS:
             out.append(emit_codelet(q))
         out.append("template <int Q, bool INV> __device__ __forceinline__ void fft_reg(float2* a) {")
-        for i, q in enumerate(sorted(CODELETS + RADIX_CODELETS)):
+        for i, q in enumerate(CODELETS):
             kw = "if" if i == 0 else "else if"
             out.append(f"  {kw} constexpr (Q == {q}) fft_reg_{q}<INV>(a);")
         out.append("}")
         # prime-factor (Good-Thomas) forms of the lengths with coprime factors:
         # the pair kernels use them (measured faster there; the forward
         # transforms keep the Stockham forms, which measured faster in them)
-        for q in sorted(CODELETS + RADIX_CODELETS):
+        for q in CODELETS:
             if pfa_plan(q):
                 out.append(emit_codelet_pfa(q))
         out.append("template <int Q, bool INV> __device__ __forceinline__ void fft_reg_pf(float2* a) {")
         first = True
-        for q in sorted(CODELETS + RADIX_CODELETS):
+        for q in CODELETS:
             if pfa_plan(q):
                 out.append(f"  {'if' if first else 'else if'} constexpr (Q == {q}) fft_pfa_{q}<INV>(a);")
                 first = False

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "kernels.cuh"
+#include "codelets_gen.cuh"
 #include "mixed_fft.cuh"
 
 namespace mc {

@@ -75,7 +75,7 @@ struct PairColsArgs {
   long long strideB;
   const int2* pairs;   // (frame of A, frame of B)
   int npairs;
-  int pairs_per_cta;
+  int pairs_per_cta;   // 0: chosen by the launch
   int n, ldn, H;
   float mbf;           // -0.5*bfactor/n/n as float
   float inv_size;      // 1 / ((n/2+1) n)
@@ -83,8 +83,6 @@ struct PairColsArgs {
   FftPlan1D qplan;     // length Q
   const float2* twQ;   // Q twiddles exp(-2 pi i m / Q)
   const float2* twO;   // [P][box] exp(+2 pi i k1 y_m / n)
-  const float2* twN;   // exp(+2 pi i e / n), n entries: when set (P*box > n), the generic
-                       // kernel reads twO[k1][m] as twN[(k1 * y_m) mod n] (the same floats)
   int box;
   int ystart;
   float2* G;           // [npairs][H][box]
@@ -281,7 +279,7 @@ struct MixedShape {
   int B, threads;
   size_t smem;
 };
-constexpr int kMixedMaxThreads = 512;
+constexpr int kMixedMaxThreads = 384;
 constexpr int kMixedMinBlocks = 2;
 MixedShape mixed_shape(const FftPlan1D& p, int count, bool gather);
 
@@ -297,12 +295,9 @@ bool pair_cols_reg_supported(int P, int Q);
 // the split n = P*Q a plan's register-codelet column stage uses for (n, box)
 // (schedule or cost model); false when n has none (mc_plan.cu)
 bool reg_pair_split(int n, int box, int* P, int* Q);
-size_t pair_cols_reg_smem(int n, int team);
 // dynamic shared memory launch_pair_cols asks for with this split
 size_t pair_cols_launch_smem(int n, int P, int Q, int box);
 
 size_t pair_cols_smem(int n, int P, int Q, int box);
-// the generic column kernel keeps a length-n twiddle table instead of P x box
-inline bool pair_cols_tabn(int n, int P, int box) { return (long long)P * box > n; }
 
 }  // namespace mc

@@ -40,7 +40,7 @@ cudaError_t allow_smem(const void* func, size_t bytes) {
 // Chosen by a model of one CTA's time: every stage runs ceil(butterflies /
 // threads) rounds, each costing a fixed latency plus its radix' traffic and
 // arithmetic, so thread counts that leave the last round of a stage nearly
-// empty lose; CTAs per SM follow from threads (64 registers each) and shared
+// empty lose; CTAs per SM follow from threads (80 registers each) and shared
 // memory.  The best is the one that finishes most transforms per SM and time.
 MixedShape mixed_shape(const FftPlan1D& p, int count, bool gather) {
   MixedShape best{1, 256, (size_t)2 * p.n * sizeof(float2)};
@@ -49,17 +49,19 @@ MixedShape mixed_shape(const FftPlan1D& p, int count, bool gather) {
     const size_t smem = (size_t)2 * B * p.n * sizeof(float2);
     if (smem > 200 * 1024 && B > 1) break;
     for (int th = 64; th <= kMixedMaxThreads; th += 32) {
-      const double res = std::min({2048 / th, 65536 / (th * 64), (int)(227 * 1024 / (smem + 1024)), 32});
+      const double res = std::min({2048 / th, 65536 / (th * 80), (int)(227 * 1024 / (smem + 1024)), 32});
       if (res < 1) continue;
       double t = 40.0;
       for (int s = 0; s < p.nst; s++) {
         const FftStage& st = p.st[s];
         const int nq = p.n / st.R, items = nq * B;
         auto rounds = [&](int k) { return (double)((k + th - 1) / th); };
-        if (st.G) {
-          const int h = (st.R - 1) / 2, ng = (h + st.G - 1) / st.G;
-          t += 40.0 + rounds(items * (h + 1)) * 24.0 + rounds(items * ng) * (20.0 + h * (4.5 * st.G + 4.0) * 0.5);
-        } else if (st.R > 16) {
+        if (st.kind == kStageSymmetric) {
+          const int h = (st.R - 1) / 2, ng = (h + kPrimePairs - 1) / kPrimePairs;
+          t += 40.0 + rounds(items * (h + 1)) * 24.0 + rounds(items * ng) * (20.0 + h * 16.0);
+        } else if (st.kind == kStageDirect) {
+          t += 40.0 + rounds(items * st.R) * 12.0 + rounds(items * ((st.R + 7) / 8)) * (20.0 + st.R * 28.0);
+        } else if (st.kind == kStageGeneric) {
           t += 40.0 + rounds(items * st.R) * (20.0 + 8.0 * st.R);
         } else {
           t += 40.0 + rounds(items) * (30.0 + 8.0 * st.R);

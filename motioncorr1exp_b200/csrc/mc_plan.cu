@@ -81,7 +81,6 @@ namespace {
 constexpr double kPi = 3.14159265358979323846;
 constexpr int kPairBatch = 512;
 constexpr int kTablePrime = 127;  // largest prime radix with a cosine/sine table (mixed_fft.cuh)
-constexpr int kPairsPerCta = 32;
 constexpr int kForwardCtas = 148 * 16;  // row CTAs (of four rows) a forward launch is filled to
 // spectrum slots: the fewest a plan works with (two blocks of two frames in
 // the pair stage), and the device memory the automatic choice leaves free
@@ -92,52 +91,74 @@ constexpr size_t kKeepFree = (size_t)256 << 20;
 inline long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 
 // ----------------------------------------------------------- FFT planning --
-// Instructions per point of a radix' butterfly (mixed_fft.cuh): its
-// arithmetic; a stage adds its shared-memory and twiddle traffic.
-double radix_arith(int r) {
-  static const double a[17] = {0, 0, 2, 5.3, 4, 7.2, 7.3, 9.4, 7.5, 13, 9.2, 13.6, 9.3, 15.7, 11.4, 12.5, 11};
-  return r <= 16 ? a[r] : (r <= kTablePrime ? 6.0 + 1.3 * r : 8.0 * r);
-}
-constexpr double kStageCost = 14.0;
-
-double radices_cost(const std::vector<int>& rad) {
-  double c = 0.0;
-  for (int r : rad) c += radix_arith(r) + kStageCost;
-  return c;
-}
-
-// The radices of length n that cost least: primes above 13 are stages of
-// their own, the rest splits into radices up to 16.
-void split_radices(int m, int top, std::vector<int>& cur, std::vector<int>& best) {
-  if (m == 1) {
-    if (best.empty() || radices_cost(cur) < radices_cost(best)) best = cur;
-    return;
-  }
-  for (int r = std::min(top, m); r >= 2; r--) {
-    if (m % r) continue;
-    cur.push_back(r);
-    split_radices(m / r, r, cur, best);
-    cur.pop_back();
-  }
-}
+const int kFixedRadices[] = {53, 13, 11, 7, 5, 3};
 
 std::vector<int> factor_radices(int n) {
-  std::vector<int> primes, cur, rad;
+  std::vector<int> r;
   int m = n;
-  for (int p = 2; p <= 13; p++)
-    while (m % p == 0) m /= p;
-  int smooth = n / m;
-  for (int p = 17; (long long)p * p <= m; p += 2)
+  for (int p : kFixedRadices)
     while (m % p == 0) {
-      primes.push_back(p);
+      r.push_back(p);
       m /= p;
     }
-  if (m > 1) primes.push_back(m);
-  if (smooth > 1) split_radices(smooth, 16, cur, rad);
-  // odd radices before even ones (mixed_fft.cuh), the primes first of all
-  std::sort(rad.begin(), rad.end(), [](int a, int b) { return a % 2 != b % 2 ? a % 2 > b % 2 : a > b; });
-  primes.insert(primes.end(), rad.begin(), rad.end());
-  return primes;
+  int twos = 0;
+  while (m % 2 == 0) {
+    twos++;
+    m /= 2;
+  }
+  // remaining primes -> runtime-radix stages (placed first: no twiddles)
+  std::vector<int> generic;
+  for (int p = 3; (long long)p * p <= m; p += 2)
+    while (m % p == 0) {
+      generic.push_back(p);
+      m /= p;
+    }
+  if (m > 1) generic.push_back(m);
+  std::vector<int> pw;
+  while (twos >= 3) {
+    if (twos == 4) {
+      pw.push_back(4);
+      pw.push_back(4);
+      twos = 0;
+      break;
+    }
+    pw.push_back(8);
+    twos -= 3;
+  }
+  if (twos == 2) pw.push_back(4);
+  if (twos == 1) pw.push_back(2);
+  std::vector<int> out = generic;
+  out.insert(out.end(), r.begin(), r.end());
+  out.insert(out.end(), pw.begin(), pw.end());
+  return out;
+}
+
+// Neighbouring radices (from rad[s] on) that run as one pass.
+int fused_pair(const std::vector<int>& rad, size_t s) {
+  if (s + 1 >= rad.size()) return 0;
+#define MC_FUSED_HAS(A, B) \
+  if (rad[s] == (A) && rad[s + 1] == (B)) return (A) * 16 + (B);
+  MC_FUSED_LIST(MC_FUSED_HAS)
+#undef MC_FUSED_HAS
+  return 0;
+}
+
+// Passes from radix s on: the fewest (fused[s] = 1: rad[s] and rad[s + 1] as one).
+int fewest_passes(const std::vector<int>& rad, size_t s, std::vector<int>& fused) {
+  if (s >= rad.size()) return 0;
+  std::vector<int> one = fused, two = fused;
+  int a = 1 + fewest_passes(rad, s + 1, one);
+  one[s] = 0;
+  if (fused_pair(rad, s)) {
+    const int b = 1 + fewest_passes(rad, s + 2, two);
+    two[s] = 1;
+    if (b <= a) {
+      fused = two;
+      return b;
+    }
+  }
+  fused = one;
+  return a;
 }
 
 // Compiled two-level length the tables of n hold step A's factors for: n, or
@@ -150,51 +171,66 @@ int two_level_part(int n) {
 }
 
 bool make_plan(int n, FftPlan1D& p) {
-  std::vector<int> rad = factor_radices(n);
-  if ((int)rad.size() > mc::kMaxStages) return false;
+  const std::vector<int> rad = factor_radices(n);
+  std::vector<int> fused(rad.size(), 0);
+  if (fewest_passes(rad, 0, fused) > mc::kMaxStages) return false;
   p.n = n;
-  p.nst = (int)rad.size();
+  p.nst = 0;
   int ns = 1, off = n + two_level_part(n);
-  for (int s = 0; s < p.nst; s++) {
-    mc::FftStage& st = p.st[s];
-    st.R = rad[s];
+  for (size_t s = 0; s < rad.size();) {
+    mc::FftStage& st = p.st[p.nst++];
+    const int r = rad[s];
+    st = mc::FftStage{};
+    st.R = r;
     st.Ns = ns;
+    st.kind = fused[s] ? fused_pair(rad, s) : r * 16 + 1;
+    if (r > 13) st.kind = r == 53 ? mc::kStageSymmetric : ns == 1 && r <= kTablePrime ? mc::kStageDirect : mc::kStageGeneric;
     st.tw = off;
-    if (ns > 1) off += (rad[s] - 1) * ns;
-    st.G = 0;
-    if (rad[s] > 16 && rad[s] <= kTablePrime) {
-      // six or eight output pairs a thread, whichever leaves fewer of them idle
-      const int h = (rad[s] - 1) / 2;
-      st.G = (h + 5) / 6 * 6 < (h + 7) / 8 * 8 ? 6 : 8;
-      st.ctp = (h + st.G - 1) / st.G * (st.G / 2);
-      off = (off + 1) / 2 * 2;
+    if (ns > 1 && st.kind != mc::kStageGeneric) off += (r - 1) * ns;
+    if (fused[s]) {
+      st.R *= rad[s + 1];
+      st.tw2 = off;
+      off += (rad[s + 1] - 1) * ns * r;
+    }
+    if (st.kind == mc::kStageDirect || st.kind == mc::kStageSymmetric) {
+      const int h = (r - 1) / 2, G = mc::kPrimePairs;
+      off = (off + 1) / 2 * 2;  // 16-byte rows
       st.ct = off;
-      off += h * st.ctp * 2;
+      st.ctp = st.kind == mc::kStageDirect ? (r + 7) / 8 * 4 : (h + G - 1) / G * (G / 2);
+      off += (st.kind == mc::kStageDirect ? r : h) * st.ctp * 2;
     }
     st.nsdiv = mc::make_fastdiv((uint32_t)ns);
-    st.nqdiv = mc::make_fastdiv((uint32_t)(n / rad[s]));
-    ns *= rad[s];
+    st.nqdiv = mc::make_fastdiv((uint32_t)(n / st.R));
+    ns *= st.R;
+    s += fused[s] ? 2 : 1;
   }
   p.ntab = off;
   return ns == n || n == 1;
 }
 
-// Cost of a codelet length's radices 7, 5, 3, 8, 4, 2 per point.
-double codelet_cost(int q) {
-  static const int rad[] = {7, 5, 3};
-  static const double cost[] = {5.0, 4.0, 3.0};
-  double c = 0.0;
-  int stages = 0;
-  for (int i = 0; i < 3; i++)
-    for (; q % rad[i] == 0; q /= rad[i]) c += cost[i] + (stages++ ? 2.0 : 0.0);
-  int twos = 0;
-  for (; q % 2 == 0; q /= 2) twos++;
-  for (; twos > 0; stages++) {
-    const int t = twos == 4 ? 2 : std::min(twos, 3);
-    c += (t == 3 ? 3.0 : t == 2 ? 2.5 : 2.0) + (stages ? 2.0 : 0.0);
-    twos -= t;
+// largest prime factor of n
+int max_prime(int n) {
+  int best = 1, m = n;
+  for (int p = 2; (long long)p * p <= m; p++)
+    while (m % p == 0) {
+      best = p;
+      m /= p;
+    }
+  return std::max(best, m);
+}
+
+double radix_cost(int r) {
+  switch (r) {
+    case 2: return 2.0;
+    case 4: return 2.5;
+    case 8: return 3.0;
+    case 3: return 3.0;
+    case 5: return 4.0;
+    case 7: return 5.0;
+    case 11: return 7.0;
+    case 13: return 8.0;
+    default: return (double)r;
   }
-  return c;
 }
 
 // Pair-stage schedules by binned side n (mc_schedule_set): the autotuner's
@@ -229,7 +265,10 @@ bool mc::reg_pair_split(int n, int box, int* Pout, int* Qout) {
   int P = 0, Q = 0;
   for (int q = 2; q <= n; q++) {
     if (n % q || !mc::pair_cols_reg_supported(n / q, q)) continue;
-    const double cost = (double)n * codelet_cost(q) + 4.0 * box * (n / q);
+    std::vector<int> rad = factor_radices(q);
+    double c = 0.0;
+    for (size_t s = 0; s < rad.size(); s++) c += radix_cost(rad[s]) + (s ? 2.0 : 0.0);
+    const double cost = (double)n * c + 4.0 * box * (n / q);
     if (cost < best) {
       best = cost;
       P = n / q;
@@ -244,38 +283,26 @@ bool mc::reg_pair_split(int n, int box, int* Pout, int* Qout) {
 
 namespace {
 
-// Sides the pair stage takes (others are MC_E_SIZE): those with a register
-// split, or with a split n = P*Q, Q of primes up to 13, whose column of
-// products, ping-pong buffer, weights and tables fit shared memory.
-bool pair_stage_takes(int n, int box) {
-  int P, Q;
-  if (mc::reg_pair_split(n, box, &P, &Q)) return true;
-  for (int q = 1; q <= n; q++) {
-    if (n % q) continue;
-    int m = q;
-    for (int p = 2; p <= 13; p++)
-      while (m % p == 0) m /= p;
-    if (m > 1) continue;
-    const size_t outer = mc::pair_cols_tabn(n, n / q, box) ? (size_t)n : (size_t)(n / q) * box;
-    if ((size_t)20 * n + 8 * (q + outer) + 16 <= 227 * 1024) return true;
-  }
-  return false;
-}
-
 // n = P*Q for the pruned inverse: Q-point FFTs + P-term output sums.
-void choose_prune(int n, int box, int& P, int& Q) {
+bool choose_prune(int n, int box, int& P, int& Q) {
   double best = 1e300;
-  if (mc::reg_pair_split(n, box, &P, &Q)) return;
+  if (mc::reg_pair_split(n, box, &P, &Q)) return true;
   // otherwise the shared-memory kernel
   P = n;
   Q = 1;
   for (int q = 1; q <= n; q++) {
     if (n % q) continue;
     const int p = n / q;
-    if (mc::pair_cols_smem(n, p, q, box) + 16 > 227 * 1024) continue;  // must fit shared memory
-    const std::vector<int> rad = factor_radices(q);
-    if (q > 1 && *std::max_element(rad.begin(), rad.end()) > kTablePrime) continue;
-    const double c = radices_cost(rad);
+    // the sides the stage takes: column of products, exchange buffer, weights
+    // and tables within a CTA's shared memory
+    const size_t outer = (size_t)std::min<long long>(n, (long long)p * box);
+    if ((size_t)20 * n + 8 * (q + outer) + 16 > 227 * 1024) continue;
+    if (q > 1 && max_prime(q) > 13) continue;
+    double c = 0.0;
+    if (q > 1) {
+      std::vector<int> rad = factor_radices(q);
+      for (size_t s = 0; s < rad.size(); s++) c += radix_cost(rad[s]) + (s ? 2.0 : 0.0);
+    }
     const double cost = (double)n * c + 4.0 * box * p;
     if (cost < best) {
       best = cost;
@@ -283,6 +310,7 @@ void choose_prune(int n, int box, int& P, int& Q) {
       Q = q;
     }
   }
+  return best < 1e300;
 }
 
 std::vector<float2> twiddles(int n, int sign) {
@@ -315,10 +343,19 @@ std::vector<float2> fft_tables(const FftPlan1D& p) {
   }
   for (int s = 0; s < p.nst; s++) {
     const mc::FftStage& st = p.st[s];
-    if (st.Ns > 1)
-      for (int r = 1; r < st.R; r++)
-        for (int m = 0; m < st.Ns; m++) t[st.tw + (r - 1) * st.Ns + m] = t[(size_t)r * m * (n / (st.Ns * st.R))];
-    if (st.G) {
+    const bool prime = st.kind < 16;
+    const int r1 = prime ? st.R : st.kind / 16, r2 = prime ? 1 : st.kind % 16;
+    if (st.Ns > 1 && st.kind != mc::kStageGeneric)
+      for (int r = 1; r < r1; r++)
+        for (int m = 0; m < st.Ns; m++) t[st.tw + (r - 1) * st.Ns + m] = t[(size_t)r * m * (n / (st.Ns * r1))];
+    if (r2 > 1)
+      for (int r = 1; r < r2; r++)
+        for (int m = 0; m < st.Ns * r1; m++)
+          t[st.tw2 + (r - 1) * st.Ns * r1 + m] = t[(size_t)r * m * (n / (st.Ns * st.R))];
+    if (st.kind == mc::kStageDirect)
+      for (int r = 0; r < st.R; r++)
+        for (int k = 0; k < st.R; k++) t[st.ct + r * st.ctp * 2 + k] = t[(size_t)(r * k % st.R) * (n / st.R)];
+    if (st.kind == mc::kStageSymmetric) {
       const int h = (st.R - 1) / 2;
       for (int r = 1; r <= h; r++)
         for (int k = 1; k <= h; k++) {
@@ -361,7 +398,7 @@ struct mc_plan {
   int nx = 0, ny = 0, nz = 0, mode = 0, wl = 0;
   int nstart = 0, nend = 0, nframe = 0;
   int cap_frames = 0, cap_pairs = 0;  // buffer capacities (mc_plan_reframe stays within them)
-  int ppc = 32;                       // pairs per CTA of the pair column stage
+  int ppc = 0;                        // pairs per CTA of the pair column stage (0: the launch's choice)
   int nu = 0, n = 0, H = 0, ldn = 0, ldu = 0, ldt2 = 0;
   int box = 0, ystart = 0, P = 1, Q = 1;
   bool two_sets = false;
@@ -405,7 +442,6 @@ struct mc_plan {
   long long slot_clock = 0, recomputes = 0;
   float* d_boxes_all = nullptr;    // slot mode: pair windows gathered in list order
   float2 *d_tw_nu = nullptr, *d_tw_n = nullptr, *d_twQ = nullptr, *d_twO = nullptr, *d_cs = nullptr;
-  float2* d_twN = nullptr;  // length-n outer table of the generic pair kernel (large P x box)
   double* d_w16 = nullptr;
   int2* d_pairs = nullptr;
   float2* d_G = nullptr;
@@ -684,7 +720,6 @@ int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, cons
     a.qplan = pl->plan_q;
     a.twQ = pl->d_twQ;
     a.twO = pl->d_twO;
-    a.twN = pl->d_twN;
     a.box = pl->box;
     a.ystart = pl->ystart;
     a.G = pl->d_G;
@@ -714,8 +749,8 @@ int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, cons
     r.npairs = nb;
     r.H = pl->H;
     r.box = pl->box;
-    r.cs = pl->d_cs;
     r.boxes = pl->d_boxes + (long long)p0 * pl->box * pl->box;
+    r.cs = pl->d_cs;
     r.twO = pl->d_twO;
     r.P = pl->P;
     r.Q = pl->Q;
@@ -1153,18 +1188,15 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
   pl->ystart = (ori + pl->n / 2) % pl->n;
   if (!make_plan(pl->nu, pl->plan_nu) || !make_plan(pl->n, pl->plan_n))
     return set_err(MC_E_SIZE, "no FFT plan for %d / %d", pl->nu, pl->n);
-  choose_prune(pl->n, pl->box, pl->P, pl->Q);
+  const bool placed = choose_prune(pl->n, pl->box, pl->P, pl->Q);
   if (!make_plan(pl->Q, pl->plan_q)) return set_err(MC_E_SIZE, "no FFT plan for Q=%d", pl->Q);
   {
-    const bool reg = mc::pair_cols_reg_supported(pl->P, pl->Q);
-    const int team = pl->P <= 32 ? 32 : (pl->P <= 64 ? 64 : 128);
-    const size_t need = std::max(mc::pair_cols_launch_smem(pl->n, pl->P, pl->Q, pl->box),
-                                 reg ? mc::pair_cols_reg_smem(pl->n, team) : (size_t)0);
-    if (need > 227 * 1024 || !pair_stage_takes(pl->n, pl->box))
+    const size_t need = mc::pair_cols_launch_smem(pl->n, pl->P, pl->Q, pl->box);
+    if (need > 227 * 1024 || !placed)
       return set_err(MC_E_SIZE, "pair stage does not fit shared memory for n=%d", pl->n);
     mc_schedule sc{};
     const bool have_sc = find_schedule(pl->n, &sc);
-    pl->ppc = (have_sc && sc.pairs_per_cta > 0) ? std::min(sc.pairs_per_cta, 512) : kPairsPerCta;
+    pl->ppc = (have_sc && sc.pairs_per_cta > 0) ? std::min(sc.pairs_per_cta, 512) : 0;
     if (have_sc) {
       if (sc.fwd_streams > 0) pl->nfs = std::min(sc.fwd_streams, (int)mc_plan::kMaxForwardStreams);
       pl->fwd_rows_pairing = sc.fwd_rows_pairing;
@@ -1262,16 +1294,6 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
     const std::vector<float2> t = fft_tables(pl->plan_q);
     CKR(pl->alloc(&pl->d_twQ, sizeof(float2) * t.size()));
     CKR(upload(pl, pl->d_twQ, t));
-  }
-  if (!mc::pair_cols_reg_supported(pl->P, pl->Q) && mc::pair_cols_tabn(pl->n, pl->P, pl->box)) {
-    // generic column kernel with a length-n outer table: exp(+2 pi i e / n)
-    std::vector<float2> tn(pl->n);
-    for (int e = 0; e < pl->n; e++) {
-      const double ang = 2.0 * kPi * (double)e / pl->n;
-      tn[e] = make_float2((float)std::cos(ang), (float)std::sin(ang));
-    }
-    CKR(pl->alloc(&pl->d_twN, sizeof(float2) * tn.size()));
-    CKR(upload(pl, pl->d_twN, tn));
   }
   {
     std::vector<float2> two((size_t)pl->P * pl->box);

@@ -17,31 +17,25 @@
 // Both keep consecutive threads on consecutive shared-memory words.
 //
 // What bounds a stage is its shared-memory and twiddle traffic, not its
-// arithmetic, so the plan takes few stages of large radix (up to 16, in
-// registers); the first stage reads its input through `ldf` (global memory or
-// a staged row) and the last hands its output to `stf`, which saves a pass
-// over shared memory at either end; a stage's twiddles lie in global memory in
-// the order its threads read them.  Odd radices come first: a first stage of
-// even radix R would write with stride R, gcd(R, 16) lanes to a bank pair.
+// arithmetic, so two neighbouring stages R1, R2 run as one pass where R1 * R2
+// values fit a thread's registers (fused below: the same operations on the same
+// factors in the same order, so the transform's bits do not depend on what is
+// fused); the first pass reads its input through `ldf` (global memory or a
+// staged row) and the last hands its output to `stf`, which saves a trip
+// through shared memory at either end; a stage's twiddles lie in global memory
+// in the order its threads read them.  Odd radices come first: a first stage of
+// even radix R writes with stride R, gcd(R, 16) lanes to a bank pair.
 //
-// Measured per frame, row / column pass, before (radices up to 13, a direct sum
-// per output for other primes, tables copied to shared memory) and now:
-// 4092^2 = 31 x 12 x 11 605 / 520 -> 130 / 104 us; 1500^2 = 15 x 10 x 10 55 /
-// 41 -> 14 / 7.5 us; 520^2 (30 frames) 13.6 / 13.9 -> 2.1 / 1.5 us.  Powers of
-// two and 3710 keep the two-level form (kcommon.cuh), which has one exchange
-// instead of two: 4096^2 84 / 44 us against 129 / 69 here.
+// Measured per frame, row / column pass, before (one stage a pass, three shared
+// buffers with the tables copied in, one output of a prime's direct sum a
+// thread) and now: 4092^2 = 31 | 11 | 3 x 4 605 / 520 -> 205 / 172 us; 1500^2 =
+// 5 x 5 | 5 x 3 | 4 55 / 41 -> 15.8 / 9.8 us; 520^2 = 13 | 5 | 8 (30 frames)
+// 13.6 / 13.9 -> 2.2 / 1.5 us.  Powers of two and 3710 keep the two-level form
+// (kcommon.cuh), which has one exchange instead of two.
 #pragma once
-#include "codelets_gen.cuh"
 #include "fft_engine.cuh"
 
 namespace mc {
-
-template <int R, bool INV>
-__device__ __forceinline__ void radix_bfly(float2* v) {
-  if constexpr (R == 9 || R == 16) fft_reg<R, INV>(v);
-  else if constexpr (R == 6 || R == 10 || R == 12 || R == 14 || R == 15) fft_reg_pf<R, INV>(v);
-  else dft_any<R, INV>(v);
-}
 
 // Butterfly index t of a batch stage -> (transform b, butterfly j).
 template <bool INTERLEAVED>
@@ -50,52 +44,127 @@ __device__ __forceinline__ void bfly_index(uint32_t t, const FftStage& s, FastDi
   else fdivmod(t, s.nqdiv, b, j);
 }
 
-// One stage of compile-time radix R over B transforms.
-template <int R, bool INV, bool INTERLEAVED, class Ld, class St>
-__device__ __forceinline__ void stage_fixed(const float2* src, float2* dst, const FftStage& s, int B, FastDiv bdiv,
+// Stages of radix R1 and R2 (R2 = 1: one stage) in one pass over B transforms.
+// With R = R1 R2, thread j holds x[j + i n/R], i = r2 + R2 r1: for every r2 the
+// radix-R1 butterfly j + r2 n/R of the first stage, whose outputs r1 are the
+// inputs r2 of the second stage's butterfly (j div Ns) Ns R1 + jm + r1 Ns.
+template <int R1, int R2, bool INV, bool INTERLEAVED, class Ld, class St>
+__device__ __forceinline__ void stage_fused(const float2* src, float2* dst, const FftStage& s, int B, FastDiv bdiv,
                                             int ld, const float2* __restrict__ tw, int tid, int nth, bool first,
                                             bool last, Ld&& ldf, St&& stf) {
+  constexpr int R = R1 * R2;
   const int nq = (int)s.nqdiv.d, Ns = s.Ns;
   const int total = nq * B;
+  auto factor = [&](const float2* w) {
+    float2 f = __ldg(w);
+    if (INV) f.y = -f.y;
+    return f;
+  };
   for (int t = tid; t < total; t += nth) {
     uint32_t j, b, jq, jm = 0;
     bfly_index<INTERLEAVED>((uint32_t)t, s, bdiv, b, j);
-    float2 v[R];
+    float2 v[R2][R1];
     if (first) {
       jq = j;
 #pragma unroll
-      for (int r = 0; r < R; r++) v[r] = ldf((int)b, (int)j + r * nq);
+      for (int i = 0; i < R; i++) v[i % R2][i / R2] = ldf((int)b, (int)j + i * nq);
     } else {
       fdivmod(j, s.nsdiv, jq, jm);
       const float2* w = tw + s.tw + jm;
 #pragma unroll
-      for (int r = 0; r < R; r++) {
-        const int i = (int)j + r * nq;
-        v[r] = INTERLEAVED ? src[b + B * i] : src[b * ld + i];
-        if (r) {
-          float2 f = __ldg(w + (r - 1) * Ns);
-          if (INV) f.y = -f.y;
-          v[r] = cmul(v[r], f);
+      for (int r1 = 0; r1 < R1; r1++) {
+        float2 f;
+        if (r1) f = factor(w + (r1 - 1) * Ns);
+#pragma unroll
+        for (int r2 = 0; r2 < R2; r2++) {
+          const int i = (int)j + (r2 + R2 * r1) * nq;
+          const float2 x = INTERLEAVED ? src[b + B * i] : src[b * ld + i];
+          v[r2][r1] = r1 ? cmul(x, f) : x;
         }
       }
     }
-    radix_bfly<R, INV>(v);
+#pragma unroll
+    for (int r2 = 0; r2 < R2; r2++) dft_any<R1, INV>(v[r2]);
     const int base = (int)jq * Ns * R + (int)jm;
-    if (last) {
+    auto put = [&](int i, float2 x) {
+      if (last) stf(dst, (int)b, i, x);
+      else dst[INTERLEAVED ? b + B * i : b * ld + i] = x;
+    };
+    if constexpr (R2 == 1) {
 #pragma unroll
-      for (int r = 0; r < R; r++) stf(dst, (int)b, base + r * Ns, v[r]);
+      for (int r1 = 0; r1 < R1; r1++) put(base + r1 * Ns, v[0][r1]);
     } else {
+      const float2* w = tw + s.tw2 + jm;
 #pragma unroll
-      for (int r = 0; r < R; r++) {
-        const int i = base + r * Ns;
-        dst[INTERLEAVED ? b + B * i : b * ld + i] = v[r];
+      for (int r1 = 0; r1 < R1; r1++) {
+        float2 u[R2];
+        u[0] = v[0][r1];
+#pragma unroll
+        for (int r2 = 1; r2 < R2; r2++) u[r2] = cmul(v[r2][r1], factor(w + ((r2 - 1) * R1 + r1) * Ns));
+        dft_any<R2, INV>(u);
+#pragma unroll
+        for (int r2 = 0; r2 < R2; r2++) put(base + (r1 + r2 * R1) * Ns, u[r2]);
       }
     }
   }
 }
 
-// Radix-p stage for a prime p with a table (17..127), in the symmetric direct
-// form: with a_r = x_r + x_{p-r}, b_r = x_r - x_{p-r}, r = 1..h = (p-1)/2,
+// Prime radix p (17..127) as the first stage, every output the direct sum
+//   X_k = sum_r x_r W_p^(r k), r ascending.
+// A thread forms G outputs of one butterfly, so an input read serves G outputs
+// and the factors (the same for all threads of a warp) come two to a 16-byte
+// load from the table [r][k].
+template <bool INV, bool INTERLEAVED, class Ld, class St>
+__device__ __forceinline__ void stage_direct(float2* cur, float2* dst, const FftStage& s, int B, FastDiv bdiv, int ld,
+                                             const float2* __restrict__ tw, int tid, int nth, bool last, Ld&& ldf,
+                                             St&& stf) {
+  constexpr int G = 8;
+  const int p = s.R, nq = (int)s.nqdiv.d, nb = nq * B, ng = (p + G - 1) / G;
+  const FastDiv nbdiv = make_fastdiv((uint32_t)nb);
+  for (int t = tid; t < nb * p; t += nth) {
+    uint32_t r, jb, j, b;
+    fdivmod((uint32_t)t, nbdiv, r, jb);
+    bfly_index<INTERLEAVED>(jb, s, bdiv, b, j);
+    const int i = (int)j + (int)r * nq;
+    cur[INTERLEAVED ? b + B * i : b * ld + i] = ldf((int)b, i);
+  }
+  __syncthreads();
+  const float4* __restrict__ tab = reinterpret_cast<const float4*>(tw + s.ct);
+  for (int t = tid; t < nb * ng; t += nth) {
+    uint32_t g, jb, j, b;
+    fdivmod((uint32_t)t, nbdiv, g, jb);
+    bfly_index<INTERLEAVED>(jb, s, bdiv, b, j);
+    const int step = INTERLEAVED ? B * nq : nq;
+    const float2* x = cur + (INTERLEAVED ? b + B * j : b * ld + j);
+    float2 A[G];
+#pragma unroll
+    for (int i = 0; i < G; i++) A[i] = x[0];
+    const float4* tr = tab + s.ctp + (int)g * (G / 2);
+    for (int r = 1; r < p; r++) {
+      x += step;
+      const float2 a = *x;
+#pragma unroll
+      for (int i = 0; i < G / 2; i++) {
+        const float4 c = __ldg(tr + i);
+        const float2 u = cmul(a, make_float2(c.x, INV ? -c.y : c.y)), v = cmul(a, make_float2(c.z, INV ? -c.w : c.w));
+        A[2 * i] = cadd(A[2 * i], u);
+        A[2 * i + 1] = cadd(A[2 * i + 1], v);
+      }
+      tr += s.ctp;
+    }
+#pragma unroll
+    for (int i = 0; i < G; i++) {
+      const int k = (int)g * G + i;
+      if (k >= p) break;
+      const int o = (int)j * p + k;  // span 1
+      if (last) stf(dst, (int)b, o, A[i]);
+      else dst[INTERLEAVED ? b + B * o : b * ld + o] = A[i];
+    }
+  }
+}
+
+// Radix 53 in the symmetric direct form: with a_r = x_r + x_{p-r},
+// b_r = x_r - x_{p-r}, r = 1..h = (p-1)/2,
 //   A_k = x_0 + sum_r a_r cos(2 pi r k / p),  B_k = sum_r b_r sin(2 pi r k / p)
 //   X_k, X_{p-k} = A_k -/+ i B_k  (forward; inverse the other way round)
 // The a and b replace the inputs in place (every thread its own two elements);
@@ -103,7 +172,7 @@ __device__ __forceinline__ void stage_fixed(const float2* src, float2* dst, cons
 // from shared memory serves G pairs, and the cosines and sines (the same for
 // all threads of a warp) come two pairs to a 16-byte load.
 template <int G, bool INV, bool INTERLEAVED, class St>
-__device__ __forceinline__ void prime_outputs(const float2* cur, float2* dst, const FftStage& s, int B, FastDiv bdiv,
+__device__ __forceinline__ void symmetric_outputs(const float2* cur, float2* dst, const FftStage& s, int B, FastDiv bdiv,
                                               int ld, const float2* __restrict__ tw, int tid, int nth, bool last,
                                               St&& stf) {
   const int p = s.R, h = (p - 1) / 2, nq = (int)s.nqdiv.d, Ns = s.Ns;
@@ -118,7 +187,7 @@ __device__ __forceinline__ void prime_outputs(const float2* cur, float2* dst, co
     const int step = INTERLEAVED ? B * nq : nq;
     const float2* x = cur + (INTERLEAVED ? b + B * j : b * ld + j);
     const float2 x0 = x[0];
-    float2 A[G], S[G], sum = x0;
+    float2 A[G], S[G], sum = make_float2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < G; i++) {
       A[i] = x0;
@@ -129,7 +198,7 @@ __device__ __forceinline__ void prime_outputs(const float2* cur, float2* dst, co
     const float2* xb = x + (p - 1) * step;
     for (int r = 0; r < h; r++) {
       const float2 a = *xa, d = *xb;
-      sum = cadd(sum, a);
+      sum = r ? cadd(sum, a) : a;
 #pragma unroll
       for (int i = 0; i < G / 2; i++) {
         const float4 c = __ldg(tr + i);
@@ -152,7 +221,7 @@ __device__ __forceinline__ void prime_outputs(const float2* cur, float2* dst, co
       if (last) stf(dst, (int)b, i, v);
       else dst[INTERLEAVED ? b + B * i : b * ld + i] = v;
     };
-    if (g == 0) put(0, sum);
+    if (g == 0) put(0, cadd(x0, sum));
 #pragma unroll
     for (int i = 0; i < G; i++) {
       const int k = (int)g * G + i + 1;
@@ -167,7 +236,7 @@ __device__ __forceinline__ void prime_outputs(const float2* cur, float2* dst, co
 }
 
 template <bool INV, bool INTERLEAVED, class Ld, class St>
-__device__ __forceinline__ void stage_prime(float2* cur, float2* dst, const FftStage& s, int B, FastDiv bdiv, int ld,
+__device__ __forceinline__ void stage_symmetric(float2* cur, float2* dst, const FftStage& s, int B, FastDiv bdiv, int ld,
                                             const float2* __restrict__ tw, int tid, int nth, bool first, bool last,
                                             Ld&& ldf, St&& stf) {
   const int p = s.R, h = (p - 1) / 2, nq = (int)s.nqdiv.d, Ns = s.Ns, nb = nq * B;
@@ -201,11 +270,10 @@ __device__ __forceinline__ void stage_prime(float2* cur, float2* dst, const FftS
     *x1 = csub(u, v);
   }
   __syncthreads();
-  if (s.G == 6) prime_outputs<6, INV, INTERLEAVED>(cur, dst, s, B, bdiv, ld, tw, tid, nth, last, stf);
-  else prime_outputs<8, INV, INTERLEAVED>(cur, dst, s, B, bdiv, ld, tw, tid, nth, last, stf);
+  symmetric_outputs<kPrimePairs, INV, INTERLEAVED>(cur, dst, s, B, bdiv, ld, tw, tid, nth, last, stf);
 }
 
-// Larger primes: every output of every butterfly as a direct sum,
+// Other primes: every output of every butterfly as a direct sum,
 //   X_k = sum_r src[j + r*n/R] * W_n^(r*((j mod Ns)*tws + k*n/R)).
 template <bool INV, bool INTERLEAVED, class Ld, class St>
 __device__ void stage_generic(float2* src, float2* dst, const FftStage& s, int n, int B, FastDiv bdiv, int ld,
@@ -264,16 +332,20 @@ __device__ __forceinline__ void fft_exec(float2* s0, float2* s1, const FftPlan1D
   for (int si = 0; si < p.nst; si++) {
     const FftStage& s = p.st[si];
     const bool first = si == 0, last = si == p.nst - 1;
-#define MC_RADIX(RR)                                                                                            \
-  case RR:                                                                                                      \
-    stage_fixed<RR, INV, INTERLEAVED>(cur, nxt, s, B, bdiv, ld, tw, tid, nth, first, last, ldf, stf);           \
+#define MC_RADIX(A, B2)                                                                                         \
+  case A * 16 + B2:                                                                                             \
+    stage_fused<A, B2, INV, INTERLEAVED>(cur, nxt, s, B, bdiv, ld, tw, tid, nth, first, last, ldf, stf);        \
     break;
-    switch (s.R) {
-      MC_RADIX(2) MC_RADIX(3) MC_RADIX(4) MC_RADIX(5) MC_RADIX(6) MC_RADIX(7) MC_RADIX(8) MC_RADIX(9)
-      MC_RADIX(10) MC_RADIX(11) MC_RADIX(12) MC_RADIX(13) MC_RADIX(14) MC_RADIX(15) MC_RADIX(16)
+    switch (s.kind) {
+      MC_RADIX(2, 1) MC_RADIX(3, 1) MC_RADIX(4, 1) MC_RADIX(5, 1) MC_RADIX(7, 1) MC_RADIX(8, 1) MC_RADIX(11, 1)
+      MC_RADIX(13, 1)
+      MC_FUSED_LIST(MC_RADIX)
+      case kStageDirect: stage_direct<INV, INTERLEAVED>(cur, nxt, s, B, bdiv, ld, tw, tid, nth, last, ldf, stf); break;
+      case kStageSymmetric:
+        stage_symmetric<INV, INTERLEAVED>(cur, nxt, s, B, bdiv, ld, tw, tid, nth, first, last, ldf, stf);
+        break;
       default:
-        if (s.G) stage_prime<INV, INTERLEAVED>(cur, nxt, s, B, bdiv, ld, tw, tid, nth, first, last, ldf, stf);
-        else stage_generic<INV, INTERLEAVED>(cur, nxt, s, p.n, B, bdiv, ld, tw, tid, nth, first, last, ldf, stf);
+        stage_generic<INV, INTERLEAVED>(cur, nxt, s, p.n, B, bdiv, ld, tw, tid, nth, first, last, ldf, stf);
     }
 #undef MC_RADIX
     if (!last) __syncthreads();

@@ -1,10 +1,10 @@
 """The mixed-radix engine (mixed_fft.cuh) at the lengths where it can go wrong:
-every register radix alone and combined, primes with a cosine/sine table (six
-and eight output pairs a thread, a square of one, two of them), a prime beyond
-the tables, the largest side, and batches that leave the last CTA partly empty.
+every register radix alone and fused with a neighbour, radix 53, primes as a
+direct sum from a table (first stage), a second such prime, a prime beyond the
+tables, the largest side, and batches that leave the last CTA partly empty.
 Against numpy's FP64 transform: every output is a sum of n terms whose FP32
 rounding errors (2^-24 each, at most ~20 operations deep or a direct sum of
-up to 127 terms) add like a random walk, below 2e-6 of the result."""
+up to 131 terms) add like a random walk, below 2e-6 of the result."""
 import numpy as np
 import pytest
 
