@@ -94,7 +94,8 @@ struct PairRowsArgs {
   const float2* G;
   int npairs, H, box;
   const float2* cs;    // [H][box]
-  float* boxes;        // [npairs][box][box]
+  float* boxes;        // [npairs][box][box], pair p's window at order[p] (null: at p)
+  const int* order;
   // when set with a compiled split n = P*Q: the pruned-transform row kernel
   // (twO and ystart as in PairColsArgs); otherwise the product kernel
   const float2* twO;

@@ -307,12 +307,13 @@ __global__ void __launch_bounds__(kRegThreads, pair_reg_min_blocks(Q)) k_pair_ro
   }
   team_barrier(1 + tm, T);
   const int ya = yb0 + 2 * tm, yb = ya + 1;
+  const int o = a.order ? a.order[p] : p;
   for (int mm = lt; mm < box; mm += T) {
     float2 s = part[mm];
 #pragma unroll
     for (int cc = 1; cc < C; cc++) s = cadd(s, part[cc * box + mm]);
-    if (ya < box) a.boxes[((long long)p * box + ya) * box + mm] = s.x;
-    if (yb < box) a.boxes[((long long)p * box + yb) * box + mm] = s.y;
+    if (ya < box) a.boxes[((long long)o * box + ya) * box + mm] = s.x;
+    if (yb < box) a.boxes[((long long)o * box + yb) * box + mm] = s.y;
   }
 }
 
@@ -441,6 +442,7 @@ __global__ void __launch_bounds__(kRowThreads) k_pair_rows(PairRowsArgs a) {
     if (more) park(s ^ 1);
     __syncthreads();
   }
+  const long long o = a.order ? a.order[p] : p;
 #pragma unroll
   for (int i = 0; i < RI; i++) {
     const int yb = yb0 + ty + i;
@@ -448,7 +450,7 @@ __global__ void __launch_bounds__(kRowThreads) k_pair_rows(PairRowsArgs a) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const int xb = xb0 + tx + (j & 1) + (j >> 1) * 16;
-      if (xb < box) a.boxes[((long long)p * box + yb) * box + xb] = acc[i][j];
+      if (xb < box) a.boxes[(o * box + yb) * box + xb] = acc[i][j];
     }
   }
 }

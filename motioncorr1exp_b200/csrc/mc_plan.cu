@@ -80,6 +80,11 @@ namespace {
 
 constexpr double kPi = 3.14159265358979323846;
 constexpr int kPairBatch = 512;
+// A host movie's upload goes in chunks of at least this (one chunk: no
+// pipelining).  Smaller chunks leave less for the end but their pair launches
+// read the earlier spectra once more each: 40 x 3710^2 uint8 with 2 / 4 / 5 / 6 /
+// 7 / 9 frames a chunk 16.6, 15.5, 15.6, 16.0, 16.0, 16.6 ms.
+constexpr size_t kChunkBytes = (size_t)48 << 20;
 constexpr int kTablePrime = 127;  // largest prime radix with a cosine/sine table (mixed_fft.cuh)
 constexpr int kForwardCtas = 148 * 16;  // row CTAs (of four rows) a forward launch is filled to
 // spectrum slots: the fewest a plan works with (two blocks of two frames in
@@ -458,6 +463,13 @@ struct mc_plan {
 
   // device-only movie pipeline (forward -> pairs -> device solve -> sum)
   int2* d_pairs_main = nullptr;  // the plan's pair list, uploaded once
+  // the pair list in the order a host movie's chunks complete it (by chunk of
+  // the later frame), and the list position of each; made on the first run of a
+  // frame configuration from host memory
+  int2* d_pairs_chunk = nullptr;
+  int* d_order_chunk = nullptr;
+  std::vector<mc::PairIJ> pairs_chunk;
+  std::vector<int> chunk_end;  // pairs_chunk entries of the chunks up to each
   double *d_M = nullptr, *d_rhs = nullptr, *d_work = nullptr, *d_ki1 = nullptr, *d_ki2 = nullptr;
   double *d_dshift = nullptr, *d_dfshift = nullptr;
   int *d_mask = nullptr, *d_order = nullptr, *d_uf = nullptr, *d_kept = nullptr, *d_nkept = nullptr;
@@ -693,11 +705,11 @@ int hold_spectra(mc_plan* pl, const std::vector<int>& frames, std::vector<int>& 
 }
 
 // pair stage over an explicit list: (a-frame, b-frame) into a/b spectrum sets
-// Launches the pair kernels for `list`, whose device copy is d_list; results
-// land in d_pshift / d_pcc / d_ppeak.  No host synchronisation.
-int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, const float2* specB, long long strideB,
-                       const std::vector<mc::PairIJ>& list, const int2* d_list) {
-  const int np = (int)list.size();
+// Launches the window kernels for the pairs list[first..first + np), whose
+// device copy starts at d_list; pair i's window goes to d_boxes at d_order[i]
+// (null: at first + i).  No host synchronisation.
+int enqueue_windows(mc_plan* pl, const float2* specA, long long strideA, const float2* specB, long long strideB,
+                    const std::vector<mc::PairIJ>& list, int first, int np, const int2* d_list, const int* d_order) {
   if (np > pl->maxp) return set_err(MC_E_STATE, "pair list larger than the plan's capacity");
   const float mbf = (float)(-0.5 * (double)pl->p.bfactor / pl->n / pl->n);
   for (int p0 = 0; p0 < np; p0 += kPairBatch) {
@@ -729,7 +741,7 @@ int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, cons
     const bool one_set = specA == specB && strideA == strideB;
     std::vector<char> seenA(pl->nframe + 1, 0), seenB(pl->nframe + 1, 0);
     long long nspec = 0;
-    for (int i = p0; i < p0 + nb; i++) {
+    for (int i = first + p0; i < first + p0 + nb; i++) {
       const int fa = strideA ? list[i].first : pl->nframe, fb = list[i].second;
       if (!seenA[fa]) {
         seenA[fa] = 1;
@@ -749,7 +761,8 @@ int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, cons
     r.npairs = nb;
     r.H = pl->H;
     r.box = pl->box;
-    r.boxes = pl->d_boxes + (long long)p0 * pl->box * pl->box;
+    r.boxes = pl->d_boxes + (d_order ? 0 : (long long)(first + p0) * pl->box * pl->box);
+    r.order = d_order ? d_order + p0 : nullptr;
     r.cs = pl->d_cs;
     r.twO = pl->d_twO;
     r.P = pl->P;
@@ -759,6 +772,11 @@ int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, cons
            gbytes + (double)pl->H * pl->box * sizeof(float2) + (double)nb * pl->box * pl->box * sizeof(float),
            mc::launch_pair_rows(r, pl->st));
   }
+  return MC_OK;
+}
+
+// The peaks of np windows in d_boxes, into d_pshift / d_pcc / d_ppeak.
+int enqueue_peaks(mc_plan* pl, int np) {
   mc::PeakArgs k{};
   k.boxes = pl->d_boxes;
   k.npairs = np;
@@ -772,6 +790,12 @@ int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, cons
   LAUNCH(pl, MC_K_PEAK, (double)np * pl->box * pl->box * sizeof(float) + (double)np * 5 * sizeof(float),
          mc::launch_peak(k, pl->st));
   return MC_OK;
+}
+
+int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, const float2* specB, long long strideB,
+                       const std::vector<mc::PairIJ>& list, const int2* d_list) {
+  CKR(enqueue_windows(pl, specA, strideA, specB, strideB, list, 0, (int)list.size(), d_list, nullptr));
+  return enqueue_peaks(pl, (int)list.size());
 }
 
 // pair stage over an explicit list of spectrum indices, synchronous,
@@ -1058,6 +1082,7 @@ static int configure_frames(mc_plan* pl, const mc_params& q, int nz, bool upload
                    (int)pairs.size(), pl->cap_frames, pl->cap_pairs);
   const bool same = pairs == pl->pairs;
   pl->pairs = pairs;
+  if (!same) pl->pairs_chunk.clear();
   if (pl->d_pairs_main && !same && upload_pairs) {
     std::vector<int2> pr(pairs.size());
     for (size_t i = 0; i < pairs.size(); i++) pr[i] = make_int2(pairs[i].first, pairs[i].second);
@@ -1240,6 +1265,8 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
     std::vector<int2> pr(pl->pairs.size());
     for (size_t i = 0; i < pr.size(); i++) pr[i] = make_int2(pl->pairs[i].first, pl->pairs[i].second);
     CKR(pl->alloc(&pl->d_pairs_main, sizeof(int2) * np));
+    CKR(pl->alloc(&pl->d_pairs_chunk, sizeof(int2) * np));
+    CKR(pl->alloc(&pl->d_order_chunk, sizeof(int) * np));
     CKR(upload(pl, pl->d_pairs_main, pr));
     CKR(pl->alloc(&pl->d_M, sizeof(double) * (size_t)nc * nc));
     CKR(pl->alloc(&pl->d_rhs, sizeof(double) * 2 * (size_t)nc));
@@ -1525,7 +1552,8 @@ int mc_plan_bind_frames_device(mc_plan* pl, const void* d_frames) {
 
 }  // extern "C"
 
-static int run_device(mc_plan* pl, float* image_host, const std::vector<cudaEvent_t>* waits, int chunk);
+static int run_device(mc_plan* pl, float* image_host);
+static int run_host_device(mc_plan* pl, const char* frames, float* image_host, int chunk);
 static bool device_path(const mc_plan* pl);
 
 // Forward transforms of every position.  With `waits`, the plan stream waits
@@ -1757,6 +1785,15 @@ static int forward_all(mc_plan* pl, const std::vector<cudaEvent_t>* waits, int c
   return MC_OK;
 }
 
+// Chunk c of a host movie's frames on the copy stream, its event recorded.
+static int copy_chunk(mc_plan* pl, const char* frames, int c, int chunk) {
+  const int f0 = c * chunk, cnt = std::min(chunk, pl->nframe - f0);
+  CK(cudaMemcpyAsync((char*)pl->d_frames + (size_t)f0 * pl->frame_bytes, frames + (size_t)f0 * pl->frame_bytes,
+                     (size_t)cnt * pl->frame_bytes, cudaMemcpyHostToDevice, pl->st_copy));
+  CK(cudaEventRecord(pl->chunk_ev[c], pl->st_copy));
+  return MC_OK;
+}
+
 extern "C" {
 
 int mc_plan_forward(mc_plan* pl) {
@@ -1772,9 +1809,21 @@ int mc_plan_run_host(mc_plan* pl, const void* frames, float* image_host) {
   CK(cudaSetDevice(pl->device));
   if (!pl->st_copy) CK(cudaStreamCreateWithFlags(&pl->st_copy, cudaStreamNonBlocking));
   // chunks of frames: copy chunk c on the copy stream while the plan stream
-  // transforms the frames of chunks < c
-  const int chunk = 4;
+  // works on the frames of chunks < c; a movie of one chunk is copied on the
+  // plan stream and runs as from device memory (its graph replayed)
+  const int chunk = (int)std::min<long long>(pl->nframe, ((long long)kChunkBytes - 1) / (long long)pl->frame_bytes + 1);
   const int nchunk = (pl->nframe + chunk - 1) / chunk;
+  const bool device = device_path(pl);
+  pl->frames_src = nullptr;
+  for (int f = 0; f < pl->nframe; f++) pl->loaded[f] = 1;
+  pl->log("Input Stack: Nx(%d) Ny(%d) Nz(%d) Mode(%d)\n\n", pl->nx, pl->ny, pl->nz, pl->mode);
+  pl->log("Crop Image: Offset(%d %d) RawDim(%d) BinnedDim(%d)\n", pl->p.crop_offsetx, pl->p.crop_offsety, pl->nu,
+          pl->n);
+  if (device && nchunk == 1) {
+    CK(cudaMemcpyAsync(pl->d_frames, frames, (size_t)pl->nframe * pl->frame_bytes, cudaMemcpyHostToDevice, pl->st));
+    return run_device(pl, image_host);
+  }
+  if (!pl->st_copy) CK(cudaStreamCreateWithFlags(&pl->st_copy, cudaStreamNonBlocking));
   while ((int)pl->chunk_ev.size() < nchunk) {
     cudaEvent_t e;
     CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1785,19 +1834,8 @@ int mc_plan_run_host(mc_plan* pl, const void* frames, float* image_host) {
   if (!pl->start_ev) CK(cudaEventCreateWithFlags(&pl->start_ev, cudaEventDisableTiming));
   CK(cudaEventRecord(pl->start_ev, pl->st));
   CK(cudaStreamWaitEvent(pl->st_copy, pl->start_ev, 0));
-  pl->frames_src = nullptr;
-  for (int c = 0; c < nchunk; c++) {
-    const int f0 = c * chunk, cnt = std::min(chunk, pl->nframe - f0);
-    CK(cudaMemcpyAsync((char*)pl->d_frames + (size_t)f0 * pl->frame_bytes,
-                       (const char*)frames + (size_t)f0 * pl->frame_bytes, (size_t)cnt * pl->frame_bytes,
-                       cudaMemcpyHostToDevice, pl->st_copy));
-    CK(cudaEventRecord(pl->chunk_ev[c], pl->st_copy));
-  }
-  for (int f = 0; f < pl->nframe; f++) pl->loaded[f] = 1;
-  pl->log("Input Stack: Nx(%d) Ny(%d) Nz(%d) Mode(%d)\n\n", pl->nx, pl->ny, pl->nz, pl->mode);
-  pl->log("Crop Image: Offset(%d %d) RawDim(%d) BinnedDim(%d)\n", pl->p.crop_offsetx, pl->p.crop_offsety, pl->nu,
-          pl->n);
-  if (device_path(pl)) return run_device(pl, image_host, &pl->chunk_ev, chunk);
+  if (device) return run_host_device(pl, static_cast<const char*>(frames), image_host, chunk);
+  for (int c = 0; c < nchunk; c++) CKR(copy_chunk(pl, static_cast<const char*>(frames), c, chunk));
   CKR(forward_all(pl, &pl->chunk_ev, chunk));
   CKR(mc_plan_pairs(pl));
   CKR(mc_plan_solve(pl));
@@ -2420,11 +2458,14 @@ int mc_plan_refine(mc_plan* pl, int iterations) {
 
 // pairs -> device solve -> sum -> result copies into the pinned staging,
 // all on the plan stream without a host synchronisation.
-static int enqueue_tail(mc_plan* pl, unsigned char* hs) {
+static int enqueue_tail(mc_plan* pl, unsigned char* hs, bool windows_done = false) {
   const int np = (int)pl->pairs.size(), nf = pl->nframe, nc = nf - 1;
   CK(cudaMemcpy2DAsync(hs + pl->st_dc, sizeof(float2), pl->d_specA, sizeof(float2) * pl->fstride, sizeof(float2),
                        nf, cudaMemcpyDeviceToHost, pl->st));
-  CKR(enqueue_pair_stage(pl, pl->d_specA, pl->fstride, pl->d_specB, pl->fstride, pl->pairs, pl->d_pairs_main));
+  if (!windows_done)
+    CKR(enqueue_windows(pl, pl->d_specA, pl->fstride, pl->d_specB, pl->fstride, pl->pairs, 0, np, pl->d_pairs_main,
+                        nullptr));
+  CKR(enqueue_peaks(pl, np));
   int nss, nes, lim;
   sum_range(pl, &nss, &nes, &lim);
   mc::SolveArgs s{};
@@ -2531,10 +2572,26 @@ static int finish_device_movie(mc_plan* pl, const unsigned char* hs) {
   return MC_OK;
 }
 
+// End of a device-only movie: its image to the host, the synchronisation, the
+// results into the plan's host state.
+static int finish_device_run(mc_plan* pl, float* image_host) {
+  CK(cudaEventRecord(pl->ev[1], pl->st));
+  if (image_host)
+    CK(cudaMemcpyAsync(image_host, pl->d_image, sizeof(float) * (size_t)pl->n * pl->n, cudaMemcpyDeviceToHost,
+                       pl->st));
+  CK(cudaStreamSynchronize(pl->st));
+  CKR(pl->collect());
+  float ms = 0.f;
+  CK(cudaEventElapsedTime(&ms, pl->ev[0], pl->ev[1]));
+  pl->tm = mc_timings{};
+  pl->tm.total_ms = ms;
+  return finish_device_movie(pl, pl->h_stage);
+}
+
 // Whole movie on the device with one synchronisation; captured once into a
 // CUDA graph and replayed (unless profiling or a capture failure).
-static int run_device(mc_plan* pl, float* image_host, const std::vector<cudaEvent_t>* waits, int chunk) {
-  const bool graph_ok = !waits && !pl->profiling && !pl->graph_failed;
+static int run_device(mc_plan* pl, float* image_host) {
+  const bool graph_ok = !pl->profiling && !pl->graph_failed;
   CKR(upload_frame_base(pl));
   CK(cudaEventRecord(pl->ev[0], pl->st));
   mc_plan::GraphEntry* ge = nullptr;
@@ -2590,20 +2647,76 @@ static int run_device(mc_plan* pl, float* image_host, const std::vector<cudaEven
       pl->kbytes[k] += ge->kbytes[k];
     }
   } else {
-    CKR(enqueue_forward(pl, waits, chunk));
+    CKR(enqueue_forward(pl, nullptr, 1));
     CKR(enqueue_tail(pl, pl->h_stage));
   }
-  CK(cudaEventRecord(pl->ev[1], pl->st));
-  if (image_host)
-    CK(cudaMemcpyAsync(image_host, pl->d_image, sizeof(float) * (size_t)pl->n * pl->n, cudaMemcpyDeviceToHost,
-                       pl->st));
+  return finish_device_run(pl, image_host);
+}
+
+// Chunks of a host movie in upload order: from both ends inwards.  A pair's
+// frames are at least `dist` apart, so the ends have the most partners: going
+// from the first frame to the last leaves most pairs to the last chunks.
+static std::vector<int> chunk_sequence(int nchunk) {
+  std::vector<int> seq;
+  for (int a = 0, b = nchunk - 1; a <= b; a++, b--) {
+    seq.push_back(a);
+    if (b > a) seq.push_back(b);
+  }
+  return seq;
+}
+
+// The pair list by the upload step that completes each pair, for the current
+// frame configuration; its device copies made when it changes.
+static int order_by_chunk(mc_plan* pl, int chunk) {
+  if (!pl->pairs_chunk.empty()) return MC_OK;
+  const int np = (int)pl->pairs.size(), nchunk = (pl->nframe + chunk - 1) / chunk;
+  const std::vector<int> seq = chunk_sequence(nchunk);
+  std::vector<int> step(nchunk), order(np);
+  for (int k = 0; k < nchunk; k++) step[seq[k]] = k;
+  auto done = [&](int p) { return std::max(step[pl->pairs[p].first / chunk], step[pl->pairs[p].second / chunk]); };
+  for (int i = 0; i < np; i++) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return done(a) < done(b); });
+  pl->chunk_end.assign(nchunk, 0);
+  std::vector<int2> pr(np);
+  std::vector<mc::PairIJ> list(np);
+  for (int i = 0; i < np; i++) {
+    list[i] = pl->pairs[order[i]];
+    pr[i] = make_int2(list[i].first, list[i].second);
+    for (int k = done(order[i]); k < nchunk; k++) pl->chunk_end[k] = i + 1;
+  }
+  CK(cudaMemcpyAsync(pl->d_pairs_chunk, pr.data(), sizeof(int2) * np, cudaMemcpyHostToDevice, pl->st));
+  CK(cudaMemcpyAsync(pl->d_order_chunk, order.data(), sizeof(int) * np, cudaMemcpyHostToDevice, pl->st));
   CK(cudaStreamSynchronize(pl->st));
-  CKR(pl->collect());
-  float ms = 0.f;
-  CK(cudaEventElapsedTime(&ms, pl->ev[0], pl->ev[1]));
-  pl->tm = mc_timings{};
-  pl->tm.total_ms = ms;
-  return finish_device_movie(pl, pl->h_stage);
+  pl->pairs_chunk = list;
+  return MC_OK;
+}
+
+// A device-only movie from host memory, pipelined with its upload: each chunk
+// of frames is transformed when it has arrived, and the windows of the pairs
+// it completes follow at once (their places in the list through the order
+// table), so little is left when the last frame is there.  40 x 3710^2 uint8,
+// 378 pairs, whole call: 19.3 ms with the pair stage behind the last upload,
+// 16.6 with the chunks uploaded first to last, 15.5 now (the upload alone 10.3).
+static int run_host_device(mc_plan* pl, const char* frames, float* image_host, int chunk) {
+  const int nchunk = (pl->nframe + chunk - 1) / chunk;
+  CKR(order_by_chunk(pl, chunk));
+  CKR(upload_frame_base(pl));
+  CK(cudaEventRecord(pl->ev[0], pl->st));
+  const std::vector<int> seq = chunk_sequence(nchunk);
+  for (int k = 0; k < nchunk; k++) {
+    const int c = seq[k];
+    CKR(copy_chunk(pl, frames, c, chunk));
+    CK(cudaStreamWaitEvent(pl->st, pl->chunk_ev[c], 0));
+    std::vector<std::pair<int, int>> jobs;
+    for (int f = c * chunk; f < std::min(pl->nframe, (c + 1) * chunk); f++) jobs.push_back({f, f});
+    CKR(enqueue_forward(pl, nullptr, 1, &jobs));
+    const int p0 = k ? pl->chunk_end[k - 1] : 0, np = pl->chunk_end[k] - p0;
+    if (np > 0)
+      CKR(enqueue_windows(pl, pl->d_specA, pl->fstride, pl->d_specB, pl->fstride, pl->pairs_chunk, p0, np,
+                          pl->d_pairs_chunk + p0, pl->d_order_chunk + p0));
+  }
+  CKR(enqueue_tail(pl, pl->h_stage, true));
+  return finish_device_run(pl, image_host);
 }
 
 static bool device_path(const mc_plan* pl) { return pl->p.iter == 0 && !pl->p.refine && !pl->slots; }
@@ -2619,7 +2732,7 @@ int mc_plan_run(mc_plan* pl, float* image_host) {
     for (int f = 0; f < pl->nframe; f++)
       if (!pl->loaded[f]) return set_err(MC_E_STATE, "frame position %d not loaded", f);
     CK(cudaSetDevice(pl->device));
-    return run_device(pl, image_host, nullptr, 1);
+    return run_device(pl, image_host);
   }
   CKR(mc_plan_forward(pl));
   CKR(mc_plan_pairs(pl));
