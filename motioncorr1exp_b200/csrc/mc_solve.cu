@@ -235,15 +235,16 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve(SolveArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Shared-memory form of the same solve (used when its working set fits):
-// the pair list, the measured shifts, the normal matrix, the residuals, the
-// rank order, the union-find parents and the final step shifts live in
-// shared memory (the one-thread sections, the threshold scan and the
-// union-find pass, then run on shared-memory latency instead of dependent
-// global loads); the normal equations are built one frame step per thread in
-// a single pass over the pairs (a histogram of the pair ends per step, then
-// suffix sums), and the per-row residual and compaction loops run in
-// parallel.  Sums run in the same order as the global-memory form.
+// Shared-memory form of the same solve (used when its working set fits), one
+// CTA.  What bounds it is latency: the factorisation's chain of square root,
+// division and update per step, and the back substitution's chain of dependent
+// multiply-adds.  So a step takes two barriers (every thread forms the pivot's
+// root for itself, the right-hand sides are eliminated along with the columns,
+// which is the forward substitution), the normal matrix comes from counts and
+// two prefix passes, and when every residual is below the threshold nothing is
+// ranked or solved again: the second system is the first.  Every sum runs in
+// the order of the global-memory form.  Measured: 8 frames / 21 pairs 34 -> 15
+// us, 16 / 55 70 -> 25, 24 / 105 117 -> 35, 40 / 378 310 -> 66 (every row kept).
 namespace {
 
 struct SolveSmem {
@@ -251,85 +252,97 @@ struct SolveSmem {
   float2* ps;      // [P]
   int* mask;       // [P]
   double* ki;      // [P]
-  int* hist;       // [nc][nf]
+  int* hist;       // [nc][nf] rows by (first, last) frame, then their suffix sums
   int* order;      // [P] rows in ascending ki1 rank
   int* uf;         // [nf] union-find parents
   double* M;       // [nc][nc]
   double* rx;      // [nc]
   double* ry;      // [nc]
+  double* ld;      // [nc] diagonal of the Cholesky factor
 };
 
 __device__ bool solve_masked_smem(const SolveSmem& m, int P, int nf, double* sx, double* sy) {
   const int nc = nf - 1, tid = threadIdx.x;
-  __shared__ int s_bad;
-  if (tid == 0) s_bad = 0;
-  // step k: rows with i <= k < j; histogram of their ends j and rhs sums
-  for (int k = tid; k < nc; k += kSolveThreads) {
-    int* h = m.hist + (size_t)k * nf;
-    for (int j = 0; j < nf; j++) h[j] = 0;
-    double x = 0.0, y = 0.0;
-    for (int r = 0; r < P; r++) {
-      const int2 q = m.pr[r];
-      if (m.mask[r] && q.x <= k && k < q.y) {
-        h[q.y]++;
-        x += (double)m.ps[r].x;
-        y += (double)m.ps[r].y;
-      }
-    }
-    m.rx[k] = x;
-    m.ry[k] = y;
-    // M[k][l] (l >= k) = rows with i <= k and j > l: suffix sums of the ends
+  double* M = m.M;
+  for (int t = tid; t < nc * nf; t += kSolveThreads) m.hist[t] = 0;
+  __syncthreads();
+  for (int r = tid; r < P; r += kSolveThreads)
+    if (m.mask[r]) atomicAdd(&m.hist[m.pr[r].x * nf + m.pr[r].y], 1);
+  __syncthreads();
+  // rows (i, j) with j > l, at [i][l + 1]
+  for (int i = tid; i < nc; i += kSolveThreads) {
     int c = 0;
-    for (int l = nc - 1; l >= k; l--) {
-      c += h[l + 1];
-      m.M[(size_t)k * nc + l] = (double)c;
-      m.M[(size_t)l * nc + k] = (double)c;
+    for (int l = nc; l >= 1; l--) m.hist[i * nf + l] = c += m.hist[i * nf + l];
+  }
+  __syncthreads();
+  // M[k][l] (l >= k) = rows with i <= k and j > l; right-hand sides: the rows
+  // covering step k summed in list order.  One job a thread, its kinds in
+  // warps of their own
+  const int ncw = (nc + 31) / 32 * 32;
+  for (int t = tid; t < 3 * ncw; t += kSolveThreads) {
+    const int kind = t / ncw, k = t - kind * ncw;
+    if (k >= nc) continue;
+    if (kind == 0) {
+      int c = 0;
+      for (int q = 0; q <= k; q++) {
+        c += m.hist[q * nf + k + 1];
+        M[(size_t)q * nc + k] = M[(size_t)k * nc + q] = (double)c;
+      }
+    } else {
+      double v = 0.0;
+#pragma unroll 4
+      for (int r = 0; r < P; r++) {
+        const int2 q = m.pr[r];
+        const float2 w = m.ps[r];
+        if (m.mask[r] && q.x <= k && k < q.y) v += (double)(kind == 1 ? w.x : w.y);
+      }
+      (kind == 1 ? m.rx : m.ry)[k] = v;
     }
   }
   __syncthreads();
   double dmax = 1.0;
-  for (int k = 0; k < nc; k++) dmax = fmax(dmax, m.M[(size_t)k * nc + k]);
+  for (int k = tid & 31; k < nc; k += 32) dmax = fmax(dmax, M[(size_t)k * nc + k]);
+  for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
   const double tiny = 1e-12 * dmax;
-  double* M = m.M;
+  bool ok = true;
+  const int tx = tid & 15, ty = tid >> 4;
   for (int k = 0; k < nc; k++) {
-    if (tid == 0) {
-      const double d = M[(size_t)k * nc + k];
-      if (!(d > tiny)) s_bad = 1;
-      M[(size_t)k * nc + k] = sqrt(fmax(d, tiny));
+    const double d = M[(size_t)k * nc + k];
+    if (!(d > tiny)) ok = false;  // the same in every thread
+    const double lkk = sqrt(fmax(d, tiny));
+    for (int t = tid; t < nc - k + 1; t += kSolveThreads) {
+      if (t < 2) {
+        double* v = (t ? m.ry : m.rx) + k;
+        *v /= lkk;
+        if (t == 0) m.ld[k] = lkk;
+      } else {
+        M[(size_t)(k + t - 1) * nc + k] /= lkk;
+      }
     }
     __syncthreads();
-    const double lkk = M[(size_t)k * nc + k];
-    for (int i = k + 1 + tid; i < nc; i += kSolveThreads) M[(size_t)i * nc + k] /= lkk;
-    __syncthreads();
-    const int w = nc - k - 1;
-    for (int idx = tid; idx < w * w; idx += kSolveThreads) {
-      const int i = k + 1 + idx / w, j = k + 1 + idx % w;
-      if (j <= i) M[(size_t)i * nc + j] -= M[(size_t)i * nc + k] * M[(size_t)j * nc + k];
+    for (int i = k + 1 + ty; i < nc; i += kSolveThreads / 16) {
+      const double lik = M[(size_t)i * nc + k];
+      for (int j = k + 1 + tx; j <= i; j += 16) M[(size_t)i * nc + j] -= lik * M[(size_t)j * nc + k];
+      if (tx == 15) m.rx[i] -= lik * m.rx[k];
+      if (tx == 14) m.ry[i] -= lik * m.ry[k];
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    for (int i = 0; i < nc; i++) {
-      double vx = m.rx[i], vy = m.ry[i];
-      for (int q = 0; q < i; q++) {
-        vx -= M[(size_t)i * nc + q] * m.rx[q];
-        vy -= M[(size_t)i * nc + q] * m.ry[q];
-      }
-      m.rx[i] = vx / M[(size_t)i * nc + i];
-      m.ry[i] = vy / M[(size_t)i * nc + i];
-    }
+  // back substitution, x and y in a warp each
+  if (tid == 0 || tid == 32) {
+    const double* b = tid ? m.ry : m.rx;
+    double* x = tid ? sy : sx;
+    double next = 0.0;  // x[i + 1]
     for (int i = nc - 1; i >= 0; i--) {
-      double vx = m.rx[i], vy = m.ry[i];
-      for (int q = i + 1; q < nc; q++) {
-        vx -= M[(size_t)q * nc + i] * sx[q];
-        vy -= M[(size_t)q * nc + i] * sy[q];
-      }
-      sx[i] = vx / M[(size_t)i * nc + i];
-      sy[i] = vy / M[(size_t)i * nc + i];
+      double v = b[i];
+      if (i + 1 < nc) v -= M[(size_t)(i + 1) * nc + i] * next;
+#pragma unroll 8
+      for (int q = i + 2; q < nc; q++) v -= M[(size_t)q * nc + i] * x[q];
+      next = x[i] = v / m.ld[i];
     }
   }
   __syncthreads();
-  return s_bad == 0;
+  return ok;
 }
 
 // residual |sum of steps i..j-1 - measured| of row r (steps summed k ascending)
@@ -342,6 +355,60 @@ __device__ double row_residual(const SolveSmem& m, const double* wx, const doubl
   }
   const double dx = ax - (double)m.ps[r].x, dy = ay - (double)m.ps[r].y;
   return sqrt(dx * dx + dy * dy);
+}
+
+// Step, frame and sum shifts of the final steps (wx, wy).
+__device__ void solve_outputs(const SolveArgs& a, const SolveSmem& m, const double* wx, const double* wy) {
+  const int nc = a.nframe - 1, tid = threadIdx.x;
+  if (tid == 0) {
+    double* sx = a.shift;
+    double ox = 0.0, oy = 0.0, px = 0.0, py = 0.0, tx = 0.0, ty = 0.0;
+    a.frame_shift[0] = 0.0;
+    a.frame_shift[1] = 0.0;
+    for (int k = 0; k < nc; k++) {
+      const double nx = ox + wx[k], ny = oy + wy[k];
+      ox = nx;
+      oy = ny;
+      const double stx = nx - px, sty = ny - py;
+      px = nx;
+      py = ny;
+      sx[2 * k] = stx;
+      sx[2 * k + 1] = sty;
+      m.rx[k] = stx;  // shared copies for the sums below (no global reads back)
+      m.ry[k] = sty;
+      tx += stx;
+      ty += sty;
+      a.frame_shift[2 * (k + 1)] = tx;
+      a.frame_shift[2 * (k + 1) + 1] = ty;
+    }
+    double mx = 0.0, my = 0.0;
+    if (a.align_to_mid)
+      for (int k = 0; k < a.mid_steps; k++) {
+        mx += m.rx[k];
+        my += m.ry[k];
+      }
+    double Tx = 0.0, Ty = 0.0;
+    for (int k = 1; k < a.sum_first + 1; k++) {
+      Tx += m.rx[k - 1];
+      Ty += m.ry[k - 1];
+    }
+    for (int k = a.sum_first; k <= a.sum_last; k++) {
+      if (k > a.sum_first) {
+        Tx += m.rx[k - 1];
+        Ty += m.ry[k - 1];
+      }
+      const int q2 = k - a.sum_first;
+      a.sum_shift[q2] = make_double2(-Tx + mx, -Ty + my);
+      a.sum_frames[q2] = k;
+      a.sum_apply[q2] = (k == a.sum_first && !a.align_to_mid) ? 0 : 1;
+    }
+    // the final solve's per-step shifts into work[], where the host reads them
+    for (int k = 0; k < nc; k++) {
+      a.work[k] = wx[k];
+      a.work[nc + k] = wy[k];
+    }
+    *a.status = 0;
+  }
 }
 
 size_t solve_smem_bytes(int P, int nf) {
@@ -361,7 +428,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_smem(SolveArgs a) {
   m.ry = m.rx + nc;
   double* wx = m.ry + nc;
   double* wy = wx + nc;
-  m.ki = wy + nc;
+  m.ld = wy + nc;
+  m.ki = m.ld + nc;
   m.ps = reinterpret_cast<float2*>(m.ki + P);
   m.pr = reinterpret_cast<int2*>(m.ps + P);
   m.mask = reinterpret_cast<int*>(m.pr + P);
@@ -378,13 +446,24 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_smem(SolveArgs a) {
     if (tid == 0) *a.status = -6;
     return;
   }
+  bool below = true;
   for (int r = tid; r < P; r += kSolveThreads) {
     const double v = row_residual(m, wx, wy, r);
     m.ki[r] = v;
     a.ki1[r] = v;
     m.order[r] = r;  // every slot holds a row even if NaN residuals share a rank
+    below = below && v < (double)a.kithresh;
   }
-  __syncthreads();
+  if (__syncthreads_and(below)) {
+    // every row is kept: the second system is the first
+    for (int r = tid; r < P; r += kSolveThreads) {
+      a.kept[r] = r;
+      a.ki2[r] = m.ki[r];
+    }
+    if (tid == 0) *a.nkept = P;
+    solve_outputs(a, m, wx, wy);
+    return;
+  }
   // stable ascending rank of ki1 (OD_Threshold's repeated first-minimum pick)
   int* order = m.order;
   for (int r = tid; r < P; r += kSolveThreads) {
@@ -455,55 +534,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_smem(SolveArgs a) {
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    double* sx = a.shift;
-    double ox = 0.0, oy = 0.0, px = 0.0, py = 0.0, tx = 0.0, ty = 0.0;
-    a.frame_shift[0] = 0.0;
-    a.frame_shift[1] = 0.0;
-    for (int k = 0; k < nc; k++) {
-      const double nx = ox + wx[k], ny = oy + wy[k];
-      ox = nx;
-      oy = ny;
-      const double stx = nx - px, sty = ny - py;
-      px = nx;
-      py = ny;
-      sx[2 * k] = stx;
-      sx[2 * k + 1] = sty;
-      m.rx[k] = stx;  // shared copies for the sums below (no global reads back)
-      m.ry[k] = sty;
-      tx += stx;
-      ty += sty;
-      a.frame_shift[2 * (k + 1)] = tx;
-      a.frame_shift[2 * (k + 1) + 1] = ty;
-    }
-    double mx = 0.0, my = 0.0;
-    if (a.align_to_mid)
-      for (int k = 0; k < a.mid_steps; k++) {
-        mx += m.rx[k];
-        my += m.ry[k];
-      }
-    double Tx = 0.0, Ty = 0.0;
-    for (int k = 1; k < a.sum_first + 1; k++) {
-      Tx += m.rx[k - 1];
-      Ty += m.ry[k - 1];
-    }
-    for (int k = a.sum_first; k <= a.sum_last; k++) {
-      if (k > a.sum_first) {
-        Tx += m.rx[k - 1];
-        Ty += m.ry[k - 1];
-      }
-      const int q2 = k - a.sum_first;
-      a.sum_shift[q2] = make_double2(-Tx + mx, -Ty + my);
-      a.sum_frames[q2] = k;
-      a.sum_apply[q2] = (k == a.sum_first && !a.align_to_mid) ? 0 : 1;
-    }
-    // the final solve's per-step shifts into work[], where the host reads them
-    for (int k = 0; k < nc; k++) {
-      a.work[k] = wx[k];
-      a.work[nc + k] = wy[k];
-    }
-    *a.status = 0;
-  }
+  solve_outputs(a, m, wx, wy);
 }
 
 cudaError_t launch_solve(const SolveArgs& a, cudaStream_t st) {
