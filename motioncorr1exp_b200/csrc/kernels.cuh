@@ -219,6 +219,10 @@ struct SolveArgs {
   int* sum_frames;
   int* sum_apply;
   int* status;           // 0 ok, -6 singular system
+  // the frames' DC terms gathered beside the other results: dc[f] = spec[f * spec_stride]
+  float2* dc;
+  const float2* spec;
+  long long spec_stride;
 };
 cudaError_t launch_solve(const SolveArgs& a, cudaStream_t st);
 cudaError_t launch_ramp(const double2* shifts, int nsum, int n, float2* ey, cudaStream_t st);

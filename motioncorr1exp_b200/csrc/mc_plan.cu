@@ -18,6 +18,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/mc.h"
@@ -475,6 +476,7 @@ struct mc_plan {
   int *d_mask = nullptr, *d_order = nullptr, *d_uf = nullptr, *d_kept = nullptr, *d_nkept = nullptr;
   int* d_status = nullptr;
   unsigned char* h_stage = nullptr;  // pinned copies of the per-movie results
+  unsigned char* d_stage = nullptr;  // their device block (d_pshift .. d_status point into it)
   const void** d_src_slot = nullptr;  // device word: base of the run's frames (read by the forward kernels)
   size_t st_dc = 0, st_pshift = 0, st_pcc = 0, st_ppeak = 0, st_ki1 = 0, st_kept = 0, st_nkept = 0, st_ki2 = 0,
          st_work = 0, st_status = 0, st_slot = 0, st_bytes = 0;
@@ -1246,9 +1248,6 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
   CKR(pl->alloc(&pl->d_pairs, sizeof(int2) * pl->maxp));
   CKR(pl->alloc(&pl->d_G, sizeof(float2) * (size_t)std::min(pl->maxp, kPairBatch) * pl->H * pl->box));
   CKR(pl->alloc(&pl->d_boxes, sizeof(float) * (size_t)pl->maxp * pl->box * pl->box));
-  CKR(pl->alloc(&pl->d_pshift, sizeof(float) * 2 * pl->maxp));
-  CKR(pl->alloc(&pl->d_pcc, sizeof(float) * pl->maxp));
-  CKR(pl->alloc(&pl->d_ppeak, sizeof(int) * 2 * pl->maxp));
   CKR(pl->alloc(&pl->d_sum, sizeof(float2) * pl->fstride));
   CKR(pl->alloc(&pl->d_T2, sizeof(float2) * (size_t)pl->n * pl->ldt2));
   CKR(pl->alloc(&pl->d_sumacc, sizeof(float2) * pl->fstride));
@@ -1270,37 +1269,43 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
     CKR(upload(pl, pl->d_pairs_main, pr));
     CKR(pl->alloc(&pl->d_M, sizeof(double) * (size_t)nc * nc));
     CKR(pl->alloc(&pl->d_rhs, sizeof(double) * 2 * (size_t)nc));
-    CKR(pl->alloc(&pl->d_work, sizeof(double) * (2 * (size_t)nc + 2 * (size_t)nf)));
-    CKR(pl->alloc(&pl->d_ki1, sizeof(double) * np));
-    CKR(pl->alloc(&pl->d_ki2, sizeof(double) * np));
     CKR(pl->alloc(&pl->d_dshift, sizeof(double) * 2 * (size_t)nc));
     CKR(pl->alloc(&pl->d_dfshift, sizeof(double) * 2 * (size_t)nf));
     CKR(pl->alloc(&pl->d_mask, sizeof(int) * np));
     CKR(pl->alloc(&pl->d_order, sizeof(int) * np));
     CKR(pl->alloc(&pl->d_uf, sizeof(int) * nf));
-    CKR(pl->alloc(&pl->d_kept, sizeof(int) * np));
-    CKR(pl->alloc(&pl->d_nkept, sizeof(int)));
-    CKR(pl->alloc(&pl->d_status, sizeof(int)));
     size_t o = 0;
     auto place = [&](size_t& off, size_t bytes) {
       off = o;
       o += (bytes + 15) / 16 * 16;
     };
     place(pl->st_dc, sizeof(float2) * nf);
-    place(pl->st_pshift, sizeof(float) * 2 * np);
-    place(pl->st_pcc, sizeof(float) * np);
-    place(pl->st_ppeak, sizeof(int) * 2 * np);
+    place(pl->st_pshift, sizeof(float) * 2 * pl->maxp);
+    place(pl->st_pcc, sizeof(float) * pl->maxp);
+    place(pl->st_ppeak, sizeof(int) * 2 * pl->maxp);
     place(pl->st_ki1, sizeof(double) * np);
     place(pl->st_kept, sizeof(int) * np);
     place(pl->st_nkept, sizeof(int));
     place(pl->st_ki2, sizeof(double) * np);
-    place(pl->st_work, sizeof(double) * 2 * (size_t)nc);
+    place(pl->st_work, sizeof(double) * (2 * (size_t)nc + 2 * (size_t)nf));
     place(pl->st_status, sizeof(int));
     place(pl->st_slot, sizeof(void*));
     pl->st_bytes = o;
     if (injected_alloc_failure())
       return set_err(MC_E_NOMEM, "cudaMallocHost(%zu bytes) failed: injected failure (mc_debug_fail_alloc)", o);
     CK(cudaMallocHost(&pl->h_stage, o));
+    // the results' device block has the staging's layout: one copy brings them all
+    CKR(pl->alloc(&pl->d_stage, pl->st_slot));
+    auto at = [&](auto** p, size_t off) { *p = reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(pl->d_stage + off); };
+    at(&pl->d_pshift, pl->st_pshift);
+    at(&pl->d_pcc, pl->st_pcc);
+    at(&pl->d_ppeak, pl->st_ppeak);
+    at(&pl->d_ki1, pl->st_ki1);
+    at(&pl->d_kept, pl->st_kept);
+    at(&pl->d_nkept, pl->st_nkept);
+    at(&pl->d_ki2, pl->st_ki2);
+    at(&pl->d_work, pl->st_work);
+    at(&pl->d_status, pl->st_status);
     CKR(pl->alloc(&pl->d_src_slot, sizeof(void*)));
   }
 
@@ -2459,9 +2464,7 @@ int mc_plan_refine(mc_plan* pl, int iterations) {
 // pairs -> device solve -> sum -> result copies into the pinned staging,
 // all on the plan stream without a host synchronisation.
 static int enqueue_tail(mc_plan* pl, unsigned char* hs, bool windows_done = false) {
-  const int np = (int)pl->pairs.size(), nf = pl->nframe, nc = nf - 1;
-  CK(cudaMemcpy2DAsync(hs + pl->st_dc, sizeof(float2), pl->d_specA, sizeof(float2) * pl->fstride, sizeof(float2),
-                       nf, cudaMemcpyDeviceToHost, pl->st));
+  const int np = (int)pl->pairs.size(), nf = pl->nframe;
   if (!windows_done)
     CKR(enqueue_windows(pl, pl->d_specA, pl->fstride, pl->d_specB, pl->fstride, pl->pairs, 0, np, pl->d_pairs_main,
                         nullptr));
@@ -2494,6 +2497,9 @@ static int enqueue_tail(mc_plan* pl, unsigned char* hs, bool windows_done = fals
   s.sum_frames = pl->d_sumframes;
   s.sum_apply = pl->d_apply;
   s.status = pl->d_status;
+  s.dc = reinterpret_cast<float2*>(pl->d_stage + pl->st_dc);
+  s.spec = pl->d_specA;
+  s.spec_stride = pl->fstride;
   LAUNCH(pl, MC_K_SOLVE, (double)np * (2 * sizeof(float) + 2 * sizeof(double) + sizeof(int)) + (double)nf * 4 * sizeof(double),
          mc::launch_solve(s, pl->st));
   mc::ShiftSumArgs a{};
@@ -2525,16 +2531,7 @@ static int enqueue_tail(mc_plan* pl, unsigned char* hs, bool windows_done = fals
   c.plan = pl->plan_n;
   c.tw = pl->d_tw_n;
   LAUNCH(pl, MC_K_C2R_ROWS, spec_bytes + (double)pl->n * pl->n * sizeof(float), mc::launch_c2r_rows(c, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_pshift, pl->d_pshift, sizeof(float) * 2 * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_pcc, pl->d_pcc, sizeof(float) * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_ppeak, pl->d_ppeak, sizeof(int) * 2 * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_ki1, pl->d_ki1, sizeof(double) * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_kept, pl->d_kept, sizeof(int) * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_nkept, pl->d_nkept, sizeof(int), cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_ki2, pl->d_ki2, sizeof(double) * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_work, pl->d_work, sizeof(double) * 2 * (size_t)nc, cudaMemcpyDeviceToHost,
-                     pl->st));
-  CK(cudaMemcpyAsync(hs + pl->st_status, pl->d_status, sizeof(int), cudaMemcpyDeviceToHost, pl->st));
+  CK(cudaMemcpyAsync(hs, pl->d_stage, pl->st_slot, cudaMemcpyDeviceToHost, pl->st));
   return MC_OK;
 }
 

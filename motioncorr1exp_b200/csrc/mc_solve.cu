@@ -20,6 +20,10 @@ namespace {
 
 constexpr int kSolveThreads = 256;
 
+__device__ void gather_dc(const SolveArgs& a) {
+  for (int f = threadIdx.x; f < a.nframe; f += kSolveThreads) a.dc[f] = a.spec[f * a.spec_stride];
+}
+
 __device__ int uf_find(int* par, int x) {
   while (par[x] != x) {
     par[x] = par[par[x]];
@@ -111,6 +115,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve(SolveArgs a) {
   double* cy = a.work + 2 * nc + nf;
   int* mask = a.mask;
   int* order = a.order;
+  gather_dc(a);
   for (int r = tid; r < P; r += kSolveThreads) mask[r] = 1;
   __syncthreads();
   if (!solve_masked(a, mask, wx, wy)) {
@@ -436,6 +441,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_smem(SolveArgs a) {
   m.hist = m.mask + P;
   m.order = m.hist + (size_t)nc * nf;
   m.uf = m.order + P;
+  gather_dc(a);
   for (int r = tid; r < P; r += kSolveThreads) {
     m.pr[r] = a.pairs[r];
     m.ps[r] = make_float2(a.pshift[2 * r], a.pshift[2 * r + 1]);
