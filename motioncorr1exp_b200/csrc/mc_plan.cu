@@ -479,7 +479,7 @@ struct mc_plan {
   unsigned char* d_stage = nullptr;  // their device block (d_pshift .. d_status point into it)
   const void** d_src_slot = nullptr;  // device word: base of the run's frames (read by the forward kernels)
   size_t st_dc = 0, st_pshift = 0, st_pcc = 0, st_ppeak = 0, st_ki1 = 0, st_kept = 0, st_nkept = 0, st_ki2 = 0,
-         st_work = 0, st_status = 0, st_slot = 0, st_bytes = 0;
+         st_work = 0, st_status = 0, st_slot = 0, st_obj = 0, st_bytes = 0;
   // captured movie graphs, one per frame configuration (frame range, sum
   // range, pair distance, threshold, reference frame) the plan has run
   struct GraphEntry {
@@ -800,6 +800,23 @@ int enqueue_pair_stage(mc_plan* pl, const float2* specA, long long strideA, cons
   return enqueue_peaks(pl, (int)list.size());
 }
 
+// The pair results' part of the result block into the pinned staging, and from
+// there (after a synchronisation) to the host's lists.
+int fetch_pairs(mc_plan* pl) {
+  CK(cudaMemcpyAsync(pl->h_stage + pl->st_pshift, pl->d_stage + pl->st_pshift, pl->st_ki1 - pl->st_pshift,
+                     cudaMemcpyDeviceToHost, pl->st));
+  return MC_OK;
+}
+
+void read_pairs(const mc_plan* pl, int np, std::vector<float>& shift, std::vector<float>& cc, std::vector<int>& peak) {
+  const float* s = reinterpret_cast<const float*>(pl->h_stage + pl->st_pshift);
+  const float* c = reinterpret_cast<const float*>(pl->h_stage + pl->st_pcc);
+  const int* k = reinterpret_cast<const int*>(pl->h_stage + pl->st_ppeak);
+  shift.assign(s, s + 2 * (size_t)np);
+  cc.assign(c, c + np);
+  peak.assign(k, k + 2 * (size_t)np);
+}
+
 // pair stage over an explicit list of spectrum indices, synchronous,
 // results to the host
 int run_pair_list_held(mc_plan* pl, const float2* specA, long long strideA, const float2* specB, long long strideB,
@@ -814,10 +831,9 @@ int run_pair_list_held(mc_plan* pl, const float2* specA, long long strideA, cons
   if (np > pl->maxp) return set_err(MC_E_STATE, "pair list larger than the plan's capacity");
   CK(cudaMemcpyAsync(pl->d_pairs, pr.data(), sizeof(int2) * np, cudaMemcpyHostToDevice, pl->st));
   CKR(enqueue_pair_stage(pl, specA, strideA, specB, strideB, list, pl->d_pairs));
-  CK(cudaMemcpyAsync(shift.data(), pl->d_pshift, sizeof(float) * 2 * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(cc.data(), pl->d_pcc, sizeof(float) * np, cudaMemcpyDeviceToHost, pl->st));
-  CK(cudaMemcpyAsync(peak.data(), pl->d_ppeak, sizeof(int) * 2 * np, cudaMemcpyDeviceToHost, pl->st));
+  CKR(fetch_pairs(pl));
   CK(cudaStreamSynchronize(pl->st));
+  read_pairs(pl, np, shift, cc, peak);
   return pl->collect();
 }
 
@@ -885,15 +901,26 @@ int run_pair_list(mc_plan* pl, const float2* specA, long long strideA, const flo
   return MC_OK;
 }
 
+// The frame list of a sum to the device: shifts, spectrum positions and apply
+// flags in one copy (pageable: the source is free when it returns).
+int upload_sum_list(mc_plan* pl, const std::vector<int>& frames, const std::vector<cplx>& shifts,
+                    const std::vector<int>& apply) {
+  const size_t ns = frames.size(), capf = pl->cap_frames;
+  std::vector<double2> block(capf + (capf + 1) / 2);
+  for (size_t i = 0; i < ns; i++) block[i] = make_double2(shifts[i].real(), shifts[i].imag());
+  int* q = reinterpret_cast<int*>(block.data() + capf);
+  std::copy(frames.begin(), frames.end(), q);
+  std::copy(apply.begin(), apply.end(), q + capf);
+  CK(cudaMemcpyAsync(pl->d_sumshift, block.data(), (sizeof(double2) + 2 * sizeof(int)) * capf, cudaMemcpyHostToDevice,
+                     pl->st));
+  return MC_OK;
+}
+
 // sum of phase-shifted frames of set A; mode 0 -> d_sum spectrum, mode 1 -> image
 int run_shift_sum_held(mc_plan* pl, const std::vector<int>& frames, const std::vector<cplx>& shifts,
                        const std::vector<int>& apply, int mode, int accumulate = 0) {
   const int ns = (int)frames.size();
-  std::vector<double2> sh(ns);
-  for (int i = 0; i < ns; i++) sh[i] = make_double2(shifts[i].real(), shifts[i].imag());
-  CK(cudaMemcpyAsync(pl->d_sumframes, frames.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, pl->st));
-  CK(cudaMemcpyAsync(pl->d_apply, apply.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, pl->st));
-  CK(cudaMemcpyAsync(pl->d_sumshift, sh.data(), sizeof(double2) * ns, cudaMemcpyHostToDevice, pl->st));
+  CKR(upload_sum_list(pl, frames, shifts, apply));
   mc::ShiftSumArgs a{};
   a.spec = pl->d_specA;
   a.stride = pl->fstride;
@@ -1253,9 +1280,10 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
   CKR(pl->alloc(&pl->d_sumacc, sizeof(float2) * pl->fstride));
   CKR(pl->alloc(&pl->d_ey, sizeof(float2) * (size_t)capf * pl->n));
   CKR(pl->alloc(&pl->d_image, sizeof(float) * (size_t)pl->n * pl->n));
-  CKR(pl->alloc(&pl->d_sumframes, sizeof(int) * capf));
-  CKR(pl->alloc(&pl->d_apply, sizeof(int) * capf));
-  CKR(pl->alloc(&pl->d_sumshift, sizeof(double2) * capf));
+  // the summed frames' shifts, positions and flags, one block (upload_sum_list)
+  CKR(pl->alloc(&pl->d_sumshift, (sizeof(double2) + 2 * sizeof(int)) * capf));
+  pl->d_sumframes = reinterpret_cast<int*>(pl->d_sumshift + capf);
+  pl->d_apply = pl->d_sumframes + capf;
   CKR(pl->alloc(&pl->d_opart, sizeof(double) * ((size_t)pl->H * capf * 5 + pl->H)));
   CKR(pl->alloc(&pl->d_oout, sizeof(double) * ((size_t)capf * 5 + 1)));
   {
@@ -1290,6 +1318,7 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
     place(pl->st_work, sizeof(double) * (2 * (size_t)nc + 2 * (size_t)nf));
     place(pl->st_status, sizeof(int));
     place(pl->st_slot, sizeof(void*));
+    place(pl->st_obj, sizeof(double) * ((size_t)nf * 5 + 1));
     pl->st_bytes = o;
     if (injected_alloc_failure())
       return set_err(MC_E_NOMEM, "cudaMallocHost(%zu bytes) failed: injected failure (mc_debug_fail_alloc)", o);
@@ -1778,9 +1807,11 @@ static int forward_all(mc_plan* pl, const std::vector<cudaEvent_t>* waits, int c
   } else {
     CKR(enqueue_forward(pl, waits, chunk));
     CK(cudaEventRecord(pl->ev[1], pl->st));
-    CK(cudaMemcpy2DAsync(dc.data(), sizeof(float2), pl->d_specA, sizeof(float2) * pl->fstride, sizeof(float2),
-                         pl->nframe, cudaMemcpyDeviceToHost, pl->st));
+    float2* hdc = reinterpret_cast<float2*>(pl->h_stage + pl->st_dc);
+    CK(cudaMemcpy2DAsync(hdc, sizeof(float2), pl->d_specA, sizeof(float2) * pl->fstride, sizeof(float2), pl->nframe,
+                         cudaMemcpyDeviceToHost, pl->st));
     CK(cudaStreamSynchronize(pl->st));
+    std::copy(hdc, hdc + pl->nframe, dc.begin());
   }
   CKR(pl->collect());
   CK(cudaEventElapsedTime(&pl->tm.forward_ms, pl->ev[0], pl->ev[1]));
@@ -1857,10 +1888,19 @@ int mc_plan_pairs(mc_plan* pl) {
   if (!pl->have_forward) return set_err(MC_E_STATE, "pairs before forward");
   CK(cudaSetDevice(pl->device));
   CK(cudaEventRecord(pl->ev[2], pl->st));
-  CKR(run_pair_list(pl, pl->d_specA, pl->fstride, pl->d_specB, pl->fstride, pl->pairs, pl->pshift, pl->pcc,
-                    pl->ppeak));
-  CK(cudaEventRecord(pl->ev[3], pl->st));
-  CK(cudaEventSynchronize(pl->ev[3]));
+  if (pl->slots) {
+    CKR(run_pair_list(pl, pl->d_specA, pl->fstride, pl->d_specB, pl->fstride, pl->pairs, pl->pshift, pl->pcc,
+                      pl->ppeak));
+    CK(cudaEventRecord(pl->ev[3], pl->st));
+    CK(cudaEventSynchronize(pl->ev[3]));
+  } else {
+    CKR(enqueue_pair_stage(pl, pl->d_specA, pl->fstride, pl->d_specB, pl->fstride, pl->pairs, pl->d_pairs_main));
+    CK(cudaEventRecord(pl->ev[3], pl->st));
+    CKR(fetch_pairs(pl));
+    CK(cudaStreamSynchronize(pl->st));
+    read_pairs(pl, (int)pl->pairs.size(), pl->pshift, pl->pcc, pl->ppeak);
+    CKR(pl->collect());
+  }
   CK(cudaEventElapsedTime(&pl->tm.pairs_ms, pl->ev[2], pl->ev[3]));
   log_pairs(pl);
   pl->have_pairs = true;
@@ -2383,8 +2423,8 @@ static int objective(mc_plan* pl, const std::vector<cplx>& s, double* J, double*
     LAUNCH_N(pl, MC_K_OBJECTIVE, (double)(nf + 1) * pl->H * pl->n * sizeof(float2), 2,
              mc::launch_objective(a, pl->st));
   }
-  std::vector<double> out((size_t)nf * 5 + 1);
-  CK(cudaMemcpyAsync(out.data(), pl->d_oout, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, pl->st));
+  double* out = reinterpret_cast<double*>(pl->h_stage + pl->st_obj);
+  CK(cudaMemcpyAsync(out, pl->d_oout, sizeof(double) * ((size_t)nf * 5 + 1), cudaMemcpyDeviceToHost, pl->st));
   CK(cudaStreamSynchronize(pl->st));
   CKR(pl->collect());
   if (J) *J = out[(size_t)nf * 5];
