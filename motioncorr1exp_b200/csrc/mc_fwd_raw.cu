@@ -55,56 +55,6 @@ __global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS / 2)
   }
 }
 
-// Forward rows: two image rows (or the two reference sets of one row) packed
-// as one complex transform, then split into the two real half spectra.
-template <int N1, int N2>
-__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_rows2l(FwdRowsArgs a) {
-  using TL = TwoLevel<N1, N2>;
-  constexpr int N = TL::N;
-  extern __shared__ float2 dyn2l[];
-  float2* xin = dyn2l;      // packed input rows, later the spectrum Z
-  float2* ysm = dyn2l + N;  // exchange buffer
-  int y0, y1;
-  if (a.two_outputs) {
-    y0 = blockIdx.x;
-    y1 = y0;
-  } else {
-    y0 = 2 * blockIdx.x;
-    y1 = y0 + 1;
-  }
-  const long long r0 = (long long)(a.offy + y0) * a.nx + a.offx;
-  const long long r1 = (long long)(a.offy + y1) * a.nx + a.offx;
-  switch (a.mode) {
-    case 0: stage_rows<int8_t>(xin, a, r0, r1, N, TL::T); break;
-    case MC_MODE_U8: stage_rows<uint8_t>(xin, a, r0, r1, N, TL::T); break;
-    case 1: stage_rows<int16_t>(xin, a, r0, r1, N, TL::T); break;
-    case 6: stage_rows<uint16_t>(xin, a, r0, r1, N, TL::T); break;
-    case MC_MODE_F16: stage_rows<__half>(xin, a, r0, r1, N, TL::T); break;
-    default: stage_rows<float>(xin, a, r0, r1, N, TL::T); break;
-  }
-  __syncthreads();
-  // step B writes Z into xin: every step-A read of xin precedes the barrier
-  // between the steps, and step B reads only ysm
-  float2* zsm = xin;
-  TL::template run<false, false>(
-      ysm, a.tw + N, [&](int x) { return xin[x]; }, [&](int k, float2 v) { zsm[k] = v; });
-  __syncthreads();
-  float2* outA = a.outA + blockIdx.y * a.out_stride;
-  float2* outB = a.two_outputs ? a.outB + blockIdx.y * a.out_stride : nullptr;
-  for (int k = threadIdx.x; k < a.hk; k += TL::T) {
-    const float2 z = zsm[k];
-    const float2 zc = zsm[k == 0 ? 0 : N - k];
-    const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
-    const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
-    if (a.two_outputs) {
-      outA[(long long)k * a.ldt + y0] = X;
-      outB[(long long)k * a.ldt + y0] = Y;
-    } else {
-      *reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0) = make_float4(X.x, X.y, Y.x, Y.y);
-    }
-  }
-}
-
 template <int A, int B, typename PX, bool PR>
 cudaError_t launch_raw_rows_p(const FwdRowsArgs& a, int grid, cudaStream_t st) {
   const size_t smem = 2 * (size_t)A * B * sizeof(float2) + 4 * (size_t)raw_row_bytes<PX>(A * B);
@@ -123,6 +73,8 @@ cudaError_t launch_raw_rows(const FwdRowsArgs& a, bool paired, int grid, cudaStr
   }
   return launch_raw_rows_p<A, B, PX, kFwdRowsPaired>(a, grid, st);
 }
+
+cudaError_t launch_fwd_rows2l_refs(const FwdRowsArgs& a, cudaStream_t st);
 
 cudaError_t launch_fwd_rows2l(const FwdRowsArgs& a, cudaStream_t st) {
   int n1 = 0, n2 = 0;
@@ -144,11 +96,7 @@ cudaError_t launch_fwd_rows2l(const FwdRowsArgs& a, cudaStream_t st) {
         default: MC_TL_RAW(A, B, float)                                                              \
       }                                                                                              \
     }                                                                                                \
-    const size_t smem = (size_t)2 * (A) * (B) * sizeof(float2);                                      \
-    cudaError_t e = allow_smem((const void*)k_fwd_rows2l<A, B>, smem);                               \
-    if (e != cudaSuccess) return e;                                                                  \
-    k_fwd_rows2l<A, B><<<dim3(grid, std::max(a.nfr, 1)), TwoLevel<A, B>::T, smem, st>>>(a);                                    \
-    return cudaGetLastError();                                                                       \
+    return launch_fwd_rows2l_refs(a, st);                                                            \
   }
   MC_TWO_LEVEL_LIST(MC_TL_LAUNCH)
 #undef MC_TL_LAUNCH
