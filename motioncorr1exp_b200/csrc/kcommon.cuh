@@ -52,10 +52,13 @@ __device__ __forceinline__ const void* fwd_frame(const FwdRowsArgs& a) {
 // (mc_schedule_set, the autotuner) can pick either.
 constexpr bool kFwdRowsPaired = true;
 constexpr bool kFwdColsPaired = true;
-// Resident CTAs per SM the two-level transforms are compiled for (register cap).
-#ifndef MC_TL_MIN_BLOCKS
-#define MC_TL_MIN_BLOCKS 4
-#endif
+// Resident CTAs per SM the two-level transforms of T threads are compiled for
+// (register cap): 168 registers at 96 and 64 threads, 128 at 32.  4096^2 column
+// pass, 24 frames, with four / five / six CTAs of 64 threads 1062, 940, 942 us,
+// 2048^2 row pass 311, 310, 263; 16 x 1024^2 row pass with 4 / 10 / 16 CTAs of 32
+// 66, 65, 61; 96 threads with five (136 registers, spills): 3710^2 column pass
+// 1.67 -> 2.14 ms.
+constexpr int tl_min_blocks(int T) { return T == 96 ? 4 : T == 64 ? 6 : 16; }
 
 template <int N1, int N2>
 struct TwoLevel {

@@ -172,7 +172,7 @@ cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, cudaStream_t st)
 
 // Batched rows: out_row[i] = scale * X[i < keep_lo ? i : i + (n - n_out)].
 template <int N1, int N2, bool INV, bool PAIRED, bool PLAIN = false>
-__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_rows_fft2l(RowsFftArgs a) {
+__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, tl_min_blocks(TwoLevel<N1, N2>::T)) k_rows_fft2l(RowsFftArgs a) {
   using TL = TwoLevel<N1, N2>;
   __shared__ float2 ysm[TL::N];
   const long long row = blockIdx.x;

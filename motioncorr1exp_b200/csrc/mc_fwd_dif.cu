@@ -25,35 +25,31 @@ __device__ __forceinline__ int dif_kmax(int lo) {
   return k < (N1 - 1) / 2 ? k : (N1 - 1) / 2;
 }
 
-// Forward rows of length L without references: two rows staged as raw
-// pixels; only the Z indices the half-spectrum split needs are kept in
-// shared memory (Z[0, hk) and Z(L - hk, L)).
+// Forward rows of length L without references: two rows packed, read by the
+// step-A loads.  Only the Z indices the half-spectrum split needs are kept,
+// Z[0, hk) and Z(L - hk, L): the even ones, of the first transform, in a buffer
+// of their own, the odd ones in the exchange buffer once the second transform
+// has read it.  44.6 KB a CTA at 7420 -> 3710 (74 with the raw rows and every
+// kept index staged): registers, not shared memory, set the four CTAs per SM.
+// @@DIF@@
 template <int N1, int N2, typename Px>
-__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_rows_dif(FwdRowsArgs a) {
+__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_fwd_rows_dif(FwdRowsArgs a) {
   using TL = TwoLevel<N1, N2>;
   constexpr int N = TL::N, L = 2 * N;
-  constexpr int RB = raw_row_bytes<Px>(L);
   extern __shared__ float2 dyndif[];
-  const int hk = a.hk;
-  float2* ysm = dyndif;
-  float2* zlo = dyndif + N;   // Z[0 .. hk-1]
-  float2* zhi = zlo + hk;     // Z[L-hk+1 .. L-1]
-  unsigned char* raw0 = reinterpret_cast<unsigned char*>(zhi + hk);
-  unsigned char* raw1 = raw0 + RB;
+  const int hk = a.hk, half = hk / 2 + 1;
+  float2* zeven = dyndif;             // [2][half]: low, then high indices
+  float2* ysm = dyndif + 2 * half;    // exchange buffer, later the odd indices
+  float2* zodd = ysm;
   const int y0 = 2 * blockIdx.x, y1 = y0 + 1;
   float2* outA = a.outA + blockIdx.y * a.out_stride;
   const Px* f = reinterpret_cast<const Px*>(fwd_frame(a));
-  const Px* row0 = f + (long long)(a.offy + y0) * a.nx + a.offx;
-  const Px* row1 = f + (long long)(a.offy + y1) * a.nx + a.offx;
-  stage_raw_row<Px>(raw0, row0, L, threadIdx.x, TL::T);
-  stage_raw_row<Px>(raw1, row1, L, threadIdx.x, TL::T);
-  __syncthreads();
-  const Px* p0 = reinterpret_cast<const Px*>(raw0 + (reinterpret_cast<uintptr_t>(row0) & 15));
-  const Px* p1 = reinterpret_cast<const Px*>(raw1 + (reinterpret_cast<uintptr_t>(row1) & 15));
+  const Px* p0 = f + (long long)(a.offy + y0) * a.nx + a.offx;
+  const Px* p1 = f + (long long)(a.offy + y1) * a.nx + a.offx;
   const float2* tw = a.tw;
-  auto keep = [&](int idx, float2 v) {
-    if (idx < hk) zlo[idx] = v;
-    else if (idx > L - hk) zhi[idx - (L - hk + 1)] = v;
+  auto keep = [&](float2* z, int idx, float2 v) {
+    if (idx < hk) z[idx >> 1] = v;
+    else if (idx > L - hk) z[half + ((idx - (L - hk + 1)) >> 1)] = v;
   };
   // wanted A/B outputs: m < hk/2 or m > N - hk/2, i.e. m = k2 + N2*k1 with
   // k1 or N1 - 1 - k1 at most (hk/2)/N2
@@ -63,19 +59,20 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_r
       [&](int n) {
         return make_float2((float)p0[n] + (float)p0[n + N], (float)p1[n] + (float)p1[n + N]);
       },
-      [&](int m, float2 v) { keep(2 * m, v); }, kmax);
+      [&](int m, float2 v) { keep(zeven, 2 * m, v); }, kmax);
   __syncthreads();
-  TL::template run<false, false, false>(
+  TL::template run<false, true, false>(
       ysm, tw + L,
       [&](int n) {
         const float2 d = make_float2((float)p0[n] - (float)p0[n + N], (float)p1[n] - (float)p1[n + N]);
         return cmul(d, __ldg(tw + n));
       },
-      [&](int m, float2 v) { keep(2 * m + 1, v); }, kmax);
+      [&](int m, float2 v) { keep(zodd, 2 * m + 1, v); }, kmax);
   __syncthreads();
   for (int k = threadIdx.x; k < hk; k += TL::T) {
-    const float2 z = zlo[k];
-    const float2 zc = k == 0 ? zlo[0] : zhi[hk - 1 - k];
+    const float2* zs = k & 1 ? zodd : zeven;
+    const float2 z = zs[k >> 1];
+    const float2 zc = k == 0 ? z : zs[half + ((hk - 1 - k) >> 1)];
     const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
     const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
     *reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0) = make_float4(X.x, X.y, Y.x, Y.y);
@@ -84,7 +81,7 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_fwd_r
 
 // Forward columns of length L: out_row[i] = scale * X[i < keep_lo ? i : i + (L - n_out)].
 template <int N1, int N2>
-__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS) k_rows_fft_dif(RowsFftArgs a) {
+__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_rows_fft_dif(RowsFftArgs a) {
   using TL = TwoLevel<N1, N2>;
   constexpr int N = TL::N, L = 2 * N;
   __shared__ float2 ysm[N];
@@ -127,8 +124,8 @@ cudaError_t launch_fwd_rows_dif(const FwdRowsArgs& a, cudaStream_t st) {
   const dim3 grid(a.nu / 2, std::max(a.nfr, 1));
 #define MC_DIF_RAW(A, B, PX)                                                                          \
   {                                                                                                   \
-    const size_t smem = ((size_t)(A) * (B) + 2 * (size_t)a.hk) * sizeof(float2) +                     \
-                        2 * (size_t)raw_row_bytes<PX>(2 * (A) * (B));                                 \
+    const size_t kept = 2 * (size_t)(a.hk / 2 + 1);                                                   \
+    const size_t smem = (kept + std::max<size_t>((size_t)(A) * (B), kept)) * sizeof(float2);          \
     cudaError_t e = allow_smem((const void*)k_fwd_rows_dif<A, B, PX>, smem);                          \
     if (e != cudaSuccess) return e;                                                                   \
     k_fwd_rows_dif<A, B, PX><<<grid, TwoLevel<A, B>::T, smem, st>>>(a);                               \

@@ -1,42 +1,35 @@
-// Forward row pass of libmc for two-level lengths (sm_100a): two rows packed
-// as one complex FFT, raw-pixel staging when no dark/gain references apply
-// (DFAlign.cu:710-806).
+// Forward row pass of libmc for two-level lengths without dark/gain references
+// (sm_100a): two rows packed as one complex FFT (DFAlign.cu:710-806).
 #include <algorithm>
 
 #include "kcommon.cuh"
 
 namespace mc {
 
-// Forward rows without references, four rows per CTA: the rows are staged
-// as raw pixels (a quarter of the float staging for 8-bit frames) and
-// decoded in the step-A loads; two teams of T threads each run one packed
-// two-row transform (the same code and barriers side by side) and write
-// their spectrum Z back into their exchange buffer after the barrier that
-// follows the step-B reads; then the CTA writes the four rows' half spectra
-// as one 32-byte sector per kx (two threads per sector) instead of two half
-// sectors from two CTAs (c2 row pass 3.33 -> 3.09 ms per movie).  The last
+// Forward rows without references, four rows per CTA: two teams of T threads
+// each run one packed two-row transform, its step-A loads decoding the pixels
+// straight from global memory (N2 independent loads of either row a thread;
+// staging the raw rows first cost the CTA a phase of its own and shared memory
+// for another CTA: 40 x 3710^2 uint8 2.61 -> 2.10 ms, 24 x 4096^2 float 2.02 ->
+// 1.20, 16 x 1024^2 float 73 -> 61 us); they write their spectrum Z back into
+// their exchange buffer after the barrier that follows the step-B reads; then
+// the CTA writes the four rows' half spectra as one 32-byte sector per kx (two
+// threads per sector) instead of two half sectors from two CTAs.  The last
 // CTA of an odd pair count runs its second team on a copy of the first pair
 // and stores only the first.
 template <int N1, int N2, typename Px, bool PAIRED>
-__global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS / 2) k_fwd_rows2l_raw4(FwdRowsArgs a) {
+__global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, tl_min_blocks(TwoLevel<N1, N2>::T) / 2) k_fwd_rows2l_raw4(FwdRowsArgs a) {
   using TL = TwoLevel<N1, N2>;
   constexpr int N = TL::N, T = TL::T;
-  constexpr int RB = raw_row_bytes<Px>(N);
   extern __shared__ float2 dynraw[];
   const int tid = threadIdx.x, team = tid / T, lt = tid - team * T;
   float2* ysm = dynraw + (size_t)team * N;
-  unsigned char* rawb = reinterpret_cast<unsigned char*>(dynraw + 2 * N);  // four staged rows
   const int y0 = 4 * blockIdx.x;
   float2* outA = a.outA + blockIdx.y * a.out_stride;
   const bool two = y0 + 2 < a.nu;  // the second row pair exists
   const Px* f = reinterpret_cast<const Px*>(fwd_frame(a));
   auto row = [&](int j) { return f + (long long)(a.offy + y0 + (two ? j : (j & 1))) * a.nx + a.offx; };
-#pragma unroll
-  for (int j = 0; j < 4; j++) stage_raw_row<Px>(rawb + j * RB, row(j), N, tid, 2 * T);
-  __syncthreads();
-  const Px* p0 = reinterpret_cast<const Px*>(rawb + (2 * team) * RB + (reinterpret_cast<uintptr_t>(row(2 * team)) & 15));
-  const Px* p1 =
-      reinterpret_cast<const Px*>(rawb + (2 * team + 1) * RB + (reinterpret_cast<uintptr_t>(row(2 * team + 1)) & 15));
+  const Px *p0 = row(2 * team), *p1 = row(2 * team + 1);
   TL::template run<false, true, PAIRED>(
       ysm, a.tw + N, [&](int x) { return make_float2((float)p0[x], (float)p1[x]); },
       [&](int k, float2 v) { ysm[k] = v; }, (N1 - 1) / 2, lt);
@@ -57,7 +50,7 @@ __global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS / 2)
 
 template <int A, int B, typename PX, bool PR>
 cudaError_t launch_raw_rows_p(const FwdRowsArgs& a, int grid, cudaStream_t st) {
-  const size_t smem = 2 * (size_t)A * B * sizeof(float2) + 4 * (size_t)raw_row_bytes<PX>(A * B);
+  const size_t smem = 2 * (size_t)A * B * sizeof(float2);
   cudaError_t e = allow_smem((const void*)k_fwd_rows2l_raw4<A, B, PX, PR>, smem);
   if (e != cudaSuccess) return e;
   k_fwd_rows2l_raw4<A, B, PX, PR><<<dim3((grid + 1) / 2, std::max(a.nfr, 1)), 2 * TwoLevel<A, B>::T, smem, st>>>(a);

@@ -17,7 +17,7 @@ namespace mc {
 // rows as 16 bytes in each set.  Measured, 16 frames of 3710^2 uint16 with dark
 // and gain: 5.63 -> 2.55 ms.
 template <int N1, int N2, typename Px>
-__global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS / 2) k_fwd_rows2l_refs(FwdRowsArgs a) {
+__global__ void __launch_bounds__(2 * TwoLevel<N1, N2>::T, tl_min_blocks(TwoLevel<N1, N2>::T) / 2) k_fwd_rows2l_refs(FwdRowsArgs a) {
   using TL = TwoLevel<N1, N2>;
   constexpr int N = TL::N, T = TL::T;
   extern __shared__ float2 dynref[];

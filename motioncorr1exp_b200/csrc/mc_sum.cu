@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kThreads) k_shift_acc(ShiftSumArgs a, const fl
 // The inverse along ky of each accumulated column, written transposed
 // (out[y * ld_out + kx]) for the C2R row pass.
 template <int N1, int N2>
-__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, MC_TL_MIN_BLOCKS)
+__global__ void __launch_bounds__(TwoLevel<N1, N2>::T, tl_min_blocks(TwoLevel<N1, N2>::T))
     k_sum_cols2l(const float2* __restrict__ in, long long ld_in, const float2* __restrict__ tw, float2* out,
                  long long ld_out) {
   using TL = TwoLevel<N1, N2>;
