@@ -108,6 +108,7 @@ struct PeakArgs {
   const float* boxes;
   int npairs, box, n, nps;
   const double* w16;   // [16][9] cosine-mask weights
+  const double2* tw;   // exp(+2 pi i m / 512) (launch_peak_table)
   float* shift;        // [npairs][2]
   float* cc;           // [npairs]
   int* peak;           // [npairs][2] integer box peak (x, y)
@@ -244,6 +245,8 @@ cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, cudaStream_t st)
 cudaError_t launch_pair_cols(const PairColsArgs& a, cudaStream_t st);
 cudaError_t launch_pair_rows(const PairRowsArgs& a, cudaStream_t st);
 cudaError_t launch_peak(const PeakArgs& a, cudaStream_t st);
+// the 512 table entries of PeakArgs.tw
+cudaError_t launch_peak_table(double2* tw, cudaStream_t st);
 // ey: scratch of nsum*n float2 for the per-frame ky phase ramps
 cudaError_t launch_shift_sum(const ShiftSumArgs& a, float2* ey, cudaStream_t st);
 int shift_sum_kernels(const ShiftSumArgs& a);  // kernels launch_shift_sum launches

@@ -31,7 +31,8 @@ __device__ __forceinline__ int dif_kmax(int lo) {
 // of their own, the odd ones in the exchange buffer once the second transform
 // has read it.  44.6 KB a CTA at 7420 -> 3710 (74 with the raw rows and every
 // kept index staged): registers, not shared memory, set the four CTAs per SM.
-// @@DIF@@
+// 24 frames of 7420^2 uint8 6.98 -> 6.69 ms (two output pairs of the pruned
+// radix-53 step per loop pass: 6.66, with 72 bytes of spills; not taken).
 template <int N1, int N2, typename Px>
 __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_fwd_rows_dif(FwdRowsArgs a) {
   using TL = TwoLevel<N1, N2>;

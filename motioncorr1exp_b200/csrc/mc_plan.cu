@@ -449,6 +449,7 @@ struct mc_plan {
   float* d_boxes_all = nullptr;    // slot mode: pair windows gathered in list order
   float2 *d_tw_nu = nullptr, *d_tw_n = nullptr, *d_twQ = nullptr, *d_twO = nullptr, *d_cs = nullptr;
   double* d_w16 = nullptr;
+  double2* d_peaktw = nullptr;
   int2* d_pairs = nullptr;
   float2* d_G = nullptr;
   float* d_boxes = nullptr;
@@ -786,6 +787,7 @@ int enqueue_peaks(mc_plan* pl, int np) {
   k.n = pl->n;
   k.nps = pl->p.NoisePeakSize;
   k.w16 = pl->d_w16;
+  k.tw = pl->d_peaktw;
   k.shift = pl->d_pshift;
   k.cc = pl->d_pcc;
   k.peak = pl->d_ppeak;
@@ -1388,6 +1390,8 @@ static int create_plan(const mc_params* pin, int nx, int ny, int nz, int mode, i
         w[j * 9 + i] = r < 8 ? std::cos(r * kPi / 8.0) / 2 + 0.5 : 0.0;
       }
     }
+    CKR(pl->alloc(&pl->d_peaktw, sizeof(double2) * 512));
+    CK(mc::launch_peak_table(pl->d_peaktw, pl->st));
     CKR(pl->alloc(&pl->d_w16, sizeof(double) * w.size()));
     CKR(upload(pl, pl->d_w16, w));
   }

@@ -33,6 +33,7 @@ constexpr int kUp = 32;
 
 struct PeakSmem {
   double2 tw[kPad];        // exp(+2 pi i m / 512)
+  double2 tw16[kSub];      // exp(+2 pi i m / 16), side by side (in tw they share their banks)
   double2 s[kSub][9];      // masked 16x16 half spectrum
   double2 sp[8][8];        // s[j] + s[16 - j] (row 0: s[0])
   double2 sn[8][8];        // s[j] - s[16 - j]
@@ -64,6 +65,14 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a, int C) {
   const int wnoise = a.nps - 1;
   const int hb = box / 2;
 
+  // ---- tables
+  for (int m = tid; m < kPad; m += nth) {
+    const double2 w = __ldg(a.tw + m);
+    S.tw[m] = w;
+    if (m % (kPad / kSub) == 0) S.tw16[m / (kPad / kSub)] = w;
+  }
+  const double wt = tid < kSub * 9 ? __ldg(a.w16 + tid) : 0.0;  // this thread's mask weight below
+
   // ---- integer peak (cufunc.cu:409-424): strict '>' from -1e9, y outer, x inner
   float bv = -1e9f;
   int bi = 0x7fffffff;
@@ -92,11 +101,6 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a, int C) {
     S.fv[wid] = bv;
     S.fi[wid] = bi;
   }
-  for (int m = tid; m < kPad; m += nth) {
-    double sn, cn;
-    sincospi((double)m / (kPad / 2), &sn, &cn);
-    S.tw[m] = make_double2(cn, sn);
-  }
   __syncthreads();
   bv = S.fv[0];
   bi = S.fi[0];
@@ -123,11 +127,11 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a, int C) {
   }
   __syncthreads();
   // R2C along x: rx[y][kx] = sum_x sub[y][x] exp(-2 pi i kx x / 16)
-  for (int t = tid; t < kSub * 9; t += nth) {
-    const int yy = t / 9, k = t - yy * 9;
+  if (tid < kSub * 9) {
+    const int yy = tid / 9, k = tid - yy * 9;
     double re = 0.0, im = 0.0;
     for (int xx = 0; xx < kSub; xx++) {
-      const double2 w = S.tw[((k * xx) & (kSub - 1)) * (kPad / kSub)];
+      const double2 w = S.tw16[(k * xx) & (kSub - 1)];
       re += S.sub[yy][xx] * w.x;
       im -= S.sub[yy][xx] * w.y;
     }
@@ -135,16 +139,15 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a, int C) {
   }
   __syncthreads();
   // along y, then the cosine mask (func.cpp:348-370)
-  for (int t = tid; t < kSub * 9; t += nth) {
-    const int j = t / 9, k = t - j * 9;
+  if (tid < kSub * 9) {
+    const int j = tid / 9, k = tid - j * 9;
     double re = 0.0, im = 0.0;
     for (int yy = 0; yy < kSub; yy++) {
-      const double2 w = S.tw[((j * yy) & (kSub - 1)) * (kPad / kSub)];  // exp(+i..)
+      const double2 w = S.tw16[(j * yy) & (kSub - 1)];  // exp(+i..)
       const double2 v = S.rx[yy][k];
       re += v.x * w.x + v.y * w.y;  // v * conj(w)
       im += v.y * w.x - v.x * w.y;
     }
-    const double wt = a.w16[j * 9 + k];
     S.s[j][k] = make_double2(re * wt, im * wt);
   }
   __syncthreads();
@@ -205,6 +208,7 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a, int C) {
   const int Xs[4] = {X, (kPad - X) & (kPad - 1), kPad / 2 - X, kPad / 2 + X};
   double qb[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   int ql[4] = {-1, -1, -1, -1};
+#pragma unroll 2
   for (int l = tid >> 7; l < nrow; l += kThreads / 128) {
     const double2* g = S.g1[l];
     double ev = g[0].x, od, es, os;
@@ -305,6 +309,17 @@ __global__ void __launch_bounds__(kThreads) k_peak(PeakArgs a, int C) {
     a.peak[2 * p + 1] = iy;
   }
   cl.sync();  // the other CTAs' maxima stay in place until CTA 0 has read them
+}
+
+__global__ void k_peak_table(double2* tw) {
+  double sn, cn;
+  sincospi((double)threadIdx.x / (kPad / 2), &sn, &cn);
+  tw[threadIdx.x] = make_double2(cn, sn);
+}
+
+cudaError_t launch_peak_table(double2* tw, cudaStream_t st) {
+  k_peak_table<<<1, kPad, 0, st>>>(tw);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_peak(const PeakArgs& a, cudaStream_t st) {
