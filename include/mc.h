@@ -167,8 +167,8 @@ int mc_plan_sum(mc_plan* plan, float* image_host); /* DFAlign.cu:1114-1292; imag
 int mc_plan_run(mc_plan* plan, float* image_host);
 /* All stages in order on frames in host memory (all positions, file pixel
  * type): the upload runs in chunks on a second stream and overlaps the
- * forward transforms of the chunks already resident (pinned memory for the
- * overlap; pageable works but serialises).  Replaces the per-frame
+ * forward transforms and the pair windows of the chunks already resident
+ * (pinned memory for the overlap; pageable works but serialises).  Replaces the per-frame
  * read/GPUMemH2D/GPUFFT2d sequence of DFAlign.cu:710-820 plus the rest of
  * the path. */
 int mc_plan_run_host(mc_plan* plan, const void* frames, float* image_host);
@@ -345,7 +345,7 @@ int mc_plan_bind_frames_device(mc_plan* plan, const void* d_frames);
 typedef struct mc_schedule {
   int n;             /* binned side the entry applies to */
   int pair_q;        /* codelet length Q of the split n = P*Q (0 = built-in cost model) */
-  int pairs_per_cta; /* pairs per CTA of the pair column stage (0 = 32) */
+  int pairs_per_cta; /* pairs per CTA of the pair column stage (0: 32 for a compiled split, else by launch) */
   int pair_variant;  /* reserved: 0 (the register-codelet column kernel) */
   int fwd_streams;   /* forked streams of the forward transforms, 1..8 (0 = 4) */
   int fwd_rows_pairing; /* radix-53 step of the forward row pass: 0 built-in, 1 one output pair */
