@@ -81,17 +81,23 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_fwd_rows_dif(FwdRows
 }
 
 // Forward columns of length L: out_row[i] = scale * X[i < keep_lo ? i : i + (L - n_out)].
-template <int N1, int N2>
+// IN_PLACE (out = in, the columns of a movie that is not binned): the second
+// transform reads the whole row again, so the first one's outputs wait in shared
+// memory until the barrier inside the second has passed every read of the row.
+template <int N1, int N2, bool IN_PLACE>
 __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_rows_fft_dif(RowsFftArgs a) {
   using TL = TwoLevel<N1, N2>;
   constexpr int N = TL::N, L = 2 * N;
-  __shared__ float2 ysm[N];
+  extern __shared__ float2 dyncol[];
+  float2* ysm = dyncol;
+  float2* zeven = dyncol + N;  // IN_PLACE: X[2m]
   const long long row = blockIdx.x;
   const float2* in = a.in + blockIdx.y * a.in_stride + row * a.ld_in;
   float2* out = a.out + blockIdx.y * a.out_stride + row * a.ld_out;
   const int shift = L - a.n_out, keep = a.keep_lo;
   const float sc = a.scale;
   const float2* tw = a.tw;
+  auto get = [&](int i) { return IN_PLACE ? in[i] : __ldg(in + i); };
   auto put = [&](int i, float2 v) {
     int o;
     if (i < keep) o = i;
@@ -100,18 +106,24 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_rows_fft_dif(RowsFft
     out[o] = make_float2(v.x * sc, v.y * sc);
   };
   // wanted outputs i < keep or i >= keep + shift: with no crop all of them
-  const int kmax = shift == 0 ? (N1 - 1) / 2 : dif_kmax<N1, N2>(keep + 1);
+  const int kmax = IN_PLACE || shift == 0 ? (N1 - 1) / 2 : dif_kmax<N1, N2>(keep + 1);
   TL::template run<false, false, false>(
-      ysm, tw + L, [&](int n) { return cadd(__ldg(in + n), __ldg(in + n + N)); },
-      [&](int m, float2 v) { put(2 * m, v); }, kmax);
+      ysm, tw + L, [&](int n) { return cadd(get(n), get(n + N)); },
+      [&](int m, float2 v) {
+        if (IN_PLACE) zeven[m] = v;
+        else put(2 * m, v);
+      },
+      kmax);
   __syncthreads();
   TL::template run<false, false, false>(
       ysm, tw + L,
       [&](int n) {
-        const float2 x0 = __ldg(in + n), x1 = __ldg(in + n + N);
+        const float2 x0 = get(n), x1 = get(n + N);
         return cmul(make_float2(x0.x - x1.x, x0.y - x1.y), __ldg(tw + n));
       },
       [&](int m, float2 v) { put(2 * m + 1, v); }, kmax);
+  if (IN_PLACE)
+    for (int m = threadIdx.x; m < N; m += TL::T) put(2 * m, zeven[m]);
 }
 
 bool dif_supported(int n) {
@@ -149,14 +161,20 @@ cudaError_t launch_fwd_rows_dif(const FwdRowsArgs& a, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
+template <int A, int B, bool IN_PLACE>
+cudaError_t launch_cols_dif(const RowsFftArgs& a, cudaStream_t st) {
+  const size_t smem = (IN_PLACE ? 2 : 1) * (size_t)A * B * sizeof(float2);
+  cudaError_t e = allow_smem((const void*)k_rows_fft_dif<A, B, IN_PLACE>, smem);
+  if (e != cudaSuccess) return e;
+  k_rows_fft_dif<A, B, IN_PLACE><<<dim3(a.nrows, std::max(a.nfr, 1)), TwoLevel<A, B>::T, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_rows_fft_dif(const RowsFftArgs& a, cudaStream_t st) {
   int n1 = 0, n2 = 0;
   if (a.plan.n % 2 || !two_level_split(a.plan.n / 2, n1, n2)) return cudaErrorInvalidValue;
-#define MC_DIF_LAUNCH(A, B)                                                        \
-  if (n1 == (A) && n2 == (B)) {                                                    \
-    k_rows_fft_dif<A, B><<<dim3(a.nrows, std::max(a.nfr, 1)), TwoLevel<A, B>::T, 0, st>>>(a); \
-    return cudaGetLastError();                                                     \
-  }
+#define MC_DIF_LAUNCH(A, B) \
+  if (n1 == (A) && n2 == (B)) return a.in == a.out ? launch_cols_dif<A, B, true>(a, st) : launch_cols_dif<A, B, false>(a, st);
   MC_TWO_LEVEL_LIST(MC_DIF_LAUNCH)
 #undef MC_DIF_LAUNCH
   return cudaErrorInvalidValue;
