@@ -29,7 +29,8 @@ __device__ __forceinline__ int dif_kmax(int lo) {
 // step-A loads.  Only the Z indices the half-spectrum split needs are kept,
 // Z[0, hk) and Z(L - hk, L): the even ones, of the first transform, in a buffer
 // of their own, the odd ones in the exchange buffer once the second transform
-// has read it.  44.6 KB a CTA at 7420 -> 3710 (74 with the raw rows and every
+// has read it.  Without a Fourier crop the two ranges meet in Z[L / 2], which
+// lies in the low one.  44.6 KB a CTA at 7420 -> 3710 (74 with the raw rows and every
 // kept index staged): registers, not shared memory, set the four CTAs per SM.
 // 24 frames of 7420^2 uint8 6.98 -> 6.69 ms (two output pairs of the pruned
 // radix-53 step per loop pass: 6.66, with 72 bytes of spills; not taken).
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_fwd_rows_dif(FwdRows
   for (int k = threadIdx.x; k < hk; k += TL::T) {
     const float2* zs = k & 1 ? zodd : zeven;
     const float2 z = zs[k >> 1];
-    const float2 zc = k == 0 ? z : zs[half + ((hk - 1 - k) >> 1)];
+    const float2 zc = k == 0 || 2 * k == L ? z : zs[half + ((hk - 1 - k) >> 1)];  // Z[-k]
     const float2 X = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
     const float2 Y = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));
     *reinterpret_cast<float4*>(outA + (long long)k * a.ldt + y0) = make_float4(X.x, X.y, Y.x, Y.y);
