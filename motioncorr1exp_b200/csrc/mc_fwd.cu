@@ -170,7 +170,10 @@ cudaError_t launch_rows_fft(const RowsFftArgs& a, bool inverse, cudaStream_t st)
   return cudaGetLastError();
 }
 
-// Batched rows: out_row[i] = scale * X[i < keep_lo ? i : i + (n - n_out)].
+// Batched rows: out_row[i] = scale * X[i < keep_lo ? i : i + (n - n_out)].  In
+// place when nothing is cropped (a barrier inside the transform separates a
+// row's reads from its stores), so the row is read with plain loads: __ldg is
+// for memory that the kernel does not write.
 template <int N1, int N2, bool INV, bool PAIRED, bool PLAIN = false>
 __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, tl_min_blocks(TwoLevel<N1, N2>::T)) k_rows_fft2l(RowsFftArgs a) {
   using TL = TwoLevel<N1, N2>;
@@ -181,12 +184,12 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, tl_min_blocks(TwoLevel<N1
   if constexpr (PLAIN) {
     // every output kept, unscaled (the forward column pass without a Fourier
     // crop): no per-output crop test or multiply (2.47 -> 2.15 ms per c2 movie)
-    TL::template run<INV, false, PAIRED>(ysm, a.tw + TL::N, [&](int i) { return __ldg(in + i); },
+    TL::template run<INV, false, PAIRED>(ysm, a.tw + TL::N, [&](int i) { return in[i]; },
                                          [&](int k, float2 v) { out[k] = v; });
   } else {
     const int shift = TL::N - a.n_out, keep = a.keep_lo;
     const float sc = a.scale;
-    TL::template run<INV, false, PAIRED>(ysm, a.tw + TL::N, [&](int i) { return __ldg(in + i); },
+    TL::template run<INV, false, PAIRED>(ysm, a.tw + TL::N, [&](int i) { return in[i]; },
                           [&](int k, float2 v) {
                             int o;
                             if (k < keep) o = k;
