@@ -1834,20 +1834,15 @@ static int copy_chunk(mc_plan* pl, const char* frames, int c, int chunk) {
   return MC_OK;
 }
 
-extern "C" {
-
-int mc_plan_forward(mc_plan* pl) {
-  if (!pl) return set_err(MC_E_ARG, "null plan");
-  for (int f = 0; f < pl->nframe; f++)
-    if (!pl->loaded[f]) return set_err(MC_E_STATE, "frame position %d not loaded", f);
-  CK(cudaSetDevice(pl->device));
-  return forward_all(pl, nullptr, 1);
+// Every copy of a host movie is queued: its frames count as loaded from here on.
+static void host_frames_queued(mc_plan* pl) {
+  pl->loaded.assign(pl->nframe, 1);
+  pl->log("Input Stack: Nx(%d) Ny(%d) Nz(%d) Mode(%d)\n\n", pl->nx, pl->ny, pl->nz, pl->mode);
+  pl->log("Crop Image: Offset(%d %d) RawDim(%d) BinnedDim(%d)\n", pl->p.crop_offsetx, pl->p.crop_offsety, pl->nu,
+          pl->n);
 }
 
-int mc_plan_run_host(mc_plan* pl, const void* frames, float* image_host) {
-  if (!pl || !frames) return set_err(MC_E_ARG, "null argument");
-  CK(cudaSetDevice(pl->device));
-  if (!pl->st_copy) CK(cudaStreamCreateWithFlags(&pl->st_copy, cudaStreamNonBlocking));
+static int run_host(mc_plan* pl, const char* frames, float* image_host) {
   // chunks of frames: copy chunk c on the copy stream while the plan stream
   // works on the frames of chunks < c; a movie of one chunk is copied on the
   // plan stream and runs as from device memory (its graph replayed)
@@ -1855,12 +1850,11 @@ int mc_plan_run_host(mc_plan* pl, const void* frames, float* image_host) {
   const int nchunk = (pl->nframe + chunk - 1) / chunk;
   const bool device = device_path(pl);
   pl->frames_src = nullptr;
-  for (int f = 0; f < pl->nframe; f++) pl->loaded[f] = 1;
-  pl->log("Input Stack: Nx(%d) Ny(%d) Nz(%d) Mode(%d)\n\n", pl->nx, pl->ny, pl->nz, pl->mode);
-  pl->log("Crop Image: Offset(%d %d) RawDim(%d) BinnedDim(%d)\n", pl->p.crop_offsetx, pl->p.crop_offsety, pl->nu,
-          pl->n);
+  // until every copy is queued (host_frames_queued) no frame counts as loaded
+  pl->loaded.assign(pl->nframe, 0);
   if (device && nchunk == 1) {
     CK(cudaMemcpyAsync(pl->d_frames, frames, (size_t)pl->nframe * pl->frame_bytes, cudaMemcpyHostToDevice, pl->st));
+    host_frames_queued(pl);
     return run_device(pl, image_host);
   }
   if (!pl->st_copy) CK(cudaStreamCreateWithFlags(&pl->st_copy, cudaStreamNonBlocking));
@@ -1874,8 +1868,9 @@ int mc_plan_run_host(mc_plan* pl, const void* frames, float* image_host) {
   if (!pl->start_ev) CK(cudaEventCreateWithFlags(&pl->start_ev, cudaEventDisableTiming));
   CK(cudaEventRecord(pl->start_ev, pl->st));
   CK(cudaStreamWaitEvent(pl->st_copy, pl->start_ev, 0));
-  if (device) return run_host_device(pl, static_cast<const char*>(frames), image_host, chunk);
-  for (int c = 0; c < nchunk; c++) CKR(copy_chunk(pl, static_cast<const char*>(frames), c, chunk));
+  if (device) return run_host_device(pl, frames, image_host, chunk);
+  for (int c = 0; c < nchunk; c++) CKR(copy_chunk(pl, frames, c, chunk));
+  host_frames_queued(pl);
   CKR(forward_all(pl, &pl->chunk_ev, chunk));
   CKR(mc_plan_pairs(pl));
   CKR(mc_plan_solve(pl));
@@ -1885,6 +1880,29 @@ int mc_plan_run_host(mc_plan* pl, const void* frames, float* image_host) {
   CKR(mc_plan_sum(pl, image_host));
   pl->tm.total_ms = pl->tm.forward_ms + pl->tm.pairs_ms + pl->tm.iterate_ms + pl->tm.refine_ms + pl->tm.sum_ms;
   return MC_OK;
+}
+
+extern "C" {
+
+int mc_plan_forward(mc_plan* pl) {
+  if (!pl) return set_err(MC_E_ARG, "null plan");
+  for (int f = 0; f < pl->nframe; f++)
+    if (!pl->loaded[f]) return set_err(MC_E_STATE, "frame position %d not loaded", f);
+  CK(cudaSetDevice(pl->device));
+  return forward_all(pl, nullptr, 1);
+}
+
+int mc_plan_run_host(mc_plan* pl, const void* frames, float* image_host) {
+  if (!pl || !frames) return set_err(MC_E_ARG, "null argument");
+  CK(cudaSetDevice(pl->device));
+  const int rc = run_host(pl, static_cast<const char*>(frames), image_host);
+  if (rc != MC_OK) {
+    // after a failure no copy from or to the caller's buffers is left in flight
+    if (pl->st_copy) cudaStreamSynchronize(pl->st_copy);
+    cudaStreamSynchronize(pl->st);
+    cudaGetLastError();
+  }
+  return rc;
 }
 
 int mc_plan_pairs(mc_plan* pl) {
@@ -2747,6 +2765,7 @@ static int run_host_device(mc_plan* pl, const char* frames, float* image_host, i
   for (int k = 0; k < nchunk; k++) {
     const int c = seq[k];
     CKR(copy_chunk(pl, frames, c, chunk));
+    if (k == nchunk - 1) host_frames_queued(pl);
     CK(cudaStreamWaitEvent(pl->st, pl->chunk_ev[c], 0));
     std::vector<std::pair<int, int>> jobs;
     for (int f = c * chunk; f < std::min(pl->nframe, (c + 1) * chunk); f++) jobs.push_back({f, f});
