@@ -1,6 +1,6 @@
 // Device code shared by the kernel translation units of libmc (mc_fwd*.cu,
-// mc_pair.cu, mc_sum.cu): constants, pixel decode, the two-level register FFT
-// and the raw-row staging helpers.
+// mc_pair*.cu, mc_sum.cu): constants, the two-level register FFT and the raw-row
+// staging helpers.
 #pragma once
 #include <cuda_fp16.h>
 #include <math.h>
@@ -15,17 +15,6 @@ namespace mc {
 namespace {
 
 constexpr int kThreads = 256;
-
-__device__ __forceinline__ float load_pixel(const void* frame, int mode, long long idx) {
-  switch (mode) {
-    case 0: return (float)((const int8_t*)frame)[idx];
-    case MC_MODE_U8: return (float)((const uint8_t*)frame)[idx];
-    case 1: return (float)((const int16_t*)frame)[idx];
-    case 6: return (float)((const uint16_t*)frame)[idx];
-    case MC_MODE_F16: return __half2float(((const __half*)frame)[idx]);
-    default: return ((const float*)frame)[idx];
-  }
-}
 
 }  // namespace
 
@@ -111,9 +100,9 @@ struct TwoLevel {
   }
 };
 
-// Stage the two packed input rows of k_fwd_rows2l or of one transform of
-// k_fwd_rows in shared memory: every
-// thread of the CTA issues independent typed loads of the raw pixels.
+// Stage the two packed input rows of one transform of k_fwd_rows in shared
+// memory: every thread of the CTA issues independent typed loads of the raw
+// pixels.
 template <typename Px>
 __device__ __forceinline__ void stage_rows(float2* xin, const FwdRowsArgs& a, long long r0, long long r1, int n,
                                            int nth) {
@@ -165,14 +154,6 @@ __device__ __forceinline__ void stage_raw_row(unsigned char* dst, const Px* src,
   uint4* d4 = reinterpret_cast<uint4*>(dst + (as - a0));
   for (int c = tid; c < chunks; c += nth) d4[c] = __ldg(g + c);
 }
-
-// Shared bytes one staged row takes: n pixels + up to 15 bytes of alignment,
-// rounded to 16.
-template <typename Px>
-constexpr int raw_row_bytes(int n) {
-  return (n * (int)sizeof(Px) + 15 + 15) / 16 * 16;
-}
-
 
 // Two-level splits compiled in (N1, N2).
 #define MC_TWO_LEVEL_LIST(X) X(53, 70) X(64, 64) X(32, 64) X(32, 32) X(16, 16) X(16, 32)

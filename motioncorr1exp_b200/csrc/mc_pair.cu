@@ -333,13 +333,6 @@ __global__ void __launch_bounds__(kRegThreads, pair_reg_min_blocks(Q)) k_pair_ro
 // the compiled (Q, P) splits of the tuned lengths: 3710, 4096, 2048, 1024
 #define MC_RP_LIST(X) X(35, 106) X(70, 53) X(64, 64) X(32, 128) X(64, 32) X(32, 64) X(16, 128) X(32, 32) X(16, 64)
 
-bool pair_cols_rp_supported(int P, int Q) {
-#define MC_RP_HAS(A, B) if (Q == (A) && P == (B)) return true;
-  MC_RP_LIST(MC_RP_HAS)
-#undef MC_RP_HAS
-  return false;
-}
-
 size_t pair_cols_launch_smem(int n, int P, int Q, int box) {
 #define MC_RP_SMEM(A, B) \
   if (Q == (A) && P == (B)) return pair_cols_rp_smem(n, RpShape<A, B>::YN, RpShape<A, B>::T, RpShape<A, B>::C, box);
