@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_fwd_rows_dif(FwdRows
 // IN_PLACE (out = in, the columns of a movie that is not binned): the second
 // transform reads the whole row again, so the first one's outputs wait in shared
 // memory until the barrier inside the second has passed every read of the row.
+// Uint8 movies, a frame's columns in place: 7420^2 288 us, 8192^2 243 (the
+// mixed-radix engine, also safe in place: 535 and 376).
 template <int N1, int N2, bool IN_PLACE>
 __global__ void __launch_bounds__(TwoLevel<N1, N2>::T, 4) k_rows_fft_dif(RowsFftArgs a) {
   using TL = TwoLevel<N1, N2>;

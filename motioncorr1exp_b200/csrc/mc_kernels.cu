@@ -1,12 +1,15 @@
 // Hand-written sm_100a kernels of the drift-correction path, in translation
 // units that compile in parallel:
-//   mc_fwd.cu, mc_fwd_raw.cu, mc_fwd_dif.cu   k_fwd_rows*, k_rows_fft*: decode +
-//        dark/gain + crop + row R2C with transposed store (DFAlign.cu:710-806),
-//        column FFT with Fourier-crop binning (cufunc.cu:162-176, 223-227)
-//   mc_pair.cu   k_pair_cols*, k_pair_rows: cross power x B-factor + pruned
-//        inverse FFTs onto the pbx window (cufunc.cu:229-233, 343-407)
-//   mc_sum.cu    k_peak, k_shift_sum*, k_c2r_rows*, k_count_sum, k_objective
-//        (cufunc.cu:372-497, DFAlign.cu:1287-1292)
+//   mc_fwd.cu, mc_fwd_raw.cu, mc_fwd_refs.cu, mc_fwd_dif.cu   k_fwd_rows*,
+//        k_rows_fft*: decode + dark/gain + crop + row R2C with transposed store
+//        (DFAlign.cu:710-806), column FFT with Fourier-crop binning
+//        (cufunc.cu:162-176, 223-227)
+//   mc_pair.cu, mc_pair_cols.cu   k_pair_cols*, k_pair_rows*: cross power x
+//        B-factor + pruned inverse FFTs onto the pbx window (cufunc.cu:229-233,
+//        343-407)
+//   mc_sum.cu    k_peak, k_ramp, k_shift_acc, k_sum_cols*, k_c2r_rows*,
+//        k_count_sum, k_objective* (cufunc.cu:372-497, DFAlign.cu:1287-1292)
+//   mc_solve.cu  k_solve, k_solve_smem: drift solve (DFAlign.cu:914-948, 1056-1139)
 //   this file    host helpers shared by all of them
 #include <math.h>
 #include <stdint.h>

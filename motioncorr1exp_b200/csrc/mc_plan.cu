@@ -86,7 +86,7 @@ constexpr int kPairBatch = 512;
 // read the earlier spectra once more each: 40 x 3710^2 uint8 with 2 / 4 / 5 / 6 /
 // 7 / 9 frames a chunk 16.6, 15.5, 15.6, 16.0, 16.0, 16.6 ms.
 constexpr size_t kChunkBytes = (size_t)48 << 20;
-constexpr int kTablePrime = 127;  // largest prime radix with a cosine/sine table (mixed_fft.cuh)
+constexpr int kTablePrime = 127;  // largest prime whose direct sum, as a first stage, runs from a table (stage_direct)
 constexpr int kForwardCtas = 148 * 16;  // row CTAs (of four rows) a forward launch is filled to
 // spectrum slots: the fewest a plan works with (two blocks of two frames in
 // the pair stage), and the device memory the automatic choice leaves free
@@ -299,8 +299,12 @@ bool choose_prune(int n, int box, int& P, int& Q) {
   for (int q = 1; q <= n; q++) {
     if (n % q) continue;
     const int p = n / q;
-    // the sides the stage takes: column of products, exchange buffer, weights
-    // and tables within a CTA's shared memory
+    // the sides the stage takes, and the split each gets (it decides the
+    // windows' last bits): by what a column, an exchange buffer, the weights and
+    // both factor tables take of a CTA's shared memory.  The kernel stages less
+    // (pair_cols_smem, asked at plan creation): up to the largest crop side every
+    // split chosen here fits it, and sides from 8302 up without a codelet split
+    // stay refused
     const size_t outer = (size_t)std::min<long long>(n, (long long)p * box);
     if ((size_t)20 * n + 8 * (q + outer) + 16 > 227 * 1024) continue;
     if (q > 1 && max_prime(q) > 13) continue;

@@ -25,8 +25,8 @@ namespace cg = cooperative_groups;
 // (26 FP64 operations for four values, 14 multiply-adds each before).  The rows
 // likewise: G(Y) and G(512 - Y) share theirs.  Rows ascend within a thread, so
 // the strict comparison keeps the first of equal values.
-// Measured per launch, one CTA per pair before / now: 21 pairs 179 -> 27 us,
-// 55 pairs 186 -> 35 us, 105 pairs 185 -> 52 us, 378 pairs 417 -> 123 us.
+// Measured per launch, one CTA per pair before / now: 21 pairs 179 -> 25 us,
+// 55 pairs 186 -> 33 us, 105 pairs 185 -> 47 us, 378 pairs 417 -> 113 us.
 constexpr int kSub = 16;
 constexpr int kPad = 512;
 constexpr int kUp = 32;
@@ -325,8 +325,8 @@ cudaError_t launch_peak_table(double2* tw, cudaStream_t st) {
 cudaError_t launch_peak(const PeakArgs& a, cudaStream_t st) {
   // CTAs per pair: four while they all run at once (two per SM), else two; the
   // work every CTA of a pair repeats (table, sub-box) outweighs a finer split
-  // (C = 1 / 2 / 4 / 8: 21 pairs 62, 37, 27, 27 us; 55 pairs 64, 41, 35, 52;
-  // 105 pairs 66, 52, 62, 79; 378 pairs 142, 123, 150, 227)
+  // (C = 1 / 2 / 4 / 8: 21 pairs 52, 35, 25, 25 us; 55 pairs 53, 35, 33, 46;
+  // 105 pairs 54, 47, 54, 69; 378 pairs 117, 113, 126, 191)
   const int C = a.npairs * 4 <= 148 * 2 ? 4 : 2;
   const size_t smem = peak_smem(C);
   cudaError_t e = allow_smem((const void*)k_peak, smem);

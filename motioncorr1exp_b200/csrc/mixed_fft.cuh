@@ -28,9 +28,9 @@
 //
 // Measured per frame, row / column pass, before (one stage a pass, three shared
 // buffers with the tables copied in, one output of a prime's direct sum a
-// thread) and now: 4092^2 = 31 | 11 | 3 x 4 605 / 520 -> 205 / 172 us; 1500^2 =
-// 5 x 5 | 5 x 3 | 4 55 / 41 -> 15.8 / 9.8 us; 520^2 = 13 | 5 | 8 (30 frames)
-// 13.6 / 13.9 -> 2.2 / 1.5 us.  Powers of two and 3710 keep the two-level form
+// thread) and now: 4092^2 = 31 | 11 | 3 x 4 605 / 520 -> 182 / 173 us; 1500^2 =
+// 5 x 5 | 5 x 3 | 4 55 / 41 -> 13.5 / 10.0 us; 520^2 = 13 | 5 | 8 (30 frames)
+// 13.6 / 13.9 -> 2.0 / 1.5 us.  Powers of two and 3710 keep the two-level form
 // (kcommon.cuh), which has one exchange instead of two.
 #pragma once
 #include "fft_engine.cuh"
@@ -109,7 +109,8 @@ __device__ __forceinline__ void stage_fused(const float2* src, float2* dst, cons
   }
 }
 
-// Prime radix p (17..127) as the first stage, every output the direct sum
+// Prime radix p (17..127) as the first stage (a second such prime, or a larger
+// one, takes stage_generic), every output the direct sum
 //   X_k = sum_r x_r W_p^(r k), r ascending.
 // A thread forms G outputs of one butterfly, so an input read serves G outputs
 // and the factors (the same for all threads of a warp) come two to a 16-byte
@@ -273,7 +274,8 @@ __device__ __forceinline__ void stage_symmetric(float2* cur, float2* dst, const 
   symmetric_outputs<kPrimePairs, INV, INTERLEAVED>(cur, dst, s, B, bdiv, ld, tw, tid, nth, last, stf);
 }
 
-// Other primes: every output of every butterfly as a direct sum,
+// Other primes, and a table prime that is not the first stage: every output of
+// every butterfly as a direct sum,
 //   X_k = sum_r src[j + r*n/R] * W_n^(r*((j mod Ns)*tws + k*n/R)).
 template <bool INV, bool INTERLEAVED, class Ld, class St>
 __device__ void stage_generic(float2* src, float2* dst, const FftStage& s, int n, int B, FastDiv bdiv, int ld,
